@@ -2,7 +2,8 @@
 
 The reference builds one shared library into ``deploy3d/libs/`` with CMake
 (trt/CMakeLists.txt:1-19, -gencode sm_75/sm_86).  This build targets sm_100a only and needs
-nothing but nvcc: one translation unit per .cu file, objects cached by content hash under
+nothing but nvcc and, for ``libs/_d3d_host.so`` (``csrc/host``, the native half of the Python binding), g++ and
+torch's headers: one translation unit per .cu file, objects cached by content hash under
 ``csrc/build/``, linked with ``nvcc -shared`` (static cudart, no other dependency).
 
 Run as ``python -m deploy3d_b200.build`` or through ``__graft_entry__.build()``.
@@ -53,6 +54,31 @@ def _digest(path, flags):
     return h.hexdigest()[:16]
 
 
+def build_host():
+    """Compile ``csrc/host/dispatch.cpp`` against the installed torch; returns the module's path."""
+    import sysconfig
+
+    import torch
+    src, out = os.path.join(CSRC, "host", "dispatch.cpp"), os.path.join(HERE, "libs", "_d3d_host.so")
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wno-unused-function",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I" + os.path.join(root, "include"),
+           "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + sysconfig.get_paths()["include"], "-I" + cuda, src, "-o", out, "-L" + os.path.join(root, "lib"),
+           "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    with open(src) as f:
+        want = _digest(src, cmd + [torch.__version__, f.read()])
+    stamp = os.path.join(OBJ, "link_host.stamp")
+    if not (os.path.exists(out) and os.path.exists(stamp) and open(stamp).read() == want):
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("g++ failed for %s:\n%s\n%s" % (src, " ".join(cmd), r.stderr))
+        with open(stamp, "w") as f:
+            f.write(want)
+    return out
+
+
 def build(verbose=False, ptxas_info=False, tuning=None, defines=(), checked=False):
     """Compile and link; returns the library path. Unchanged translation units are reused.
     `tuning` names a tuning build (see the module docstring): `defines` apply to spconv_mm_tc.cu only."""
@@ -100,6 +126,8 @@ def build(verbose=False, ptxas_info=False, tuning=None, defines=(), checked=Fals
             raise RuntimeError("link failed:\n%s" % r.stderr)
         with open(stamp, "w") as f:
             f.write(want)
+    if not tuning:
+        build_host()
     # drop objects of older source revisions (the regular build decides; tuning builds leave the cache alone)
     if not tuning:
         keep = set(objs) | {stamp}

@@ -1,7 +1,10 @@
 """``nms3d`` and ``yolox3d_decode`` (deploy3d/symfun/ops/decoder/nms3d.py, yolox3d_decode.py)."""
 import numpy as np
 
-from .spconv import _plugin
+from ..plugins import deserialize_plugin
+from .spconv import _plugin_by_args
+
+_NMS = {}  # one plugin per threshold
 
 
 def nms3d(scores, boxes, iou_threshold=None):
@@ -9,12 +12,15 @@ def nms3d(scores, boxes, iou_threshold=None):
 
     The reference plugin has no parameters and a fixed IoU threshold of 0.1 (trt/decoder/nms3d.cu:138);
     ``iou_threshold`` overrides it for callers that go through this module."""
-    plug = _plugin("NMS3d", b"")
-    if iou_threshold is not None:
-        import copy
-        plug = copy.copy(plug)
-        plug.p = type(plug.p)(float(iou_threshold))
-        plug._workspace = None
+    thr = None if iou_threshold is None else float(iou_threshold)
+    plug = _NMS.get(thr)
+    if plug is None:
+        if len(_NMS) > 64:
+            _NMS.clear()
+        plug = _NMS[thr] = deserialize_plugin("NMS3d", b"")
+        if thr is not None:
+            plug.p = type(plug.p)(thr)
+    plug._workspace = None  # a mask of its own for every call: calls on several streams may overlap
     return plug.enqueue(scores, boxes)[0]
 
 
@@ -30,5 +36,5 @@ def yolox3d_decode(cls_scores, bbox_preds, voxel_config, stride, class_ids, topk
     """cls_scores [B, C, Y, X], bbox_preds [B, 9+a, Y, X] (same dtype), voxel_config float32 [6]; returns
     (topk_class_ids, topk_scores, topk_boxes) for every class id, in order
     (deploy3d/symfun/ops/decoder/yolox3d_decode.py:20-37)."""
-    plug = _plugin("YoloX3dDecode", data_s_yolox3d_decode(stride, class_ids, topk))
+    plug = _plugin_by_args("YoloX3dDecode", (stride, tuple(class_ids), topk), data_s_yolox3d_decode)
     return plug.enqueue(cls_scores, bbox_preds, voxel_config)

@@ -1,7 +1,7 @@
 """``scatter_to``, ``gather_back`` (deploy3d/symfun/ops/point_voxel_mapping/*.py)."""
 import numpy as np
 
-from .spconv import _plugin
+from .spconv import _plugin, _plugin_by_args
 
 
 def data_s_scatter_to(reduce_type):
@@ -10,7 +10,7 @@ def data_s_scatter_to(reduce_type):
 
 def scatter_to(batch_point_feats, scatter_to, scatter_count, reduce_type):
     """reduce_type 0: max, otherwise mean (deploy3d/symfun/ops/point_voxel_mapping/scatter_to.py:19-28)."""
-    plug = _plugin("ScatterTo", data_s_scatter_to(reduce_type))
+    plug = _plugin_by_args("ScatterTo", (reduce_type,), data_s_scatter_to)
     return plug.enqueue(batch_point_feats, scatter_to, scatter_count)[0]
 
 
@@ -24,5 +24,6 @@ def data_s_gather_back(fill_val=None):
 def gather_back(reduces_feats, scatter_to, fill_val=None, out=None):
     """Rows whose index is negative are filled with ``fill_val`` when given, otherwise left untouched
     (deploy3d/symfun/ops/point_voxel_mapping/gather_back.py:19-27)."""
-    plug = _plugin("GatherBack", data_s_gather_back(fill_val))
+    plug = _plugin_by_args("GatherBack", (fill_val,), data_s_gather_back) if fill_val else \
+        _plugin("GatherBack", data_s_gather_back(fill_val))  # 0.0 and -0.0 are equal as keys
     return plug.enqueue(reduces_feats, scatter_to, outputs=None if out is None else [out])[0]

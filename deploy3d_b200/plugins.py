@@ -13,7 +13,7 @@ import ctypes
 import numpy as np
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._lib import (D3D_BF16, D3D_FLOAT, D3D_HALF, D3D_INT32, check, desc_array, lib, make_desc, ptr_array)
 
 PLUGIN_VERSION = "2.0"  # e.g. trt/spconv/index_trt.cu:24
@@ -43,18 +43,26 @@ class _Plugin:
 
     def __init__(self):
         self._workspace = None
+        self._call = None  # native enqueue of this plugin (entry points resolved at the first call)
 
     # -- to be provided by subclasses
     def _params_ref(self):
         raise NotImplementedError
 
+    def _params_address(self):
+        """(address the library takes the parameters from, their size; size 0: an opaque handle)."""
+        return ctypes.addressof(self.p), ctypes.sizeof(self.p)
+
     num_outputs = 1
+
+    def _num_outputs(self):
+        return self.num_outputs
 
     def output_descs(self, in_descs):
         """getOutputDimensions / getOutputDataType, from the library (one source with the TensorRT shells)."""
         fn = getattr(lib(), self._prefix + "_output_desc")
         outs = []
-        for i in range(self.num_outputs):
+        for i in range(self._num_outputs()):
             d = _lib.TensorDesc()
             check(self._prefix + "_output_desc", fn(self._params_ref(), desc_array(in_descs), len(in_descs), i,
                                                     ctypes.byref(d)))
@@ -79,29 +87,11 @@ class _Plugin:
 
     def enqueue(self, *inputs, outputs=None, stream=None):
         """Runs the plugin on the current (or given) CUDA stream and returns the tuple of output tensors."""
-        if not inputs or not inputs[0].is_cuda:
-            raise RuntimeError("%s: inputs must be CUDA tensors; this library has no CPU path" % self.name)
-        inputs = [t if t.is_contiguous() else t.contiguous() for t in inputs]
-        device = inputs[0].device
-        in_descs = [_desc_of(t) for t in inputs]
-        out_descs = self.output_descs(in_descs)
-        if outputs is None:
-            outputs = [torch.empty(tuple(d.dims[:d.nb_dims]), dtype=_D3D2TORCH[d.dtype], device=device)
-                       for d in out_descs]
-        else:  # the caller's buffers say which of the accepted output types it wants (GatherBack can widen)
-            for d, t in zip(out_descs, outputs):
-                d.dtype = _TORCH2D3D[t.dtype]
-        ws_bytes = self.workspace_size(in_descs)
-        ws = self._get_workspace(ws_bytes, device)
-        fn = getattr(lib(), self._prefix + "_enqueue")
-        with torch.cuda.device(device):
-            status = fn(self._params_ref(), desc_array(in_descs), len(in_descs), desc_array(out_descs),
-                        len(out_descs), ptr_array([t.data_ptr() for t in inputs]),
-                        ptr_array([t.data_ptr() for t in outputs]),
-                        ctypes.c_void_p(ws.data_ptr() if ws is not None else 0), ctypes.c_size_t(ws_bytes),
-                        _stream_ptr(stream))
-        check(self._prefix + "_enqueue", status)
-        return tuple(outputs)
+        call = self._call
+        if call is None:
+            call = self._call = _host.call(self.name, self._prefix)
+        address, size = self._params_address()
+        return call.enqueue(self, address, size, self._num_outputs(), inputs, outputs, stream)
 
 
 class SPConvIdxPlugin(_Plugin):
@@ -119,17 +109,8 @@ class SPConvIdxPlugin(_Plugin):
     def _params_ref(self):
         return ctypes.byref(self.p)
 
-    def output_descs(self, in_descs):
-        n = lib().d3d_spconv_index_num_outputs(ctypes.byref(self.p))
-        outs = []
-        for i in range(n):
-            d = _lib.TensorDesc()
-            check("d3d_spconv_index_output_desc",
-                  lib().d3d_spconv_index_output_desc(ctypes.byref(self.p), desc_array(in_descs), len(in_descs), i,
-                                                     ctypes.byref(d)))
-            outs.append(d)
-        return outs
-
+    def _num_outputs(self):
+        return 2 if self.p.subm else 5  # d3d_spconv_index_num_outputs
 
     def subm_table_ok(self):
         """True when enqueue_ex can write SPConvMM's neighbour table itself (mirror-symmetric 3-D SubM rulebook)."""
@@ -167,6 +148,7 @@ class SPConvMMPlugin(_Plugin):
     def __init__(self, name, data_s):
         super().__init__()
         self.handle = ctypes.c_void_p(0)
+        self._configured = None  # (dtype, device) of the uploaded weights
         buf = ctypes.create_string_buffer(bytes(data_s), len(data_s))
         check("d3d_spconv_mm_create", lib().d3d_spconv_mm_create(buf, len(data_s), ctypes.byref(self.handle)))
         self.p = _lib.SpconvMMParams()
@@ -183,6 +165,9 @@ class SPConvMMPlugin(_Plugin):
     def _params_ref(self):
         return self.handle
 
+    def _params_address(self):
+        return self.handle.value, 0
+
     def serialize(self):
         n = ctypes.c_size_t(0)
         check("d3d_spconv_mm_serialize", lib().d3d_spconv_mm_serialize(self.handle, None, ctypes.byref(n)))
@@ -193,13 +178,17 @@ class SPConvMMPlugin(_Plugin):
     def enqueue(self, *inputs, outputs=None, stream=None):
         """configurePlugin for the dtype of ``inFeats`` (a no-op when already done), then enqueue: the C entry
         point itself refuses a handle that was not configured, as it may not allocate."""
-        with torch.cuda.device(inputs[0].device):
-            self.configure(inputs[0].dtype)
+        x = inputs[0]
+        if (x.dtype, x.device) != self._configured:
+            with torch.cuda.device(x.device):
+                self.configure(x.dtype)
         return super().enqueue(*inputs, outputs=outputs, stream=stream)
 
     def configure(self, torch_dtype):
         """configurePlugin: upload the weights in the compute dtype (trt/spconv/mm_trt.cu:127-142)."""
+        self._configured = None
         check("d3d_spconv_mm_configure", lib().d3d_spconv_mm_configure(self.handle, _TORCH2D3D[torch_dtype]))
+        self._configured = (torch_dtype, torch.device("cuda", torch.cuda.current_device()))
 
     def set_kernel(self, which):
         """0 automatic, 1 SIMT, 2 tcgen05, 3 tcgen05 with one CTA per SM."""
@@ -360,16 +349,8 @@ class YoloX3dDecodePlugin(_PodPlugin):
     _prefix = "d3d_yolox3d_decode"
     _params_t = _lib.YoloX3dDecodeParams
 
-    def output_descs(self, d):
-        n = lib().d3d_yolox3d_decode_num_outputs(ctypes.byref(self.p))
-        out = []
-        for i in range(n):
-            desc = _lib.TensorDesc()
-            check("d3d_yolox3d_decode_output_desc",
-                  lib().d3d_yolox3d_decode_output_desc(ctypes.byref(self.p), desc_array(d), len(d), i,
-                                                       ctypes.byref(desc)))
-            out.append(desc)
-        return out
+    def _num_outputs(self):
+        return lib().d3d_yolox3d_decode_num_outputs(ctypes.byref(self.p))
 
 
 _REGISTRY = {

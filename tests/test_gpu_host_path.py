@@ -1,0 +1,66 @@
+"""The native enqueue and the operator layer's plugin look-up: what is kept between calls never outlives its inputs."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("cin,cout,dtype", [(16, 16, torch.float32), (32, 64, torch.float16)])
+def test_changed_weights_are_seen(d3d, cin, cout, dtype):
+    """The same array objects with new contents, and other arrays with the same contents, give what fresh ones give."""
+    r = np.random.Generator(np.random.PCG64(3))
+    n = 700
+    grid = (8, 20, 20)
+    ids = r.choice(8 * 20 * 20, n, replace=False)
+    coors = np.stack([0 * ids, ids // 400, ids // 20 % 20, ids % 20], 1).astype(np.int32)
+    num = torch.tensor([n], dtype=torch.int32, device=DEV)
+    one = (1, 1, 1)
+    index, num_index = d3d.spconv_index(torch.from_numpy(coors).to(DEV), num,
+                                        torch.empty((1, 0) + grid, dtype=torch.int32, device=DEV), (3, 3, 3), one, one,
+                                        one, (0, 0, 0), n, True, False)
+    x = torch.randn((n, cin), device=DEV).to(dtype)
+
+    def run(w, b):
+        return d3d.spconv_mm(x, num, num, index, num_index, (3, 3, 3), cin, cout, n, True, False, w, b).clone()
+
+    w = r.standard_normal((27, cin, cout)).astype(np.float32)
+    b = r.standard_normal(cout).astype(np.float32)
+    first = run(w, b)
+    assert torch.equal(first, run(w, b)) and torch.equal(first, run(w.copy(), b.copy()))
+    old = w[26, cin - 1, cout - 1]
+    w[26] *= -1  # the last offset only: the compare has to reach the end
+    changed = run(w, b)
+    assert torch.equal(changed, run(w.copy(), b)) and not torch.equal(changed, first)
+    w[26] *= -1
+    assert w[26, cin - 1, cout - 1] == old and torch.equal(first, run(w, b))
+    b[cout - 1] += 1
+    moved = run(w, b)
+    assert torch.equal(moved[:, :-1], first[:, :-1]) and not torch.equal(moved[:, -1], first[:, -1])
+    assert torch.equal(moved, run(np.asfortranarray(w), b.copy()))  # a layout that is not the blob's
+
+
+def test_shapes_and_types_in_turn(d3d):
+    """More signatures than a plugin keeps, the first of them again at the end."""
+    pts = [torch.randn((5 + i, 3 + i % 4), device=DEV) for i in range(12)]
+    to = [torch.arange(len(p), dtype=torch.int32, device=DEV).flip(0) for p in pts]
+    for _ in range(2):
+        for p, t in zip(pts, to):
+            assert torch.equal(d3d.gather_back(p, t, 0.0), p.flip(0))
+            h = p.half()
+            assert d3d.gather_back(h, t, 0.0).dtype == torch.float16
+    neg = torch.full((4,), -1, dtype=torch.int32, device=DEV)
+    assert torch.signbit(d3d.gather_back(pts[0], neg, -0.0)).all()
+    assert not torch.signbit(d3d.gather_back(pts[0], neg, 0.0)).any()
+
+
+def test_refusals(d3d):
+    from deploy3d_b200._lib import D3DError
+    with pytest.raises(RuntimeError, match="CUDA tensors"):
+        d3d.gather_back(torch.zeros((3, 2)), torch.zeros(3, dtype=torch.int32))
+    with pytest.raises(TypeError, match="dtype"):
+        d3d.gather_back(torch.zeros((3, 2), dtype=torch.float64, device=DEV),
+                        torch.zeros(3, dtype=torch.int32, device=DEV))
+    with pytest.raises(D3DError):
+        d3d.nms3d(torch.zeros((1, 4), device=DEV), torch.zeros((1, 4, 5), device=DEV))
