@@ -2,20 +2,34 @@
 //
 // Replaces decoder::YoloX3dDecodePlugin of the reference (trt/decoder/yolox3d_decode.cu:147-412): there a
 // segmented radix sort of all B*C*Y*X scores (cub, :341-355) followed by one decode launch per class (:357-367).
-// Only the first K entries of every sorted segment are ever read, so here one CTA per (class, batch row) selects
-// them directly: a 4-pass radix select finds the K-th largest key, the cells above it (and, among equal scores,
-// the lowest positions, which is what the stable sort of the reference yields) are collected in shared memory,
-// sorted there, and decoded in the same kernel.  No workspace, one launch for all classes.
+// Only the first K entries of every sorted segment are ever read, so here one cluster of eight CTAs per (class, batch
+// row) selects them directly: each CTA keeps the keys of its eighth of the map in shared memory; a three-pass radix
+// select over the cluster's histograms finds the K-th largest key; the cells above it (and, among equal scores, the
+// lowest positions, which is what the stable sort of the reference yields) are collected, every CTA ranks an eighth of
+// them by counting the larger ones, and decodes its boxes to their ranks.  No workspace, one launch for all classes.
+//
+// What bounds it: a head has few (class, row) pairs -- six of 180 x 180 cells fill six CTAs of the former one-CTA
+// version, which read the map five times, searched its histograms serially and sorted with a barrier per step.  The
+// chain that is left is one pass over the map, five cluster barriers and the decode (2 x 3 x 180 x 180, top 500, fp16:
+// 62.6 -> 19.7 us).
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <string.h>
+
+#include <atomic>
 
 #include "common.cuh"
 
 namespace d3d {
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kMaxTopK = 4096;  // candidates are sorted in shared memory
+namespace cg = cooperative_groups;
+
+constexpr int kThreads = 512;
+constexpr int kCluster = 8;     // CTAs per (class, batch row); the largest portable cluster
+constexpr int kMaxTopK = 4096;  // candidates are ranked in shared memory
+constexpr int kBins = 2048;     // digits of 11, 11 and 10 bits
+constexpr int kMaxHeldKeys = 24 * 1024;  // keys a CTA keeps in shared memory; larger maps are read again (from L2)
 
 // Order-preserving map of a float to an unsigned key (larger score = larger key); -0 and +0 share a key.
 __device__ __forceinline__ uint32_t score_key(float f) {
@@ -87,80 +101,148 @@ __device__ __forceinline__ void decode_cell(const DecodeArgs& a, const T* preds_
   for (int e = 9; e < a.box_in_params; ++e) box_out[e - 2] = load_f32(pred + (int64_t)e * n);
 }
 
-template <class T>
-__global__ void __launch_bounds__(kThreads)
-topk_decode_kernel(const DecodeArgs a) {
-  extern __shared__ unsigned long long cand[];  // [padded K] (key << 32) | ~position: descending = the output order
-  __shared__ int hist[256];
-  __shared__ int scratch[40];
-  __shared__ uint32_t sel_prefix, sel_mask;
-  __shared__ int sel_need, n_greater;
-  const int c = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+// Cluster rank r owns the cells [r * per, (r + 1) * per).  Dynamic shared memory: candidates [topk], then (kHold) keys.
+template <class T, bool kHold>
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
+topk_decode_kernel(const DecodeArgs a, const int per) {
+  extern __shared__ unsigned long long cand[];  // (key << 32) | ~position: descending = the output order
+  __shared__ int hist[3][kBins];
+  __shared__ int warp_sum[kThreads / 32];
+  __shared__ int sel_digit, sel_need, n_greater;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = blockIdx.x / kCluster, b = blockIdx.y;
   const int n = a.size_y * a.size_x, k_out = a.topk;
   const T* scores = reinterpret_cast<const T*>(a.cls_scores) + ((int64_t)b * a.num_class + c) * n;
   const T* preds_b = reinterpret_cast<const T*>(a.bbox_preds) + (int64_t)b * a.box_in_params * n;
-  if (tid == 0) sel_prefix = 0u, sel_mask = 0u, sel_need = k_out, n_greater = 0;
-  // ---- radix select: after the four passes sel_prefix is the K-th largest key, sel_need how many cells with
-  // exactly that key belong to the top K
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int d = tid; d < 256; d += kThreads) hist[d] = 0;
-    __syncthreads();
-    const uint32_t prefix = sel_prefix, mask = sel_mask;
-    for (int i = tid; i < n; i += kThreads) {
-      const uint32_t key = score_key(load_f32(scores + i));
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int need = sel_need, d = 255;
-      for (; d > 0 && hist[d] < need; --d) need -= hist[d];
-      sel_need = need;
-      sel_prefix = prefix | ((uint32_t)d << shift);
-      sel_mask = mask | (255u << shift);
-    }
-    __syncthreads();
-  }
-  const uint32_t threshold = sel_prefix;
-  const int need = sel_need, greater = k_out - need;
-  // ---- collect: everything above the threshold (any order), then the `need` lowest positions at the threshold
-  int tie_base = 0;
-  for (int base = 0; base < n; base += kThreads) {
-    const int i = base + tid;
-    uint32_t key = 0u;
-    bool tie = false;
-    if (i < n) {
-      key = score_key(load_f32(scores + i));
-      tie = key == threshold;
-      if (key > threshold) cand[atomicAdd(&n_greater, 1)] = ((unsigned long long)key << 32) | (0xFFFFFFFFu - (uint32_t)i);
-    }
-    int total;
-    const int rank = tie_base + block_exclusive_scan(tie ? 1 : 0, scratch, &total);
-    if (tie && rank < need) cand[greater + rank] = ((unsigned long long)key << 32) | (0xFFFFFFFFu - (uint32_t)i);
-    tie_base += total;
-  }
-  int padded = 1;
-  while (padded < k_out) padded <<= 1;
-  for (int i = k_out + tid; i < padded; i += kThreads) cand[i] = 0ull;
+  uint32_t* held = reinterpret_cast<uint32_t*>(cand + k_out);
+  const int first = min(rank * per, n), count = min(per, n - first);
+  auto key_at = [&](int i) -> uint32_t { return kHold ? held[i] : score_key(load_f32(scores + first + i)); };
+  for (int i = tid; i < 3 * kBins; i += kThreads) (&hist[0][0])[i] = 0;
+  if (tid == 0) n_greater = 0;
+  if (kHold)
+    for (int i = tid; i < count; i += kThreads) held[i] = score_key(load_f32(scores + first + i));
   __syncthreads();
-  // ---- bitonic sort, descending
-  for (int size = 2; size <= padded; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = tid; t < (padded >> 1); t += kThreads) {
-        const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
-        const bool descending = (lo & size) == 0;
-        const unsigned long long x = cand[lo], y = cand[hi];
-        if ((x < y) == descending) cand[lo] = y, cand[hi] = x;
-      }
-      __syncthreads();
+  // ---- radix select: after the three passes `prefix` is the K-th largest key, `need` how many cells with exactly
+  // that key belong to the top K
+  uint32_t prefix = 0u, mask = 0u;
+  int need = k_out;
+#pragma unroll
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+    const uint32_t digits = pass == 2 ? 1023u : 2047u;
+    for (int i = tid; i < count; i += kThreads) {
+      const uint32_t key = key_at(i);
+      if ((key & mask) == prefix) atomicAdd(&hist[pass][(key >> shift) & digits], 1);
+    }
+    cluster.sync();
+    // every CTA adds up the cluster's bins for itself: thread t holds the bins [4 t, 4 t + 4)
+    int v[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < kCluster; ++r) {
+      const int4 w = *reinterpret_cast<const int4*>(cluster.map_shared_rank(&hist[pass][4 * tid], r));
+      v[0] += w.x, v[1] += w.y, v[2] += w.z, v[3] += w.w;
+    }
+    const int mine = v[0] + v[1] + v[2] + v[3];
+    int above = mine;  // cells in this thread's bins and all higher ones: suffix sum over the CTA
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int t = __shfl_down_sync(0xffffffffu, above, d);
+      if (lane + d < 32) above += t;
+    }
+    if (lane == 0) warp_sum[warp] = above;
+    __syncthreads();
+    for (int w = warp + 1; w < kThreads / 32; ++w) above += warp_sum[w];
+    above -= mine;  // strictly higher bins
+#pragma unroll
+    for (int q = 3; q >= 0; --q) {
+      if (above < need && above + v[q] >= need) sel_digit = 4 * tid + q, sel_need = need - above;  // one thread, one q
+      above += v[q];
+    }
+    __syncthreads();
+    prefix |= (uint32_t)sel_digit << shift;
+    mask |= digits << shift;
+    need = sel_need;
+    __syncthreads();
+  }
+  const uint32_t threshold = prefix;
+  const int greater = k_out - need;
+  // ---- collect into CTA 0: everything above the threshold (any order), then the `need` lowest positions at it
+  unsigned long long* all = cluster.map_shared_rank(cand, 0);
+  int* taken = cluster.map_shared_rank(&n_greater, 0);
+  int tie_base = 0;  // ties of the lower ranks: their last histogram knows them
+  for (int r = 0; r < rank; ++r) tie_base += *cluster.map_shared_rank(&hist[2][threshold & 1023u], r);
+  // a warp owns a run of cells; its ties are counted first so that they can be numbered by position
+  const int run = (count + kThreads / 32 - 1) / (kThreads / 32);
+  const int w0 = min(warp * run, count), w1 = min(w0 + run, count);
+  int ties = 0;
+  for (int i0 = w0; i0 < w1; i0 += 32) {
+    const bool in = i0 + lane < w1;
+    ties += __popc(__ballot_sync(0xffffffffu, in && key_at(in ? i0 + lane : 0) == threshold));
+  }
+  if (lane == 0) warp_sum[warp] = ties;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) tie_base += warp_sum[w];
+  for (int i0 = w0; i0 < w1; i0 += 32) {
+    const bool in = i0 + lane < w1;
+    const uint32_t key = in ? key_at(i0 + lane) : 0u;
+    const unsigned long long entry = ((unsigned long long)key << 32) | (0xFFFFFFFFu - (uint32_t)(first + i0 + lane));
+    const unsigned up = __ballot_sync(0xffffffffu, in && key > threshold);
+    const unsigned tie = __ballot_sync(0xffffffffu, in && key == threshold);
+    int base = 0;
+    if (up) {
+      if (lane == 0) base = atomicAdd(taken, __popc(up));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if ((up >> lane) & 1u) all[base + __popc(up & lanemask_lt())] = entry;
+    }
+    if ((tie >> lane) & 1u) {
+      const int t = tie_base + __popc(tie & lanemask_lt());
+      if (t < need) all[greater + t] = entry;
+    }
+    tie_base += __popc(tie);
+  }
+  cluster.sync();
+  if (rank != 0)
+    for (int i = tid; i < k_out; i += kThreads) cand[i] = all[i];
+  cluster.sync();  // CTA 0 may leave once the others have their copies
+  // ---- rank and decode: the entries are distinct, so an entry's rank is the number of larger ones; eight lanes count
+  // for one entry
+  const int share = (k_out + kCluster - 1) / kCluster;
+  const int e0 = min(rank * share, k_out), e1 = min(e0 + share, k_out);
+  for (int e = e0 + (tid >> 3); e < ((e1 - e0 + 3) & ~3) + e0; e += kThreads / 8) {  // whole warps
+    const unsigned long long me = cand[e < e1 ? e : e0];
+    int larger = 0;
+    for (int i = tid & 7; i < k_out; i += 8) larger += cand[i] > me;
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) larger += __shfl_xor_sync(0xffffffffu, larger, d);
+    if ((tid & 7) == 0 && e < e1) {
+      const int pos = (int)(0xFFFFFFFFu - (uint32_t)me);
+      const int64_t o = (int64_t)b * k_out + larger;
+      decode_cell<T>(a, preds_b, pos, load_f32(scores + pos), a.out_ids[c] + o, a.out_scores[c] + o,
+                     a.out_boxes[c] + o * (a.box_in_params - 2), a.class_ids[c]);
     }
   }
-  // ---- decode
-  for (int r = tid; r < k_out; r += kThreads) {
-    const int pos = (int)(0xFFFFFFFFu - (uint32_t)cand[r]);
-    const int64_t o = (int64_t)b * k_out + r;
-    decode_cell<T>(a, preds_b, pos, load_f32(scores + pos), a.out_ids[c] + o, a.out_scores[c] + o,
-                   a.out_boxes[c] + o * (a.box_in_params - 2), a.class_ids[c]);
+}
+
+template <class T> int launch_topk(const DecodeArgs& a, int b, cudaStream_t st) {
+  const int n = a.size_y * a.size_x, per = (n + kCluster - 1) / kCluster;
+  const bool hold = per <= kMaxHeldKeys;
+  const size_t smem = (size_t)a.topk * sizeof(unsigned long long) + (hold ? (size_t)per * sizeof(uint32_t) : 0);
+  auto kern = hold ? topk_decode_kernel<T, true> : topk_decode_kernel<T, false>;
+  if (smem > 20 * 1024) {  // beside the histograms' 24 KB
+    static std::atomic<bool> raised[64][2];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return D3D_ERR_CUDA;
+    if (!raised[dev][hold].load(std::memory_order_acquire)) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTopK * 8 + kMaxHeldKeys * 4) !=
+          cudaSuccess)
+        return D3D_ERR_CUDA;
+      raised[dev][hold].store(true, std::memory_order_release);
+    }
   }
+  kern<<<dim3(a.num_class * kCluster, b), kThreads, smem, st>>>(a, per);
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
 }
 
 int num_classes(const d3d_yolox3d_decode_params* p) {
@@ -253,14 +335,6 @@ extern "C" int d3d_yolox3d_decode_enqueue(const d3d_yolox3d_decode_params* p, co
     a.out_boxes[i] = i < c ? reinterpret_cast<float*>(outputs[3 * i + 2]) : nullptr;
     D3D_REQUIRE(i >= c || (a.out_ids[i] && a.out_scores[i] && a.out_boxes[i]), D3D_ERR_INVALID_ARGUMENT);
   }
-  int padded = 1;
-  while (padded < k) padded <<= 1;
-  const size_t smem = (size_t)padded * sizeof(unsigned long long);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (in[0].dtype == D3D_FLOAT)
-    topk_decode_kernel<float><<<dim3(c, b), kThreads, smem, st>>>(a);
-  else
-    topk_decode_kernel<__half><<<dim3(c, b), kThreads, smem, st>>>(a);
-  D3D_CHECK_LAUNCH();
-  return D3D_OK;
+  return in[0].dtype == D3D_FLOAT ? launch_topk<float>(a, b, st) : launch_topk<__half>(a, b, st);
 }
