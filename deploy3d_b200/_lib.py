@@ -17,7 +17,7 @@ D3D_MAX_DIMS = 8
 D3D_MAX_NDIM = 4
 
 D3D_FLOAT, D3D_HALF, D3D_INT8, D3D_INT32, D3D_BOOL, D3D_BF16 = 0, 1, 2, 3, 4, 7
-D3D_STATUS_HASH_FULL, D3D_STATUS_OUTPUT_OVERFLOW = 1, 2
+D3D_STATUS_HASH_FULL, D3D_STATUS_OUTPUT_OVERFLOW, D3D_STATUS_STALLED = 1, 2, 4
 
 
 class TensorDesc(ctypes.Structure):
@@ -113,6 +113,12 @@ SIGNATURES = {
     "d3d_spconv_index_subm_table_ok": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams)]),
     "d3d_spconv_index_enqueue_ex": (ctypes.c_int, _enqueue_sig(ctypes.POINTER(SpconvIndexParams)) +
                                     [ctypes.POINTER(SpconvIndexExtras)]),
+    "d3d_spconv_subm_tables_workspace": (ctypes.c_int, [_descp, ctypes.c_int, _szp]),
+    "d3d_spconv_subm_tables": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_int32), _vpp, _descp, ctypes.c_int,
+                                              _vpp, _vp, _sz, _vp, _vp]),
+    "d3d_spconv_conv_tables_ok": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int]),
+    "d3d_spconv_conv_tables": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int, _vpp, _vp, _vp,
+                                              _vp, _vp, _vp, _sz, _vp, _vp]),
     "d3d_spconv_mm_create": (ctypes.c_int, [_vp, _sz, ctypes.POINTER(_vp)]),
     "d3d_spconv_mm_get_params": (ctypes.c_int, [_vp, ctypes.POINTER(SpconvMMParams)]),
     "d3d_spconv_mm_serialize": (ctypes.c_int, [_vp, _vp, _szp]),

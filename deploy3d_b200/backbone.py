@@ -12,7 +12,7 @@ import torch
 
 from . import synth
 from .ops import data_s_spconv_index, data_s_spconv_mm
-from .plugins import SPConvMMPlugin, deserialize_plugin
+from .plugins import SPConvMMPlugin, SubmTables, deserialize_plugin
 
 
 class Layer:
@@ -182,7 +182,57 @@ def make_weights(layers, seed=0):
 
 
 class _Rulebook:
-    pass
+    """What the layers of one `key` share.  The convolutions read neighbour tables only, so a net builds those straight
+    from the coordinates; `index` / `num_index` are the SPConvIdx outputs of the current voxels, made when somebody asks
+    for them (plugin order, where every SPConvMM node reads them, fills them on every frame)."""
+    group = None      # submanifold: the rulebooks over the same voxel set, built in one pass
+    direct = False    # strided: tables from the coordinates
+    _index = _num_index = None
+
+    def buffers(self):
+        """Index buffers, allocated at first use."""
+        if self._index is None:
+            dev = self.shape_tensor.device
+            self._index = torch.empty((3, self.kvol * (self.sets[self.in_set]["cap"] + 128)), dtype=torch.int32,
+                                      device=dev)
+            self._num_index = torch.zeros(1, dtype=torch.int32, device=dev)
+        return self._index, self._num_index
+
+    def _current(self):
+        if self.group is not None or self.direct:
+            src = self.sets[self.in_set]
+            outs = list(self.buffers())
+            if self.kind != "subm":  # the same output voxels again, beside the live ones
+                dst = self.sets[self.out_set]
+                outs += [torch.empty_like(dst["coors"]), torch.empty_like(dst["num"]), self.out_shape_tensor]
+            self.plugin.enqueue(src["coors"], src["num"], self.shape_tensor, outputs=outs)
+        return self.buffers()
+
+    @property
+    def index(self):
+        return self._current()[0]
+
+    @property
+    def num_index(self):
+        return self._current()[1]
+
+
+class _SubmGroup:
+    """The submanifold rulebooks over one voxel set whose tables one pass can build; equal kernels share a table."""
+
+    def __init__(self):
+        self.by_ksize, self.pass_ = {}, None
+
+    def table_of(self, rb, make):
+        if rb.ksize not in self.by_ksize:
+            self.by_ksize[rb.ksize] = make()
+        return self.by_ksize[rb.ksize]
+
+    def enqueue(self, coors, num, shape):
+        sizes = list(self.by_ksize)
+        if self.pass_ is None or len(self.pass_.kernel_sizes) != len(sizes):
+            self.pass_ = SubmTables(sizes)
+        self.pass_.enqueue(coors, num, shape, tables=[self.by_ksize[k] for k in sizes])
 
 
 class SparseNet:
@@ -216,6 +266,7 @@ class SparseNet:
         self.kernel = kernel
         weights = make_weights(layers, seed)
         self.rulebooks = {}
+        self.groups = {}  # voxel set -> _SubmGroup
         self.mm = []
         self.sets = {"in": dict(cap=int(caps["in"]), shape=[int(v) for v in spatial], coors=None, num=None)}
         cur = "in"
@@ -239,6 +290,7 @@ class SparseNet:
                 if L.key not in self.rulebooks:
                     assert L.kind != "inverse", "an inverse layer needs the rulebook of its conv"
                     rb = _Rulebook()
+                    rb.sets = self.sets  # (not the net: no reference cycles, a dropped net frees its plugins at once)
                     rb.kind, rb.in_set, rb.ksize = L.kind, cur, L.ksize
                     # SubM with an odd kernel and 'same' padding: offsets k and kVol-1-k mirror each other
                     rb.mirror = (L.kind == "subm" and all(k % 2 == 1 for k in L.ksize) and
@@ -259,22 +311,32 @@ class SparseNet:
                         L.ksize, L.stride, L.padding, (1, 1, 1), (0, 0, 0), out["cap"], subm, False))
                     rb.shape_tensor = torch.empty([src["shape"][0], 0] + src["shape"][1:], dtype=torch.int32,
                                                   device=self.device)
-                    row_len = rb.kvol * (src["cap"] + 128)
                     rb.out_shape_tensor = torch.empty([out["shape"][0], 0] + out["shape"][1:], dtype=torch.int32,
                                                       device=self.device)
-                    rb.index = torch.empty((3, row_len), dtype=torch.int32, device=self.device)
-                    rb.num_index = torch.zeros(1, dtype=torch.int32, device=self.device)
                     if not subm:
                         out["coors"] = torch.zeros((out["cap"], 4), dtype=torch.int32, device=self.device)
                         out["num"] = torch.zeros(1, dtype=torch.int32, device=self.device)
-                    rb.table_fwd = None if plugin_order else torch.empty(
-                        max(SPConvMMPlugin.table_bytes(rb.kvol, out["cap"]), 16), dtype=torch.uint8,
-                        device=self.device)
+                    new_table = lambda: torch.empty(max(SPConvMMPlugin.table_bytes(rb.kvol, out["cap"]), 16),
+                                                    dtype=torch.uint8, device=self.device)
+                    if plugin_order:
+                        rb.table_fwd = None
+                    elif subm and rb.mirror and all(k in (1, 3) for k in L.ksize):
+                        # one pass per voxel set builds the tables of all its submanifold kernels
+                        rb.group = self.groups.setdefault(cur, _SubmGroup())
+                        if len(rb.group.by_ksize) >= SubmTables.MAX_TABLES and rb.ksize not in rb.group.by_ksize:
+                            rb.group = self.groups[cur] = _SubmGroup()
+                        rb.table_fwd = rb.group.table_of(rb, new_table)
+                    else:
+                        rb.table_fwd = new_table()
+                        rb.direct = not subm and rb.plugin.tables_ok(
+                            torch.empty((src["cap"], 4), dtype=torch.int32, device="meta"),
+                            torch.empty(1, dtype=torch.int32, device="meta"), rb.shape_tensor)
                     rb.table_inv = None
                     rb.raw_fwd = rb.raw_inv = rb.scratch_fwd = rb.scratch_inv = None
                     rb.regroup = self.regroup and rb.kvol <= 32
                     if rb.regroup:  # the builders write the plain table, the layers read the regrouped one
-                        rb.raw_fwd = torch.empty_like(rb.table_fwd)
+                        rb.raw_fwd = rb.table_fwd
+                        rb.table_fwd = torch.empty_like(rb.raw_fwd)
                         rb.scratch_fwd = torch.empty(
                             max(SPConvMMPlugin.regroup_scratch_bytes(rb.kvol, out["cap"]), 16), dtype=torch.uint8,
                             device=self.device)
@@ -330,33 +392,40 @@ class SparseNet:
         self.sets["in"]["coors"], self.sets["in"]["num"] = coors, num
 
     def _build_rulebook(self, rb):
+        """Whatever the layers of `rb` read; for a group of submanifold rulebooks, the tables of all of them."""
         src, dst = self.sets[rb.in_set], self.sets[rb.out_set]
         if self.plugin_order:  # the plain plugin entry point; every SPConvMM node builds its own table
-            outs = [rb.index, rb.num_index] if rb.kind == "subm" else \
-                [rb.index, rb.num_index, dst["coors"], dst["num"], rb.out_shape_tensor]
+            outs = list(rb.buffers()) if rb.kind == "subm" else \
+                list(rb.buffers()) + [dst["coors"], dst["num"], rb.out_shape_tensor]
             rb.plugin.enqueue(src["coors"], src["num"], rb.shape_tensor, outputs=outs)
             return
-        first = rb.calls == 0
-        rb.calls += 1
+        if rb.group is not None:
+            rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor)
+            for other in self.rulebooks.values():
+                if other.group is rb.group and other.regroup:
+                    SPConvMMPlugin.regroup(other.kvol, dst["cap"], other.raw_fwd, other.table_fwd, other.scratch_fwd)
+            return
         plain_fwd = rb.raw_fwd if rb.regroup else rb.table_fwd
-        if rb.kind == "subm":
-            rb.plugin.enqueue_ex(src["coors"], src["num"], rb.shape_tensor, outputs=[rb.index, rb.num_index],
-                                 persistent=True, first_call=first,
-                                 subm_table=plain_fwd if rb.fused_table else None)
-        else:
-            rb.plugin.enqueue_ex(src["coors"], src["num"], rb.shape_tensor,
-                                 outputs=[rb.index, rb.num_index, dst["coors"], dst["num"], rb.out_shape_tensor],
-                                 persistent=True, first_call=first)
-        if not rb.fused_table:
-            SPConvMMPlugin.prepare(rb.kvol, False, dst["cap"], rb.index, rb.num_index, table=plain_fwd,
-                                   mirror=rb.mirror)
+        plain_inv = rb.raw_inv if rb.regroup else rb.table_inv
+        if rb.direct:
+            rb.plugin.tables(src["coors"], src["num"], rb.shape_tensor, out_coors=dst["coors"],
+                             num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv)
+        else:  # kernels or grids the direct builders do not take
+            first = rb.calls == 0
+            rb.calls += 1
+            outs = list(rb.buffers())
+            if rb.kind != "subm":
+                outs += [dst["coors"], dst["num"], rb.out_shape_tensor]
+            rb.plugin.enqueue_ex(src["coors"], src["num"], rb.shape_tensor, outputs=outs, persistent=True,
+                                 first_call=first, subm_table=plain_fwd if rb.fused_table else None)
+            if not rb.fused_table:
+                SPConvMMPlugin.prepare(rb.kvol, False, dst["cap"], outs[0], outs[1], table=plain_fwd, mirror=rb.mirror)
+            if plain_inv is not None:
+                SPConvMMPlugin.prepare(rb.kvol, True, src["cap"], outs[0], outs[1], table=plain_inv)
         if rb.regroup:
             SPConvMMPlugin.regroup(rb.kvol, dst["cap"], plain_fwd, rb.table_fwd, rb.scratch_fwd)
-        if rb.table_inv is not None:
-            SPConvMMPlugin.prepare(rb.kvol, True, src["cap"], rb.index, rb.num_index,
-                                   table=rb.raw_inv if rb.regroup else rb.table_inv)
-            if rb.regroup:
-                SPConvMMPlugin.regroup(rb.kvol, src["cap"], rb.raw_inv, rb.table_inv, rb.scratch_inv)
+            if plain_inv is not None:
+                SPConvMMPlugin.regroup(rb.kvol, src["cap"], plain_inv, rb.table_inv, rb.scratch_inv)
 
     def forward(self, feats):
         """feats [cap_in, Cin] in the net dtype; coordinates / count as given to set_input.  Returns
@@ -377,8 +446,9 @@ class SparseNet:
             for L in self.layers:
                 if L.kind == "ew" or L.key in done:
                     continue
-                done.add(L.key)
                 rb = self.rulebooks[L.key]
+                keys = [L.key] if rb.group is None else [k for k, r in self.rulebooks.items() if r.group is rb.group]
+                done.update(keys)
                 stream = self.side_subm if rb.kind == "subm" else self.side
                 with torch.cuda.stream(stream):
                     # rb.in_set is named after the strided rulebook that wrote its coordinates ('in': the caller)
@@ -387,7 +457,7 @@ class SparseNet:
                     self._build_rulebook(rb)
                     ev = torch.cuda.Event()
                     ev.record(stream)
-                    ready[L.key] = ev
+                    ready.update((k, ev) for k in keys)
         built = set()
         saved = {"input": feats}
         x = feats
@@ -407,12 +477,13 @@ class SparseNet:
                     main.wait_event(ready[L.key])
                 else:
                     self._build_rulebook(rb)
+                    if rb.group is not None:
+                        built.update(k for k, r in self.rulebooks.items() if r.group is rb.group)
                 built.add(L.key)
             res = saved[L.residual] if L.residual else None
             if self.plugin_order:
                 in_set = rb.out_set if L.kind == "inverse" else rb.in_set
-                plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], rb.index, rb.num_index,
-                             outputs=[out_buf])
+                plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], *rb.buffers(), outputs=[out_buf])
                 if L.relu and L.act_first:
                     out_buf.relu_()
                 if res is not None:
@@ -447,7 +518,8 @@ class SparseNet:
                 continue
             rb = self.rulebooks[L.key]
             if L.key not in pairs:
-                k = rb.index[2, :int(rb.num_index.item())]
+                index, num_index = rb._current()
+                k = index[2, :int(num_index.item())]
                 pairs[L.key] = int((k >= 0).sum().item())
             out.append((plug.p.in_channels, plug.p.out_channels, rb.kvol, int(self.sets[out_set]["num"].item()),
                         pairs[L.key]))

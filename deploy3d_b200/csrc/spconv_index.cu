@@ -12,7 +12,10 @@
 // Work decomposition: one thread per (input voxel, kernel row), a kernel row being the run of offsets along the
 // fastest axis; a warp holds 32 consecutive inputs of one row so the pair table is written with 128-byte
 // coalesced stores and the probes of one thread fall into one 32-byte hash bucket (see common.cuh).
+#include <algorithm>
+
 #include "common.cuh"
+#include "spconv_mm_internal.h"
 
 namespace d3d {
 namespace {
@@ -640,6 +643,8 @@ __global__ void __launch_bounds__(1024) segment_scan_kernel(int32_t* __restrict_
   __shared__ int warp_sum[32];
   __shared__ int carry_s, chunk_total;
   __shared__ bool last;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int n = live_count(num_act_in, n_max);
   const int live_blk = (n + kIdxThreads - 1) / kIdxThreads;
   const int warp = threadIdx.x >> 5, lane = lane_id();
@@ -866,12 +871,11 @@ compact_packed_kernel(const int32_t* __restrict__ pair_out, const int32_t* __res
 
 // Everything that is not a pair is -1: the unused tail of each 128-aligned segment and the rows beyond
 // numIndex (the reference memsets the three rows beforehand, trt/spconv/index.cu:352-354).
-__global__ void fill_padding_kernel(const int32_t* __restrict__ seg, int kvol, int32_t* __restrict__ index,
-                                    int64_t row_len, const int32_t* __restrict__ state) {
+__device__ __forceinline__ void fill_padding(const int32_t* __restrict__ seg, int kvol, int32_t* __restrict__ index,
+                                             int64_t row_len, const int32_t* __restrict__ state, int64_t tid,
+                                             int64_t nthreads) {
   int num_index = seg[kvol];
   const int64_t fill_end = state[0];  // row_len, or where the previous rulebook in this buffer ended
-  int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   // in-segment padding: at most 127 entries per offset
   for (int64_t t = tid; t < (int64_t)kvol * kSegment; t += nthreads) {
     int k = (int)(t / kSegment), j = (int)(t % kSegment);
@@ -906,6 +910,20 @@ __global__ void fill_padding_kernel(const int32_t* __restrict__ seg, int kvol, i
   }
 }
 
+__global__ void fill_padding_kernel(const int32_t* __restrict__ seg, int kvol, int32_t* __restrict__ index,
+                                    int64_t row_len, const int32_t* __restrict__ state) {
+  fill_padding(seg, kvol, index, row_len, state, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+               (int64_t)gridDim.x * blockDim.x);
+}
+
+}  // namespace
+}  // namespace d3d
+
+#include "spconv_index3.cuh"
+
+namespace d3d {
+namespace {
+
 struct Plan {
   Geometry g;
   int64_t n_max;
@@ -922,11 +940,39 @@ struct Plan {
   int32_t* winners;
   uint32_t* win_bits;  // per input: which of its offsets won an output voxel (kvol <= 32)
   int32_t* state;      // words that survive between calls, and the ticket of segment_scan_kernel
+  // 3-D kernels of at most three taps per axis (spconv_index3.cuh); kHash: the kernels of this file
+  enum Path { kHash, kBits, kDirect } path;
+  int64_t cells;
+  bool two_taps;       // at most two taps per axis reach an output from one input
+  int32_t* grid;
+  uint32_t* bits;
+  uint8_t* list_local;
+  unsigned long long* chain;
   bool packed;         // strided rulebook kept as kPackedSlots entries per input instead of kvol
   size_t bytes;
 };
 
-int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* workspace, Plan* plan) {
+// Which lookup a 3-D rulebook uses, by grid cells per voxel buffer row.
+//   strided    clearing the grid (4 bytes per cell, 5 TB/s) against what the hash path costs beyond it, 0.4 ns per
+//              input measured on B200: even at about 500 cells per input.
+//   submanifold  the same clearing against the bit map's hash insertion and its second round of loads, 0.05 ns per
+//              voxel: even at about 64 cells per voxel.  The bit map itself (a bit per cell) saves two thirds of the
+//              probe kernel; below one voxel per 128 k cells clearing it costs more than that.
+// `tables`: for d3d_spconv_subm_tables, which has no other kernels to fall back to.
+Plan::Path pick_lookup(const d3d_spconv_index_params* p, const Geometry& g, int64_t cells, int64_t n_max, bool tables) {
+  if (g.ndim != 3 || n_max < 1) return Plan::kHash;
+  for (int d = 0; d < 3; ++d)
+    if (g.ksize[d] > 3) return Plan::kHash;
+  if (!p->subm) return cells <= 512 * n_max ? Plan::kDirect : Plan::kHash;
+  for (int d = 0; d < 3; ++d)
+    if (g.stride[d] != 1) return Plan::kHash;
+  if (cells <= 64 * n_max) return Plan::kDirect;
+  if (tables) return Plan::kBits;
+  return cells <= (128 << 10) * n_max && 2 * g.dil[2] < 32 ? Plan::kBits : Plan::kHash;
+}
+
+int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* workspace, Plan* plan,
+              bool tables = false) {
   D3D_REQUIRE(p && in && n_in >= 3, D3D_ERR_INVALID_ARGUMENT);
   int ndim = p->ndim;
   D3D_REQUIRE(ndim >= 1 && ndim <= D3D_MAX_NDIM, D3D_ERR_INVALID_ARGUMENT);
@@ -976,12 +1022,25 @@ int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n
   size_t cap = next_pow2((size_t)(plan->n_max > 8 ? plan->n_max : 8) * plan->fan * 2);
   D3D_REQUIRE(cap <= (1ull << 30), D3D_ERR_TOO_LARGE);
   plan->cap_max = (uint32_t)(cap < 16 ? 16 : cap);
+  plan->cells = vol;
+  plan->two_taps = true;
+  for (int d = 0; d < ndim; ++d) {
+    int common = g.stride[d], rest = g.dil[d] % g.stride[d];
+    while (rest) { const int t = common % rest; common = rest, rest = t; }  // gcd(stride, dilation)
+    const int taps = (g.transpose || common != 1) ? g.ksize[d] : (g.ksize[d] + g.stride[d] - 1) / g.stride[d];
+    if (taps > 2) plan->two_taps = false;
+  }
+  plan->path = pick_lookup(p, g, vol, plan->n_max, tables);
   Carver w(workspace);
-  plan->table = w.take<unsigned long long>(plan->cap_max);
-  plan->pair_out = w.take<int32_t>((size_t)g.kvol * (plan->n_max > 0 ? plan->n_max : 1));
+  plan->table = plan->path == Plan::kDirect ? nullptr : w.take<unsigned long long>(plan->cap_max);
+  plan->grid = plan->path == Plan::kDirect ? w.take<int32_t>((size_t)(vol + 63) / 64 * 64) : nullptr;
+  plan->bits = plan->path == Plan::kBits ? w.take<uint32_t>((size_t)((vol + 31) / 32 + 63) / 64 * 64) : nullptr;
+  plan->pair_out = w.take<int32_t>((size_t)g.kvol * (plan->n_max > 0 ? (size_t)plan->nblk * kIdxThreads : 1));
+  plan->list_local = plan->path == Plan::kHash ? nullptr : w.take<uint8_t>((size_t)g.kvol * plan->nblk * kIdxThreads);
+  plan->chain = plan->path == Plan::kDirect ? w.take<unsigned long long>(plan->nblk) : nullptr;
   plan->block_counts = w.take<int32_t>((size_t)g.kvol * plan->nblk);
   plan->seg = w.take<int32_t>(2 * (size_t)g.kvol + 2);
-  plan->slot_out = p->subm ? nullptr : w.take<int32_t>(plan->cap_max);
+  plan->slot_out = p->subm || plan->path == Plan::kDirect ? nullptr : w.take<int32_t>(plan->cap_max);
   plan->winners = p->subm ? nullptr : w.take<int32_t>((size_t)plan->nblk + 1);
   plan->win_bits = p->subm ? nullptr : w.take<uint32_t>((size_t)(plan->n_max > 0 ? plan->n_max : 1));
   plan->packed = !p->subm && !g.transpose && ndim == 3 && g.ksize[0] <= 3 && g.ksize[1] <= 3 && g.ksize[2] <= 3 &&
@@ -989,6 +1048,104 @@ int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n
                  p->max_num_act_out <= (1 << kPackedShift);
   plan->state = w.take<int32_t>(4);
   plan->bytes = w.off;
+  return D3D_OK;
+}
+
+// Launch in `st`, optionally as a programmatic dependent of the kernel before it (every kernel of spconv_index3.cuh
+// waits for that kernel itself): the launch gap inside a chain of 3-5 us kernels goes from about 1.2 to 0.4 us.
+template <class... P, class... A>
+int launch3(bool chained, void (*kern)(P...), int64_t grid, int threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3(threads), cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...) == cudaSuccess ? D3D_OK : D3D_ERR_CUDA;
+}
+#define D3D_LAUNCH3(...)                     \
+  do {                                       \
+    const int rc_ = launch3(__VA_ARGS__);    \
+    if (rc_ != D3D_OK) return rc_;           \
+  } while (0)
+
+TableTarget make_target(void* table, int kvol, int64_t m_max) {
+  const TableParts t = table_parts(table, kvol, m_max);
+  TableTarget r;
+  r.ids = t.ids, r.mask = t.tile_mask, r.rows = t.row_masks, r.perm = t.perm, r.kvol = kvol;
+  for (int s = 0; s < kTaps3; ++s) r.g_of_slot[s] = 0, r.slot_of_g[s] = -1;
+  return r;
+}
+// Slots of the table of a submanifold kernel with extents `ks` inside a pass over `outer` (equal, or 3 where ks is 1):
+// the voxel found for offset k feeds its input through offset kvol - 1 - k.
+void mirror_slots(TableTarget* t, const int* ks, const int* outer) {
+  for (int a = 0; a < ks[0]; ++a)
+    for (int b = 0; b < ks[1]; ++b)
+      for (int c = 0; c < ks[2]; ++c) {
+        const int k = (a * ks[1] + b) * ks[2] + c;
+        const int ga = a + (outer[0] - ks[0]) / 2, gb = b + (outer[1] - ks[1]) / 2, gc = c + (outer[2] - ks[2]) / 2;
+        const int g = (ga * 3 + gb) * 3 + gc;
+        t->g_of_slot[t->kvol - 1 - k] = (signed char)g, t->slot_of_g[g] = (signed char)(t->kvol - 1 - k);
+      }
+}
+void plain_slots(TableTarget* t, const Geometry& g) {
+  for (int q = 0; q < kTaps3; ++q) {
+    const int a = q / 9, b = q / 3 % 3, c = q % 3;
+    if (a < g.ksize[0] && b < g.ksize[1] && c < g.ksize[2]) {
+      const int k = (a * g.ksize[1] + b) * g.ksize[2] + c;
+      t->g_of_slot[k] = (signed char)q, t->slot_of_g[q] = (signed char)k;
+    }
+  }
+}
+
+ClearArgs clear_args(const Plan& plan) {
+  ClearArgs a = {};
+  a.look.direct = plan.grid, a.look.slots = plan.table, a.look.cap_max = plan.cap_max, a.look.bits = plan.bits;
+  a.direct_words = (plan.cells + 63) / 64 * 64;
+  a.bit_words = ((plan.cells + 31) / 32 + 63) / 64 * 64;
+  a.fan = plan.fan;
+  a.chain = plan.chain, a.chain_words = plan.chain ? plan.nblk : 0;
+  a.state = plan.state;
+  return a;
+}
+int64_t clear_grid(const ClearArgs& a) {
+  const int64_t words = (a.look.direct ? a.direct_words : 0) + (a.look.bits ? a.bit_words : 0) +
+                        (a.look.slots ? 2ll * a.look.cap_max : 0) + a.row_words + 4 * a.perm_words;
+  return stream_grid(words / 16, 256);  // four 16-byte stores per thread
+}
+
+// Lookup structure of the inputs, then their neighbours.
+int launch_subm3(const Plan& plan, const int32_t* coors, const int32_t* num_act_in, bool chained,
+                 const PairLists& lists, const Targets& targets, int32_t* status, cudaStream_t st) {
+  const ClearArgs a = clear_args(plan);
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  D3D_LAUNCH3(chained, subm_mark3_kernel, plan.nblk, kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g,
+              status);
+  // one block per 256 rows up to the end of the tables, so that rows beyond the live count get their masks
+  const int64_t blocks = targets.count ? std::max<int64_t>(plan.nblk, ceil_div(targets.tiles * 128, kIdxThreads))
+                                       : plan.nblk;
+  D3D_LAUNCH3(chained, plan.path == Plan::kDirect ? subm_find3_kernel<true> : subm_find3_kernel<false>, blocks,
+              kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g, lists, targets);
+  return D3D_OK;
+}
+
+int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_in, int32_t max_out, bool chained,
+                 const PairLists& lists, const TableParts* fwd, int64_t fwd_rows, const Targets& inverse,
+                 int32_t* out_coors, int32_t* num_act_out, int32_t* status, cudaStream_t st) {
+  ClearArgs a = clear_args(plan);
+  if (fwd) {
+    a.rows = fwd->row_masks, a.row_words = fwd->tiles * plan.g.kvol * 4;
+    a.perm = fwd->perm, a.perm_words = fwd->tiles * 128, a.m_max = fwd_rows;
+  }
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  const bool two = plan.two_taps;
+  D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
+  D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
+              coors, num_act_in, plan.n_max, plan.g, max_out, plan.chain, out_coors, num_act_out, status);
+  const int64_t blocks = inverse.count ? std::max<int64_t>(plan.nblk, ceil_div(inverse.tiles * 128, kIdxThreads))
+                                       : plan.nblk;
+  D3D_LAUNCH3(chained, two ? conv_find3_kernel<2> : conv_find3_kernel<3>, blocks, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g,
+              lists, fwd ? fwd->ids : nullptr, fwd ? fwd->row_masks : nullptr, inverse);
   return D3D_OK;
 }
 
@@ -1106,6 +1263,35 @@ extern "C" int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, con
   }
   D3D_REQUIRE(coors && num_act_in && index && num_index, D3D_ERR_INVALID_ARGUMENT);
   const int nblk = plan.nblk;
+  if (plan.path != Plan::kHash) {
+    // The plain entry point is called from one stream, kernel after kernel: chained launches.  A caller with buffers of
+    // its own runs other work beside the rulebooks, which blocks that wait early would keep from the SMs.
+    const bool chained = !persistent;
+    const PairLists lists = {plan.pair_out, plan.list_local, plan.block_counts, nblk};
+    Targets targets = {};
+    if (p->subm) {
+      if (nbr) {
+        targets.count = 1, targets.tiles = (n_max + 127) / 128;
+        targets.t[0] = make_target(nbr, g.kvol, n_max);
+        mirror_slots(&targets.t[0], g.ksize, g.ksize);
+      }
+      rc = launch_subm3(plan, coors, num_act_in, chained, lists, targets, status, st);
+    } else {
+      int32_t* out_coors = reinterpret_cast<int32_t*>(outputs[2]);
+      int32_t* num_act_out = reinterpret_cast<int32_t*>(outputs[3]);
+      D3D_REQUIRE(out_coors && num_act_out, D3D_ERR_INVALID_ARGUMENT);
+      D3D_REQUIRE(out[2].dims[0] >= p->max_num_act_out, D3D_ERR_INVALID_ARGUMENT);
+      rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, chained, lists, nullptr, 0, targets, out_coors,
+                        num_act_out, status, st);
+    }
+    if (rc != D3D_OK) return rc;
+    D3D_LAUNCH3(chained, segment_scan_kernel, g.kvol, 1024, st, plan.block_counts, nblk, g.kvol, num_act_in, n_max,
+                plan.seg, num_index, plan.state, persistent, first, plan.row_len);
+    D3D_LAUNCH3(chained, emit_index3_kernel, nblk + stream_grid(3 * plan.row_len / 16, kIdxThreads, 4), kIdxThreads, st,
+                lists, plan.seg, num_act_in, n_max, g.kvol, index, plan.row_len, plan.state);
+    D3D_CHECK_LAUNCH();
+    return D3D_OK;
+  }
   reset_table_kernel<<<stream_grid(plan.cap_max / 2, 256), 256, 0, st>>>(plan.table, num_act_in, n_max, plan.fan,
                                                                          plan.cap_max, plan.state);
   if (p->subm) {
@@ -1179,6 +1365,104 @@ extern "C" int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, con
                                                                num_act_in, n_max, nblk, index, plan.row_len);
   fill_padding_kernel<<<stream_grid(3 * plan.row_len, 256), 256, 0, st>>>(plan.seg, g.kvol, index, plan.row_len,
                                                                           plan.state);
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
+// ---- neighbour tables without the rulebook ---------------------------------------------------------------------------
+namespace {
+void subm_params(d3d_spconv_index_params* p, const int* ks) {
+  memset(p, 0, sizeof(*p));
+  p->ndim = 3, p->subm = 1;
+  for (int d = 0; d < 3; ++d) p->kernel_size[d] = ks[d], p->stride[d] = p->dilation[d] = 1, p->padding[d] = ks[d] / 2;
+}
+}  // namespace
+
+extern "C" int d3d_spconv_subm_tables_workspace(const d3d_tensor_desc* in, int n_in, size_t* bytes) {
+  const int ks[3] = {3, 3, 3};
+  d3d_spconv_index_params p;
+  subm_params(&p, ks);
+  D3D_REQUIRE(bytes, D3D_ERR_INVALID_ARGUMENT);
+  Plan plan;
+  const int rc = make_plan(&p, in, n_in, nullptr, &plan, true);
+  if (rc == D3D_OK) *bytes = plan.bytes;
+  return rc;
+}
+
+extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables,
+                                      const d3d_tensor_desc* in, int n_in, const void* const* inputs, void* workspace,
+                                      size_t workspace_bytes, void* stream, int32_t* status) {
+  D3D_NVTX_RANGE("d3d_spconv_subm_tables");
+  D3D_REQUIRE(n_tables >= 1 && n_tables <= kMaxTargets && kernel_size && tables && inputs, D3D_ERR_INVALID_ARGUMENT);
+  int outer[3] = {1, 1, 1};
+  for (int t = 0; t < n_tables; ++t)
+    for (int d = 0; d < 3; ++d) {
+      const int k = kernel_size[3 * t + d];
+      D3D_REQUIRE((k == 1 || k == 3) && tables[t], D3D_ERR_INVALID_ARGUMENT);
+      if (k > outer[d]) outer[d] = k;
+    }
+  d3d_spconv_index_params p;
+  const int ks3[3] = {3, 3, 3};
+  subm_params(&p, ks3);  // the workspace's layout
+  Plan plan;
+  int rc = make_plan(&p, in, n_in, workspace, &plan, true);
+  if (rc != D3D_OK) return rc;
+  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  const int64_t n_max = plan.n_max;
+  if (n_max == 0) return D3D_OK;
+  const int32_t* coors = reinterpret_cast<const int32_t*>(inputs[0]);
+  const int32_t* num_act_in = reinterpret_cast<const int32_t*>(inputs[1]);
+  D3D_REQUIRE(coors && num_act_in, D3D_ERR_INVALID_ARGUMENT);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  Targets targets = {};
+  targets.count = n_tables, targets.tiles = (n_max + 127) / 128;
+  plan.g.kvol = 1;
+  for (int d = 0; d < 3; ++d) plan.g.ksize[d] = outer[d], plan.g.pad[d] = outer[d] / 2, plan.g.kvol *= outer[d];
+  for (int t = 0; t < n_tables; ++t) {
+    const int ks[3] = {kernel_size[3 * t], kernel_size[3 * t + 1], kernel_size[3 * t + 2]};
+    targets.t[t] = make_target(tables[t], ks[0] * ks[1] * ks[2], n_max);
+    mirror_slots(&targets.t[t], ks, outer);
+  }
+  rc = launch_subm3(plan, coors, num_act_in, false, PairLists{}, targets, status, st);
+  if (rc != D3D_OK) return rc;
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
+extern "C" int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in) {
+  Plan plan;
+  if (!p || p->subm || make_plan(p, in, n_in, nullptr, &plan) != D3D_OK) return 0;
+  return plan.path == Plan::kDirect && plan.g.kvol <= 32;
+}
+
+extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                                      const void* const* inputs, int32_t* out_coors, int32_t* num_act_out, void* table,
+                                      void* table_inverse, void* workspace, size_t workspace_bytes, void* stream,
+                                      int32_t* status) {
+  D3D_NVTX_RANGE("d3d_spconv_conv_tables");
+  D3D_REQUIRE(p && inputs && out_coors && num_act_out && table, D3D_ERR_INVALID_ARGUMENT);
+  Plan plan;
+  int rc = make_plan(p, in, n_in, workspace, &plan);
+  if (rc != D3D_OK) return rc;
+  D3D_REQUIRE(!p->subm && plan.path == Plan::kDirect && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
+  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  const int32_t* coors = reinterpret_cast<const int32_t*>(inputs[0]);
+  const int32_t* num_act_in = reinterpret_cast<const int32_t*>(inputs[1]);
+  D3D_REQUIRE(coors && num_act_in, D3D_ERR_INVALID_ARGUMENT);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int kvol = plan.g.kvol;
+  const TableParts fwd = table_parts(table, kvol, p->max_num_act_out);
+  Targets inverse = {};
+  if (table_inverse) {
+    inverse.count = 1, inverse.tiles = (plan.n_max + 127) / 128;
+    inverse.t[0] = make_target(table_inverse, kvol, plan.n_max);
+    plain_slots(&inverse.t[0], plan.g);
+  }
+  rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, false, PairLists{}, &fwd, p->max_num_act_out, inverse,
+                    out_coors, num_act_out, status, st);
+  if (rc != D3D_OK) return rc;
+  rc = pack_table_masks(fwd, kvol, st);
+  if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }

@@ -303,6 +303,13 @@ template <class T> int launch_simt_typed(const MmLaunch& a) {
 
 }  // namespace
 
+int pack_table_masks(const TableParts& t, int kernel_vol, void* stream) {
+  pack_mask_kernel<<<(unsigned)ceil_div(t.tiles * 32, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const uint4*>(t.row_masks), t.tiles, kernel_vol, t.tile_mask);
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
 int launch_spconv_mm_simt(const MmLaunch& a) {
   switch (a.dtype) {
     case D3D_FLOAT: return launch_simt_typed<float>(a);

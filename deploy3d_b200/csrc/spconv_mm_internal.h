@@ -81,6 +81,9 @@ inline size_t table_perm_bytes(int64_t max_num_act_out) {
   return (tiles * 128 * sizeof(int32_t) + 255) / 256 * 256;
 }
 
+// Derives the offset mask of every tile from its row masks (cudaStream_t as void*).
+int pack_table_masks(const TableParts& t, int kernel_vol, void* stream);
+
 int launch_spconv_mm_simt(const MmLaunch& a);
 // Returns D3D_ERR_INVALID_ARGUMENT when the shape/dtype is not eligible for the tensor-core path.
 bool spconv_mm_tc_eligible(const d3d_spconv_mm_s* h, int dtype);

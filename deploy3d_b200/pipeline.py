@@ -163,7 +163,8 @@ class DetectionPipeline:
                   self.scores, self.nms_scores, self.vfe._workspace, self.densify._workspace, self.nms._workspace):
             add(t)
         for rb in self.net.rulebooks.values():
-            for t in (rb.index, rb.table_fwd, rb.table_inv, rb.plugin._workspace):
+            for t in (rb._index, rb.table_fwd, rb.table_inv, rb.plugin._workspace,
+                      rb.group.pass_._workspace if rb.group is not None and rb.group.pass_ is not None else None):
                 add(t)
         for _, buf, _ in self.net.mm:
             add(buf)

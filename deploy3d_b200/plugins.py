@@ -140,6 +140,55 @@ class SPConvIdxPlugin(_Plugin):
         return tuple(outputs)
 
 
+    def tables_ok(self, *inputs):
+        """True when `tables` can build this strided kernel's neighbour tables without the rulebook."""
+        d = [_desc_of(t) for t in inputs]
+        return bool(lib().d3d_spconv_conv_tables_ok(ctypes.byref(self.p), desc_array(d), len(d)))
+
+    def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None):
+        """Output voxels and neighbour tables of a strided kernel straight from the coordinates, no `index`
+        (d3d_spconv_conv_tables)."""
+        device = inputs[0].device
+        d = [_desc_of(t) for t in inputs]
+        nbytes = self.workspace_size(d)
+        ws = self._get_workspace(nbytes, device)
+        with torch.cuda.device(device):
+            check("d3d_spconv_conv_tables", lib().d3d_spconv_conv_tables(
+                ctypes.byref(self.p), desc_array(d), len(d), ptr_array([t.data_ptr() for t in inputs]),
+                out_coors.data_ptr(), num_act_out.data_ptr(), table.data_ptr(),
+                table_inverse.data_ptr() if table_inverse is not None else None, ws.data_ptr(), nbytes,
+                _stream_ptr(stream), status.data_ptr() if status is not None else None))
+
+
+class SubmTables:
+    """Neighbour tables of up to eight submanifold kernels (extents 1 or 3, dilation 1, 'same' padding) over one voxel
+    set, built in one pass over its voxels and without their rulebooks (d3d_spconv_subm_tables)."""
+    MAX_TABLES = 8
+
+    def __init__(self, kernel_sizes):
+        assert 1 <= len(kernel_sizes) <= self.MAX_TABLES
+        self.kernel_sizes = [tuple(int(v) for v in k) for k in kernel_sizes]
+        flat = [v for k in self.kernel_sizes for v in k]
+        self._flat = (ctypes.c_int32 * len(flat))(*flat)
+        self._workspace = None
+
+    def enqueue(self, *inputs, tables, status=None, stream=None):
+        """inputs: coordinates, count, shape carrier (as SPConvIdx3d); `tables`: one buffer per kernel size."""
+        assert len(tables) == len(self.kernel_sizes)
+        device = inputs[0].device
+        d = [_desc_of(t) for t in inputs]
+        n = ctypes.c_size_t(0)
+        check("d3d_spconv_subm_tables_workspace",
+              lib().d3d_spconv_subm_tables_workspace(desc_array(d), len(d), ctypes.byref(n)))
+        if self._workspace is None or self._workspace.numel() < n.value or self._workspace.device != device:
+            self._workspace = torch.empty(n.value, dtype=torch.uint8, device=device)
+        with torch.cuda.device(device):
+            check("d3d_spconv_subm_tables", lib().d3d_spconv_subm_tables(
+                len(tables), self._flat, ptr_array([t.data_ptr() for t in tables]), desc_array(d), len(d),
+                ptr_array([t.data_ptr() for t in inputs]), self._workspace.data_ptr(), n.value, _stream_ptr(stream),
+                status.data_ptr() if status is not None else None))
+
+
 class SPConvMMPlugin(_Plugin):
     """``SPConvMM`` (trt/spconv/mm_trt.cu:39-206); owns the weight handle."""
     name = "SPConvMM"

@@ -46,6 +46,7 @@ typedef enum {
  * (trt/include/common/hash32.h:70) and outputs beyond maxNumActOut are dropped (trt/spconv/index.cu:163-168). */
 #define D3D_STATUS_HASH_FULL 1       /* a key found no free slot: its pairs / points were dropped */
 #define D3D_STATUS_OUTPUT_OVERFLOW 2 /* more output voxels than maxNumActOut: the surplus was dropped */
+#define D3D_STATUS_STALLED 4         /* a bounded wait inside a kernel ran out: the results are not valid */
 
 /* Values follow nvinfer1::DataType so a plugin shell can pass PluginTensorDesc::type through. */
 typedef enum {
@@ -154,6 +155,28 @@ int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, const d3d_tens
                                 const d3d_tensor_desc* out, int n_out, const void* const* inputs,
                                 void* const* outputs, void* workspace, size_t workspace_bytes, void* stream,
                                 const d3d_spconv_index_extras* extras);
+
+/* Neighbour tables without the rulebook (no reference counterpart: its convolution reads the rulebook itself).  A caller
+ * that runs SPConvMM in its two-step form needs the tables only; these entry points build them from the coordinates,
+ * with the contents d3d_spconv_mm_prepare would give them, and write no `index`.
+ *  d3d_spconv_subm_tables  n_tables submanifold kernels over ONE voxel set in one pass (at most 8): kernel_size[t] has
+ *      extents of 1 or 3, stride and dilation 1, padding (k - 1) / 2; tables[t] holds d3d_spconv_mm_table_bytes(kVol_t,
+ *      maxNumActIn) bytes.  in / inputs as SPConvIdx3d (coordinates without duplicates, count, shape carrier).
+ *  d3d_spconv_conv_tables  one strided or transposed 3-D kernel of at most three taps per axis (p->subm == 0): writes
+ *      the output coordinates and their number (SPConvIdx's outputs 2 and 3) and `table` (over the outputs); when
+ *      non-null, also `table_inverse` (over the inputs, for the inverse convolution).
+ *  d3d_spconv_conv_tables_ok  1 when d3d_spconv_conv_tables accepts this kernel and grid; otherwise build the rulebook
+ *      and use d3d_spconv_mm_prepare.
+ * Workspace: d3d_spconv_subm_tables_workspace; for conv_tables, d3d_spconv_index_workspace. */
+int d3d_spconv_subm_tables_workspace(const d3d_tensor_desc* in, int n_in, size_t* bytes);
+int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables, const d3d_tensor_desc* in,
+                           int n_in, const void* const* inputs, void* workspace, size_t workspace_bytes, void* stream,
+                           int32_t* status);
+int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in);
+int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                           const void* const* inputs, int32_t* out_coors, int32_t* num_act_out, void* table,
+                           void* table_inverse, void* workspace, size_t workspace_bytes, void* stream,
+                           int32_t* status);
 
 /* ---------------------------------------------------------------------------------------------
  * SPConvMM -- gather / GEMM / scatter over the rulebook.

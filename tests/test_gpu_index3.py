@@ -1,0 +1,134 @@
+"""The rulebook kernels for 3-D kernels of at most three taps per axis: every lookup they choose between (the grid itself,
+bit map + hash table, hash table), block edges, truncation, and the neighbour tables built without the rulebook."""
+import numpy as np
+import pytest
+import torch
+
+from tests._util import assert_table_consistent, assert_tables_equal, rng, table_pairs, table_parts, unique_coors
+from tests.test_gpu_spconv import DEV, _t, check_index, run_index
+
+pytestmark = pytest.mark.gpu
+ONE, ZERO = (1, 1, 1), (0, 0, 0)
+GRIDS = {"direct": [1, 9, 20, 21], "bits": [2, 40, 160, 150], "hash": [1, 41, 1600, 1408]}
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 600])
+@pytest.mark.parametrize("ks,dil", [((3, 3, 3), ONE), ((1, 3, 3), (1, 2, 1)), ((3, 1, 2), (3, 1, 2)), ((2, 3, 1), ONE)])
+def test_subm_rulebook(d3d, orc, grid, n, ks, dil):
+    shape = GRIDS[grid]
+    coors = unique_coors(rng(n), n, shape) if np.prod(shape) < 1 << 24 else \
+        np.unique(np.stack([rng(n + d).integers(0, s, n) for d, s in enumerate(shape)], 1), axis=0).astype(np.int32)
+    coors[: n // 2, 1:] = coors[: n // 2, 1:] // 4  # some of them crowded, so that neighbours exist
+    coors = np.unique(coors, axis=0)
+    coors = coors[rng(1).permutation(len(coors))]
+    pd = tuple(d * (k // 2) for k, d in zip(ks, dil))
+    n_max = len(coors) + (0 if n % 2 else 77)
+    outs, _ = run_index(d3d, coors, n_max, [shape[0], 0] + shape[1:], ks, ONE, pd, dil, ZERO, n_max, True, False)
+    check_index(orc, outs, coors, n_max, shape, ks, ONE, pd, dil, ZERO, n_max, True, False)
+
+
+@pytest.mark.parametrize("grid", ["direct", "bits"])
+def test_subm_rulebook_with_duplicates_and_stray_voxels(d3d, orc, grid):
+    """Voxels that occur twice (the smaller index stands for both) and coordinates outside the grid."""
+    shape = GRIDS[grid]
+    coors = unique_coors(rng(5), 400, shape)
+    coors[200:300] = coors[:100]
+    coors[350:360, 3] = shape[3] + 5
+    coors[360:365, 0] = -1
+    outs, _ = run_index(d3d, coors, 400, [shape[0], 0] + shape[1:], (3, 3, 3), ONE, ONE, ONE, ZERO, 400, True, False)
+    first = {}
+    for i, c in enumerate(map(tuple, coors.tolist())):
+        if all(0 <= v < e for v, e in zip(c, shape)):
+            first.setdefault(c, i)
+    index, num = outs[0].cpu().numpy(), int(outs[1].item())
+    orc.check_layout(index, num, 27)
+    for k in range(27):
+        tap = np.array([0, k // 9, k // 3 % 3, k % 3]) - [0, 1, 1, 1]
+        pairs = [(i, first[c]) for i, c in enumerate(map(tuple, (coors - tap).tolist())) if c in first]
+        got = index[:2, :num][:, index[2, :num] == k].T
+        assert got.tolist() == [list(p) for p in pairs], k
+
+
+CONVS = [((3, 3, 3), (2, 2, 2), ONE, ONE, False), ((3, 1, 1), (2, 1, 1), ZERO, ONE, False),
+         ((3, 3, 3), ONE, ONE, ONE, False), ((3, 3, 3), (2, 2, 1), ONE, (2, 1, 1), False),
+         ((2, 2, 2), (2, 2, 2), ZERO, ONE, True), ((3, 3, 3), (3, 2, 1), ONE, ONE, True)]
+
+
+@pytest.mark.parametrize("n", [1, 256, 257, 1500])
+@pytest.mark.parametrize("ks,st,pd,dil,tr", CONVS)
+@pytest.mark.parametrize("room", [1.0, 0.3])
+def test_conv_rulebook(d3d, orc, n, ks, st, pd, dil, tr, room):
+    shape = [2, 13, 24, 25]
+    coors = unique_coors(rng(n), n, shape)
+    m = orc.rulebook_conv(coors, shape, ks, st, pd, dil, ZERO, tr, 10 ** 7, max_num_act_in=n)[3]
+    max_out = max(1, int(m * room))
+    outs, _ = run_index(d3d, coors, n, [2, 0] + shape[1:], ks, st, pd, dil, ZERO, max_out, False, tr)
+    check_index(orc, outs, coors, n, shape, ks, st, pd, dil, ZERO, max_out, False, tr)
+    assert int(outs[3].item()) == min(m, max_out)
+
+
+def test_conv_numbering_is_by_first_touch_across_many_blocks(d3d):
+    """A thousand blocks: the numbers are those of a serial walk over the inputs and, for each, over the offsets."""
+    shape, n = [1, 21, 400, 352], 300000
+    coors = unique_coors(rng(8), n, shape)
+    outs, _ = run_index(d3d, coors, n, [1, 0] + shape[1:], (3, 3, 3), (2, 2, 2), ONE, ONE, ZERO, 600000, False, False)
+    tap = np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(27, 3)
+    at = coors[:, None, 1:] + 1 - tap[None]
+    ok = ((at % 2 == 0) & (at >= 0) & (at // 2 < np.array([11, 200, 176]))).all(-1)
+    key = ((at[..., 0] // 2 * 200 + at[..., 1] // 2) * 176 + at[..., 2] // 2)[ok]
+    _, first = np.unique(key, return_index=True)
+    want = key[np.sort(first)]
+    m = int(outs[3].item())
+    got = outs[2].cpu().numpy()[:m]
+    assert m == len(want) and ((got[:, 1] * 200 + got[:, 2]) * 176 + got[:, 3] == want).all()
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("n", [1, 128, 129, 400])
+def test_subm_tables_of_several_kernels(d3d, grid, n):
+    from deploy3d_b200.plugins import SPConvMMPlugin, SubmTables
+    shape, cap = GRIDS[grid], 500
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, [shape[0], 9, 12, 13])
+    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
+    shp = torch.empty([shape[0], 0] + shape[1:], dtype=torch.int32, device=DEV)
+    kernels = [(3, 3, 3), (1, 3, 3), (3, 1, 3), (3, 1, 1), (1, 3, 1), (1, 1, 3), (1, 1, 1)]
+    for sub in (kernels, kernels[1:2], kernels[3:5]):
+        vols = [int(np.prod(k)) for k in sub]
+        tables = [torch.full((SPConvMMPlugin.table_bytes(v, cap),), 93, dtype=torch.uint8, device=DEV) for v in vols]
+        SubmTables(sub).enqueue(coors_t, num, shp, tables=tables)
+        for k, v, t in zip(sub, vols, tables):
+            index, num_index = d3d.spconv_index(coors_t, num, shp, k, ONE, tuple(x // 2 for x in k), ONE, ZERO, cap,
+                                                True, False)
+            want = SPConvMMPlugin.prepare(v, False, cap, index, num_index)
+            got = table_parts(t, v, cap)
+            assert_tables_equal(got, table_parts(want, v, cap), "%s" % (k,))
+            assert_table_consistent(*got)
+
+
+@pytest.mark.parametrize("ks,st,pd,dil,tr", CONVS)
+@pytest.mark.parametrize("n,room", [(1, 1.0), (700, 1.3), (700, 0.4)])
+def test_conv_tables(d3d, orc, ks, st, pd, dil, tr, n, room):
+    from deploy3d_b200.plugins import SPConvMMPlugin, deserialize_plugin
+    shape, cap, kvol = [1, 13, 24, 25], 750, int(np.prod(ks))
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, shape)
+    m = orc.rulebook_conv(coors[:n], shape, ks, st, pd, dil, ZERO, tr, 10 ** 7, max_num_act_in=n)[3]
+    max_out = max(1, int(m * room))
+    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
+    shp = torch.empty([1, 0] + shape[1:], dtype=torch.int32, device=DEV)
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, dil, ZERO, max_out, False, tr))
+    assert plug.tables_ok(coors_t, num, shp)
+    fwd = torch.full((SPConvMMPlugin.table_bytes(kvol, max_out),), 55, dtype=torch.uint8, device=DEV)
+    inv = torch.full((SPConvMMPlugin.table_bytes(kvol, cap),), 55, dtype=torch.uint8, device=DEV)
+    oc, on = torch.zeros((max_out, 4), dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(2):
+        plug.tables(coors_t, num, shp, out_coors=oc, num_act_out=on, table=fwd, table_inverse=inv)
+    index, num_index, woc, won, _ = plug.enqueue(coors_t, num, shp)
+    live = int(won.item())
+    assert int(on.item()) == live and torch.equal(oc[:live], woc[:live])
+    for inverse, rows, t in ((False, max_out, fwd), (True, cap, inv)):
+        want = SPConvMMPlugin.prepare(kvol, inverse, rows, index, num_index)
+        assert_tables_equal(table_parts(t, kvol, rows), table_parts(want, kvol, rows), "inverse %s" % inverse)
+        assert len(table_pairs(table_parts(t, kvol, rows))) == int((index[2, :int(num_index.item())] >= 0).sum())
