@@ -17,7 +17,7 @@ D3D_MAX_DIMS = 8
 D3D_MAX_NDIM = 4
 
 D3D_FLOAT, D3D_HALF, D3D_INT8, D3D_INT32, D3D_BOOL, D3D_BF16 = 0, 1, 2, 3, 4, 7
-D3D_STATUS_HASH_FULL, D3D_STATUS_OUTPUT_OVERFLOW, D3D_STATUS_STALLED = 1, 2, 4
+D3D_STATUS_HASH_FULL, D3D_STATUS_OUTPUT_OVERFLOW = 1, 2
 
 
 class TensorDesc(ctypes.Structure):

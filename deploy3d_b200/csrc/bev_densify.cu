@@ -12,12 +12,15 @@ namespace d3d {
 namespace {
 
 __global__ void map_fill_kernel(int32_t* map, int64_t n) {
+  pdl_release();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     map[i] = -1;
 }
 
 __global__ void map_scatter_kernel(int32_t* __restrict__ map, const int32_t* __restrict__ coors,
                                    const int32_t* num_act_in, int64_t n_max, int b, int z, int y, int x) {
+  pdl_release();
+  pdl_wait();
   int n = *num_act_in;
   n = n > n_max ? (int)n_max : n;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -39,6 +42,7 @@ __global__ void densify_kernel(const int32_t* __restrict__ map, const T* __restr
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* tile = reinterpret_cast<T*>(smem_raw);  // [kStrip][c + pad]
   __shared__ int32_t vid[kStrip];
+  pdl_wait();
   const int pitch = c + (sizeof(T) == 2 ? 2 : 1);
   const int x0 = blockIdx.x * kStrip, yy = blockIdx.y, bz = blockIdx.z;
   const int b = bz / z, zz = bz % z;
@@ -69,6 +73,7 @@ densify_wide_kernel(const int32_t* __restrict__ map, const unsigned short* __res
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t* tile = reinterpret_cast<uint32_t*>(smem_raw);  // [kWideStrip][c / 2 + 1] words: odd pitch
   __shared__ int32_t vid[kWideStrip];
+  pdl_wait();
   const int pitch = c / 2 + 1;
   const int x0 = blockIdx.x * kWideStrip, yy = blockIdx.y, bz = blockIdx.z;
   const int b = bz / z, zz = bz % z;
@@ -147,23 +152,24 @@ extern "C" int d3d_bev_densify_enqueue(const d3d_bev_densify_params* p, const d3
   int32_t* map = reinterpret_cast<int32_t*>(workspace);
   map_fill_kernel<<<stream_grid(elems, 256), 256, 0, st>>>(map, elems);
   if (n_max > 0)
-    map_scatter_kernel<<<(unsigned)ceil_div(n_max, 256), 256, 0, st>>>(
-        map, reinterpret_cast<const int32_t*>(inputs[1]), reinterpret_cast<const int32_t*>(inputs[2]), n_max, b, z, y,
-        x);
+    D3D_LAUNCH(true, map_scatter_kernel, (unsigned)ceil_div(n_max, 256), 256, 0, st, map,
+               reinterpret_cast<const int32_t*>(inputs[1]), reinterpret_cast<const int32_t*>(inputs[2]), n_max, b, z, y,
+               x);
   dim3 grid((unsigned)ceil_div(x, kStrip), (unsigned)y, (unsigned)(b * z));
   if (dtype == D3D_FLOAT) {
     size_t smem = (size_t)kStrip * (c + 1) * 4;
     D3D_REQUIRE(smem <= 48 * 1024, D3D_ERR_TOO_LARGE);
-    densify_kernel<float><<<grid, 256, smem, st>>>(map, reinterpret_cast<const float*>(inputs[0]), c, z, y, x,
-                                                   reinterpret_cast<float*>(outputs[0]));
+    D3D_LAUNCH(true, densify_kernel<float>, grid, 256, smem, st, map, reinterpret_cast<const float*>(inputs[0]), c, z, y,
+               x, reinterpret_cast<float*>(outputs[0]));
   } else {
     // half and bf16 are both moved as 16-bit words
     const size_t wide_smem = (size_t)kWideStrip * (c / 2 + 1) * 4;
     if (c % 8 == 0 && x % 2 == 0 && wide_smem <= 48 * 1024 && reinterpret_cast<uintptr_t>(inputs[0]) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(outputs[0]) % 4 == 0) {
       dim3 wide((unsigned)ceil_div(x, kWideStrip), (unsigned)y, (unsigned)(b * z));
-      densify_wide_kernel<<<wide, 256, wide_smem, st>>>(map, reinterpret_cast<const unsigned short*>(inputs[0]), c, z,
-                                                        y, x, reinterpret_cast<unsigned short*>(outputs[0]));
+      D3D_LAUNCH(true, densify_wide_kernel, wide, 256, wide_smem, st, map,
+                 reinterpret_cast<const unsigned short*>(inputs[0]), c, z, y, x,
+                 reinterpret_cast<unsigned short*>(outputs[0]));
       D3D_CHECK_LAUNCH();
       return D3D_OK;
     }

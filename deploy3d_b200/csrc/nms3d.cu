@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256)
 overlap_mask_kernel(const float* __restrict__ boxes, int k, int box_dim, float thr, int nw,
                     unsigned long long* __restrict__ mask) {
   constexpr int kCols = kNmsBlock / kSplit, kPerThread = kCols / 4;  // columns of the CTA, of a thread
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_release();
   const int cb = blockIdx.x / kSplit, part = blockIdx.x % kSplit, rb = blockIdx.y, b = blockIdx.z;
   if (rb > cb) return;
   __shared__ Box cols[kCols], rows[kNmsBlock];
@@ -412,7 +412,7 @@ suppress_blocks_kernel(const unsigned long long* __restrict__ mask, const float*
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   if (tid < kSweepMaxWords) removed[tid] = 0ull;
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the mask of the preceding kernel
+  pdl_wait();  // the mask of the preceding kernel
   for (int blk = 0; blk < kRing - 1; ++blk) load(blk);
   for (int blk = 0; blk < nw; ++blk) {
     load(blk + kRing - 1);  // its slot was last read before the barrier at the end of the previous turn
@@ -513,15 +513,7 @@ static int launch_nms(const d3d_nms3d_params* p, int b, int k, int bd, int nw, c
       raised[dev].store(true, std::memory_order_release);
     }
     // started while the mask kernel drains; it waits for the mask itself
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(b), cfg.blockDim = dim3(kSweepThreads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr, cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, suppress_blocks_kernel, (const unsigned long long*)mask, scores, k, nw, out) !=
-        cudaSuccess)
-      return D3D_ERR_CUDA;
+    D3D_LAUNCH(true, suppress_blocks_kernel, (unsigned)b, kSweepThreads, smem, st, mask, scores, k, nw, out);
   } else {
     suppress_kernel<<<b, 32, 0, st>>>(mask, scores, k, nw, out);
   }

@@ -13,6 +13,7 @@ namespace d3d {
 namespace {
 
 __global__ void fill_kernel(float* out, int64_t n, float v) {
+  pdl_release();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = v;
 }
@@ -29,6 +30,7 @@ template <bool kMean, bool kVec>
 __global__ void scatter_reduce_kernel(const float* __restrict__ in_feats, const int32_t* __restrict__ scatter_to,
                                       const int32_t* __restrict__ scatter_count, int64_t n, int c, int64_t m,
                                       float* __restrict__ out) {
+  pdl_wait();
   const int groups = kVec ? c / 4 : c;
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n * groups) return;
@@ -121,11 +123,9 @@ extern "C" int d3d_scatter_to_enqueue(const d3d_scatter_to_params* p, const d3d_
     const bool vec = (c % 4 == 0) && (reinterpret_cast<uintptr_t>(feats) % 16 == 0) &&
                      (reinterpret_cast<uintptr_t>(o) % 16 == 0);
     int64_t work = n * (vec ? c / 4 : c);
-    unsigned grid = (unsigned)ceil_div(work, 256);
-    if (mean && vec) scatter_reduce_kernel<true, true><<<grid, 256, 0, st>>>(feats, idx, cnt, n, c, m, o);
-    else if (mean) scatter_reduce_kernel<true, false><<<grid, 256, 0, st>>>(feats, idx, cnt, n, c, m, o);
-    else if (vec) scatter_reduce_kernel<false, true><<<grid, 256, 0, st>>>(feats, idx, cnt, n, c, m, o);
-    else scatter_reduce_kernel<false, false><<<grid, 256, 0, st>>>(feats, idx, cnt, n, c, m, o);
+    auto kern = mean ? (vec ? scatter_reduce_kernel<true, true> : scatter_reduce_kernel<true, false>)
+                     : (vec ? scatter_reduce_kernel<false, true> : scatter_reduce_kernel<false, false>);
+    D3D_LAUNCH(true, kern, (unsigned)ceil_div(work, 256), 256, 0, st, feats, idx, cnt, n, c, m, o);
   }
   D3D_CHECK_LAUNCH();
   return D3D_OK;

@@ -643,8 +643,8 @@ __global__ void __launch_bounds__(1024) segment_scan_kernel(int32_t* __restrict_
   __shared__ int warp_sum[32];
   __shared__ int carry_s, chunk_total;
   __shared__ bool last;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_release();
+  pdl_wait();
   const int n = live_count(num_act_in, n_max);
   const int live_blk = (n + kIdxThreads - 1) / kIdxThreads;
   const int warp = threadIdx.x >> 5, lane = lane_id();
@@ -947,7 +947,6 @@ struct Plan {
   int32_t* grid;
   uint32_t* bits;
   uint8_t* list_local;
-  unsigned long long* chain;
   bool packed;         // strided rulebook kept as kPackedSlots entries per input instead of kvol
   size_t bytes;
 };
@@ -1037,7 +1036,6 @@ int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n
   plan->bits = plan->path == Plan::kBits ? w.take<uint32_t>((size_t)((vol + 31) / 32 + 63) / 64 * 64) : nullptr;
   plan->pair_out = w.take<int32_t>((size_t)g.kvol * (plan->n_max > 0 ? (size_t)plan->nblk * kIdxThreads : 1));
   plan->list_local = plan->path == Plan::kHash ? nullptr : w.take<uint8_t>((size_t)g.kvol * plan->nblk * kIdxThreads);
-  plan->chain = plan->path == Plan::kDirect ? w.take<unsigned long long>(plan->nblk) : nullptr;
   plan->block_counts = w.take<int32_t>((size_t)g.kvol * plan->nblk);
   plan->seg = w.take<int32_t>(2 * (size_t)g.kvol + 2);
   plan->slot_out = p->subm || plan->path == Plan::kDirect ? nullptr : w.take<int32_t>(plan->cap_max);
@@ -1051,23 +1049,7 @@ int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n
   return D3D_OK;
 }
 
-// Launch in `st`, optionally as a programmatic dependent of the kernel before it (every kernel of spconv_index3.cuh
-// waits for that kernel itself): the launch gap inside a chain of 3-5 us kernels goes from about 1.2 to 0.4 us.
-template <class... P, class... A>
-int launch3(bool chained, void (*kern)(P...), int64_t grid, int threads, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3(threads), cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, P(args)...) == cudaSuccess ? D3D_OK : D3D_ERR_CUDA;
-}
-#define D3D_LAUNCH3(...)                     \
-  do {                                       \
-    const int rc_ = launch3(__VA_ARGS__);    \
-    if (rc_ != D3D_OK) return rc_;           \
-  } while (0)
+#define D3D_LAUNCH3(chained, kern, grid, threads, st, ...) D3D_LAUNCH(chained, (kern), grid, threads, 0, st, __VA_ARGS__)
 
 TableTarget make_target(void* table, int kvol, int64_t m_max) {
   const TableParts t = table_parts(table, kvol, m_max);
@@ -1104,7 +1086,6 @@ ClearArgs clear_args(const Plan& plan) {
   a.direct_words = (plan.cells + 63) / 64 * 64;
   a.bit_words = ((plan.cells + 31) / 32 + 63) / 64 * 64;
   a.fan = plan.fan;
-  a.chain = plan.chain, a.chain_words = plan.chain ? plan.nblk : 0;
   a.state = plan.state;
   return a;
 }
@@ -1140,8 +1121,10 @@ int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
   D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
   const bool two = plan.two_taps;
   D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
+  D3D_LAUNCH3(chained, two ? conv_count3_kernel<2> : conv_count3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
+              num_act_in, plan.n_max, plan.g, plan.win_bits, plan.winners);
   D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
-              coors, num_act_in, plan.n_max, plan.g, max_out, plan.chain, out_coors, num_act_out, status);
+              coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, out_coors, num_act_out, status);
   const int64_t blocks = inverse.count ? std::max<int64_t>(plan.nblk, ceil_div(inverse.tiles * 128, kIdxThreads))
                                        : plan.nblk;
   D3D_LAUNCH3(chained, two ? conv_find3_kernel<2> : conv_find3_kernel<3>, blocks, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g,

@@ -20,9 +20,6 @@ namespace {
 constexpr int kTaps3 = 27;  // offsets of the enclosing 3 x 3 x 3 kernel: g = (a * 3 + b) * 3 + c
 constexpr int kBlockWarps = kIdxThreads / 32;
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // A neighbour table (SPConvMM's layout) a pass fills for tiles of the voxels it walks: slot s of the table is offset
 // g_of_slot[s] of the pass.
 struct TableTarget {
@@ -55,14 +52,11 @@ struct Lookup3 {
 };
 
 // Clears what a rulebook starts from: the lookup (live part of the hash table, all of the grid or of the bit map), the
-// words a scan is chained through, the ticket of segment_scan_kernel, and the row masks / output map of a neighbour
-// table that is filled by scattering.
+// ticket of segment_scan_kernel, and the row masks / output map of a neighbour table that is filled by scattering.
 struct ClearArgs {
   Lookup3 look;
   int64_t direct_words, bit_words;
   int fan;
-  unsigned long long* chain;
-  int chain_words;
   int32_t* state;
   uint32_t* rows;
   int64_t row_words;
@@ -87,7 +81,6 @@ __global__ void __launch_bounds__(256) clear3_kernel(const ClearArgs a, const in
     const uint32_t cap = hash_capacity((long long)live_count(num_act_in, n_max) * a.fan, a.look.cap_max);
     fill(a.look.slots, cap / 2, ones);
   }
-  for (int64_t i = tid; i < a.chain_words; i += nth) a.chain[i] = 0ull;
   if (a.rows) fill(a.rows, a.row_words / 4, zero);
   for (int64_t i = tid; i < a.perm_words; i += nth) a.perm[i] = i < a.m_max ? (int32_t)i : -1;
 }
@@ -436,63 +429,20 @@ conv_mark3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors,
   }
 }
 
-// Exclusive prefix over the blocks in front of this one, which publish their sums in `chain` (zeroed before).  The whole
-// block looks back, 256 blocks at a time: with 32 at a time the prefix travelled through the thousand blocks of a first
-// wave at 32 blocks per round trip to L2 (number kernel of 281 k inputs 28 us).  Blocks are dispatched in order, so those
-// in front are running or done; the wait is bounded all the same.  Called by all threads; `scratch` holds 2 x 8 words.
-constexpr unsigned long long kChainSum = 1ull << 62, kChainPrefix = 2ull << 62, kChainValue = (1ull << 62) - 1;
-__device__ __forceinline__ long long chained_prefix(unsigned long long* chain, int blk, long long sum, int32_t* status,
-                                                    long long* scratch) {
-  const int lane = lane_id(), warp = threadIdx.x >> 5;
-  volatile unsigned long long* word = chain;
-  if (threadIdx.x == 0) word[blk] = (blk == 0 ? kChainPrefix : kChainSum) | (unsigned long long)sum;
-  long long prefix = 0;
-  for (int base = blk - 1; base >= 0; base -= kIdxThreads) {
-    const int j = base - (int)threadIdx.x;
-    unsigned long long s = kChainPrefix;
-    if (j >= 0) s = word[j];
-    for (int spins = 0; s < kChainSum; ++spins) {
-      if (spins > (1 << 21)) {
-        report_status(status, D3D_STATUS_STALLED);
-        s = kChainPrefix;
-        break;
-      }
-      s = word[j];
-    }
-    // the nearest block that already knows its whole prefix ends the walk
-    const unsigned done = __ballot_sync(0xffffffffu, s >= kChainPrefix);
-    const int last = done ? __ffs(done) - 1 : 31;
-    long long v = lane <= last ? (long long)(s & kChainValue) : 0;
-#pragma unroll
-    for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-    if (lane == 0) scratch[warp] = v, scratch[kBlockWarps + warp] = done != 0u;
-    __syncthreads();
-    bool found = false;
-    for (int w = 0; w < kBlockWarps && !found; ++w) prefix += scratch[w], found = scratch[kBlockWarps + w] != 0;
-    __syncthreads();
-    if (found) break;
-  }
-  if (threadIdx.x == 0 && blk != 0) word[blk] = kChainPrefix | (unsigned long long)(prefix + sum);
-  return prefix;
-}
-
-// Cells after numbering: an output's id with the sign bit set (never equal to a pair id, so that blocks still comparing
-// are not misled), or kDropped beyond maxNumActOut.
+// Cells after numbering: an output's id with the sign bit set, or kDropped beyond maxNumActOut.
 constexpr int kDropped = -2;
 constexpr int kIdBit = -2147483647 - 1;
 
-// The pair whose id is left in a cell numbers that output: in pair order, i.e. by first touch (index.cu:104-121).
+// The pair whose id is left in a cell numbers that output: in pair order, i.e. by first touch (index.cu:104-121).  First
+// the winning combinations of every input and their number per block, then the numbers themselves.
 template <int kTaps>
 __global__ void __launch_bounds__(kIdxThreads)
-conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
-                    int64_t n_max, const Geometry g, int32_t max_out, unsigned long long* chain,
-                    int32_t* __restrict__ out_coors, int32_t* __restrict__ num_act_out, int32_t* status) {
-  __shared__ int scratch[40];
-  __shared__ long long chain_scratch[2 * kBlockWarps];
+conv_count3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
+                   int64_t n_max, const Geometry g, uint32_t* __restrict__ wins, int32_t* __restrict__ counts) {
+  __shared__ int sums[kBlockWarps];
   pdl_release();
   pdl_wait();
   const int n = live_count(num_act_in, n_max);
-  if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) *num_act_out = 0;
   if ((int64_t)blockIdx.x * kIdxThreads >= n) return;
   const int i = blockIdx.x * kIdxThreads + threadIdx.x;
   int4 c = make_int4(-1, 0, 0, 0);
@@ -503,24 +453,53 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
     const Combo<kTaps> r = combo(t, e);
-    left[e] = r.ok ? __ldcg(grid + cell_of(g, r, c.x)) : -1;  // cells hold ids >= 0 or, numbered already, negatives
+    left[e] = r.ok ? __ldg(grid + cell_of(g, r, c.x)) : -1;
   }
-  uint32_t wins = 0u;
+  uint32_t bits = 0u;
 #pragma unroll
   for (int e = 0; e < kCombos; ++e)
-    if (left[e] >= 0 && left[e] == i * g.kvol + offset_of(g, combo(t, e))) wins |= 1u << e;
+    if (left[e] >= 0 && left[e] == i * g.kvol + offset_of(g, combo(t, e))) bits |= 1u << e;
+  if (i < n) wins[i] = bits;
+  const int sum = __reduce_add_sync(0xffffffffu, __popc(bits));
+  if (lane_id() == 0) sums[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int w = 0; w < kBlockWarps; ++w) total += sums[w];
+    counts[blockIdx.x] = total;
+  }
+}
+
+template <int kTaps>
+__global__ void __launch_bounds__(kIdxThreads)
+conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
+                    int64_t n_max, const Geometry g, int32_t max_out, const uint32_t* __restrict__ wins,
+                    const int32_t* __restrict__ counts, int32_t* __restrict__ out_coors,
+                    int32_t* __restrict__ num_act_out, int32_t* status) {
+  __shared__ int scratch[40], sums[kBlockWarps];
+  pdl_release();
+  pdl_wait();
+  const int n = live_count(num_act_in, n_max);
+  if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) *num_act_out = 0;
+  if ((int64_t)blockIdx.x * kIdxThreads >= n) return;
+  const int i = blockIdx.x * kIdxThreads + threadIdx.x;
+  const uint32_t bits = i < n ? __ldg(wins + i) : 0u;
+  int4 c = make_int4(-1, 0, 0, 0);
+  if (bits) c = __ldg(reinterpret_cast<const int4*>(coors) + i);
+  const int base = preceding_sum<kIdxThreads>(counts, blockIdx.x, sums);
   int total;
-  int id = block_exclusive_scan(__popc(wins), scratch, &total);
-  const long long base = chained_prefix(chain, blockIdx.x, total, status, chain_scratch);
+  int id = base + block_exclusive_scan(__popc(bits), scratch, &total);
   if (threadIdx.x == 0 && ((int64_t)blockIdx.x + 1) * kIdxThreads >= n) {
-    const long long all = base + total;  // the last live block knows the number of outputs
+    const long long all = (long long)base + total;  // the last live block knows the number of outputs
     *num_act_out = (int32_t)(all < max_out ? all : max_out);
     if (all > max_out) report_status(status, D3D_STATUS_OUTPUT_OVERFLOW);
   }
-  id += (int)base;
+  if (!bits) return;
+  constexpr int kCombos = kTaps * kTaps * kTaps;
+  const Taps<kTaps> t = taps_of<kTaps>(g, c, true);
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
-    if (!((wins >> e) & 1u)) continue;
+    if (!((bits >> e) & 1u)) continue;
     const Combo<kTaps> r = combo(t, e);
     if (id < max_out) {
       grid[cell_of(g, r, c.x)] = kIdBit | id;

@@ -46,7 +46,6 @@ typedef enum {
  * (trt/include/common/hash32.h:70) and outputs beyond maxNumActOut are dropped (trt/spconv/index.cu:163-168). */
 #define D3D_STATUS_HASH_FULL 1       /* a key found no free slot: its pairs / points were dropped */
 #define D3D_STATUS_OUTPUT_OVERFLOW 2 /* more output voxels than maxNumActOut: the surplus was dropped */
-#define D3D_STATUS_STALLED 4         /* a bounded wait inside a kernel ran out: the results are not valid */
 
 /* Values follow nvinfer1::DataType so a plugin shell can pass PluginTensorDesc::type through. */
 typedef enum {
