@@ -12,7 +12,7 @@ import torch
 
 from . import synth
 from .ops import data_s_spconv_index, data_s_spconv_mm
-from .plugins import SPConvMMPlugin, SubmTables, deserialize_plugin
+from .plugins import SPConvMMPlugin, SubmTables, activation, deserialize_plugin
 
 
 class Layer:
@@ -484,12 +484,8 @@ class SparseNet:
             if self.plugin_order:
                 in_set = rb.out_set if L.kind == "inverse" else rb.in_set
                 plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], *rb.buffers(), outputs=[out_buf])
-                if L.relu and L.act_first:
-                    out_buf.relu_()
-                if res is not None:
-                    out_buf.add_(res)
-                if L.relu and not L.act_first:
-                    out_buf.relu_()
+                if L.relu or res is not None:  # the element-wise layer an engine fuses sum and activation into
+                    activation(out_buf, res, L.relu_mode)
                 x = out_buf
             else:
                 table = rb.table_inv if L.kind == "inverse" else rb.table_fwd

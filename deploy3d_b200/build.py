@@ -62,7 +62,7 @@ def build_host():
     src, out = os.path.join(CSRC, "host", "dispatch.cpp"), os.path.join(HERE, "libs", "_d3d_host.so")
     root = os.path.dirname(torch.__file__)
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wno-unused-function",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-pthread", "-Wall", "-Wno-unused-function",
            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I" + os.path.join(root, "include"),
            "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I" + sysconfig.get_paths()["include"], "-I" + cuda, src, "-o", out, "-L" + os.path.join(root, "lib"),

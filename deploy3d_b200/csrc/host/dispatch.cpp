@@ -18,8 +18,13 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <string.h>
+#include <unistd.h>
 
+#include <atomic>
+#include <condition_variable>
+#include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../../include/deploy3d_b200.h"
@@ -303,6 +308,68 @@ PyMethodDef call_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 PyTypeObject call_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
+// Compares two large buffers with three helper threads beside the caller: one core reads two 1.8 MB weight arrays in
+// 93 us (they come from its neighbours' caches), four in 30-40 us.  Helpers sleep between calls; a second caller that
+// finds them busy compares alone.  They are started at first use, and not in a forked child.
+class Comparer {
+ public:
+  static constexpr int kHelpers = 3;
+  static constexpr size_t kWorthIt = 256 << 10;
+
+  bool same(const char* a, const char* b, size_t n) {
+    if (n < kWorthIt || getpid() != pid_ || !turn_.try_lock()) return memcmp(a, b, n) == 0;
+    std::lock_guard<std::mutex> turn(turn_, std::adopt_lock);
+    if (!started_) {
+      for (int i = 0; i < kHelpers; ++i) std::thread([this, i] { help(i); }).detach();
+      started_ = true;
+    }
+    part_ = (n / (kHelpers + 1) + 63) & ~size_t(63);
+    differ_.store(false, std::memory_order_relaxed);
+    left_.store(kHelpers, std::memory_order_relaxed);
+    {
+      std::lock_guard<std::mutex> g(lock_);
+      a_ = a, b_ = b, n_ = n;
+      ++job_;
+    }
+    wake_.notify_all();
+    const bool same = memcmp(a, b, part_) == 0;
+    while (left_.load(std::memory_order_acquire) > 0) std::this_thread::yield();
+    return same && !differ_.load(std::memory_order_relaxed);
+  }
+
+ private:
+  void help(int i) {
+    unsigned long seen = 0;
+    for (;;) {
+      const char *a, *b;
+      size_t from, to;
+      {
+        std::unique_lock<std::mutex> g(lock_);
+        wake_.wait(g, [&] { return job_ != seen; });
+        seen = job_;
+        a = a_, b = b_;
+        from = part_ * (i + 1);
+        to = i + 1 == kHelpers ? n_ : from + part_;
+      }
+      if (memcmp(a + from, b + from, to - from) != 0) differ_.store(true, std::memory_order_relaxed);
+      left_.fetch_sub(1, std::memory_order_release);
+    }
+  }
+  const pid_t pid_ = getpid();
+  std::mutex turn_, lock_;
+  std::condition_variable wake_;
+  std::atomic<int> left_{0};
+  std::atomic<bool> differ_{false};
+  bool started_ = false;
+  unsigned long job_ = 0;
+  const char *a_ = nullptr, *b_ = nullptr;
+  size_t n_ = 0, part_ = 0;
+};
+Comparer* comparer() {
+  static Comparer* c = new Comparer();  // never destroyed: the helpers outlive the module's statics
+  return c;
+}
+
 // same_bytes(a, b, offset of b): whether the buffer `a` equals the bytes of `b` from `offset` on.
 PyObject* same_bytes(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Py_buffer a, b;
@@ -320,7 +387,7 @@ PyObject* same_bytes(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   bool same = off >= 0 && off <= b.len && a.len <= b.len - off;
   if (same) {
     Py_BEGIN_ALLOW_THREADS;
-    same = memcmp(a.buf, static_cast<const char*>(b.buf) + off, (size_t)a.len) == 0;
+    same = comparer()->same(static_cast<const char*>(a.buf), static_cast<const char*>(b.buf) + off, (size_t)a.len);
     Py_END_ALLOW_THREADS;
   }
   PyBuffer_Release(&a);

@@ -29,8 +29,9 @@ namespace {
 // where its row-mask bit is set.  The scatter kernel sets ids and bits; the per-tile offset masks are derived from
 // the row masks afterwards.
 __global__ void table_fill_kernel(uint32_t* row_masks, int64_t mask_words, int32_t* perm, int64_t perm_words,
-                                  int64_t m_max) {
+                                  int64_t m_max, unsigned long long* checks) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
+  if (checks && tid < 2) checks[tid] = 0ull;
   for (int64_t w = tid; w < perm_words; w += nthreads) perm[w] = w < m_max ? (int32_t)w : -1;
   for (int64_t w = tid; w < mask_words; w += nthreads) row_masks[w] = 0u;
 }
@@ -53,7 +54,9 @@ __global__ void pack_mask_kernel(const uint4* __restrict__ row_masks, int64_t ti
 // convolution kernel copies only those rows and lets the tensor core update only those accumulator lanes.
 __global__ void table_scatter_kernel(const int32_t* __restrict__ index, int64_t row_len,
                                      const int32_t* __restrict__ num_index, int inverse, int mirror, int kvol,
-                                     int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks) {
+                                     int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks,
+                                     const unsigned long long* __restrict__ unless_equal) {
+  if (unless_equal && unless_equal[0] == unless_equal[1]) return;  // done by table_scatter_mirrored_kernel
   int64_t n = *num_index;
   n = n > row_len ? row_len : n;
   // grid-stride over the live part of the rulebook only (the rows are sized for the worst case, mostly unused)
@@ -98,6 +101,89 @@ __global__ void table_scatter_kernel(const int32_t* __restrict__ index, int64_t 
                  1u << (s[u] & 31));
     }
   }
+}
+
+// The table of a rulebook that SPConvMM was told is submanifold, read as its own mirror image.
+//
+// A submanifold rulebook over an odd kernel with "same" padding holds (g, s) under offset k exactly when it holds (s, g)
+// under kvol - 1 - k.  Read that way its entries fill the table in ascending order of their segments: neighbouring lanes
+// write neighbouring ids, and the row-mask bits of a warp's lanes fall into a few words, so that one atomic per word
+// replaces one per entry (5.35 M entries at 463 k voxels: 62 -> 26 us).  Whether the rulebook has that symmetry is not
+// taken on trust: the same pass adds up a 64-bit mix of every entry and of its mirror image, which are equal sums for
+// a symmetric rulebook and otherwise differ but for a chance of about 2^-64 (checks[0] and [1]; zero before the launch).
+// table_redo_kernel and the plain scatter behind it do the work over where they differ, and return at once where not.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+  x ^= x >> 32;
+  x *= 0xd6e8feb86659fd93ull;
+  x ^= x >> 32;
+  x *= 0xd6e8feb86659fd93ull;
+  x ^= x >> 32;
+  return x;
+}
+__device__ __forceinline__ unsigned long long entry_mix(int g, int s, int k) {
+  return mix64(((unsigned long long)(unsigned)g << 32 | (unsigned)s) + (unsigned long long)(k + 1) * 0x9e3779b97f4a7c15ull);
+}
+__global__ void __launch_bounds__(256)
+table_scatter_mirrored_kernel(const int32_t* __restrict__ index, int64_t row_len, const int32_t* __restrict__ num_index,
+                              int kvol, int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks,
+                              unsigned long long* __restrict__ checks) {
+  int64_t n = *num_index;
+  n = n > row_len ? row_len : n;
+  const int64_t n_warp = (n + 31) & ~(int64_t)31, stride = (int64_t)gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  constexpr int kUnroll = 4;
+  unsigned long long sum = 0, mirrored = 0;
+  for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < n_warp; p0 += kUnroll * stride) {
+    int k[kUnroll], g[kUnroll], s[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int64_t p = p0 + u * stride;
+      const bool in = p < n;
+      k[u] = in ? __ldg(index + 2 * row_len + p) : -1;
+      g[u] = in ? __ldg(index + p) : -1;
+      s[u] = in ? __ldg(index + row_len + p) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      if (p0 + u * stride >= n_warp) break;  // warp-uniform
+      const bool live = k[u] >= 0 && k[u] < kvol;
+      if (live) {
+        (void)(D3D_BOUNDS_OK(g[u], 0, 0x7fffffffll, kSiteTableEntry) && D3D_BOUNDS_OK(s[u], 0, m_max, kSiteTableEntry));
+        sum += entry_mix(g[u], s[u], k[u]), mirrored += entry_mix(s[u], g[u], kvol - 1 - k[u]);
+      }
+      // entry (g, s, k) read as (s, g, kvol - 1 - k): row g of the table gets id s
+      const bool valid = live && s[u] >= 0 && g[u] >= 0 && g[u] < m_max;
+      const int64_t blk = valid ? (int64_t)(g[u] >> 7) * kvol + (kvol - 1 - k[u]) : -1;
+      if (valid) table[blk * 128 + (g[u] & 127)] = s[u];
+      // bits of the lanes that share a row-mask word: runs of equal words, OR-ed into the run's first lane
+      const long long word = valid ? blk * 4 + ((g[u] & 127) >> 5) : -1;
+      unsigned bits = valid ? 1u << (g[u] & 31) : 0u;
+      const long long prev = __shfl_up_sync(0xffffffffu, word, 1);
+      const bool head = lane == 0 || prev != word;
+      const unsigned heads = __ballot_sync(0xffffffffu, head);
+      const unsigned above = lane == 31 ? 0u : heads >> (lane + 1);
+      const int run = above ? __ffs(above) : 32 - lane;  // lanes from this one to the end of its run
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned t = __shfl_down_sync(0xffffffffu, bits, d);
+        if (d < run) bits |= t;
+      }
+      if (head && word >= 0) atomicOr(row_masks + word, bits);
+    }
+  }
+#pragma unroll
+  for (int d = 16; d; d >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    mirrored += __shfl_xor_sync(0xffffffffu, mirrored, d);
+  }
+  if (lane == 0 && (sum | mirrored)) atomicAdd(checks, sum), atomicAdd(checks + 1, mirrored);
+}
+// The rulebook was not symmetric after all: the row masks start over.
+__global__ void table_redo_kernel(const unsigned long long* __restrict__ checks, uint32_t* __restrict__ row_masks,
+                                  int64_t mask_words) {
+  if (checks[0] == checks[1]) return;
+  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < mask_words; w += (int64_t)gridDim.x * blockDim.x)
+    row_masks[w] = 0u;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -180,7 +266,16 @@ RegroupScratch regroup_scratch(void* scratch, int kernel_vol, int64_t m_max) {
 
 // ---------------------------------------------------------------------------------------------
 // SIMT kernel: tile of 32 outputs per CTA, 256 threads, thread = (row, 8-strided column group).
+//
+// A tile is worked off offset by offset -- features and weights through shared memory, two barriers and a round trip to L2
+// for every offset that any of its rows has -- or, in layers of at most 32 output channels, row by row: a group of lanes
+// per row, a lane per channel, that only walks the row's own inputs.  A fine voxel grid gives a row one to three inputs,
+// and its tiles nearly as many offsets as a dense one's (20 k voxels, 16 -> 16, 1.3 inputs per row: 36 us by offsets).
+// Each tile chooses for itself; the row walk costs as much as the offsets at 10 to 15 inputs per row and 27 offsets
+// (measured at 16 and 32 channels: 6 inputs 62 against 131 us, 19 inputs 475 against 310), hence kWalkRows.  Either way a
+// sum runs over offsets and channels in the same ascending order.
 // ---------------------------------------------------------------------------------------------
+constexpr int kWalkRows = 12;  // row by row when the tile has fewer than this many inputs per offset it takes part in
 constexpr int kTileM = 32;
 constexpr int kChunkK = 32;
 constexpr int kSimtThreads = 256;
@@ -195,7 +290,7 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
 template <class T, int CPT>
-__global__ void __launch_bounds__(kSimtThreads)
+__global__ void __launch_bounds__(kSimtThreads, CPT <= 4 ? 8 : 1)
 spconv_mm_simt_kernel(const T* __restrict__ in_feats, int64_t n_in_max, const T* __restrict__ weight,
                       const float* __restrict__ bias, const int32_t* __restrict__ table,
                       const uint32_t* __restrict__ row_masks, const int32_t* __restrict__ perm, int64_t m_max,
@@ -213,6 +308,11 @@ spconv_mm_simt_kernel(const T* __restrict__ in_feats, int64_t n_in_max, const T*
   const int64_t blk0 = (tile0 >> 7) * kvol;
   const int quarter = (int)((tile0 & 127) >> 5);
 
+  constexpr int kLanes = CPT == 2 ? 16 : CPT == 4 ? 32 : 0;  // lanes of a row walk, 0: none
+  __shared__ int pairs_s, offsets_s;
+  if (tid == 0) pairs_s = 0, offsets_s = 0;
+  __syncthreads();
+  int pairs = 0, offsets = 0;
   for (int k = warp; k < kvol; k += kSimtThreads / 32) {
     const unsigned rows = __ldg(row_masks + (blk0 + k) * 4 + quarter);
     int v = ((rows >> lane) & 1u) ? __ldg(table + (blk0 + k) * 128 + quarter * 32 + lane) : -1;
@@ -220,8 +320,68 @@ spconv_mm_simt_kernel(const T* __restrict__ in_feats, int64_t n_in_max, const T*
     idx_s[k * kTileM + lane] = v;
     unsigned any = __ballot_sync(0xffffffffu, v >= 0);
     if (lane == 0) kvalid_s[k] = any != 0;
+    pairs += __popc(any), offsets += any != 0;
   }
+  if (kLanes && lane == 0) atomicAdd(&pairs_s, pairs), atomicAdd(&offsets_s, offsets);
   __syncthreads();
+
+  if (kLanes && kvol <= 32 && pairs_s < kWalkRows * offsets_s) {
+    constexpr int kSpan = kLanes ? kLanes : 32;  // (a valid width where this branch is compiled out)
+    constexpr int kHalves = 32 / kSpan, kRowsPerGroup = kTileM * kSpan / kSimtThreads;
+    constexpr unsigned kLaneBits = kSpan == 32 ? 0xffffffffu : 0xffffu;
+    const int c = tid % kSpan, base_lane = lane / kSpan * kSpan;
+    const unsigned group = kLaneBits << base_lane;
+    for (int q = 0; q < kRowsPerGroup; ++q) {
+      const int row = tid / kSpan + q * (kSimtThreads / kSpan);
+      int id[kHalves];
+      unsigned have = 0u;  // bit k: offset k has an input
+#pragma unroll
+      for (int h = 0; h < kHalves; ++h) {
+        const int k = h * kSpan + c;
+        id[h] = k < kvol ? idx_s[k * kTileM + row] : -1;
+        have |= ((__ballot_sync(group, id[h] >= 0) >> base_lane) & kLaneBits) << (h * kSpan);
+      }
+      float sum = 0.f;
+      while (have) {
+        const int k = __ffs(have) - 1;
+        have &= have - 1u;
+        int src_row = __shfl_sync(group, id[0], base_lane + (k & (kSpan - 1)));
+        if (kHalves == 2) {
+          const int upper = __shfl_sync(group, id[kHalves - 1], base_lane + (k & (kSpan - 1)));
+          if (k >= kSpan) src_row = upper;
+        }
+        const T* src = in_feats + (int64_t)src_row * cin;
+        const T* w = weight + (int64_t)k * cin * cout + c;
+        for (int c0 = 0; c0 < cin; c0 += kSpan) {
+          const int n = cin - c0 < kSpan ? cin - c0 : kSpan;
+          const float x = c < n ? to_f32(src[c0 + c]) : 0.f;
+          if (n == kSpan) {
+            constexpr int kBatch = 8;  // weights in flight per lane (more cost registers, and with them CTAs per SM)
+#pragma unroll
+            for (int e0 = 0; e0 < kSpan; e0 += kBatch) {
+              float wv[kBatch];
+#pragma unroll
+              for (int e = 0; e < kBatch; ++e) wv[e] = c < cout ? to_f32(w[(c0 + e0 + e) * cout]) : 0.f;
+#pragma unroll
+              for (int e = 0; e < kBatch; ++e) sum = fmaf(__shfl_sync(group, x, base_lane + e0 + e), wv[e], sum);
+            }
+          } else {
+            for (int e = 0; e < n; ++e)
+              sum = fmaf(__shfl_sync(group, x, base_lane + e), c < cout ? to_f32(w[(c0 + e) * cout]) : 0.f, sum);
+          }
+        }
+      }
+      const int64_t o = __ldg(perm + tile0 + row);
+      if (o >= 0 && o < m_max && c < cout) {
+        float v = sum + bias[c];
+        if (relu == 2) v = fmaxf(v, 0.f);
+        if (residual) v += to_f32(residual[o * cout + c]);
+        if (relu == 1) v = fmaxf(v, 0.f);
+        out_feats[o * cout + c] = from_f32<T>(v);
+      }
+    }
+    return;
+  }
 
   float acc[CPT];
 #pragma unroll
@@ -493,11 +653,39 @@ extern "C" size_t d3d_spconv_mm_table_bytes(int kernel_vol, int64_t max_num_act_
          table_rows_bytes(kernel_vol, max_num_act_out) + table_perm_bytes(max_num_act_out);
 }
 
+// The table and, behind it, the two check words of a mirrored build.
+static size_t enqueue_workspace(const d3d_spconv_mm_s* h) {
+  return align_up(d3d_spconv_mm_table_bytes(h->p.kernel_vol, h->p.max_num_act_out), 256) + 256;
+}
+
 extern "C" int d3d_spconv_mm_workspace(d3d_spconv_mm_t h, const d3d_tensor_desc* in, int n_in, size_t* bytes) {
   D3D_REQUIRE(h && bytes, D3D_ERR_INVALID_ARGUMENT);
   (void)in, (void)n_in;
-  *bytes = d3d_spconv_mm_table_bytes(h->p.kernel_vol, h->p.max_num_act_out);
+  *bytes = enqueue_workspace(h);
   return D3D_OK;
+}
+
+// Builds a neighbour table.  `checks` (two 64-bit words, for rulebooks the caller calls submanifold): read the rulebook
+// as its mirror image if that is what it is, see table_scatter_mirrored_kernel.
+static int build_table(int kernel_vol, int inverse, int mirror, int64_t max_num_act_out, const int32_t* index,
+                       int64_t index_row_len, const int32_t* num_index, void* table, unsigned long long* checks,
+                       cudaStream_t st) {
+  const int64_t pitch = (max_num_act_out + 127) / 128 * 128;
+  const TableParts t = table_parts(table, kernel_vol, max_num_act_out);
+  const int64_t mask_words = t.tiles * kernel_vol * 4;
+  table_fill_kernel<<<stream_grid(mask_words, 256), 256, 0, st>>>(t.row_masks, mask_words, t.perm, t.tiles * 128,
+                                                                 max_num_act_out, checks);
+  if (index_row_len > 0) {
+    const int grid = stream_grid(index_row_len, 256);
+    if (checks) {
+      table_scatter_mirrored_kernel<<<grid, 256, 0, st>>>(index, index_row_len, num_index, kernel_vol, pitch, t.ids,
+                                                          t.row_masks, checks);
+      table_redo_kernel<<<stream_grid(mask_words, 256, 2), 256, 0, st>>>(checks, t.row_masks, mask_words);
+    }
+    table_scatter_kernel<<<grid, 256, 0, st>>>(index, index_row_len, num_index, inverse, mirror, kernel_vol, pitch,
+                                               t.ids, t.row_masks, checks);
+  }
+  return pack_table_masks(t, kernel_vol, st);
 }
 
 extern "C" int d3d_spconv_mm_prepare(int kernel_vol, int mode, int64_t max_num_act_out, const int32_t* index,
@@ -509,18 +697,8 @@ extern "C" int d3d_spconv_mm_prepare(int kernel_vol, int mode, int64_t max_num_a
   D3D_REQUIRE(index && num_index && table, D3D_ERR_INVALID_ARGUMENT);
   const int inverse = mode & 1;
   const int mirror = (mode & 2) && !inverse;  // a symmetric rulebook is its own inverse
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int64_t pitch = (max_num_act_out + 127) / 128 * 128;
-  const TableParts t = table_parts(table, kernel_vol, max_num_act_out);
-  table_fill_kernel<<<stream_grid(t.tiles * kernel_vol * 4, 256), 256, 0, st>>>(t.row_masks, t.tiles * kernel_vol * 4,
-                                                                               t.perm, t.tiles * 128, max_num_act_out);
-  if (index_row_len > 0)
-    table_scatter_kernel<<<stream_grid(index_row_len, 256), 256, 0, st>>>(
-        index, index_row_len, num_index, inverse, mirror, kernel_vol, pitch, t.ids, t.row_masks);
-  pack_mask_kernel<<<(unsigned)ceil_div(t.tiles * 32, 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(t.row_masks),
-                                                                          t.tiles, kernel_vol, t.tile_mask);
-  D3D_CHECK_LAUNCH();
-  return D3D_OK;
+  return build_table(kernel_vol, inverse, mirror, max_num_act_out, index, index_row_len, num_index, table, nullptr,
+                     reinterpret_cast<cudaStream_t>(stream));
 }
 
 // No plugin counterpart: see the header.
@@ -550,6 +728,61 @@ extern "C" int d3d_spconv_mm_regroup(int kernel_vol, int64_t max_num_act_out, co
   regroup_gather_kernel<<<(unsigned)out.tiles, 128, 0, st>>>(in.ids, r.keys_sorted, r.vals_sorted, kernel_vol,
                                                               max_num_act_out, out.ids, out.row_masks, out.tile_mask,
                                                               out.perm);
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
+// The element-wise layer that follows an SPConvMM node in a graph (residual sum and ReLU, in that order or the other):
+// one pass over the tensor where a sum and an activation layer are two.  The sum is rounded once: ReLU commutes with
+// rounding, so the bytes are those of the two layers.
+namespace d3d {
+namespace {
+template <class T>
+__global__ void __launch_bounds__(256) activation_kernel(T* __restrict__ x, const T* __restrict__ residual, int64_t n, int relu) {
+  constexpr int kVec = 16 / sizeof(T);
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
+  auto one = [&](T v, T r) -> T {
+    float f = to_f32(v);
+    if (relu == 2) f = f < 0.f ? 0.f : f;  // NaN stays NaN, as in an activation layer
+    if (residual) f += to_f32(r);
+    if (relu == 1) f = f < 0.f ? 0.f : f;
+    return from_f32<T>(f);
+  };
+  const int64_t nv = n / kVec;
+  for (int64_t i = tid; i < nv; i += nth) {
+    uint4 a = reinterpret_cast<uint4*>(x)[i], b = make_uint4(0u, 0u, 0u, 0u);
+    if (residual) b = __ldg(reinterpret_cast<const uint4*>(residual) + i);
+    T* pa = reinterpret_cast<T*>(&a);
+    const T* pb = reinterpret_cast<const T*>(&b);
+#pragma unroll
+    for (int e = 0; e < kVec; ++e) pa[e] = one(pa[e], pb[e]);
+    reinterpret_cast<uint4*>(x)[i] = a;
+  }
+  for (int64_t i = nv * kVec + tid; i < n; i += nth) x[i] = one(x[i], residual ? residual[i] : x[i]);
+}
+}  // namespace
+}  // namespace d3d
+
+extern "C" int d3d_activation(int dtype, void* x, const void* residual, int64_t elements, int relu, void* stream) {
+  D3D_NVTX_RANGE("d3d_activation");
+  D3D_REQUIRE(elements >= 0 && relu >= 0 && relu <= 2, D3D_ERR_INVALID_ARGUMENT);
+  if (elements == 0 || (relu == 0 && !residual)) return D3D_OK;
+  D3D_REQUIRE(x && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(residual) % 16 == 0,
+              D3D_ERR_INVALID_ARGUMENT);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int grid = stream_grid(elements * (int64_t)dtype_size(dtype) / 16, 256);
+  switch (dtype) {
+    case D3D_FLOAT:
+      activation_kernel<float><<<grid, 256, 0, st>>>((float*)x, (const float*)residual, elements, relu);
+      break;
+    case D3D_HALF:
+      activation_kernel<__half><<<grid, 256, 0, st>>>((__half*)x, (const __half*)residual, elements, relu);
+      break;
+    case D3D_BF16:
+      activation_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((__nv_bfloat16*)x, (const __nv_bfloat16*)residual, elements, relu);
+      break;
+    default: return D3D_ERR_UNSUPPORTED_DTYPE;
+  }
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }
@@ -591,16 +824,28 @@ extern "C" int d3d_spconv_mm_enqueue(d3d_spconv_mm_t h, const d3d_tensor_desc* i
   D3D_REQUIRE(in[3].nb_dims == 2 && in[3].dims[0] == 3, D3D_ERR_INVALID_ARGUMENT);
   D3D_REQUIRE(out[0].nb_dims == 2 && out[0].dims[0] == h->p.max_num_act_out && out[0].dims[1] == h->p.out_channels,
               D3D_ERR_INVALID_ARGUMENT);
-  size_t need = d3d_spconv_mm_table_bytes(h->p.kernel_vol, h->p.max_num_act_out);
+  const size_t need = enqueue_workspace(h);
   D3D_REQUIRE(h->p.max_num_act_out == 0 || (workspace && workspace_bytes >= need), D3D_ERR_WORKSPACE_TOO_SMALL);
   // configurePlugin (d3d_spconv_mm_configure) uploads the weights; enqueue itself allocates nothing and copies
   // nothing from the host (the reference uploads in configurePlugin too, trt/spconv/mm_trt.cu:127-142)
   int dev = -1;
   D3D_REQUIRE(cudaGetDevice(&dev) == cudaSuccess, D3D_ERR_CUDA);
   D3D_REQUIRE(h->dtype == dtype && h->device == dev, D3D_ERR_INVALID_ARGUMENT);
-  int rc = d3d_spconv_mm_prepare(h->p.kernel_vol, h->p.inverse, h->p.max_num_act_out,
-                             reinterpret_cast<const int32_t*>(inputs[3]), in[3].dims[1],
-                             reinterpret_cast<const int32_t*>(inputs[4]), workspace, stream);
+  int rc = D3D_OK;
+  if (h->p.max_num_act_out > 0) {
+    const int64_t row_len = in[3].dims[1];
+    D3D_REQUIRE(row_len >= 0 && inputs[3] && inputs[4], D3D_ERR_INVALID_ARGUMENT);
+    // worth a look where the rulebook may be symmetric and is large enough for the two extra launches (150 k voxels of a
+    // 3x3x3 kernel: at 66 k the plain scatter takes 11 us)
+    const bool may_mirror = h->p.subm && !h->p.inverse && h->p.kernel_vol % 2 == 1 && h->p.kernel_vol > 1 &&
+                            row_len >= (1 << 22);
+    unsigned long long* checks = may_mirror ? reinterpret_cast<unsigned long long*>(
+                                                  static_cast<unsigned char*>(workspace) + need - 256)
+                                            : nullptr;
+    rc = build_table(h->p.kernel_vol, h->p.inverse, 0, h->p.max_num_act_out,
+                     reinterpret_cast<const int32_t*>(inputs[3]), row_len, reinterpret_cast<const int32_t*>(inputs[4]),
+                     workspace, checks, reinterpret_cast<cudaStream_t>(stream));
+  }
   if (rc != D3D_OK) return rc;
   return d3d_spconv_mm_run(h, dtype, inputs[0], in[0].dims[0], reinterpret_cast<const int32_t*>(inputs[2]),
                            workspace, outputs[0], nullptr, stream);

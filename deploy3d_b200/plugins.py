@@ -160,6 +160,15 @@ class SPConvIdxPlugin(_Plugin):
                 _stream_ptr(stream), status.data_ptr() if status is not None else None))
 
 
+def activation(x, residual=None, relu=1, stream=None):
+    """x (+= residual), ReLU after (relu=1) or before (2) the sum, in place and in one pass (d3d_activation)."""
+    with torch.cuda.device(x.device):
+        check("d3d_activation", lib().d3d_activation(_TORCH2D3D[x.dtype], x.data_ptr(),
+                                                     residual.data_ptr() if residual is not None else None, x.numel(),
+                                                     int(relu), _stream_ptr(stream)))
+    return x
+
+
 class SubmTables:
     """Neighbour tables of up to eight submanifold kernels (extents 1 or 3, dilation 1, 'same' padding) over one voxel
     set, built in one pass over its voxels and without their rulebooks (d3d_spconv_subm_tables)."""

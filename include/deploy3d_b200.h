@@ -215,6 +215,11 @@ typedef struct {
   int32_t regrouped;
 } d3d_spconv_mm_epilogue;
 
+/* The element-wise layer behind an SPConvMM node, in place and in one pass: x += residual (when non-null) and ReLU after
+ * (relu = 1) or before (2) the sum; 0 = none.  Stand-in for the element-wise layers an engine runs between plugins;
+ * x and residual start on 16 bytes. */
+int d3d_activation(int dtype, void* x, const void* residual, int64_t elements, int relu, void* stream);
+
 int d3d_spconv_mm_create(const void* data_s, size_t len, d3d_spconv_mm_t* handle);
 int d3d_spconv_mm_get_params(d3d_spconv_mm_t handle, d3d_spconv_mm_params* p);
 /* serialize (mm_trt.cu:71-74): writes the blob back; *len receives the size (buffer may be NULL). */
