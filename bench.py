@@ -701,26 +701,35 @@ def aggregate_frames_per_second(world, steps, frames_per_step, elapsed_max):
 
 def count_launches(pipe, kind="detection"):
     """Kernels of this library launched per frame, counted from the pipeline's plan (every enqueue is a fixed launch
-    list: 105 launches per config-4 frame, as a profiler's launch list of this script shows)."""
+    list)."""
     net = pipe.net
     n = 0
+    groups = set()
     for rb in net.rulebooks.values():
-        # SubM: reset, insert, probe, segment scan, compact, padding fill; strided: reset, insert, count winners,
-        # scan, assign, translate, segment scan, compact, padding fill
-        n += 6 if rb.kind == "subm" else 9
-        if not getattr(rb, "fused_table", False):
-            n += 3  # neighbour table: fill, scatter, offset masks
-        if getattr(rb, "table_inv", None) is not None:
-            n += 3  # the inverse layers' table of the same rulebook
+        if rb.group is not None:
+            if id(rb.group) not in groups:
+                groups.add(id(rb.group))
+                n += 3  # the tables of a voxel set's submanifold kernels: clear, mark, find
+        elif rb.direct:
+            n += 6  # strided tables, forward and inverse: clear, mark, count, number, find, offset masks
+        else:
+            # SubM: reset, insert, probe, segment scan, compact, padding fill; strided: reset, insert, count winners,
+            # scan, assign, translate, segment scan, compact, padding fill
+            n += 6 if rb.kind == "subm" else 9
+            if not rb.fused_table:
+                n += 3  # neighbour table: fill, scatter, offset masks
+            if rb.table_inv is not None:
+                n += 3  # the inverse layers' table of the same rulebook
     n += sum(1 for L in net.layers if L.kind != "ew")  # SPConvMM
     if kind == "detection":
-        n += 7  # SimpleMeanEncoder: reset, voxelize, owners, scan, number, accumulate, divide
+        n += 6  # SimpleMeanEncoder: clear, voxelize, owners, number, accumulate, divide
         n += 3  # BEVDensify: map fill, map scatter, densify
         n += 2  # NMS3d: overlap mask, suppression
     else:
-        n += 6  # CylinderEncoder: reset, cylinderize, owners, scan, number, scatter ids
+        n += 5  # CylinderEncoder: clear, cylinderize, owners, number, scatter ids
         n += 2  # ScatterTo: fill, scatter-reduce
-        n += 1  # GatherBack
+        n += 1  # ReconBlock and concatenation
+        n += 1  # gather back and labels
     return n
 
 

@@ -132,6 +132,10 @@ SIGNATURES = {
                                               _vp, _vp]),
     "d3d_spconv_mm_run": (ctypes.c_int, [_vp, ctypes.c_int, _vp, ctypes.c_int64, _vp, _vp, _vp,
                                           ctypes.POINTER(SpconvMMEpilogue), _vp]),
+    "d3d_recon": (ctypes.c_int, [ctypes.c_int, _vp, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int, _vp, ctypes.c_int64,
+                                 ctypes.c_int, _vp]),
+    "d3d_gather_labels": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_int64, ctypes.c_int, ctypes.c_int64, _vp,
+                                         ctypes.c_int64, ctypes.c_float, _vp, _vp, _vp]),
     "d3d_activation": (ctypes.c_int, [ctypes.c_int, _vp, _vp, ctypes.c_int64, ctypes.c_int, _vp]),
     "d3d_spconv_mm_set_kernel": (ctypes.c_int, [_vp, ctypes.c_int]),
     "d3d_spconv_mm_set_dependent_launch": (ctypes.c_int, [_vp, ctypes.c_int]),

@@ -12,7 +12,7 @@ import torch
 
 from . import synth
 from .ops import data_s_spconv_index, data_s_spconv_mm
-from .plugins import SPConvMMPlugin, SubmTables, activation, deserialize_plugin
+from .plugins import SPConvMMPlugin, SubmTables, activation, deserialize_plugin, recon
 
 
 class Layer:
@@ -267,6 +267,7 @@ class SparseNet:
         weights = make_weights(layers, seed)
         self.rulebooks = {}
         self.groups = {}  # voxel set -> _SubmGroup
+        self._concatenated = None  # the concatenation layer whose result is in place already
         self.mm = []
         self.sets = {"in": dict(cap=int(caps["in"]), shape=[int(v) for v in spatial], coors=None, num=None)}
         cur = "in"
@@ -427,6 +428,24 @@ class SparseNet:
             if plain_inv is not None:
                 SPConvMMPlugin.regroup(rb.kvol, src["cap"], plain_inv, rb.table_inv, rb.scratch_inv)
 
+    def _elementwise(self, li, L, out_buf, xs):
+        """One element-wise graph op, in fp32, rounded to the net's type.  A ReconBlock is one pass, and the concatenation
+        of its result with its input right behind it is part of that pass."""
+        if L.ew[0] == "recon" and L.cout * out_buf.element_size() % 16 == 0:
+            nxt = self.layers[li + 1] if li + 1 < len(self.layers) else None
+            users = [U for U in self.layers if L.save is not None and
+                     (L.save in (U.source, U.residual) or (U.kind == "ew" and L.save in U.ew[1]))]
+            if users == [nxt] and nxt.kind == "ew" and nxt.ew == ("concat", [L.save, L.ew[1][3]]):
+                self._concatenated = li + 1
+                wide = self.mm[li + 1][1]
+                return recon(*xs, out=wide[:, :L.cout], copy_x=True)
+            return recon(*xs, out=out_buf)
+        if L.ew[0] == "concat" and self._concatenated == li:
+            self._concatenated = None
+            return out_buf
+        out_buf.copy_(ew_apply(L.ew[0], [x.float() for x in xs], torch))
+        return out_buf
+
     def forward(self, feats):
         """feats [cap_in, Cin] in the net dtype; coordinates / count as given to set_input.  Returns
         (out_feats, out_coors, num_act_out); every tensor is a static buffer of the net.
@@ -461,11 +480,9 @@ class SparseNet:
         built = set()
         saved = {"input": feats}
         x = feats
-        for L, (plug, out_buf, out_set) in zip(self.layers, self.mm):
+        for li, (L, (plug, out_buf, out_set)) in enumerate(zip(self.layers, self.mm)):
             if L.kind == "ew":  # element-wise graph op between plugins, in fp32 like the CPU restatement
-                y = ew_apply(L.ew[0], [saved[t].float() for t in L.ew[1]], torch)
-                out_buf.copy_(y)
-                x = out_buf
+                x = self._elementwise(li, L, out_buf, [saved[t] for t in L.ew[1]])
                 if L.save:
                     saved[L.save] = x
                 continue

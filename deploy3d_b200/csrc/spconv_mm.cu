@@ -280,14 +280,6 @@ constexpr int kTileM = 32;
 constexpr int kChunkK = 32;
 constexpr int kSimtThreads = 256;
 
-template <class T> __device__ __forceinline__ float to_f32(T v);
-template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <class T> __device__ __forceinline__ T from_f32(float v);
-template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
 template <class T, int CPT>
 __global__ void __launch_bounds__(kSimtThreads, CPT <= 4 ? 8 : 1)
@@ -728,61 +720,6 @@ extern "C" int d3d_spconv_mm_regroup(int kernel_vol, int64_t max_num_act_out, co
   regroup_gather_kernel<<<(unsigned)out.tiles, 128, 0, st>>>(in.ids, r.keys_sorted, r.vals_sorted, kernel_vol,
                                                               max_num_act_out, out.ids, out.row_masks, out.tile_mask,
                                                               out.perm);
-  D3D_CHECK_LAUNCH();
-  return D3D_OK;
-}
-
-// The element-wise layer that follows an SPConvMM node in a graph (residual sum and ReLU, in that order or the other):
-// one pass over the tensor where a sum and an activation layer are two.  The sum is rounded once: ReLU commutes with
-// rounding, so the bytes are those of the two layers.
-namespace d3d {
-namespace {
-template <class T>
-__global__ void __launch_bounds__(256) activation_kernel(T* __restrict__ x, const T* __restrict__ residual, int64_t n, int relu) {
-  constexpr int kVec = 16 / sizeof(T);
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
-  auto one = [&](T v, T r) -> T {
-    float f = to_f32(v);
-    if (relu == 2) f = f < 0.f ? 0.f : f;  // NaN stays NaN, as in an activation layer
-    if (residual) f += to_f32(r);
-    if (relu == 1) f = f < 0.f ? 0.f : f;
-    return from_f32<T>(f);
-  };
-  const int64_t nv = n / kVec;
-  for (int64_t i = tid; i < nv; i += nth) {
-    uint4 a = reinterpret_cast<uint4*>(x)[i], b = make_uint4(0u, 0u, 0u, 0u);
-    if (residual) b = __ldg(reinterpret_cast<const uint4*>(residual) + i);
-    T* pa = reinterpret_cast<T*>(&a);
-    const T* pb = reinterpret_cast<const T*>(&b);
-#pragma unroll
-    for (int e = 0; e < kVec; ++e) pa[e] = one(pa[e], pb[e]);
-    reinterpret_cast<uint4*>(x)[i] = a;
-  }
-  for (int64_t i = nv * kVec + tid; i < n; i += nth) x[i] = one(x[i], residual ? residual[i] : x[i]);
-}
-}  // namespace
-}  // namespace d3d
-
-extern "C" int d3d_activation(int dtype, void* x, const void* residual, int64_t elements, int relu, void* stream) {
-  D3D_NVTX_RANGE("d3d_activation");
-  D3D_REQUIRE(elements >= 0 && relu >= 0 && relu <= 2, D3D_ERR_INVALID_ARGUMENT);
-  if (elements == 0 || (relu == 0 && !residual)) return D3D_OK;
-  D3D_REQUIRE(x && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(residual) % 16 == 0,
-              D3D_ERR_INVALID_ARGUMENT);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = stream_grid(elements * (int64_t)dtype_size(dtype) / 16, 256);
-  switch (dtype) {
-    case D3D_FLOAT:
-      activation_kernel<float><<<grid, 256, 0, st>>>((float*)x, (const float*)residual, elements, relu);
-      break;
-    case D3D_HALF:
-      activation_kernel<__half><<<grid, 256, 0, st>>>((__half*)x, (const __half*)residual, elements, relu);
-      break;
-    case D3D_BF16:
-      activation_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((__nv_bfloat16*)x, (const __nv_bfloat16*)residual, elements, relu);
-      break;
-    default: return D3D_ERR_UNSUPPORTED_DTYPE;
-  }
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }

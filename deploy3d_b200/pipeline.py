@@ -9,7 +9,7 @@ import torch
 
 from . import backbone, synth
 from .ops import data_s_bev_densify, data_s_voxel_encoder
-from .plugins import deserialize_plugin
+from .plugins import MAX_LABEL_CLASSES, deserialize_plugin, gather_labels
 
 
 def _roundup(v, m):
@@ -217,7 +217,7 @@ class SegmentationPipeline:
             self.vox_feats_lp = torch.zeros((cap, self.net.in_channels), dtype=dtype, device=dev)
             self.net.set_input(self.vox_coors, self.vox_num)
             self.gather = deserialize_plugin("GatherBack", data_s_gather_back(0.0))
-            # GatherBack reads the half-precision network output and writes float logits
+            # the gather back reads the half-precision network output and writes float logits
             self.logits = torch.zeros((self.n_pts, n_class), dtype=torch.float32, device=dev)
             self.labels = torch.zeros(self.n_pts, dtype=torch.int32, device=dev)
         self.graph = None
@@ -250,8 +250,12 @@ class SegmentationPipeline:
         self.scatter.enqueue(self.pts_feats, self.scatter_index, self.scatter_count, outputs=[self.vox_feats])
         self.vox_feats_lp[:, :self.c_pts + 5].copy_(self.vox_feats)
         feats, _, _ = self.net.forward(self.vox_feats_lp)
-        self.gather.enqueue(feats, self.scatter_index, outputs=[self.logits])
-        self.labels.copy_(torch.argmax(self.logits, dim=1))  # the label pass of the reference (test_cylinder3d.py:322)
+        # GatherBack and the label pass of the reference (test_cylinder3d.py:322) in one
+        if feats.shape[1] <= MAX_LABEL_CLASSES:
+            gather_labels(feats, self.scatter_index, 0.0, self.logits, self.labels)
+        else:
+            self.gather.enqueue(feats, self.scatter_index, outputs=[self.logits])
+            self.labels.copy_(torch.argmax(self.logits, dim=1))
         return self.logits
 
     def capture(self):

@@ -169,6 +169,30 @@ def activation(x, residual=None, relu=1, stream=None):
     return x
 
 
+def recon(a, b, c, x, out, copy_x=False, stream=None):
+    """out[:, :C] = (sigmoid(a) + sigmoid(b) + sigmoid(c)) * x and, with copy_x, out[:, C:2C] = x (d3d_recon).  a, b, c, x
+    contiguous [M, C]; `out` may be columns of a wider tensor."""
+    assert out.stride(1) == 1 and all(t.is_contiguous() and t.shape == x.shape for t in (a, b, c, x))
+    with torch.cuda.device(x.device):
+        check("d3d_recon", lib().d3d_recon(_TORCH2D3D[x.dtype], a.data_ptr(), b.data_ptr(), c.data_ptr(), x.data_ptr(),
+                                           x.shape[0], x.shape[1], out.data_ptr(), out.stride(0), int(copy_x),
+                                           _stream_ptr(stream)))
+    return out
+
+
+MAX_LABEL_CLASSES = 128  # d3d_gather_labels keeps the rows of 64 points in shared memory
+
+
+def gather_labels(feats, ids, fill, logits, labels, stream=None):
+    """logits = feats[ids] in float, labels = their arg-max (d3d_gather_labels); feats [M, classes], maybe the first columns
+    of wider rows."""
+    with torch.cuda.device(feats.device):
+        check("d3d_gather_labels", lib().d3d_gather_labels(
+            _TORCH2D3D[feats.dtype], feats.data_ptr(), feats.stride(0), feats.shape[1], feats.shape[0], ids.data_ptr(),
+            ids.shape[0], float(fill), logits.data_ptr(), labels.data_ptr(), _stream_ptr(stream)))
+    return logits, labels
+
+
 class SubmTables:
     """Neighbour tables of up to eight submanifold kernels (extents 1 or 3, dilation 1, 'same' padding) over one voxel
     set, built in one pass over its voxels and without their rulebooks (d3d_spconv_subm_tables)."""

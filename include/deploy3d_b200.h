@@ -220,6 +220,15 @@ typedef struct {
  * x and residual start on 16 bytes. */
 int d3d_activation(int dtype, void* x, const void* residual, int64_t elements, int relu, void* stream);
 
+/* ReconBlock: out = (sigmoid(a) + sigmoid(b) + sigmoid(c)) * x over rows x channels, in fp32, rounded once; out rows are
+ * out_ld elements apart and with copy_x the row of x follows the result (channel concatenation).  Rows of 16-byte multiples. */
+int d3d_recon(int dtype, const void* a, const void* b, const void* c, const void* x, int64_t rows, int channels, void* out,
+              int64_t out_ld, int copy_x, void* stream);
+/* GatherBack of per-voxel logits together with the label pass: logits[i] = feats[ids[i]] (the first `classes` of `ld` columns,
+ * widened to float; `fill` where ids[i] is negative or beyond m) and labels[i] = index of the row's first largest value. */
+int d3d_gather_labels(int dtype, const void* feats, int64_t ld, int classes, int64_t m, const int32_t* ids, int64_t n,
+                      float fill, float* logits, int32_t* labels, void* stream);
+
 int d3d_spconv_mm_create(const void* data_s, size_t len, d3d_spconv_mm_t* handle);
 int d3d_spconv_mm_get_params(d3d_spconv_mm_t handle, d3d_spconv_mm_params* p);
 /* serialize (mm_trt.cu:71-74): writes the blob back; *len receives the size (buffer may be NULL). */
