@@ -1444,7 +1444,7 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
   rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, false, PairLists{}, &fwd, p->max_num_act_out, inverse,
                     out_coors, num_act_out, status, st);
   if (rc != D3D_OK) return rc;
-  rc = pack_table_masks(fwd, kvol, st);
+  rc = pack_table_masks(fwd, kvol, st, false);
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;

@@ -30,6 +30,8 @@ namespace {
 // the row masks afterwards.
 __global__ void table_fill_kernel(uint32_t* row_masks, int64_t mask_words, int32_t* perm, int64_t perm_words,
                                   int64_t m_max, unsigned long long* checks) {
+  pdl_release();
+  pdl_wait();
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
   if (checks && tid < 2) checks[tid] = 0ull;
   for (int64_t w = tid; w < perm_words; w += nthreads) perm[w] = w < m_max ? (int32_t)w : -1;
@@ -39,6 +41,8 @@ __global__ void table_fill_kernel(uint32_t* row_masks, int64_t mask_words, int32
 // One warp per tile: lane k looks at the four row-mask words of offset k.
 __global__ void pack_mask_kernel(const uint4* __restrict__ row_masks, int64_t tiles, int kvol,
                                  uint32_t* __restrict__ tile_mask) {
+  pdl_release();
+  pdl_wait();
   const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (tile >= tiles) return;
   const int k = threadIdx.x & 31;
@@ -56,6 +60,8 @@ __global__ void table_scatter_kernel(const int32_t* __restrict__ index, int64_t 
                                      const int32_t* __restrict__ num_index, int inverse, int mirror, int kvol,
                                      int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks,
                                      const unsigned long long* __restrict__ unless_equal) {
+  pdl_release();
+  pdl_wait();
   if (unless_equal && unless_equal[0] == unless_equal[1]) return;  // done by table_scatter_mirrored_kernel
   int64_t n = *num_index;
   n = n > row_len ? row_len : n;
@@ -127,6 +133,8 @@ __global__ void __launch_bounds__(256)
 table_scatter_mirrored_kernel(const int32_t* __restrict__ index, int64_t row_len, const int32_t* __restrict__ num_index,
                               int kvol, int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks,
                               unsigned long long* __restrict__ checks) {
+  pdl_release();
+  pdl_wait();
   int64_t n = *num_index;
   n = n > row_len ? row_len : n;
   const int64_t n_warp = (n + 31) & ~(int64_t)31, stride = (int64_t)gridDim.x * blockDim.x;
@@ -181,6 +189,8 @@ table_scatter_mirrored_kernel(const int32_t* __restrict__ index, int64_t row_len
 // The rulebook was not symmetric after all: the row masks start over.
 __global__ void table_redo_kernel(const unsigned long long* __restrict__ checks, uint32_t* __restrict__ row_masks,
                                   int64_t mask_words) {
+  pdl_release();
+  pdl_wait();
   if (checks[0] == checks[1]) return;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < mask_words; w += (int64_t)gridDim.x * blockDim.x)
     row_masks[w] = 0u;
@@ -302,7 +312,9 @@ spconv_mm_simt_kernel(const T* __restrict__ in_feats, int64_t n_in_max, const T*
 
   constexpr int kLanes = CPT == 2 ? 16 : CPT == 4 ? 32 : 0;  // lanes of a row walk, 0: none
   __shared__ int pairs_s, offsets_s;
+  pdl_release();
   if (tid == 0) pairs_s = 0, offsets_s = 0;
+  pdl_wait();
   __syncthreads();
   int pairs = 0, offsets = 0;
   for (int k = warp; k < kvol; k += kSimtThreads / 32) {
@@ -437,10 +449,10 @@ template <class T> int launch_simt_typed(const MmLaunch& a) {
   {                                                                                                                \
     auto kern = spconv_mm_simt_kernel<T, N>;                                                                       \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
-    kern<<<grid, kSimtThreads, smem, st>>>(reinterpret_cast<const T*>(a.in_feats), a.max_num_act_in,               \
-                                           reinterpret_cast<const T*>(h->w_dev), h->b_dev, tp.ids, tp.row_masks,    \
-                                           tp.perm, m_max, kvol, cin, cout, reinterpret_cast<T*>(a.out_feats),      \
-                                           a.relu, reinterpret_cast<const T*>(a.residual));                        \
+    D3D_LAUNCH(a.chained, kern, grid, kSimtThreads, smem, st, reinterpret_cast<const T*>(a.in_feats),              \
+               a.max_num_act_in, reinterpret_cast<const T*>(h->w_dev), h->b_dev, tp.ids, tp.row_masks, tp.perm,     \
+               m_max, kvol, cin, cout, reinterpret_cast<T*>(a.out_feats), a.relu,                                  \
+               reinterpret_cast<const T*>(a.residual));                                                            \
   }
   if (cpt <= 2) D3D_SIMT_CASE(2)
   else if (cpt <= 4) D3D_SIMT_CASE(4)
@@ -455,9 +467,10 @@ template <class T> int launch_simt_typed(const MmLaunch& a) {
 
 }  // namespace
 
-int pack_table_masks(const TableParts& t, int kernel_vol, void* stream) {
-  pack_mask_kernel<<<(unsigned)ceil_div(t.tiles * 32, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint4*>(t.row_masks), t.tiles, kernel_vol, t.tile_mask);
+int pack_table_masks(const TableParts& t, int kernel_vol, void* stream, bool chained) {
+  D3D_LAUNCH(chained, pack_mask_kernel, (unsigned)ceil_div(t.tiles * 32, 256), 256, 0,
+             reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const uint4*>(t.row_masks), t.tiles, kernel_vol,
+             t.tile_mask);
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }
@@ -661,23 +674,23 @@ extern "C" int d3d_spconv_mm_workspace(d3d_spconv_mm_t h, const d3d_tensor_desc*
 // as its mirror image if that is what it is, see table_scatter_mirrored_kernel.
 static int build_table(int kernel_vol, int inverse, int mirror, int64_t max_num_act_out, const int32_t* index,
                        int64_t index_row_len, const int32_t* num_index, void* table, unsigned long long* checks,
-                       cudaStream_t st) {
+                       bool chained, cudaStream_t st) {
   const int64_t pitch = (max_num_act_out + 127) / 128 * 128;
   const TableParts t = table_parts(table, kernel_vol, max_num_act_out);
   const int64_t mask_words = t.tiles * kernel_vol * 4;
-  table_fill_kernel<<<stream_grid(mask_words, 256), 256, 0, st>>>(t.row_masks, mask_words, t.perm, t.tiles * 128,
-                                                                 max_num_act_out, checks);
+  D3D_LAUNCH(chained, table_fill_kernel, stream_grid(mask_words, 256), 256, 0, st, t.row_masks, mask_words, t.perm,
+             t.tiles * 128, max_num_act_out, checks);
   if (index_row_len > 0) {
     const int grid = stream_grid(index_row_len, 256);
     if (checks) {
-      table_scatter_mirrored_kernel<<<grid, 256, 0, st>>>(index, index_row_len, num_index, kernel_vol, pitch, t.ids,
-                                                          t.row_masks, checks);
-      table_redo_kernel<<<stream_grid(mask_words, 256, 2), 256, 0, st>>>(checks, t.row_masks, mask_words);
+      D3D_LAUNCH(chained, table_scatter_mirrored_kernel, grid, 256, 0, st, index, index_row_len, num_index, kernel_vol,
+                 pitch, t.ids, t.row_masks, checks);
+      D3D_LAUNCH(chained, table_redo_kernel, stream_grid(mask_words, 256, 2), 256, 0, st, checks, t.row_masks, mask_words);
     }
-    table_scatter_kernel<<<grid, 256, 0, st>>>(index, index_row_len, num_index, inverse, mirror, kernel_vol, pitch,
-                                               t.ids, t.row_masks, checks);
+    D3D_LAUNCH(chained, table_scatter_kernel, grid, 256, 0, st, index, index_row_len, num_index, inverse, mirror,
+               kernel_vol, pitch, t.ids, t.row_masks, checks);
   }
-  return pack_table_masks(t, kernel_vol, st);
+  return pack_table_masks(t, kernel_vol, st, chained);
 }
 
 extern "C" int d3d_spconv_mm_prepare(int kernel_vol, int mode, int64_t max_num_act_out, const int32_t* index,
@@ -689,7 +702,7 @@ extern "C" int d3d_spconv_mm_prepare(int kernel_vol, int mode, int64_t max_num_a
   D3D_REQUIRE(index && num_index && table, D3D_ERR_INVALID_ARGUMENT);
   const int inverse = mode & 1;
   const int mirror = (mode & 2) && !inverse;  // a symmetric rulebook is its own inverse
-  return build_table(kernel_vol, inverse, mirror, max_num_act_out, index, index_row_len, num_index, table, nullptr,
+  return build_table(kernel_vol, inverse, mirror, max_num_act_out, index, index_row_len, num_index, table, nullptr, false,
                      reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -724,10 +737,9 @@ extern "C" int d3d_spconv_mm_regroup(int kernel_vol, int64_t max_num_act_out, co
   return D3D_OK;
 }
 
-extern "C" int d3d_spconv_mm_run(d3d_spconv_mm_t h, int dtype, const void* in_feats, int64_t max_num_act_in,
-                                 const int32_t* num_act_out, const void* table, void* out_feats,
-                                 const d3d_spconv_mm_epilogue* epilogue, void* stream) {
-  D3D_NVTX_RANGE("d3d_spconv_mm_run");
+// `chained`: the kernel in front in the stream is this call's own table build; it may be waited for inside the kernel.
+static int run(d3d_spconv_mm_t h, int dtype, const void* in_feats, int64_t max_num_act_in, const int32_t* num_act_out,
+               const void* table, void* out_feats, const d3d_spconv_mm_epilogue* epilogue, void* stream, bool chained) {
   D3D_REQUIRE(h, D3D_ERR_INVALID_ARGUMENT);
   D3D_REQUIRE(dtype == D3D_FLOAT || dtype == D3D_HALF || dtype == D3D_BF16, D3D_ERR_UNSUPPORTED_DTYPE);
   D3D_REQUIRE(h->dtype == dtype, D3D_ERR_INVALID_ARGUMENT);  // configure() must have run for this dtype
@@ -740,6 +752,7 @@ extern "C" int d3d_spconv_mm_run(d3d_spconv_mm_t h, int dtype, const void* in_fe
   a.residual = epilogue ? epilogue->residual : nullptr;
   a.regrouped = epilogue ? epilogue->regrouped : 0;
   a.stream = stream;
+  a.chained = chained || h->dependent_launch;
   bool tc_ok = spconv_mm_tc_eligible(h, dtype);
   if (h->kernel_choice == 2 || h->kernel_choice == 3) {
     D3D_REQUIRE(tc_ok, D3D_ERR_INVALID_ARGUMENT);
@@ -747,6 +760,13 @@ extern "C" int d3d_spconv_mm_run(d3d_spconv_mm_t h, int dtype, const void* in_fe
   }
   if (h->kernel_choice == 0 && tc_ok) return launch_spconv_mm_tc(a);
   return launch_spconv_mm_simt(a);
+}
+
+extern "C" int d3d_spconv_mm_run(d3d_spconv_mm_t h, int dtype, const void* in_feats, int64_t max_num_act_in,
+                                 const int32_t* num_act_out, const void* table, void* out_feats,
+                                 const d3d_spconv_mm_epilogue* epilogue, void* stream) {
+  D3D_NVTX_RANGE("d3d_spconv_mm_run");
+  return run(h, dtype, in_feats, max_num_act_in, num_act_out, table, out_feats, epilogue, stream, false);
 }
 
 extern "C" int d3d_spconv_mm_enqueue(d3d_spconv_mm_t h, const d3d_tensor_desc* in, int n_in,
@@ -781,9 +801,9 @@ extern "C" int d3d_spconv_mm_enqueue(d3d_spconv_mm_t h, const d3d_tensor_desc* i
                                             : nullptr;
     rc = build_table(h->p.kernel_vol, h->p.inverse, 0, h->p.max_num_act_out,
                      reinterpret_cast<const int32_t*>(inputs[3]), row_len, reinterpret_cast<const int32_t*>(inputs[4]),
-                     workspace, checks, reinterpret_cast<cudaStream_t>(stream));
+                     workspace, checks, true, reinterpret_cast<cudaStream_t>(stream));
   }
   if (rc != D3D_OK) return rc;
-  return d3d_spconv_mm_run(h, dtype, inputs[0], in[0].dims[0], reinterpret_cast<const int32_t*>(inputs[2]),
-                           workspace, outputs[0], nullptr, stream);
+  return run(h, dtype, inputs[0], in[0].dims[0], reinterpret_cast<const int32_t*>(inputs[2]), workspace, outputs[0],
+             nullptr, stream, true);
 }

@@ -37,6 +37,7 @@ struct MmLaunch {
   const void* residual;
   int regrouped;  // hint: the table's outputs were regrouped (few offsets per tile)
   void* stream;
+  bool chained;  // launch as a programmatic dependent of the kernel in front
 };
 
 // Bytes of the id part of the neighbour table; the per-tile offset masks (one uint32 per tile) start right after.
@@ -82,7 +83,7 @@ inline size_t table_perm_bytes(int64_t max_num_act_out) {
 }
 
 // Derives the offset mask of every tile from its row masks (cudaStream_t as void*).
-int pack_table_masks(const TableParts& t, int kernel_vol, void* stream);
+int pack_table_masks(const TableParts& t, int kernel_vol, void* stream, bool chained);
 
 int launch_spconv_mm_simt(const MmLaunch& a);
 // Returns D3D_ERR_INVALID_ARGUMENT when the shape/dtype is not eligible for the tensor-core path.

@@ -1161,7 +1161,7 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = h->dependent_launch ? 1 : 0;
+  cfg.attrs = attr, cfg.numAttrs = a.chained ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, kernel, st->map_b, p) != cudaSuccess) return D3D_ERR_CUDA;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
