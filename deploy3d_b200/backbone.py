@@ -7,6 +7,8 @@ workspace allocated at its static maximum size, exactly as TensorRT would own th
 frame after frame with no allocation and no host synchronisation, so a whole frame can be captured
 in a CUDA graph.  Layers that share a rulebook also share one output-stationary neighbour table.
 """
+import contextlib
+
 import numpy as np
 import torch
 
@@ -263,6 +265,10 @@ class SparseNet:
         self.overlap_rulebooks = overlap_rulebooks
         self.side = torch.cuda.Stream(device=self.device) if overlap_rulebooks else None
         self.side_subm = torch.cuda.Stream(device=self.device) if overlap_rulebooks else None
+        self.branch_of, self.inputs_of = self._plan_branches(layers)
+        if not overlap_rulebooks:
+            self.branch_of = [0] * len(layers)
+        self.branch = torch.cuda.Stream(device=self.device) if any(self.branch_of) else None
         self.kernel = kernel
         weights = make_weights(layers, seed)
         self.rulebooks = {}
@@ -389,6 +395,25 @@ class SparseNet:
                     set_of_tag[L.save] = cur
             self.out_set = cur
 
+    @staticmethod
+    def _plan_branches(layers):
+        """Which of two streams each layer runs on, and the layers it reads.  Layers that do not feed each other -- the two
+        branches of a residual block, the three convolutions of a ReconBlock -- go to different streams: the tail of one
+        launch, where CTAs have run out of tiles, and the ramp of the next then overlap.  A layer follows the one that
+        made its input if that is the last of a stream, else it goes where the last layer is the older one."""
+        made, branch, inputs, last, prev = {"input": -1}, [], [], [-1, -1], -1
+        for i, L in enumerate(layers):
+            reads = [made[t] for t in L.ew[1]] if L.kind == "ew" else \
+                [prev if L.source is None else made[L.source]] + ([made[L.residual]] if L.residual else [])
+            follow = max(reads) if L.kind == "ew" else reads[0]
+            b = last.index(follow) if follow in last else (0 if last[0] <= last[1] else 1)
+            branch.append(b)
+            inputs.append(sorted(set(r for r in reads if r >= 0)))
+            last[b] = prev = i
+            if L.save:
+                made[L.save] = i
+        return branch, inputs
+
     def set_input(self, coors, num):
         self.sets["in"]["coors"], self.sets["in"]["num"] = coors, num
 
@@ -480,36 +505,25 @@ class SparseNet:
         built = set()
         saved = {"input": feats}
         x = feats
+        streams = [main, self.branch]
+        if self.branch is not None:
+            self.branch.wait_stream(main)
+        finished = {}  # layer -> event, for layers that the other stream reads
+        crossing = {r for i, reads in enumerate(self.inputs_of) for r in reads if self.branch_of[r] != self.branch_of[i]}
         for li, (L, (plug, out_buf, out_set)) in enumerate(zip(self.layers, self.mm)):
-            if L.kind == "ew":  # element-wise graph op between plugins, in fp32 like the CPU restatement
-                x = self._elementwise(li, L, out_buf, [saved[t] for t in L.ew[1]])
-                if L.save:
-                    saved[L.save] = x
-                continue
-            if L.source is not None:
-                x = saved[L.source]
-            rb = self.rulebooks[L.key]
-            if L.key not in built:
-                if self.overlap_rulebooks:
-                    main.wait_event(ready[L.key])
-                else:
-                    self._build_rulebook(rb)
-                    if rb.group is not None:
-                        built.update(k for k, r in self.rulebooks.items() if r.group is rb.group)
-                built.add(L.key)
-            res = saved[L.residual] if L.residual else None
-            if self.plugin_order:
-                in_set = rb.out_set if L.kind == "inverse" else rb.in_set
-                plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], *rb.buffers(), outputs=[out_buf])
-                if L.relu or res is not None:  # the element-wise layer an engine fuses sum and activation into
-                    activation(out_buf, res, L.relu_mode)
-                x = out_buf
-            else:
-                table = rb.table_inv if L.kind == "inverse" else rb.table_fwd
-                x = plug.run(x, self.sets[out_set]["num"], table, out=out_buf, relu=L.relu_mode, residual=res,
-                             regrouped=rb.regroup)
+            here = streams[self.branch_of[li]]
+            for r in self.inputs_of[li]:
+                if self.branch_of[r] != self.branch_of[li]:
+                    here.wait_event(finished[r])
+            with torch.cuda.stream(here) if here is not main else contextlib.nullcontext():
+                x = self._layer(li, L, plug, out_buf, out_set, x, saved, here, ready, built)
             if L.save:
                 saved[L.save] = x
+            if li in crossing:
+                finished[li] = torch.cuda.Event()
+                finished[li].record(here)
+        if self.branch is not None:
+            main.wait_stream(self.branch)
         if self.overlap_rulebooks:
             main.wait_stream(self.side)
             main.wait_stream(self.side_subm)
@@ -517,6 +531,30 @@ class SparseNet:
         if x.shape[1] != self.out_channels:
             x = x[:, :self.out_channels]
         return x, o["coors"], o["num"]
+
+    def _layer(self, li, L, plug, out_buf, out_set, x, saved, stream, ready, built):
+        """One layer on `stream` (the current one); returns its output."""
+        if L.kind == "ew":  # element-wise graph op between plugins, in fp32 like the CPU restatement
+            return self._elementwise(li, L, out_buf, [saved[t] for t in L.ew[1]])
+        if L.source is not None:
+            x = saved[L.source]
+        rb = self.rulebooks[L.key]
+        if self.overlap_rulebooks:
+            if (stream, L.key) not in built:
+                stream.wait_event(ready[L.key])
+                built.add((stream, L.key))
+        elif L.key not in built:
+            self._build_rulebook(rb)
+            built.update([L.key] if rb.group is None else [k for k, r in self.rulebooks.items() if r.group is rb.group])
+        res = saved[L.residual] if L.residual else None
+        if self.plugin_order:
+            in_set = rb.out_set if L.kind == "inverse" else rb.in_set
+            plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], *rb.buffers(), outputs=[out_buf])
+            if L.relu or res is not None:  # the element-wise layer an engine fuses sum and activation into
+                activation(out_buf, res, L.relu_mode)
+            return out_buf
+        return plug.run(x, self.sets[out_set]["num"], rb.table_inv if L.kind == "inverse" else rb.table_fwd, out=out_buf,
+                        relu=L.relu_mode, residual=res, regrouped=rb.regroup)
 
     def counts(self):
         """Active voxels of every set (host sync; for calibration and reporting only)."""
