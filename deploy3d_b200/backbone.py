@@ -230,11 +230,25 @@ class _SubmGroup:
             self.by_ksize[rb.ksize] = make()
         return self.by_ksize[rb.ksize]
 
-    def enqueue(self, coors, num, shape):
+    def _pass(self):
         sizes = list(self.by_ksize)
         if self.pass_ is None or len(self.pass_.kernel_sizes) != len(sizes):
             self.pass_ = SubmTables(sizes)
-        self.pass_.enqueue(coors, num, shape, tables=[self.by_ksize[k] for k in sizes])
+        return self.pass_
+
+    def clear(self, src, shape, device):
+        self._pass().clear(*_shapes_of(src), shape, device=device)
+
+    def enqueue(self, coors, num, shape, voxel_grid=None, cleared=False):
+        p = self._pass()
+        p.enqueue(coors, num, shape, tables=[self.by_ksize[k] for k in p.kernel_sizes], voxel_grid=voxel_grid,
+                  cleared=cleared)
+
+
+def _shapes_of(voxels):
+    """Stand-ins for the coordinates and the count of a voxel set, for calls that read shapes only."""
+    return (torch.empty((voxels["cap"], 4), dtype=torch.int32, device="meta"),
+            torch.empty(1, dtype=torch.int32, device="meta"))
 
 
 class SparseNet:
@@ -273,6 +287,8 @@ class SparseNet:
         weights = make_weights(layers, seed)
         self.rulebooks = {}
         self.groups = {}  # voxel set -> _SubmGroup
+        self._cleared = False
+        self.tables_done = None  # event of the last forward: all tables built (overlap_rulebooks)
         self._concatenated = None  # the concatenation layer whose result is in place already
         self.mm = []
         self.sets = {"in": dict(cap=int(caps["in"]), shape=[int(v) for v in spatial], coors=None, num=None)}
@@ -335,9 +351,7 @@ class SparseNet:
                         rb.table_fwd = rb.group.table_of(rb, new_table)
                     else:
                         rb.table_fwd = new_table()
-                        rb.direct = not subm and rb.plugin.tables_ok(
-                            torch.empty((src["cap"], 4), dtype=torch.int32, device="meta"),
-                            torch.empty(1, dtype=torch.int32, device="meta"), rb.shape_tensor)
+                        rb.direct = not subm and rb.plugin.tables_ok(*_shapes_of(src), rb.shape_tensor)
                     rb.table_inv = None
                     rb.raw_fwd = rb.raw_inv = rb.scratch_fwd = rb.scratch_inv = None
                     rb.regroup = self.regroup and rb.kvol <= 32
@@ -417,6 +431,32 @@ class SparseNet:
     def set_input(self, coors, num):
         self.sets["in"]["coors"], self.sets["in"]["num"] = coors, num
 
+    def begin(self):
+        """Optional, ahead of `forward` and of whatever makes its input: clears the grids of the rulebooks on the side
+        streams, which does not depend on the voxels and so runs beside the encoder (cylinder 10, centerpoint 50 us of
+        kernels).  `forward` clears them itself otherwise."""
+        if not self.overlap_rulebooks:
+            return
+        main = torch.cuda.current_stream(self.device)
+        self.side.wait_stream(main)
+        self.side_subm.wait_stream(main)
+        seen = set()
+        for rb in self.rulebooks.values():
+            if rb.direct:
+                with torch.cuda.stream(self.side):
+                    rb.plugin.tables_clear(*_shapes_of(self.sets[rb.in_set]), rb.shape_tensor, device=self.device,
+                                           table=rb.raw_fwd if rb.regroup else rb.table_fwd)
+            elif rb.group is not None and rb.group not in seen and not self._made_on_grid(rb.in_set):
+                seen.add(rb.group)
+                with torch.cuda.stream(self.side_subm):
+                    rb.group.clear(self.sets[rb.in_set], rb.shape_tensor, self.device)
+        self._cleared = True
+
+    def _made_on_grid(self, name):
+        """Whether the strided pass that makes voxel set `name` leaves the grid of its voxels behind."""
+        maker = self.rulebooks.get(name)
+        return maker is not None and maker.direct
+
     def _build_rulebook(self, rb):
         """Whatever the layers of `rb` read; for a group of submanifold rulebooks, the tables of all of them."""
         src, dst = self.sets[rb.in_set], self.sets[rb.out_set]
@@ -426,7 +466,11 @@ class SparseNet:
             rb.plugin.enqueue(src["coors"], src["num"], rb.shape_tensor, outputs=outs)
             return
         if rb.group is not None:
-            rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor)
+            grid = None
+            if self._made_on_grid(rb.in_set):
+                maker = self.rulebooks[rb.in_set]
+                grid = maker.plugin.tables_grid(*_shapes_of(self.sets[maker.in_set]), maker.shape_tensor)
+            rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor, voxel_grid=grid, cleared=self._cleared)
             for other in self.rulebooks.values():
                 if other.group is rb.group and other.regroup:
                     SPConvMMPlugin.regroup(other.kvol, dst["cap"], other.raw_fwd, other.table_fwd, other.scratch_fwd)
@@ -435,7 +479,7 @@ class SparseNet:
         plain_inv = rb.raw_inv if rb.regroup else rb.table_inv
         if rb.direct:
             rb.plugin.tables(src["coors"], src["num"], rb.shape_tensor, out_coors=dst["coors"],
-                             num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv)
+                             num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv, cleared=self._cleared)
         else:  # kernels or grids the direct builders do not take
             first = rb.calls == 0
             rb.calls += 1
@@ -480,6 +524,8 @@ class SparseNet:
         of its own rulebook.  Inside a CUDA graph capture these become further branches of the graph."""
         main = torch.cuda.current_stream(self.device)
         ready = {}
+        if not self._cleared:
+            self.begin()
         if self.overlap_rulebooks:
             # two chains: the strided rulebooks follow each other (each creates the voxel set of the next); the SubM
             # rulebook of a level needs only that level's coordinates, so it runs beside the next strided one.
@@ -502,6 +548,10 @@ class SparseNet:
                     ev = torch.cuda.Event()
                     ev.record(stream)
                     ready.update((k, ev) for k in keys)
+            self._cleared = False
+            self.side.wait_stream(self.side_subm)
+            self.tables_done = torch.cuda.Event()
+            self.tables_done.record(self.side)
         built = set()
         saved = {"input": feats}
         x = feats
@@ -525,8 +575,7 @@ class SparseNet:
         if self.branch is not None:
             main.wait_stream(self.branch)
         if self.overlap_rulebooks:
-            main.wait_stream(self.side)
-            main.wait_stream(self.side_subm)
+            main.wait_event(self.tables_done)
         o = self.sets[self.out_set]
         if x.shape[1] != self.out_channels:
             x = x[:, :self.out_channels]

@@ -1095,13 +1095,17 @@ int64_t clear_grid(const ClearArgs& a) {
   return stream_grid(words / 16, 256);  // four 16-byte stores per thread
 }
 
+// How much of a pass's lookup is there already: nothing, the cleared memory, or the finished grid.
+enum Ready { kNothing, kCleared, kFinished };
+
 // Lookup structure of the inputs, then their neighbours.
-int launch_subm3(const Plan& plan, const int32_t* coors, const int32_t* num_act_in, bool chained,
+int launch_subm3(const Plan& plan, Ready ready, const int32_t* coors, const int32_t* num_act_in, bool chained,
                  const PairLists& lists, const Targets& targets, int32_t* status, cudaStream_t st) {
   const ClearArgs a = clear_args(plan);
-  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
-  D3D_LAUNCH3(chained, subm_mark3_kernel, plan.nblk, kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g,
-              status);
+  if (ready == kNothing) D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  if (ready != kFinished)
+    D3D_LAUNCH3(chained, subm_mark3_kernel, plan.nblk, kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g,
+                status);
   // one block per 256 rows up to the end of the tables, so that rows beyond the live count get their masks
   const int64_t blocks = targets.count ? std::max<int64_t>(plan.nblk, ceil_div(targets.tiles * 128, kIdxThreads))
                                        : plan.nblk;
@@ -1110,15 +1114,24 @@ int launch_subm3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
   return D3D_OK;
 }
 
-int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_in, int32_t max_out, bool chained,
-                 const PairLists& lists, const TableParts* fwd, int64_t fwd_rows, const Targets& inverse,
-                 int32_t* out_coors, int32_t* num_act_out, int32_t* status, cudaStream_t st) {
+// The grid of a strided pass and what its forward table needs cleared: nothing here depends on the voxels.
+int clear_conv3(const Plan& plan, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
   ClearArgs a = clear_args(plan);
   if (fwd) {
     a.rows = fwd->row_masks, a.row_words = fwd->tiles * plan.g.kvol * 4;
     a.perm = fwd->perm, a.perm_words = fwd->tiles * 128, a.m_max = fwd_rows;
   }
-  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, (const int32_t*)nullptr, plan.n_max);
+  return D3D_OK;
+}
+
+int launch_conv3(const Plan& plan, Ready ready, const int32_t* coors, const int32_t* num_act_in, int32_t max_out,
+                 bool chained, const PairLists& lists, const TableParts* fwd, int64_t fwd_rows, const Targets& inverse,
+                 int32_t* out_coors, int32_t* num_act_out, int32_t* status, cudaStream_t st) {
+  if (ready == kNothing) {
+    const int rc = clear_conv3(plan, fwd, fwd_rows, st);
+    if (rc != D3D_OK) return rc;
+  }
   const bool two = plan.two_taps;
   D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
   D3D_LAUNCH3(chained, two ? conv_count3_kernel<2> : conv_count3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
@@ -1258,14 +1271,14 @@ extern "C" int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, con
         targets.t[0] = make_target(nbr, g.kvol, n_max);
         mirror_slots(&targets.t[0], g.ksize, g.ksize);
       }
-      rc = launch_subm3(plan, coors, num_act_in, chained, lists, targets, status, st);
+      rc = launch_subm3(plan, kNothing, coors, num_act_in, chained, lists, targets, status, st);
     } else {
       int32_t* out_coors = reinterpret_cast<int32_t*>(outputs[2]);
       int32_t* num_act_out = reinterpret_cast<int32_t*>(outputs[3]);
       D3D_REQUIRE(out_coors && num_act_out, D3D_ERR_INVALID_ARGUMENT);
       D3D_REQUIRE(out[2].dims[0] >= p->max_num_act_out, D3D_ERR_INVALID_ARGUMENT);
-      rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, chained, lists, nullptr, 0, targets, out_coors,
-                        num_act_out, status, st);
+      rc = launch_conv3(plan, kNothing, coors, num_act_in, p->max_num_act_out, chained, lists, nullptr, 0, targets,
+                        out_coors, num_act_out, status, st);
     }
     if (rc != D3D_OK) return rc;
     D3D_LAUNCH3(chained, segment_scan_kernel, g.kvol, 1024, st, plan.block_counts, nblk, g.kvol, num_act_in, n_max,
@@ -1372,9 +1385,28 @@ extern "C" int d3d_spconv_subm_tables_workspace(const d3d_tensor_desc* in, int n
   return rc;
 }
 
+extern "C" int d3d_spconv_subm_tables_clear(const d3d_tensor_desc* in, int n_in, void* workspace,
+                                            size_t workspace_bytes, void* stream) {
+  D3D_NVTX_RANGE("d3d_spconv_subm_tables_clear");
+  const int ks[3] = {3, 3, 3};
+  d3d_spconv_index_params p;
+  subm_params(&p, ks);
+  Plan plan;
+  const int rc = make_plan(&p, in, n_in, workspace, &plan, true);
+  if (rc != D3D_OK) return rc;
+  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  if (plan.n_max == 0) return D3D_OK;
+  const ClearArgs a = clear_args(plan);
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, reinterpret_cast<cudaStream_t>(stream), a,
+              (const int32_t*)nullptr, plan.n_max);
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
 extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables,
                                       const d3d_tensor_desc* in, int n_in, const void* const* inputs, void* workspace,
-                                      size_t workspace_bytes, void* stream, int32_t* status) {
+                                      size_t workspace_bytes, void* stream, int32_t* status, const int32_t* voxel_grid,
+                                      int cleared) {
   D3D_NVTX_RANGE("d3d_spconv_subm_tables");
   D3D_REQUIRE(n_tables >= 1 && n_tables <= kMaxTargets && kernel_size && tables && inputs, D3D_ERR_INVALID_ARGUMENT);
   int outer[3] = {1, 1, 1};
@@ -1390,9 +1422,10 @@ extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, 
   Plan plan;
   int rc = make_plan(&p, in, n_in, workspace, &plan, true);
   if (rc != D3D_OK) return rc;
-  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  D3D_REQUIRE(voxel_grid || (workspace && workspace_bytes >= plan.bytes), D3D_ERR_WORKSPACE_TOO_SMALL);
   const int64_t n_max = plan.n_max;
   if (n_max == 0) return D3D_OK;
+  if (voxel_grid) plan.path = Plan::kDirect, plan.grid = const_cast<int32_t*>(voxel_grid);  // read only
   const int32_t* coors = reinterpret_cast<const int32_t*>(inputs[0]);
   const int32_t* num_act_in = reinterpret_cast<const int32_t*>(inputs[1]);
   D3D_REQUIRE(coors && num_act_in, D3D_ERR_INVALID_ARGUMENT);
@@ -1406,7 +1439,8 @@ extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, 
     targets.t[t] = make_target(tables[t], ks[0] * ks[1] * ks[2], n_max);
     mirror_slots(&targets.t[t], ks, outer);
   }
-  rc = launch_subm3(plan, coors, num_act_in, false, PairLists{}, targets, status, st);
+  rc = launch_subm3(plan, voxel_grid ? kFinished : cleared ? kCleared : kNothing, coors, num_act_in, false, PairLists{},
+                    targets, status, st);
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
@@ -1418,10 +1452,33 @@ extern "C" int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const
   return plan.path == Plan::kDirect && plan.g.kvol <= 32;
 }
 
+extern "C" const int32_t* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in,
+                                                      int n_in, void* workspace) {
+  Plan plan;
+  if (!workspace || !d3d_spconv_conv_tables_ok(p, in, n_in) || make_plan(p, in, n_in, workspace, &plan) != D3D_OK)
+    return nullptr;
+  return plan.grid;
+}
+
+extern "C" int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                                            void* table, void* workspace, size_t workspace_bytes, void* stream) {
+  D3D_NVTX_RANGE("d3d_spconv_conv_tables_clear");
+  D3D_REQUIRE(p && table && d3d_spconv_conv_tables_ok(p, in, n_in) && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
+  Plan plan;
+  int rc = make_plan(p, in, n_in, workspace, &plan);
+  if (rc != D3D_OK) return rc;
+  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  const TableParts fwd = table_parts(table, plan.g.kvol, p->max_num_act_out);
+  rc = clear_conv3(plan, &fwd, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
+  if (rc != D3D_OK) return rc;
+  D3D_CHECK_LAUNCH();
+  return D3D_OK;
+}
+
 extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                       const void* const* inputs, int32_t* out_coors, int32_t* num_act_out, void* table,
                                       void* table_inverse, void* workspace, size_t workspace_bytes, void* stream,
-                                      int32_t* status) {
+                                      int32_t* status, int cleared) {
   D3D_NVTX_RANGE("d3d_spconv_conv_tables");
   D3D_REQUIRE(p && inputs && out_coors && num_act_out && table, D3D_ERR_INVALID_ARGUMENT);
   Plan plan;
@@ -1441,8 +1498,8 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
     inverse.t[0] = make_target(table_inverse, kvol, plan.n_max);
     plain_slots(&inverse.t[0], plan.g);
   }
-  rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, false, PairLists{}, &fwd, p->max_num_act_out, inverse,
-                    out_coors, num_act_out, status, st);
+  rc = launch_conv3(plan, cleared ? kCleared : kNothing, coors, num_act_in, p->max_num_act_out, false, PairLists{}, &fwd,
+                    p->max_num_act_out, inverse, out_coors, num_act_out, status, st);
   if (rc != D3D_OK) return rc;
   rc = pack_table_masks(fwd, kvol, st, false);
   if (rc != D3D_OK) return rc;

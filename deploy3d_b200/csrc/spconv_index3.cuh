@@ -45,11 +45,20 @@ struct PairLists {
 };
 
 struct Lookup3 {
-  int32_t* direct;             // null: bits + slots
+  int32_t* direct;             // null: bits + slots; may be the grid a strided pass has left (see id_in_cell)
   unsigned long long* slots;
   uint32_t cap_max;
   uint32_t* bits;
 };
+
+// Cells a strided pass has numbered: an output's id with the sign bit set, or kDropped beyond maxNumActOut.
+constexpr int kDropped = -2;
+constexpr int kIdBit = -2147483647 - 1;
+
+// The voxel a cell of either kind of grid (plain ids of a submanifold pass, numbered outputs of a strided one) holds; -1: none.
+__device__ __forceinline__ int id_in_cell(int cell) {
+  return (unsigned)cell >= (unsigned)kDropped ? -1 : cell & ~kIdBit;
+}
 
 // Clears what a rulebook starts from: the lookup (live part of the hash table, all of the grid or of the bit map), the
 // ticket of segment_scan_kernel, and the row masks / output map of a neighbour table that is filled by scattering.
@@ -77,8 +86,8 @@ __global__ void __launch_bounds__(256) clear3_kernel(const ClearArgs a, const in
   };
   if (a.look.direct) fill(a.look.direct, a.direct_words / 4, ones);  // sizes are padded to 256 bytes
   if (a.look.bits) fill(a.look.bits, a.bit_words / 4, zero);
-  if (a.look.slots) {
-    const uint32_t cap = hash_capacity((long long)live_count(num_act_in, n_max) * a.fan, a.look.cap_max);
+  if (a.look.slots) {  // without a count (cleared ahead of the frame's voxels): all of them
+    const uint32_t cap = !num_act_in ? a.look.cap_max : hash_capacity((long long)live_count(num_act_in, n_max) * a.fan, a.look.cap_max);
     fill(a.look.slots, cap / 2, ones);
   }
   if (a.rows) fill(a.rows, a.row_words / 4, zero);
@@ -216,7 +225,9 @@ __device__ __forceinline__ void write_empty_targets(const Targets& targets, int6
 }
 
 // Submanifold neighbours: the voxel at coor + pad - tap * dilation for every tap (trt/spconv/index.cu:48-84), one thread
-// per voxel.  kDirect: 27 independent loads from the grid.  Otherwise nine words of the bit map (one per (z, y) row; a
+// per voxel.  kDirect: 27 independent loads from the grid -- the one subm_mark3_kernel has filled, or the one the strided
+// pass that made these voxels has left: then nothing is cleared or marked (level 2 of a detector, 463 k voxels: 25 us of
+// kernels less).  Otherwise nine words of the bit map (one per (z, y) row; a
 // second one where the taps straddle a word), then the hash slots of the hits, four in flight.
 // lists.value == null: no rulebook is wanted, only the tables.
 template <bool kDirect>
@@ -248,7 +259,7 @@ subm_find3_kernel(const Lookup3 look, const int32_t* __restrict__ coors, const i
       const bool ok = batch_ok && a < g.ksize[0] && b < g.ksize[1] && t < g.ksize[2] &&
                       (uint32_t)(b0 - a * g.dil[0]) < s1 && (uint32_t)(b1 - b * g.dil[1]) < s2 &&
                       (uint32_t)(b2 - t * g.dil[2]) < s3;
-      v[q] = ok ? __ldg(look.direct + (key0 - a * step0 - b * step1 - t * step2)) : -1;
+      v[q] = ok ? id_in_cell(__ldg(look.direct + (key0 - a * step0 - b * step1 - t * step2))) : -1;
     }
 #pragma unroll
     for (int q = 0; q < kTaps3; ++q) {
@@ -428,10 +439,6 @@ conv_mark3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors,
       atomicMin(reinterpret_cast<unsigned*>(grid) + cell_of(g, r, c.x), (unsigned)(i * g.kvol + offset_of(g, r)));
   }
 }
-
-// Cells after numbering: an output's id with the sign bit set, or kDropped beyond maxNumActOut.
-constexpr int kDropped = -2;
-constexpr int kIdBit = -2147483647 - 1;
 
 // The pair whose id is left in a cell numbers that output: in pair order, i.e. by first touch (index.cu:104-121).  First
 // the winning combinations of every input and their number per block, then the numbers themselves.

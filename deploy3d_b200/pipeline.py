@@ -106,15 +106,14 @@ class DetectionPipeline:
         """Enqueue one frame on the current stream (no host sync, no allocation after the first call).
 
         The NMS of the frame's candidate boxes is a parallel branch on a side stream: its inputs (decoded boxes) do
-        not come from the backbone of the same frame in this workload, and it is a chain of two small, latency-bound
-        kernels that fits beside the rulebook kernels.  (A deployed detector gets the same overlap by running the
-        NMS of frame i beside the backbone of frame i+1.)  The branch joins before enqueue returns, so the caller
-        still sees one stream; inside a CUDA graph capture it becomes a fork / join of the graph."""
+        not come from the backbone of the same frame in this workload.  (A deployed detector gets the same overlap by
+        running the NMS of frame i beside the backbone of frame i+1.)  It starts behind the last neighbour table: from
+        there to the end of the frame the convolutions leave SMs idle at their tails, while at the head of the frame
+        its mask kernel keeps the encoder and the first tables, which everything waits for, from the SMs.  The branch
+        joins before enqueue returns, so the caller still sees one stream; inside a CUDA graph capture it becomes a
+        fork / join of the graph."""
         main = torch.cuda.current_stream(self.device)
-        if not self.plugin_order:
-            self.side.wait_stream(main)
-            with torch.cuda.stream(self.side):
-                self.nms.enqueue(self.scores, self.boxes, outputs=[self.nms_scores])
+        self.net.begin()
         if self.plugin_order or self.dtype == torch.float32:
             self.vfe.enqueue(self.points, self.batch, self.cfg, self.shape_tensor,
                              outputs=[self.vox_feats, self.vox_coors, self.vox_num])
@@ -124,11 +123,19 @@ class DetectionPipeline:
             self.vfe.enqueue_lp(self.points, self.batch, self.cfg, self.shape_tensor,
                                 outputs=[self.vox_feats, self.vox_coors, self.vox_num], lp_feats=self.vox_feats_lp)
         feats, coors, num = self.net.forward(self.vox_feats_lp)
+        beside = not self.plugin_order
+        if beside:
+            if self.net.tables_done is not None:
+                self.side.wait_event(self.net.tables_done)
+            else:
+                self.side.wait_stream(main)
+            with torch.cuda.stream(self.side):
+                self.nms.enqueue(self.scores, self.boxes, outputs=[self.nms_scores])
         self.densify.enqueue(feats, coors, num, self.out_shape_tensor, outputs=[self.bev])
-        if self.plugin_order:
-            self.nms.enqueue(self.scores, self.boxes, outputs=[self.nms_scores])
-        else:
+        if beside:
             main.wait_stream(self.side)
+        else:
+            self.nms.enqueue(self.scores, self.boxes, outputs=[self.nms_scores])
         return feats, coors, num
 
     def capture(self):
@@ -244,6 +251,7 @@ class SegmentationPipeline:
     def enqueue(self):
         """One frame on the current stream: no host synchronisation, no allocation by this library (the
         element-wise graph ops between plugins are torch's)."""
+        self.net.begin()
         self.encoder.enqueue(self.points, self.batch, self.cfg, self.shape_tensor,
                              outputs=[self.pts_feats, self.scatter_index, self.scatter_count, self.vox_coors,
                                       self.vox_num])

@@ -145,9 +145,26 @@ class SPConvIdxPlugin(_Plugin):
         d = [_desc_of(t) for t in inputs]
         return bool(lib().d3d_spconv_conv_tables_ok(ctypes.byref(self.p), desc_array(d), len(d)))
 
-    def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None):
+    def tables_clear(self, *inputs, table, device, stream=None):
+        """The part of `tables` that does not depend on the voxels, ahead of them (d3d_spconv_conv_tables_clear); `inputs`
+        give shapes only."""
+        d = [_desc_of(t) for t in inputs]
+        nbytes = self.workspace_size(d)
+        ws = self._get_workspace(nbytes, device)
+        with torch.cuda.device(device):
+            check("d3d_spconv_conv_tables_clear", lib().d3d_spconv_conv_tables_clear(
+                ctypes.byref(self.p), desc_array(d), len(d), table.data_ptr(), ws.data_ptr(), nbytes,
+                _stream_ptr(stream)))
+
+    def tables_grid(self, *inputs):
+        """Address of the grid of numbered outputs the last `tables` over such inputs has left in this plugin's workspace."""
+        d = [_desc_of(t) for t in inputs]
+        return lib().d3d_spconv_conv_tables_grid(ctypes.byref(self.p), desc_array(d), len(d), self._workspace.data_ptr())
+
+    def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None,
+               cleared=False):
         """Output voxels and neighbour tables of a strided kernel straight from the coordinates, no `index`
-        (d3d_spconv_conv_tables)."""
+        (d3d_spconv_conv_tables); `cleared`: tables_clear was called for this build."""
         device = inputs[0].device
         d = [_desc_of(t) for t in inputs]
         nbytes = self.workspace_size(d)
@@ -157,7 +174,7 @@ class SPConvIdxPlugin(_Plugin):
                 ctypes.byref(self.p), desc_array(d), len(d), ptr_array([t.data_ptr() for t in inputs]),
                 out_coors.data_ptr(), num_act_out.data_ptr(), table.data_ptr(),
                 table_inverse.data_ptr() if table_inverse is not None else None, ws.data_ptr(), nbytes,
-                _stream_ptr(stream), status.data_ptr() if status is not None else None))
+                _stream_ptr(stream), status.data_ptr() if status is not None else None, int(bool(cleared))))
 
 
 def activation(x, residual=None, relu=1, stream=None):
@@ -205,21 +222,35 @@ class SubmTables:
         self._flat = (ctypes.c_int32 * len(flat))(*flat)
         self._workspace = None
 
-    def enqueue(self, *inputs, tables, status=None, stream=None):
-        """inputs: coordinates, count, shape carrier (as SPConvIdx3d); `tables`: one buffer per kernel size."""
-        assert len(tables) == len(self.kernel_sizes)
-        device = inputs[0].device
-        d = [_desc_of(t) for t in inputs]
+    def _get_workspace(self, d, device):
         n = ctypes.c_size_t(0)
         check("d3d_spconv_subm_tables_workspace",
               lib().d3d_spconv_subm_tables_workspace(desc_array(d), len(d), ctypes.byref(n)))
         if self._workspace is None or self._workspace.numel() < n.value or self._workspace.device != device:
             self._workspace = torch.empty(n.value, dtype=torch.uint8, device=device)
+        return self._workspace.data_ptr(), n.value
+
+    def clear(self, *inputs, device, stream=None):
+        """The part of `enqueue` that does not depend on the voxels, ahead of them (d3d_spconv_subm_tables_clear);
+        `inputs` give shapes only."""
+        d = [_desc_of(t) for t in inputs]
+        with torch.cuda.device(device):
+            check("d3d_spconv_subm_tables_clear", lib().d3d_spconv_subm_tables_clear(
+                desc_array(d), len(d), *self._get_workspace(d, device), _stream_ptr(stream)))
+
+    def enqueue(self, *inputs, tables, status=None, stream=None, voxel_grid=None, cleared=False):
+        """inputs: coordinates, count, shape carrier (as SPConvIdx3d); `tables`: one buffer per kernel size.  `voxel_grid`:
+        SPConvIdxPlugin.tables_grid of the strided kernel that made these voxels; `cleared`: `clear` was called for this
+        build."""
+        assert len(tables) == len(self.kernel_sizes)
+        device = inputs[0].device
+        d = [_desc_of(t) for t in inputs]
+        workspace, nbytes = (None, 0) if voxel_grid else self._get_workspace(d, device)
         with torch.cuda.device(device):
             check("d3d_spconv_subm_tables", lib().d3d_spconv_subm_tables(
                 len(tables), self._flat, ptr_array([t.data_ptr() for t in tables]), desc_array(d), len(d),
-                ptr_array([t.data_ptr() for t in inputs]), self._workspace.data_ptr(), n.value, _stream_ptr(stream),
-                status.data_ptr() if status is not None else None))
+                ptr_array([t.data_ptr() for t in inputs]), workspace, nbytes, _stream_ptr(stream),
+                status.data_ptr() if status is not None else None, voxel_grid, int(bool(cleared))))
 
 
 class SPConvMMPlugin(_Plugin):

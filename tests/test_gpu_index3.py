@@ -132,3 +132,51 @@ def test_conv_tables(d3d, orc, ks, st, pd, dil, tr, n, room):
         want = SPConvMMPlugin.prepare(kvol, inverse, rows, index, num_index)
         assert_tables_equal(table_parts(t, kvol, rows), table_parts(want, kvol, rows), "inverse %s" % inverse)
         assert len(table_pairs(table_parts(t, kvol, rows))) == int((index[2, :int(num_index.item())] >= 0).sum())
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("n", [1, 400])
+def test_subm_tables_cleared_ahead(d3d, grid, n):
+    from deploy3d_b200.plugins import SPConvMMPlugin, SubmTables
+    shape, cap = GRIDS[grid], 500
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, [shape[0], 9, 12, 13])
+    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
+    shp = torch.empty([shape[0], 0] + shape[1:], dtype=torch.int32, device=DEV)
+    want, got = (torch.full((SPConvMMPlugin.table_bytes(27, cap),), 93, dtype=torch.uint8, device=DEV) for _ in range(2))
+    p = SubmTables([(3, 3, 3)])
+    p.enqueue(coors_t, num, shp, tables=[want])
+    p._workspace.fill_(1)  # nothing of the first build may be needed
+    p.clear(coors_t, num, shp, device=torch.device(DEV))
+    p.enqueue(coors_t, num, shp, tables=[got], cleared=True)
+    assert_tables_equal(table_parts(got, 27, cap), table_parts(want, 27, cap))
+
+
+@pytest.mark.parametrize("n,room", [(1, 1.0), (127, 1.0), (700, 1.3), (700, 0.4)])
+def test_subm_tables_on_the_grid_of_a_strided_pass(d3d, orc, n, room):
+    from deploy3d_b200.plugins import SPConvMMPlugin, SubmTables, deserialize_plugin
+    shape, cap, ks, st, pd = [2, 13, 24, 25], 750, (3, 3, 3), (2, 2, 2), (1, 1, 1)
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, shape)
+    m = orc.rulebook_conv(coors[:n], shape, ks, st, pd, ONE, ZERO, False, 10 ** 7, max_num_act_in=n)[3]
+    max_out = max(1, int(m * room))
+    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
+    shp = torch.empty([2, 0] + shape[1:], dtype=torch.int32, device=DEV)
+    out_shp = torch.empty([2, 0] + [(v + 2 - 3) // 2 + 1 for v in shape[1:]], dtype=torch.int32, device=DEV)
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, ONE, ZERO, max_out, False, False))
+    fwd = torch.zeros(SPConvMMPlugin.table_bytes(27, max_out), dtype=torch.uint8, device=DEV)
+    oc, on = torch.zeros((max_out, 4), dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for cleared in (False, True):
+        if cleared:
+            plug._workspace.fill_(1)
+            fwd.fill_(7)
+            plug.tables_clear(coors_t, num, shp, table=fwd, device=torch.device(DEV))
+        plug.tables(coors_t, num, shp, out_coors=oc, num_act_out=on, table=fwd, cleared=cleared)
+        want, got = (torch.full((SPConvMMPlugin.table_bytes(27, max_out),), 93, dtype=torch.uint8, device=DEV)
+                     for _ in range(2))
+        SubmTables([ks]).enqueue(oc, on, out_shp, tables=[want])
+        SubmTables([ks]).enqueue(oc, on, out_shp, tables=[got], voxel_grid=plug.tables_grid(coors_t, num, shp))
+        assert_tables_equal(table_parts(got, 27, max_out), table_parts(want, 27, max_out))
+        index, num_index = plug.enqueue(coors_t, num, shp)[:2]
+        assert_tables_equal(table_parts(fwd, 27, max_out),
+                            table_parts(SPConvMMPlugin.prepare(27, False, max_out, index, num_index), 27, max_out))
