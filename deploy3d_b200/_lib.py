@@ -122,7 +122,7 @@ SIGNATURES = {
                                                     _sz, _vp]),
     "d3d_spconv_conv_tables_ok": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int]),
     "d3d_spconv_conv_tables": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int, _vpp, _vp, _vp,
-                                              _vp, _vp, _vp, _sz, _vp, _vp, ctypes.c_int]),
+                                              _vp, _vp, _vp, _sz, _vp, _vp, _vp, ctypes.c_int]),
     "d3d_spconv_mm_create": (ctypes.c_int, [_vp, _sz, ctypes.POINTER(_vp)]),
     "d3d_spconv_mm_get_params": (ctypes.c_int, [_vp, ctypes.POINTER(SpconvMMParams)]),
     "d3d_spconv_mm_serialize": (ctypes.c_int, [_vp, _vp, _szp]),

@@ -208,7 +208,21 @@ class _Rulebook:
                 dst = self.sets[self.out_set]
                 outs += [torch.empty_like(dst["coors"]), torch.empty_like(dst["num"]), self.out_shape_tensor]
             self.plugin.enqueue(src["coors"], src["num"], self.shape_tensor, outputs=outs)
+            if self.kind != "subm":
+                self._renumber(outs[0], outs[2][:int(outs[3])], dst["coors"][:int(dst["num"])])
         return self.buffers()
+
+    def _renumber(self, index, by_touch, by_cell):
+        """The rulebook numbers its outputs by first touch, the live tables in the order of their cells."""
+        shape = [int(v) for v in self.out_shape_tensor.shape]
+        key = lambda c: ((c[:, 0].long() * shape[2] + c[:, 1]) * shape[3] + c[:, 2]) * shape[4] + c[:, 3]
+        order = torch.argsort(key(by_touch))
+        if not torch.equal(key(by_touch)[order], key(by_cell)):
+            raise RuntimeError("the voxel set overflowed its buffer: its rulebook would keep other voxels")
+        ids = torch.empty_like(order)
+        ids[order] = torch.arange(len(order), device=order.device)
+        live = index[1] >= 0
+        index[1, live] = ids[index[1, live].long()].int()
 
     @property
     def index(self):
@@ -433,8 +447,7 @@ class SparseNet:
 
     def begin(self):
         """Optional, ahead of `forward` and of whatever makes its input: clears the grids of the rulebooks on the side
-        streams, which does not depend on the voxels and so runs beside the encoder (cylinder 10, centerpoint 50 us of
-        kernels).  `forward` clears them itself otherwise."""
+        streams, which does not depend on the voxels and so runs beside the encoder.  `forward` clears them itself otherwise."""
         if not self.overlap_rulebooks:
             return
         main = torch.cuda.current_stream(self.device)
@@ -444,18 +457,21 @@ class SparseNet:
         for rb in self.rulebooks.values():
             if rb.direct:
                 with torch.cuda.stream(self.side):
+                    table = None if self._voxel_grid(rb.in_set) else rb.raw_fwd if rb.regroup else rb.table_fwd
                     rb.plugin.tables_clear(*_shapes_of(self.sets[rb.in_set]), rb.shape_tensor, device=self.device,
-                                           table=rb.raw_fwd if rb.regroup else rb.table_fwd)
-            elif rb.group is not None and rb.group not in seen and not self._made_on_grid(rb.in_set):
+                                           table=table)
+            elif rb.group is not None and rb.group not in seen and not self._voxel_grid(rb.in_set):
                 seen.add(rb.group)
                 with torch.cuda.stream(self.side_subm):
                     rb.group.clear(self.sets[rb.in_set], rb.shape_tensor, self.device)
         self._cleared = True
 
-    def _made_on_grid(self, name):
-        """Whether the strided pass that makes voxel set `name` leaves the grid of its voxels behind."""
+    def _voxel_grid(self, name):
+        """The look-up that the strided pass which makes voxel set `name` leaves behind, if it does."""
         maker = self.rulebooks.get(name)
-        return maker is not None and maker.direct
+        if maker is None or not maker.direct:
+            return None
+        return maker.plugin.tables_grid(*_shapes_of(self.sets[maker.in_set]), maker.shape_tensor, device=self.device)
 
     def _build_rulebook(self, rb):
         """Whatever the layers of `rb` read; for a group of submanifold rulebooks, the tables of all of them."""
@@ -466,11 +482,8 @@ class SparseNet:
             rb.plugin.enqueue(src["coors"], src["num"], rb.shape_tensor, outputs=outs)
             return
         if rb.group is not None:
-            grid = None
-            if self._made_on_grid(rb.in_set):
-                maker = self.rulebooks[rb.in_set]
-                grid = maker.plugin.tables_grid(*_shapes_of(self.sets[maker.in_set]), maker.shape_tensor)
-            rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor, voxel_grid=grid, cleared=self._cleared)
+            rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor, voxel_grid=self._voxel_grid(rb.in_set),
+                             cleared=self._cleared)
             for other in self.rulebooks.values():
                 if other.group is rb.group and other.regroup:
                     SPConvMMPlugin.regroup(other.kvol, dst["cap"], other.raw_fwd, other.table_fwd, other.scratch_fwd)
@@ -479,7 +492,8 @@ class SparseNet:
         plain_inv = rb.raw_inv if rb.regroup else rb.table_inv
         if rb.direct:
             rb.plugin.tables(src["coors"], src["num"], rb.shape_tensor, out_coors=dst["coors"],
-                             num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv, cleared=self._cleared)
+                             num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv,
+                             voxel_grid=self._voxel_grid(rb.in_set), cleared=self._cleared)
         else:  # kernels or grids the direct builders do not take
             first = rb.calls == 0
             rb.calls += 1

@@ -920,6 +920,7 @@ __global__ void fill_padding_kernel(const int32_t* __restrict__ seg, int kvol, i
 }  // namespace d3d
 
 #include "spconv_index3.cuh"
+#include "spconv_rank3.cuh"
 
 namespace d3d {
 namespace {
@@ -1095,17 +1096,13 @@ int64_t clear_grid(const ClearArgs& a) {
   return stream_grid(words / 16, 256);  // four 16-byte stores per thread
 }
 
-// How much of a pass's lookup is there already: nothing, the cleared memory, or the finished grid.
-enum Ready { kNothing, kCleared, kFinished };
-
 // Lookup structure of the inputs, then their neighbours.
-int launch_subm3(const Plan& plan, Ready ready, const int32_t* coors, const int32_t* num_act_in, bool chained,
+int launch_subm3(const Plan& plan, bool cleared, const int32_t* coors, const int32_t* num_act_in, bool chained,
                  const PairLists& lists, const Targets& targets, int32_t* status, cudaStream_t st) {
   const ClearArgs a = clear_args(plan);
-  if (ready == kNothing) D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
-  if (ready != kFinished)
-    D3D_LAUNCH3(chained, subm_mark3_kernel, plan.nblk, kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g,
-                status);
+  if (!cleared) D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  D3D_LAUNCH3(chained, subm_mark3_kernel, plan.nblk, kIdxThreads, st, a.look, coors, num_act_in, plan.n_max, plan.g,
+              status);
   // one block per 256 rows up to the end of the tables, so that rows beyond the live count get their masks
   const int64_t blocks = targets.count ? std::max<int64_t>(plan.nblk, ceil_div(targets.tiles * 128, kIdxThreads))
                                        : plan.nblk;
@@ -1114,9 +1111,28 @@ int launch_subm3(const Plan& plan, Ready ready, const int32_t* coors, const int3
   return D3D_OK;
 }
 
-// The grid of a strided pass and what its forward table needs cleared: nothing here depends on the voxels.
-int clear_conv3(const Plan& plan, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
-  ClearArgs a = clear_args(plan);
+int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_in, int32_t max_out, bool chained,
+                 const PairLists& lists, int32_t* out_coors, int32_t* num_act_out, int32_t* status, cudaStream_t st) {
+  const ClearArgs a = clear_args(plan);
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, num_act_in, plan.n_max);
+  const bool two = plan.two_taps;
+  D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
+  D3D_LAUNCH3(chained, two ? conv_count3_kernel<2> : conv_count3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
+              num_act_in, plan.n_max, plan.g, plan.win_bits, plan.winners);
+  D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
+              coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, out_coors, num_act_out, status);
+  D3D_LAUNCH3(chained, two ? conv_find3_kernel<2> : conv_find3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
+              num_act_in, plan.n_max, plan.g, lists);
+  return D3D_OK;
+}
+
+// Strided tables by ranks (spconv_rank3.cuh), in the memory of the grid; launched plainly, beside other streams' work.
+uint2* rank_words(const Plan& plan) { return reinterpret_cast<uint2*>(plan.grid); }
+int64_t rank_count(const Plan& plan) { return ((plan.cells + 31) / 32 + 3) / 4 * 4; }
+// `fwd`: the forward table will be scattered into; nothing here depends on the voxels.
+int clear_rank3(const Plan& plan, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
+  ClearArgs a = {};
+  a.look.bits = reinterpret_cast<uint32_t*>(plan.grid), a.bit_words = 2 * rank_count(plan);
   if (fwd) {
     a.rows = fwd->row_masks, a.row_words = fwd->tiles * plan.g.kvol * 4;
     a.perm = fwd->perm, a.perm_words = fwd->tiles * 128, a.m_max = fwd_rows;
@@ -1124,24 +1140,10 @@ int clear_conv3(const Plan& plan, const TableParts* fwd, int64_t fwd_rows, cudaS
   D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, (const int32_t*)nullptr, plan.n_max);
   return D3D_OK;
 }
-
-int launch_conv3(const Plan& plan, Ready ready, const int32_t* coors, const int32_t* num_act_in, int32_t max_out,
-                 bool chained, const PairLists& lists, const TableParts* fwd, int64_t fwd_rows, const Targets& inverse,
-                 int32_t* out_coors, int32_t* num_act_out, int32_t* status, cudaStream_t st) {
-  if (ready == kNothing) {
-    const int rc = clear_conv3(plan, fwd, fwd_rows, st);
-    if (rc != D3D_OK) return rc;
-  }
-  const bool two = plan.two_taps;
-  D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
-  D3D_LAUNCH3(chained, two ? conv_count3_kernel<2> : conv_count3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
-              num_act_in, plan.n_max, plan.g, plan.win_bits, plan.winners);
-  D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
-              coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, out_coors, num_act_out, status);
-  const int64_t blocks = inverse.count ? std::max<int64_t>(plan.nblk, ceil_div(inverse.tiles * 128, kIdxThreads))
-                                       : plan.nblk;
-  D3D_LAUNCH3(chained, two ? conv_find3_kernel<2> : conv_find3_kernel<3>, blocks, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g,
-              lists, fwd ? fwd->ids : nullptr, fwd ? fwd->row_masks : nullptr, inverse);
+int launch_find_rank3(const RankWalk& walk, const int32_t* coors, const int32_t* num_act, int64_t n_max,
+                      const Targets& targets, cudaStream_t st) {
+  D3D_LAUNCH3(false, rank_find3_kernel, ceil_div(targets.tiles * 128, kIdxThreads), kIdxThreads, st, walk, coors, num_act,
+              n_max, targets);
   return D3D_OK;
 }
 
@@ -1271,14 +1273,13 @@ extern "C" int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, con
         targets.t[0] = make_target(nbr, g.kvol, n_max);
         mirror_slots(&targets.t[0], g.ksize, g.ksize);
       }
-      rc = launch_subm3(plan, kNothing, coors, num_act_in, chained, lists, targets, status, st);
+      rc = launch_subm3(plan, false, coors, num_act_in, chained, lists, targets, status, st);
     } else {
       int32_t* out_coors = reinterpret_cast<int32_t*>(outputs[2]);
       int32_t* num_act_out = reinterpret_cast<int32_t*>(outputs[3]);
       D3D_REQUIRE(out_coors && num_act_out, D3D_ERR_INVALID_ARGUMENT);
       D3D_REQUIRE(out[2].dims[0] >= p->max_num_act_out, D3D_ERR_INVALID_ARGUMENT);
-      rc = launch_conv3(plan, kNothing, coors, num_act_in, p->max_num_act_out, chained, lists, nullptr, 0, targets,
-                        out_coors, num_act_out, status, st);
+      rc = launch_conv3(plan, coors, num_act_in, p->max_num_act_out, chained, lists, out_coors, num_act_out, status, st);
     }
     if (rc != D3D_OK) return rc;
     D3D_LAUNCH3(chained, segment_scan_kernel, g.kvol, 1024, st, plan.block_counts, nblk, g.kvol, num_act_in, n_max,
@@ -1405,7 +1406,7 @@ extern "C" int d3d_spconv_subm_tables_clear(const d3d_tensor_desc* in, int n_in,
 
 extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables,
                                       const d3d_tensor_desc* in, int n_in, const void* const* inputs, void* workspace,
-                                      size_t workspace_bytes, void* stream, int32_t* status, const int32_t* voxel_grid,
+                                      size_t workspace_bytes, void* stream, int32_t* status, const void* voxel_grid,
                                       int cleared) {
   D3D_NVTX_RANGE("d3d_spconv_subm_tables");
   D3D_REQUIRE(n_tables >= 1 && n_tables <= kMaxTargets && kernel_size && tables && inputs, D3D_ERR_INVALID_ARGUMENT);
@@ -1425,7 +1426,6 @@ extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, 
   D3D_REQUIRE(voxel_grid || (workspace && workspace_bytes >= plan.bytes), D3D_ERR_WORKSPACE_TOO_SMALL);
   const int64_t n_max = plan.n_max;
   if (n_max == 0) return D3D_OK;
-  if (voxel_grid) plan.path = Plan::kDirect, plan.grid = const_cast<int32_t*>(voxel_grid);  // read only
   const int32_t* coors = reinterpret_cast<const int32_t*>(inputs[0]);
   const int32_t* num_act_in = reinterpret_cast<const int32_t*>(inputs[1]);
   D3D_REQUIRE(coors && num_act_in, D3D_ERR_INVALID_ARGUMENT);
@@ -1439,8 +1439,16 @@ extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, 
     targets.t[t] = make_target(tables[t], ks[0] * ks[1] * ks[2], n_max);
     mirror_slots(&targets.t[t], ks, outer);
   }
-  rc = launch_subm3(plan, voxel_grid ? kFinished : cleared ? kCleared : kNothing, coors, num_act_in, false, PairLists{},
-                    targets, status, st);
+  if (voxel_grid) {
+    RankWalk w;
+    w.grid.words = reinterpret_cast<const uint2*>(voxel_grid);
+    w.grid_count = num_act_in, w.grid_max = (int32_t)n_max;
+    for (int d = 0; d < 4; ++d) w.grid.shape[d] = plan.g.shape[d];
+    for (int d = 0; d < 3; ++d) w.mul[d] = 1, w.add[d] = outer[d] / 2, w.step[d] = -1, w.ksize[d] = outer[d];
+    rc = launch_find_rank3(w, coors, num_act_in, n_max, targets, st);
+  } else {
+    rc = launch_subm3(plan, cleared != 0, coors, num_act_in, false, PairLists{}, targets, status, st);
+  }
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
@@ -1452,8 +1460,8 @@ extern "C" int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const
   return plan.path == Plan::kDirect && plan.g.kvol <= 32;
 }
 
-extern "C" const int32_t* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in,
-                                                      int n_in, void* workspace) {
+extern "C" const void* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                                                   void* workspace) {
   Plan plan;
   if (!workspace || !d3d_spconv_conv_tables_ok(p, in, n_in) || make_plan(p, in, n_in, workspace, &plan) != D3D_OK)
     return nullptr;
@@ -1463,13 +1471,13 @@ extern "C" const int32_t* d3d_spconv_conv_tables_grid(const d3d_spconv_index_par
 extern "C" int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                             void* table, void* workspace, size_t workspace_bytes, void* stream) {
   D3D_NVTX_RANGE("d3d_spconv_conv_tables_clear");
-  D3D_REQUIRE(p && table && d3d_spconv_conv_tables_ok(p, in, n_in) && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
+  D3D_REQUIRE(p && d3d_spconv_conv_tables_ok(p, in, n_in) && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
   Plan plan;
   int rc = make_plan(p, in, n_in, workspace, &plan);
   if (rc != D3D_OK) return rc;
   D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
   const TableParts fwd = table_parts(table, plan.g.kvol, p->max_num_act_out);
-  rc = clear_conv3(plan, &fwd, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
+  rc = clear_rank3(plan, table ? &fwd : nullptr, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
@@ -1478,7 +1486,7 @@ extern "C" int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, co
 extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                       const void* const* inputs, int32_t* out_coors, int32_t* num_act_out, void* table,
                                       void* table_inverse, void* workspace, size_t workspace_bytes, void* stream,
-                                      int32_t* status, int cleared) {
+                                      int32_t* status, const void* voxel_grid, int cleared) {
   D3D_NVTX_RANGE("d3d_spconv_conv_tables");
   D3D_REQUIRE(p && inputs && out_coors && num_act_out && table, D3D_ERR_INVALID_ARGUMENT);
   Plan plan;
@@ -1498,11 +1506,51 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
     inverse.t[0] = make_target(table_inverse, kvol, plan.n_max);
     plain_slots(&inverse.t[0], plan.g);
   }
-  rc = launch_conv3(plan, cleared ? kCleared : kNothing, coors, num_act_in, p->max_num_act_out, false, PairLists{}, &fwd,
-                    p->max_num_act_out, inverse, out_coors, num_act_out, status, st);
-  if (rc != D3D_OK) return rc;
-  rc = pack_table_masks(fwd, kvol, st, false);
-  if (rc != D3D_OK) return rc;
+  const int32_t max_out = p->max_num_act_out;
+  const Geometry& g = plan.g;
+  // The forward table is filled from the outputs when the inputs have ranks: no clearing, no atomics, whole columns.
+  const bool walk_outputs = voxel_grid && !g.transpose && g.dil[2] < 16;
+  if (!cleared) {
+    rc = clear_rank3(plan, walk_outputs ? nullptr : &fwd, max_out, st);
+    if (rc != D3D_OK) return rc;
+  }
+  uint2* words = rank_words(plan);
+  const int64_t count = rank_count(plan);
+  const unsigned blocks = (unsigned)ceil_div(count, kRankWords);  // <= n_max / 16 + 1, see pick_lookup: fits win_bits
+  int32_t* block_counts = reinterpret_cast<int32_t*>(plan.win_bits);
+  const bool two = plan.two_taps;
+  D3D_LAUNCH3(false, two ? rank_mark3_kernel<2> : rank_mark3_kernel<3>, plan.nblk, kIdxThreads, st, words, coors,
+              num_act_in, plan.n_max, g);
+  D3D_LAUNCH3(false, rank_count3_kernel, blocks, kRankWords, st, words, count, block_counts);
+  D3D_LAUNCH3(false, rank_number3_kernel, blocks, kRankWords, st, words, count, block_counts, g, max_out, out_coors,
+              num_act_out, status);
+  if (walk_outputs) {
+    Targets forward = {};
+    forward.count = 1, forward.tiles = fwd.tiles;
+    forward.t[0] = make_target(table, kvol, max_out);
+    plain_slots(&forward.t[0], g);
+    RankWalk w;
+    w.grid.words = reinterpret_cast<const uint2*>(voxel_grid);
+    w.grid_count = num_act_in, w.grid_max = (int32_t)plan.n_max;
+    w.grid.shape[0] = g.shape[0];
+    for (int d = 0; d < 3; ++d) {
+      w.grid.shape[d + 1] = (int)in[2].dims[d + 2];
+      w.mul[d] = g.stride[d], w.add[d] = -g.pad[d], w.step[d] = g.dil[d], w.ksize[d] = g.ksize[d];
+    }
+    rc = launch_find_rank3(w, out_coors, num_act_out, max_out, forward, st);
+    if (rc != D3D_OK) return rc;
+  }
+  if (!walk_outputs || inverse.count) {
+    const int64_t rows = inverse.count ? std::max<int64_t>(plan.nblk, ceil_div(inverse.tiles * 128, kIdxThreads))
+                                       : plan.nblk;
+    D3D_LAUNCH3(false, two ? rank_scatter3_kernel<2> : rank_scatter3_kernel<3>, rows, kIdxThreads, st, words, num_act_out,
+                max_out, coors, num_act_in, plan.n_max, g, walk_outputs ? nullptr : fwd.ids,
+                walk_outputs ? nullptr : fwd.row_masks, inverse);
+  }
+  if (!walk_outputs) {
+    rc = pack_table_masks(fwd, kvol, st, false);
+    if (rc != D3D_OK) return rc;
+  }
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }

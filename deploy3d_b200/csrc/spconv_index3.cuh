@@ -45,20 +45,11 @@ struct PairLists {
 };
 
 struct Lookup3 {
-  int32_t* direct;             // null: bits + slots; may be the grid a strided pass has left (see id_in_cell)
+  int32_t* direct;             // null: bits + slots
   unsigned long long* slots;
   uint32_t cap_max;
   uint32_t* bits;
 };
-
-// Cells a strided pass has numbered: an output's id with the sign bit set, or kDropped beyond maxNumActOut.
-constexpr int kDropped = -2;
-constexpr int kIdBit = -2147483647 - 1;
-
-// The voxel a cell of either kind of grid (plain ids of a submanifold pass, numbered outputs of a strided one) holds; -1: none.
-__device__ __forceinline__ int id_in_cell(int cell) {
-  return (unsigned)cell >= (unsigned)kDropped ? -1 : cell & ~kIdBit;
-}
 
 // Clears what a rulebook starts from: the lookup (live part of the hash table, all of the grid or of the bit map), the
 // ticket of segment_scan_kernel, and the row masks / output map of a neighbour table that is filled by scattering.
@@ -176,37 +167,43 @@ __device__ __forceinline__ void write_lists(Found& f, const Geometry& g, uint32_
   }
 }
 
-// The block's columns of the neighbour tables: ids where a neighbour exists, the ballots as row masks (so neither needs
-// initialising), offset masks per tile, and the identity output map.  A block covers two tiles of 128.
-__device__ __forceinline__ void write_targets(const Found& f, uint32_t mask, const Targets& targets, int64_t n_max) {
-  const int64_t tile0 = (int64_t)blockIdx.x * (kIdxThreads / 128);
-  const int t_local = threadIdx.x >> 7, row = threadIdx.x & 127;
-  const int64_t tile = tile0 + t_local, pos = tile * 128 + row;
-  const bool mine = tile < targets.tiles;
+// The block's part of the neighbour tables but for the ids: the ballots as row masks, offset masks per tile, and the
+// identity output map.  A block covers two tiles of 128.
+__device__ __forceinline__ void write_target_masks(const uint32_t (&hits)[kTaps3][kBlockWarps], const Targets& targets,
+                                                   int64_t n_max) {
+  const int64_t tile0 = (int64_t)blockIdx.x * (kIdxThreads / 128), pos = tile0 * 128 + threadIdx.x;
   const int tiles_here = (int)min((int64_t)(kIdxThreads / 128), targets.tiles - tile0);
   for (int q = 0; q < targets.count; ++q) {
     const TableTarget& t = targets.t[q];
-    if (mine) {
-      t.perm[pos] = pos < n_max ? (int32_t)pos : -1;
-      int32_t* col = t.ids + tile * t.kvol * 128 + row;
-#pragma unroll
-      for (int g = 0; g < kTaps3; ++g)
-        if (((mask >> g) & 1u) && t.slot_of_g[g] >= 0) col[t.slot_of_g[g] * 128] = f.values[g][threadIdx.x];
-    }
+    if ((int)threadIdx.x < tiles_here * 128) t.perm[pos] = pos < n_max ? (int32_t)pos : -1;
     // rows[tile][slot][4]: consecutive words across the block's tiles
     uint32_t* rows = t.rows + tile0 * t.kvol * 4;
     for (int w = threadIdx.x; w < tiles_here * t.kvol * 4; w += kIdxThreads) {
       const int tl = w / (t.kvol * 4), s = w / 4 % t.kvol, quarter = w & 3;
-      rows[w] = f.hits[t.g_of_slot[s]][tl * 4 + quarter];
+      rows[w] = hits[t.g_of_slot[s]][tl * 4 + quarter];
     }
     if ((int)threadIdx.x < tiles_here) {
       uint32_t any = 0u;
       for (int s = 0; s < t.kvol; ++s) {
-        const uint32_t* h = &f.hits[t.g_of_slot[s]][threadIdx.x * 4];
+        const uint32_t* h = &hits[t.g_of_slot[s]][threadIdx.x * 4];
         if (h[0] | h[1] | h[2] | h[3]) any |= 1u << s;
       }
       t.mask[tile0 + threadIdx.x] = any;
     }
+  }
+}
+
+// The ids of a submanifold pass's block in its columns, where a neighbour exists (nothing needs initialising).
+__device__ __forceinline__ void write_targets(const Found& f, uint32_t mask, const Targets& targets, int64_t n_max) {
+  write_target_masks(f.hits, targets, n_max);
+  const int64_t pos = (int64_t)blockIdx.x * kIdxThreads + threadIdx.x, tile = pos >> 7;
+  if (tile >= targets.tiles) return;
+  for (int q = 0; q < targets.count; ++q) {
+    const TableTarget& t = targets.t[q];
+    int32_t* col = t.ids + tile * t.kvol * 128 + (pos & 127);
+#pragma unroll
+    for (int g = 0; g < kTaps3; ++g)
+      if (((mask >> g) & 1u) && t.slot_of_g[g] >= 0) col[t.slot_of_g[g] * 128] = f.values[g][threadIdx.x];
   }
 }
 
@@ -225,9 +222,7 @@ __device__ __forceinline__ void write_empty_targets(const Targets& targets, int6
 }
 
 // Submanifold neighbours: the voxel at coor + pad - tap * dilation for every tap (trt/spconv/index.cu:48-84), one thread
-// per voxel.  kDirect: 27 independent loads from the grid -- the one subm_mark3_kernel has filled, or the one the strided
-// pass that made these voxels has left: then nothing is cleared or marked (level 2 of a detector, 463 k voxels: 25 us of
-// kernels less).  Otherwise nine words of the bit map (one per (z, y) row; a
+// per voxel.  kDirect: 27 independent loads from the grid.  Otherwise nine words of the bit map (one per (z, y) row; a
 // second one where the taps straddle a word), then the hash slots of the hits, four in flight.
 // lists.value == null: no rulebook is wanted, only the tables.
 template <bool kDirect>
@@ -259,7 +254,7 @@ subm_find3_kernel(const Lookup3 look, const int32_t* __restrict__ coors, const i
       const bool ok = batch_ok && a < g.ksize[0] && b < g.ksize[1] && t < g.ksize[2] &&
                       (uint32_t)(b0 - a * g.dil[0]) < s1 && (uint32_t)(b1 - b * g.dil[1]) < s2 &&
                       (uint32_t)(b2 - t * g.dil[2]) < s3;
-      v[q] = ok ? id_in_cell(__ldg(look.direct + (key0 - a * step0 - b * step1 - t * step2))) : -1;
+      v[q] = ok ? __ldg(look.direct + (key0 - a * step0 - b * step1 - t * step2)) : -1;
     }
 #pragma unroll
     for (int q = 0; q < kTaps3; ++q) {
@@ -440,6 +435,10 @@ conv_mark3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors,
   }
 }
 
+// Cells after numbering: an output's id with the sign bit set, or kDropped beyond maxNumActOut.
+constexpr int kDropped = -2;
+constexpr int kIdBit = -2147483647 - 1;
+
 // The pair whose id is left in a cell numbers that output: in pair order, i.e. by first touch (index.cu:104-121).  First
 // the winning combinations of every input and their number per block, then the numbers themselves.
 template <int kTaps>
@@ -518,22 +517,16 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
   }
 }
 
-// The pairs of the numbered outputs: lists for the rulebook, and / or the neighbour tables themselves -- `fwd` (outputs
-// gather from inputs) by scattering ids and row-mask bits, `inverse` (inputs gather from outputs) in columns like a
-// submanifold table.
+// The pairs of the numbered outputs as lists for the rulebook.
 template <int kTaps>
 __global__ void __launch_bounds__(kIdxThreads)
 conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
-                  int64_t n_max, const Geometry g, const PairLists lists, int32_t* __restrict__ fwd_ids,
-                  uint32_t* __restrict__ fwd_rows, const Targets inverse) {
+                  int64_t n_max, const Geometry g, const PairLists lists) {
   __shared__ Found f;
   pdl_release();
   pdl_wait();
   const int n = live_count(num_act_in, n_max);
-  if ((int64_t)blockIdx.x * kIdxThreads >= n) {
-    write_empty_targets(inverse, n_max);
-    return;
-  }
+  if ((int64_t)blockIdx.x * kIdxThreads >= n) return;
   const int i = blockIdx.x * kIdxThreads + threadIdx.x;
   int4 c = make_int4(-1, 0, 0, 0);
   if (i < n) c = __ldg(reinterpret_cast<const int4*>(coors) + i);
@@ -545,17 +538,6 @@ conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ 
     const Combo<kTaps> r = combo(t, e);
     id[e] = r.ok ? __ldg(grid + cell_of(g, r, c.x)) : kDropped;
   }
-  if (fwd_ids) {
-#pragma unroll
-    for (int e = 0; e < kCombos; ++e) {
-      if (id[e] == kDropped) continue;
-      const int o = id[e] & ~kIdBit;
-      const int64_t blk = (int64_t)(o >> 7) * g.kvol + offset_of(g, combo(t, e));
-      fwd_ids[blk * 128 + (o & 127)] = i;
-      atomicOr(fwd_rows + blk * 4 + ((o & 127) >> 5), 1u << (o & 31));
-    }
-  }
-  if (!lists.value && inverse.count == 0) return;
   uint32_t mask = 0u;
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
@@ -566,8 +548,7 @@ conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ 
     f.values[q][threadIdx.x] = id[e] & ~kIdBit;
   }
   publish_hits(f, mask);
-  write_targets(f, mask, inverse, n_max);
-  if (lists.value) write_lists(f, g, mask, lists);
+  write_lists(f, g, mask, lists);
 }
 
 }  // namespace

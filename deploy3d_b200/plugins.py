@@ -147,24 +147,26 @@ class SPConvIdxPlugin(_Plugin):
 
     def tables_clear(self, *inputs, table, device, stream=None):
         """The part of `tables` that does not depend on the voxels, ahead of them (d3d_spconv_conv_tables_clear); `inputs`
-        give shapes only."""
+        give shapes only.  `table`: None when the build will be given a voxel_grid."""
         d = [_desc_of(t) for t in inputs]
         nbytes = self.workspace_size(d)
         ws = self._get_workspace(nbytes, device)
         with torch.cuda.device(device):
             check("d3d_spconv_conv_tables_clear", lib().d3d_spconv_conv_tables_clear(
-                ctypes.byref(self.p), desc_array(d), len(d), table.data_ptr(), ws.data_ptr(), nbytes,
-                _stream_ptr(stream)))
+                ctypes.byref(self.p), desc_array(d), len(d), table.data_ptr() if table is not None else None,
+                ws.data_ptr(), nbytes, _stream_ptr(stream)))
 
-    def tables_grid(self, *inputs):
-        """Address of the grid of numbered outputs the last `tables` over such inputs has left in this plugin's workspace."""
+    def tables_grid(self, *inputs, device):
+        """Address of the look-up of its outputs the last `tables` over such inputs has left in this plugin's workspace."""
         d = [_desc_of(t) for t in inputs]
-        return lib().d3d_spconv_conv_tables_grid(ctypes.byref(self.p), desc_array(d), len(d), self._workspace.data_ptr())
+        ws = self._get_workspace(self.workspace_size(d), torch.device(device))
+        return lib().d3d_spconv_conv_tables_grid(ctypes.byref(self.p), desc_array(d), len(d), ws.data_ptr())
 
     def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None,
-               cleared=False):
-        """Output voxels and neighbour tables of a strided kernel straight from the coordinates, no `index`
-        (d3d_spconv_conv_tables); `cleared`: tables_clear was called for this build."""
+               voxel_grid=None, cleared=False):
+        """Output voxels, in the order of their cells, and neighbour tables of a strided kernel straight from the
+        coordinates, no `index` (d3d_spconv_conv_tables).  `voxel_grid`: tables_grid of the strided kernel that made the
+        inputs; `cleared`: tables_clear was called for this build."""
         device = inputs[0].device
         d = [_desc_of(t) for t in inputs]
         nbytes = self.workspace_size(d)
@@ -174,7 +176,8 @@ class SPConvIdxPlugin(_Plugin):
                 ctypes.byref(self.p), desc_array(d), len(d), ptr_array([t.data_ptr() for t in inputs]),
                 out_coors.data_ptr(), num_act_out.data_ptr(), table.data_ptr(),
                 table_inverse.data_ptr() if table_inverse is not None else None, ws.data_ptr(), nbytes,
-                _stream_ptr(stream), status.data_ptr() if status is not None else None, int(bool(cleared))))
+                _stream_ptr(stream), status.data_ptr() if status is not None else None, voxel_grid,
+                int(bool(cleared))))
 
 
 def activation(x, residual=None, relu=1, stream=None):

@@ -162,31 +162,33 @@ int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, const d3d_tens
  *      extents of 1 or 3, stride and dilation 1, padding (k - 1) / 2; tables[t] holds d3d_spconv_mm_table_bytes(kVol_t,
  *      maxNumActIn) bytes.  in / inputs as SPConvIdx3d (coordinates without duplicates, count, shape carrier).
  *  d3d_spconv_conv_tables  one strided or transposed 3-D kernel of at most three taps per axis (p->subm == 0): writes
- *      the output coordinates and their number (SPConvIdx's outputs 2 and 3) and `table` (over the outputs); when
- *      non-null, also `table_inverse` (over the inputs, for the inverse convolution).
+ *      the output coordinates, in the order of their cells, and their number (SPConvIdx's outputs 2 and 3 number the same
+ *      voxels by first touch) and `table` (over the outputs); when non-null, also `table_inverse` (over the inputs, for
+ *      the inverse convolution).
  *  d3d_spconv_conv_tables_ok  1 when d3d_spconv_conv_tables accepts this kernel and grid; otherwise build the rulebook
  *      and use d3d_spconv_mm_prepare.
  *  Ahead of the voxels: the _clear calls do the part that does not depend on them (on any stream ordered before the
  *      build, e.g. beside the voxel encoder); the build is then told so with `cleared` = 1, once per clear.
- *  d3d_spconv_conv_tables_grid  where in its workspace a strided pass leaves the grid of its numbered outputs.  Given as
- *      `voxel_grid` (else NULL) to d3d_spconv_subm_tables over those outputs, nothing is cleared or inserted again; the
- *      workspace must stay as that pass left it until then, and d3d_spconv_subm_tables needs none of its own.
+ *      d3d_spconv_conv_tables_clear wants `table` unless the build will be given a voxel_grid, and NULL then.
+ *  d3d_spconv_conv_tables_grid  where in its workspace a strided pass leaves the look-up of its outputs.  Given as
+ *      `voxel_grid` (else NULL) to the passes over those voxels they are not inserted again; that workspace must stay
+ *      as it was left until then, and d3d_spconv_subm_tables needs none of its own.
  * Workspace: d3d_spconv_subm_tables_workspace; for conv_tables, d3d_spconv_index_workspace. */
 int d3d_spconv_subm_tables_workspace(const d3d_tensor_desc* in, int n_in, size_t* bytes);
 int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables, const d3d_tensor_desc* in,
                            int n_in, const void* const* inputs, void* workspace, size_t workspace_bytes, void* stream,
-                           int32_t* status, const int32_t* voxel_grid, int cleared);
+                           int32_t* status, const void* voxel_grid, int cleared);
 int d3d_spconv_subm_tables_clear(const d3d_tensor_desc* in, int n_in, void* workspace, size_t workspace_bytes,
                                  void* stream);
 int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in);
-const int32_t* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
-                                           void* workspace);
+const void* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                                        void* workspace);
 int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* table,
                                  void* workspace, size_t workspace_bytes, void* stream);
 int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                            const void* const* inputs, int32_t* out_coors, int32_t* num_act_out, void* table,
                            void* table_inverse, void* workspace, size_t workspace_bytes, void* stream,
-                           int32_t* status, int cleared);
+                           int32_t* status, const void* voxel_grid, int cleared);
 
 /* ---------------------------------------------------------------------------------------------
  * SPConvMM -- gather / GEMM / scatter over the rulebook.

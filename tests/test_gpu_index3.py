@@ -107,31 +107,107 @@ def test_subm_tables_of_several_kernels(d3d, grid, n):
             assert_table_consistent(*got)
 
 
-@pytest.mark.parametrize("ks,st,pd,dil,tr", CONVS)
-@pytest.mark.parametrize("n,room", [(1, 1.0), (700, 1.3), (700, 0.4)])
-def test_conv_tables(d3d, orc, ks, st, pd, dil, tr, n, room):
-    from deploy3d_b200.plugins import SPConvMMPlugin, deserialize_plugin
-    shape, cap, kvol = [1, 13, 24, 25], 750, int(np.prod(ks))
-    coors = np.zeros((cap, 4), np.int32)
-    coors[:n] = unique_coors(rng(n), n, shape)
-    m = orc.rulebook_conv(coors[:n], shape, ks, st, pd, dil, ZERO, tr, 10 ** 7, max_num_act_in=n)[3]
-    max_out = max(1, int(m * room))
-    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
-    shp = torch.empty([1, 0] + shape[1:], dtype=torch.int32, device=DEV)
-    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, dil, ZERO, max_out, False, tr))
-    assert plug.tables_ok(coors_t, num, shp)
+def _conv_tables_expected(d3d, coors, num, shp, out_shape, params, max_out):
+    """Output voxels in cell order and the (output, offset, input) triples of a strided kernel, from its rulebook: of more
+    than max_out outputs the first are kept."""
+    index, num_index, oc, on, _ = d3d.spconv_index(coors, num, shp, *params[:4], ZERO, 200000, False, params[4])
+    m, o = int(on.item()), [int(v) for v in out_shape]
+    oc = oc[:m].long()
+    key = ((oc[:, 0] * o[1] + oc[:, 1]) * o[2] + oc[:, 2]) * o[3] + oc[:, 3]
+    order = torch.argsort(key)
+    ids = torch.empty_like(order)
+    ids[order] = torch.arange(m, device=DEV)
+    pairs = index[:, :int(num_index.item())].long()
+    pairs = pairs[:, pairs[2] >= 0]
+    trip = torch.stack([ids[pairs[1]], pairs[2], pairs[0]], 1)
+    return m, oc[order][:max_out].int(), trip[trip[:, 0] < max_out]
+
+
+def _sorted(trip):
+    return trip[torch.argsort((trip[:, 0] * 64 + trip[:, 1]) * (1 << 32) + trip[:, 2])]
+
+
+def _conv_tables(d3d, plug, coors, num, shp, max_out, kvol, **how):
+    from deploy3d_b200.plugins import SPConvMMPlugin
+    cap = coors.shape[0]
     fwd = torch.full((SPConvMMPlugin.table_bytes(kvol, max_out),), 55, dtype=torch.uint8, device=DEV)
     inv = torch.full((SPConvMMPlugin.table_bytes(kvol, cap),), 55, dtype=torch.uint8, device=DEV)
     oc, on = torch.zeros((max_out, 4), dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
-    for _ in range(2):
-        plug.tables(coors_t, num, shp, out_coors=oc, num_act_out=on, table=fwd, table_inverse=inv)
-    index, num_index, woc, won, _ = plug.enqueue(coors_t, num, shp)
-    live = int(won.item())
-    assert int(on.item()) == live and torch.equal(oc[:live], woc[:live])
-    for inverse, rows, t in ((False, max_out, fwd), (True, cap, inv)):
-        want = SPConvMMPlugin.prepare(kvol, inverse, rows, index, num_index)
-        assert_tables_equal(table_parts(t, kvol, rows), table_parts(want, kvol, rows), "inverse %s" % inverse)
-        assert len(table_pairs(table_parts(t, kvol, rows))) == int((index[2, :int(num_index.item())] >= 0).sum())
+    if how.get("cleared"):
+        plug.tables_clear(coors, num, shp, table=None if how.get("voxel_grid") else fwd, device=DEV)
+    plug.tables(coors, num, shp, out_coors=oc, num_act_out=on, table=fwd, table_inverse=inv, **how)
+    return oc, on, table_parts(fwd, kvol, max_out), table_parts(inv, kvol, cap)
+
+
+def _check_conv_tables(got, want, max_out):
+    (oc, on, fwd, inv), (m, want_oc, trip) = got, want
+    live = min(m, max_out)
+    assert int(on.item()) == live and torch.equal(oc[:live], want_oc)
+    assert_table_consistent(*fwd)
+    assert_table_consistent(*inv)
+    assert torch.equal(table_pairs(fwd), _sorted(trip))
+    assert torch.equal(table_pairs(inv), _sorted(trip[:, [2, 1, 0]]))
+
+
+def _out_shape(shape, ks, st, pd, dil, tr):
+    if tr:
+        return [shape[0]] + [(e - 1) * s - 2 * p + (k - 1) * d + 1 for e, k, s, p, d in zip(shape[1:], ks, st, pd, dil)]
+    return [shape[0]] + [(e + 2 * p - d * (k - 1) - 1) // s + 1 for e, k, s, p, d in zip(shape[1:], ks, st, pd, dil)]
+
+
+def _carrier(shape):
+    return torch.empty([shape[0], 0] + list(shape[1:]), dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("ks,st,pd,dil,tr", CONVS)
+@pytest.mark.parametrize("n,room", [(1, 1.0), (700, 1.3), (700, 0.4)])
+def test_conv_tables(d3d, ks, st, pd, dil, tr, n, room):
+    from deploy3d_b200.plugins import deserialize_plugin
+    shape, cap, kvol = [1, 13, 24, 25], 750, int(np.prod(ks))
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, shape)
+    coors_t, num, shp = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape)
+    params, out = (ks, st, pd, dil, tr), _out_shape(shape, ks, st, pd, dil, tr)
+    max_out = max(1, int(_conv_tables_expected(d3d, coors_t, num, shp, out, params, 1)[0] * room))
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, dil, ZERO, max_out, False, tr))
+    assert plug.tables_ok(coors_t, num, shp)
+    want = _conv_tables_expected(d3d, coors_t, num, shp, out, params, max_out)
+    for cleared in (False, True):
+        _check_conv_tables(_conv_tables(d3d, plug, coors_t, num, shp, max_out, kvol, cleared=cleared), want, max_out)
+        plug._workspace.fill_(1)  # nothing of the first build may be needed
+
+
+@pytest.mark.parametrize("ks,st,pd,dil,tr", CONVS)
+@pytest.mark.parametrize("n,room", [(1, 1.0), (30, 1.0), (700, 1.3), (700, 0.4)])
+def test_tables_on_the_voxels_of_a_strided_pass(d3d, ks, st, pd, dil, tr, n, room):
+    """A second strided kernel and submanifold kernels that look their voxels up where the first kernel has left them."""
+    from deploy3d_b200.plugins import SPConvMMPlugin, SubmTables, deserialize_plugin
+    shape, cap, first = [2, 13, 24, 67], 750, ((3, 3, 3), (1, 2, 1), ONE, ONE, False)
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(n), n, shape)
+    coors_t, num, shp = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape)
+    mid = _out_shape(shape, *first)
+    mid_max = max(700, int(_conv_tables_expected(d3d, coors_t, num, shp, mid, first, 1)[0] * room))
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(*first[:4], ZERO, mid_max, False, False))
+    oc, on, _, _ = _conv_tables(d3d, plug, coors_t, num, shp, mid_max, 27)
+    grid = plug.tables_grid(coors_t, num, shp, device=DEV)
+
+    kernels = [(3, 3, 3), (1, 3, 3), (3, 1, 1), (1, 1, 1)]
+    for sub in (kernels, kernels[1:3]):
+        a, b = ([torch.full((SPConvMMPlugin.table_bytes(int(np.prod(k)), mid_max),), 93, dtype=torch.uint8, device=DEV)
+                 for k in sub] for _ in range(2))
+        SubmTables(sub).enqueue(oc, on, _carrier(mid), tables=a)
+        SubmTables(sub).enqueue(oc, on, _carrier(mid), tables=b, voxel_grid=grid)
+        for k, x, y in zip(sub, a, b):
+            v = int(np.prod(k))
+            assert_tables_equal(table_parts(y, v, mid_max), table_parts(x, v, mid_max), "%s" % (k,))
+
+    params, out = (ks, st, pd, dil, tr), _out_shape(mid, ks, st, pd, dil, tr)
+    max_out = max(1, int(_conv_tables_expected(d3d, oc, on, _carrier(mid), out, params, 1)[0] * room))
+    want = _conv_tables_expected(d3d, oc, on, _carrier(mid), out, params, max_out)
+    second = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, dil, ZERO, max_out, False, tr))
+    got = _conv_tables(d3d, second, oc, on, _carrier(mid), max_out, int(np.prod(ks)), voxel_grid=grid, cleared=not tr)
+    _check_conv_tables(got, want, max_out)
 
 
 @pytest.mark.parametrize("grid", GRIDS)
@@ -150,33 +226,3 @@ def test_subm_tables_cleared_ahead(d3d, grid, n):
     p.clear(coors_t, num, shp, device=torch.device(DEV))
     p.enqueue(coors_t, num, shp, tables=[got], cleared=True)
     assert_tables_equal(table_parts(got, 27, cap), table_parts(want, 27, cap))
-
-
-@pytest.mark.parametrize("n,room", [(1, 1.0), (127, 1.0), (700, 1.3), (700, 0.4)])
-def test_subm_tables_on_the_grid_of_a_strided_pass(d3d, orc, n, room):
-    from deploy3d_b200.plugins import SPConvMMPlugin, SubmTables, deserialize_plugin
-    shape, cap, ks, st, pd = [2, 13, 24, 25], 750, (3, 3, 3), (2, 2, 2), (1, 1, 1)
-    coors = np.zeros((cap, 4), np.int32)
-    coors[:n] = unique_coors(rng(n), n, shape)
-    m = orc.rulebook_conv(coors[:n], shape, ks, st, pd, ONE, ZERO, False, 10 ** 7, max_num_act_in=n)[3]
-    max_out = max(1, int(m * room))
-    coors_t, num = _t(coors), torch.tensor([n], dtype=torch.int32, device=DEV)
-    shp = torch.empty([2, 0] + shape[1:], dtype=torch.int32, device=DEV)
-    out_shp = torch.empty([2, 0] + [(v + 2 - 3) // 2 + 1 for v in shape[1:]], dtype=torch.int32, device=DEV)
-    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, ONE, ZERO, max_out, False, False))
-    fwd = torch.zeros(SPConvMMPlugin.table_bytes(27, max_out), dtype=torch.uint8, device=DEV)
-    oc, on = torch.zeros((max_out, 4), dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
-    for cleared in (False, True):
-        if cleared:
-            plug._workspace.fill_(1)
-            fwd.fill_(7)
-            plug.tables_clear(coors_t, num, shp, table=fwd, device=torch.device(DEV))
-        plug.tables(coors_t, num, shp, out_coors=oc, num_act_out=on, table=fwd, cleared=cleared)
-        want, got = (torch.full((SPConvMMPlugin.table_bytes(27, max_out),), 93, dtype=torch.uint8, device=DEV)
-                     for _ in range(2))
-        SubmTables([ks]).enqueue(oc, on, out_shp, tables=[want])
-        SubmTables([ks]).enqueue(oc, on, out_shp, tables=[got], voxel_grid=plug.tables_grid(coors_t, num, shp))
-        assert_tables_equal(table_parts(got, 27, max_out), table_parts(want, 27, max_out))
-        index, num_index = plug.enqueue(coors_t, num, shp)[:2]
-        assert_tables_equal(table_parts(fwd, 27, max_out),
-                            table_parts(SPConvMMPlugin.prepare(27, False, max_out, index, num_index), 27, max_out))
