@@ -254,7 +254,8 @@ subm_find3_kernel(const Lookup3 look, const int32_t* __restrict__ coors, const i
       const bool ok = batch_ok && a < g.ksize[0] && b < g.ksize[1] && t < g.ksize[2] &&
                       (uint32_t)(b0 - a * g.dil[0]) < s1 && (uint32_t)(b1 - b * g.dil[1]) < s2 &&
                       (uint32_t)(b2 - t * g.dil[2]) < s3;
-      v[q] = ok ? __ldg(look.direct + (key0 - a * step0 - b * step1 - t * step2)) : -1;
+      v[q] = __ldg(look.direct + (ok ? key0 - a * step0 - b * step1 - t * step2 : 0u));  // always a load: all in flight
+      if (!ok) v[q] = -1;
     }
 #pragma unroll
     for (int q = 0; q < kTaps3; ++q) {
@@ -538,6 +539,7 @@ conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ 
     const Combo<kTaps> r = combo(t, e);
     id[e] = r.ok ? __ldg(grid + cell_of(g, r, c.x)) : kDropped;
   }
+  __syncthreads();  // the loads stay together in front of their uses (otherwise scheduled one by one: 18 -> 28 us)
   uint32_t mask = 0u;
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {

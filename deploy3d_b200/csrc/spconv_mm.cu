@@ -117,17 +117,21 @@ __global__ void table_scatter_kernel(const int32_t* __restrict__ index, int64_t 
 // replaces one per entry (5.35 M entries at 463 k voxels: 62 -> 26 us).  Whether the rulebook has that symmetry is not
 // taken on trust: the same pass adds up a 64-bit mix of every entry and of its mirror image, which are equal sums for
 // a symmetric rulebook and otherwise differ but for a chance of about 2^-64 (checks[0] and [1]; zero before the launch).
+// A block adds its sums up before it touches them: 19 k warps on the same two words took 10 us, whatever the rulebook
+// (0.85 M entries: 17 -> 9 us).
 // table_redo_kernel and the plain scatter behind it do the work over where they differ, and return at once where not.
-__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
-  x ^= x >> 32;
-  x *= 0xd6e8feb86659fd93ull;
-  x ^= x >> 32;
-  x *= 0xd6e8feb86659fd93ull;
-  x ^= x >> 32;
-  return x;
+__device__ __forceinline__ unsigned mix32(unsigned x, unsigned m) {
+  x ^= x >> 16;
+  x *= m;
+  x ^= x >> 15;
+  x *= 0x846ca68bu;
+  return x ^ x >> 16;
 }
+// Two 32-bit mixes over different odd multiples (64-bit multiplications cost four times as many instructions).
 __device__ __forceinline__ unsigned long long entry_mix(int g, int s, int k) {
-  return mix64(((unsigned long long)(unsigned)g << 32 | (unsigned)s) + (unsigned long long)(k + 1) * 0x9e3779b97f4a7c15ull);
+  const unsigned a = (unsigned)g * 0x9e3779b1u + (unsigned)s * 0x85ebca77u + (unsigned)k * 0xc2b2ae3du;
+  const unsigned b = (unsigned)g * 0x27d4eb2fu + (unsigned)s * 0x165667b1u + (unsigned)k * 0xd3a2646du;
+  return (unsigned long long)mix32(a, 0x7feb352du) << 32 | mix32(b, 0x21f0aaadu);
 }
 __global__ void __launch_bounds__(256)
 table_scatter_mirrored_kernel(const int32_t* __restrict__ index, int64_t row_len, const int32_t* __restrict__ num_index,
@@ -184,7 +188,15 @@ table_scatter_mirrored_kernel(const int32_t* __restrict__ index, int64_t row_len
     sum += __shfl_xor_sync(0xffffffffu, sum, d);
     mirrored += __shfl_xor_sync(0xffffffffu, mirrored, d);
   }
-  if (lane == 0 && (sum | mirrored)) atomicAdd(checks, sum), atomicAdd(checks + 1, mirrored);
+  __shared__ unsigned long long sums[2][8];
+  if (lane == 0) sums[0][threadIdx.x >> 5] = sum, sums[1][threadIdx.x >> 5] = mirrored;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    sum = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += sums[threadIdx.x][w];
+    if (sum) atomicAdd(checks + threadIdx.x, sum);
+  }
 }
 // The rulebook was not symmetric after all: the row masks start over.
 __global__ void table_redo_kernel(const unsigned long long* __restrict__ checks, uint32_t* __restrict__ row_masks,

@@ -199,7 +199,8 @@ rank_scatter3_kernel(const uint2* __restrict__ words, const int32_t* __restrict_
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
     const Combo<kTaps> r = combo(t, e);
-    w[e] = r.ok ? __ldg(words + (cell_of(g, r, c.x) >> 5)) : make_uint2(0u, 0u);
+    w[e] = __ldg(words + (r.ok ? cell_of(g, r, c.x) >> 5 : 0u));  // always a load: all are in flight together
+    if (!r.ok) w[e].x = 0u;
   }
   int id[kCombos];
   uint32_t mask = 0u;
