@@ -1121,8 +1121,8 @@ int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
               num_act_in, plan.n_max, plan.g, plan.win_bits, plan.winners);
   D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
               coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, out_coors, num_act_out, status);
-  D3D_LAUNCH3(chained, two ? conv_find3_kernel<2> : conv_find3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
-              num_act_in, plan.n_max, plan.g, lists);
+  D3D_LAUNCH(chained, (two ? conv_find3_kernel<2> : conv_find3_kernel<3>), plan.nblk, kIdxThreads, kFindSpare, st, plan.grid,
+             coors, num_act_in, plan.n_max, plan.g, lists);
   return D3D_OK;
 }
 

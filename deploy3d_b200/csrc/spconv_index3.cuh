@@ -518,7 +518,10 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
   }
 }
 
-// The pairs of the numbered outputs as lists for the rulebook.
+// The pairs of the numbered outputs as lists for the rulebook.  kFindSpare: shared memory asked for on top, which keeps an SM
+// from taking more than four blocks -- launched ahead of their turn they settle wherever the kernel in front has left
+// room, and a few hundred blocks then crowd on some SMs (120 k inputs: 31 us with eight to an SM, 20 with four).
+constexpr int kFindSpare = 18 * 1024;
 template <int kTaps>
 __global__ void __launch_bounds__(kIdxThreads)
 conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
@@ -537,9 +540,9 @@ conv_find3_kernel(const int32_t* __restrict__ grid, const int32_t* __restrict__ 
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
     const Combo<kTaps> r = combo(t, e);
-    id[e] = r.ok ? __ldg(grid + cell_of(g, r, c.x)) : kDropped;
+    id[e] = __ldg(grid + (r.ok ? cell_of(g, r, c.x) : 0u));  // always a load: all are in flight together
+    if (!r.ok) id[e] = kDropped;
   }
-  __syncthreads();  // the loads stay together in front of their uses (otherwise scheduled one by one: 18 -> 28 us)
   uint32_t mask = 0u;
 #pragma unroll
   for (int e = 0; e < kCombos; ++e) {
