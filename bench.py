@@ -709,9 +709,12 @@ def count_launches(pipe, kind="detection"):
         if rb.group is not None:
             if id(rb.group) not in groups:
                 groups.add(id(rb.group))
-                n += 3  # the tables of a voxel set's submanifold kernels: clear, mark, find
+                # the tables of a voxel set's submanifold kernels: find, and clear, mark where no strided pass made the set
+                n += 1 if net.ranked(rb.in_set) else 3
         elif rb.direct:
-            n += 6  # strided tables, forward and inverse: clear, mark, count, number, find, offset masks
+            # strided tables: clear, mark, count, number, and forward from ranked voxels (and inverse) one more each,
+            # otherwise both in one pass and the offset masks
+            n += 4 + (1 + (rb.table_inv is not None) if net.ranked(rb.in_set) else 2)
         else:
             # SubM: reset, insert, probe, segment scan, compact, padding fill; strided: reset, insert, count winners,
             # scan, assign, translate, segment scan, compact, padding fill

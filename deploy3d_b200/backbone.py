@@ -466,11 +466,16 @@ class SparseNet:
                     rb.group.clear(self.sets[rb.in_set], rb.shape_tensor, self.device)
         self._cleared = True
 
-    def _voxel_grid(self, name):
-        """The look-up that the strided pass which makes voxel set `name` leaves behind, if it does."""
+    def ranked(self, name):
+        """Whether voxel set `name` is made by a strided pass that leaves a look-up of its voxels behind."""
         maker = self.rulebooks.get(name)
-        if maker is None or not maker.direct:
+        return maker is not None and maker.direct
+
+    def _voxel_grid(self, name):
+        """That look-up, or None."""
+        if not self.ranked(name):
             return None
+        maker = self.rulebooks[name]
         return maker.plugin.tables_grid(*_shapes_of(self.sets[maker.in_set]), maker.shape_tensor, device=self.device)
 
     def _build_rulebook(self, rb):
