@@ -6,8 +6,10 @@
 //     words[cell / 32] = {bits, voxels in front of the word}
 // answers "is there a voxel, and which" with one 8-byte load, for all the taps of a kernel row at once.  The structure is
 // 16 times smaller than the grid of ids (11 M cells: 2.7 MB, all of it in L2), so nothing large is cleared, and since
-// neighbouring threads now work on neighbouring voxels their loads share sectors.  B200, detector frame with 463 k voxels
-// at the second level: see the numbers at the kernels.
+// neighbouring threads now work on neighbouring voxels their loads share sectors.  What bounds the passes is the latency
+// of scattered loads.  B200, detector frame, second level of 463 k voxels: submanifold look-up 65 us from the grid of ids,
+// 31 from ranks (beside convolutions); forward table of the third level 30 us by scattering, 21 from its outputs; frames
+// 1687 -> 1582 us (300 k points) and 852 -> 756 us (120 k).
 #pragma once
 
 namespace d3d {
