@@ -14,7 +14,7 @@ import torch
 
 from . import synth
 from .ops import data_s_spconv_index, data_s_spconv_mm
-from .plugins import SPConvMMPlugin, SubmTables, activation, deserialize_plugin, recon
+from .plugins import SPConvMMPlugin, SubmTables, activation, cuda_device, deserialize_plugin, recon
 
 
 class Layer:
@@ -280,7 +280,7 @@ class SparseNet:
 
     def __init__(self, layers, spatial, caps, dtype=torch.float16, device="cuda:0", seed=0, kernel=0,
                  pad_input=True, overlap_rulebooks=False, plugin_order=False, regroup=False):
-        self.layers, self.device, self.dtype = layers, torch.device(device), dtype
+        self.layers, self.device, self.dtype = layers, cuda_device(device), dtype
         # regroup: every neighbour table is rebuilt with its outputs grouped by offset mask (same results, fewer
         # (tile, offset) blocks for the convolutions to walk); never in plugin order, where a table serves one layer
         self.regroup = regroup and not plugin_order
@@ -457,10 +457,10 @@ class SparseNet:
         for rb in self.rulebooks.values():
             if rb.direct:
                 with torch.cuda.stream(self.side):
-                    table = None if self._voxel_grid(rb.in_set) else rb.raw_fwd if rb.regroup else rb.table_fwd
+                    table = None if self.ranked(rb.in_set) else rb.raw_fwd if rb.regroup else rb.table_fwd
                     rb.plugin.tables_clear(*_shapes_of(self.sets[rb.in_set]), rb.shape_tensor, device=self.device,
                                            table=table)
-            elif rb.group is not None and rb.group not in seen and not self._voxel_grid(rb.in_set):
+            elif rb.group is not None and rb.group not in seen and not self.ranked(rb.in_set):
                 seen.add(rb.group)
                 with torch.cuda.stream(self.side_subm):
                     rb.group.clear(self.sets[rb.in_set], rb.shape_tensor, self.device)

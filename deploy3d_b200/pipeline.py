@@ -9,7 +9,7 @@ import torch
 
 from . import backbone, synth
 from .ops import data_s_bev_densify, data_s_voxel_encoder
-from .plugins import MAX_LABEL_CLASSES, deserialize_plugin, gather_labels
+from .plugins import MAX_LABEL_CLASSES, cuda_device, deserialize_plugin, gather_labels
 
 
 def _roundup(v, m):
@@ -22,7 +22,7 @@ class DetectionPipeline:
     def __init__(self, kind="centerpoint", device="cuda:0", caps=None, kernel=0, n_class=10, topk=1000,
                  iou_threshold=0.2, dtype=torch.float16, n_pts=None, overlap_rulebooks=True, plugin_order=False,
                  regroup=False):
-        self.kind, self.device, self.dtype = kind, torch.device(device), dtype
+        self.kind, self.device, self.dtype = kind, cuda_device(device), dtype
         # plugin order: one stream, nodes in ONNX order through the plugin-level entry points only (see SparseNet)
         self.plugin_order = plugin_order
         if kind == "centerpoint":
@@ -193,7 +193,7 @@ class SegmentationPipeline:
                  net="cylinder3d", overlap_rulebooks=True, regroup=False):
         from .ops import data_s_gather_back, data_s_scatter_to
         frame = synth.config5_points()
-        self.device, self.dtype, self.n_pts = torch.device(device), dtype, int(n_pts)
+        self.device, self.dtype, self.n_pts = cuda_device(device), dtype, int(n_pts)
         self.c_pts = frame["points"].shape[1]
         self.spatial = frame["spatial_shape"]
         self.cylinder_config = frame["cylinder_config"]

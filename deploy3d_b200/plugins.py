@@ -35,6 +35,14 @@ def _stream_ptr(stream):
     return ctypes.c_void_p(stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream))
 
 
+def cuda_device(device):
+    """`device` with its index: a bare "cuda" is the current device, and never equal to the device of a tensor."""
+    device = torch.device(device)
+    if device.type == "cuda" and device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device())
+    return device
+
+
 class _Plugin:
     """Common enqueue plumbing: descriptors, output allocation, workspace, status check."""
     name = None
@@ -81,9 +89,18 @@ class _Plugin:
     def _get_workspace(self, nbytes, device):
         if nbytes == 0:
             return None
+        device = cuda_device(device)
         if self._workspace is None or self._workspace.numel() < nbytes or self._workspace.device != device:
             self._workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
         return self._workspace
+
+    def _filled_workspace(self, nbytes, device):
+        """The workspace an earlier call has left something in; never a new one."""
+        ws = self._workspace
+        if ws is None or ws.numel() < nbytes or ws.device != cuda_device(device):
+            raise RuntimeError("%s: no earlier call has filled a workspace of %d bytes on %s" % (self.name, nbytes,
+                                                                                               device))
+        return ws
 
     def enqueue(self, *inputs, outputs=None, stream=None):
         """Runs the plugin on the current (or given) CUDA stream and returns the tuple of output tensors."""
@@ -157,9 +174,10 @@ class SPConvIdxPlugin(_Plugin):
                 ws.data_ptr(), nbytes, _stream_ptr(stream)))
 
     def tables_grid(self, *inputs, device):
-        """Address of the look-up of its outputs the last `tables` over such inputs has left in this plugin's workspace."""
+        """Address of the look-up of its outputs the last `tables` over such inputs has left in this plugin's workspace;
+        raises when there is none."""
         d = [_desc_of(t) for t in inputs]
-        ws = self._get_workspace(self.workspace_size(d), torch.device(device))
+        ws = self._filled_workspace(self.workspace_size(d), device)
         return lib().d3d_spconv_conv_tables_grid(ctypes.byref(self.p), desc_array(d), len(d), ws.data_ptr())
 
     def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None,
@@ -170,7 +188,7 @@ class SPConvIdxPlugin(_Plugin):
         device = inputs[0].device
         d = [_desc_of(t) for t in inputs]
         nbytes = self.workspace_size(d)
-        ws = self._get_workspace(nbytes, device)
+        ws = self._filled_workspace(nbytes, device) if cleared else self._get_workspace(nbytes, device)
         with torch.cuda.device(device):
             check("d3d_spconv_conv_tables", lib().d3d_spconv_conv_tables(
                 ctypes.byref(self.p), desc_array(d), len(d), ptr_array([t.data_ptr() for t in inputs]),
@@ -225,11 +243,14 @@ class SubmTables:
         self._flat = (ctypes.c_int32 * len(flat))(*flat)
         self._workspace = None
 
-    def _get_workspace(self, d, device):
+    def _get_workspace(self, d, device, cleared=False):
         n = ctypes.c_size_t(0)
         check("d3d_spconv_subm_tables_workspace",
               lib().d3d_spconv_subm_tables_workspace(desc_array(d), len(d), ctypes.byref(n)))
+        device = cuda_device(device)
         if self._workspace is None or self._workspace.numel() < n.value or self._workspace.device != device:
+            if cleared:
+                raise RuntimeError("no earlier call has cleared a workspace of %d bytes on %s" % (n.value, device))
             self._workspace = torch.empty(n.value, dtype=torch.uint8, device=device)
         return self._workspace.data_ptr(), n.value
 
@@ -248,7 +269,7 @@ class SubmTables:
         assert len(tables) == len(self.kernel_sizes)
         device = inputs[0].device
         d = [_desc_of(t) for t in inputs]
-        workspace, nbytes = (None, 0) if voxel_grid else self._get_workspace(d, device)
+        workspace, nbytes = (None, 0) if voxel_grid else self._get_workspace(d, device, cleared)
         with torch.cuda.device(device):
             check("d3d_spconv_subm_tables", lib().d3d_spconv_subm_tables(
                 len(tables), self._flat, ptr_array([t.data_ptr() for t in tables]), desc_array(d), len(d),

@@ -1,0 +1,48 @@
+"""What the frame pipelines and networks keep between their calls, on a small detection frame."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _frame(n=4000, seed=7):
+    from deploy3d_b200 import synth
+    frame = synth.config3_points()
+    r = np.random.Generator(np.random.PCG64(seed))
+    pts = frame["points"][r.permutation(len(frame["points"]))[:n]]
+    return dict(points=np.ascontiguousarray(pts), batch=np.zeros(n, np.int32))
+
+
+def _pipe(frame, device=DEV, caps=None, **how):
+    from deploy3d_b200.pipeline import DetectionPipeline
+    n = len(frame["points"])
+    caps = caps or {"in": n, "down2": 8 * n, "down3": 8 * n, "down4": 8 * n, "out": 8 * n}
+    pipe = DetectionPipeline("second", device, n_class=1, topk=64, n_pts=n, caps=caps, **how)
+    pipe.load_frame(frame)
+    return pipe
+
+
+def _run(pipe):
+    feats, coors, num = pipe.enqueue()
+    torch.cuda.synchronize()
+    n = int(num.item())
+    return feats[:n].float(), coors[:n].clone(), pipe.net.counts(), pipe.bev.float()
+
+
+def _assert_same_frame(got, want):
+    """Features to the order of the encoder's atomic sums (fp32, rounded to fp16 in 12 layers)."""
+    assert got[2] == want[2]
+    assert torch.equal(got[1], want[1])
+    for a, b in ((got[0], want[0]), (got[3], want[3])):
+        assert (a - b).norm() <= 1e-2 * b.norm()
+
+
+def test_device_without_an_index(d3d):
+    frame = _frame()
+    want = _run(_pipe(frame))
+    assert min(want[2].values()) > 100
+    pipe = _pipe(frame, device="cuda")
+    for _ in range(2):
+        _assert_same_frame(_run(pipe), want)
