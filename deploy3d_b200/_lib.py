@@ -43,7 +43,7 @@ class SpconvIndexExtras(ctypes.Structure):
 
 class MeanEncoderExtras(ctypes.Structure):
     _fields_ = [("lp_feats", ctypes.c_void_p), ("lp_dtype", ctypes.c_int32), ("lp_channels", ctypes.c_int32),
-                ("status", ctypes.c_void_p), ("coors_event", ctypes.c_void_p)]
+                ("status", ctypes.c_void_p)]
 
 
 class SpconvMMParams(ctypes.Structure):

@@ -391,7 +391,6 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   D3D_REQUIRE(inputs && outputs && out && n_out >= 3, D3D_ERR_INVALID_ARGUMENT);
   void* lp = extras ? extras->lp_feats : nullptr;
   int32_t* status = extras ? extras->status : nullptr;
-  cudaEvent_t coors_event = extras ? reinterpret_cast<cudaEvent_t>(extras->coors_event) : nullptr;
   D3D_REQUIRE(!lp || ((extras->lp_dtype == D3D_HALF || extras->lp_dtype == D3D_BF16) &&
                       extras->lp_channels >= in[0].dims[1]),
               D3D_ERR_INVALID_ARGUMENT);
@@ -411,7 +410,6 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   if (pl.n == 0) {
     cudaMemsetAsync(num_act_out, 0, sizeof(int32_t), st);
     if (m_max > 0) cudaMemsetAsync(out_feats, 0, (size_t)m_max * pl.c * sizeof(float), st);
-    if (coors_event && cudaEventRecord(coors_event, st) != cudaSuccess) return D3D_ERR_CUDA;
     D3D_CHECK_LAUNCH();
     return D3D_OK;
   }
@@ -425,7 +423,6 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   D3D_LAUNCH(chained, number_voxels_kernel<true>, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, m_max,
              pl.dims[1], pl.dims[2], pl.dims[3], pl.owners, pts, pl.c, out_coors, pl.count, out_feats, nullptr,
              num_act_out, status);
-  if (coors_event && cudaEventRecord(coors_event, st) != cudaSuccess) return D3D_ERR_CUDA;
   if (m_max > 0) {
     D3D_LAUNCH(chained, mean_accumulate_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pts, pl.n, pl.c,
                out_feats, pl.count);

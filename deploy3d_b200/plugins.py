@@ -427,10 +427,9 @@ class SimpleMeanEncoderPlugin(_PodPlugin):
     num_outputs = 3
 
 
-    def enqueue_lp(self, *inputs, outputs, lp_feats=None, status=None, stream=None, coors_event=None):
+    def enqueue_lp(self, *inputs, outputs, lp_feats=None, status=None, stream=None):
         """enqueue that also writes the voxel means in half / bfloat16, zero-padded to lp_feats.shape[1] channels,
-        and / or reports soft failures (D3D_STATUS_* bits) in the int32 device tensor `status`.  `coors_event`, a
-        torch.cuda.Event, is recorded once the coordinates are final, in front of the means."""
+        and / or reports soft failures (D3D_STATUS_* bits) in the int32 device tensor `status`."""
         inputs = [t if t.is_contiguous() else t.contiguous() for t in inputs]
         device = inputs[0].device
         in_descs = [_desc_of(t) for t in inputs]
@@ -442,9 +441,6 @@ class SimpleMeanEncoderPlugin(_PodPlugin):
                                         int(lp_feats.shape[1]) if lp_feats is not None else 0,
                                         status.data_ptr() if status is not None else None)
         with torch.cuda.device(device):
-            if coors_event is not None:
-                coors_event.record(stream) if stream is not None else coors_event.record()  # makes the handle
-                extras.coors_event = coors_event.cuda_event
             status = lib().d3d_simple_mean_encoder_enqueue_ex(
                 ctypes.byref(self.p), desc_array(in_descs), len(in_descs), desc_array(out_descs), len(out_descs),
                 ptr_array([t.data_ptr() for t in inputs]), ptr_array([t.data_ptr() for t in outputs]),

@@ -350,7 +350,6 @@ typedef struct {
   int32_t lp_dtype;    /* D3D_HALF or D3D_BF16 */
   int32_t lp_channels; /* >= C */
   int32_t* status;     /* optional device word that receives D3D_STATUS_* bits, or NULL */
-  void* coors_event;   /* cudaEvent_t recorded as soon as coordinates and numActOut are final (the means are not), or NULL */
 } d3d_mean_encoder_extras;
 int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
                                        const d3d_tensor_desc* out, int n_out, const void* const* inputs,

@@ -32,3 +32,11 @@ def test_what_an_earlier_call_left_is_never_allocated_anew(d3d):
         plug.tables(*voxels, out_coors=voxels[0], num_act_out=voxels[1], table=voxels[0], cleared=True)
     with pytest.raises(RuntimeError, match="no earlier call"):
         SubmTables([(3, 3, 3)]).enqueue(*voxels, tables=[voxels[0]], cleared=True)
+
+
+def test_extras_of_the_mean_encoder_keep_their_size():
+    """A C caller built against the header passes these 24 bytes; reading past them would take its stack for pointers."""
+    import ctypes
+    from deploy3d_b200 import _lib
+    assert ctypes.sizeof(_lib.MeanEncoderExtras) == 24
+    assert [f[0] for f in _lib.MeanEncoderExtras._fields_] == ["lp_feats", "lp_dtype", "lp_channels", "status"]
