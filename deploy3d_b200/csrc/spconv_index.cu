@@ -1129,10 +1129,13 @@ int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
 // Strided tables by ranks (spconv_rank3.cuh), in the memory of the grid; launched plainly, beside other streams' work.
 uint2* rank_words(const Plan& plan) { return reinterpret_cast<uint2*>(plan.grid); }
 int64_t rank_count(const Plan& plan) { return ((plan.cells + 31) / 32 + 3) / 4 * 4; }
-// `fwd`: the forward table will be scattered into; nothing here depends on the voxels.
-int clear_rank3(const Plan& plan, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
+// Whether the forward table is filled from the outputs (when the inputs have ranks): no clearing, no atomics, whole columns.
+// Otherwise the inputs scatter into it, and its row masks and output map have to be clear.
+bool walks_outputs(const Geometry& g, const void* voxel_grid) { return voxel_grid && !g.transpose && g.dil[2] < 16; }
+// `words`: the ranks; `fwd`: the forward table will be scattered into.  Nothing here depends on the voxels.
+int clear_rank3(const Plan& plan, bool words, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
   ClearArgs a = {};
-  a.look.bits = reinterpret_cast<uint32_t*>(plan.grid), a.bit_words = 2 * rank_count(plan);
+  if (words) a.look.bits = reinterpret_cast<uint32_t*>(plan.grid), a.bit_words = 2 * rank_count(plan);
   if (fwd) {
     a.rows = fwd->row_masks, a.row_words = fwd->tiles * plan.g.kvol * 4;
     a.perm = fwd->perm, a.perm_words = fwd->tiles * 128, a.m_max = fwd_rows;
@@ -1477,7 +1480,7 @@ extern "C" int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, co
   if (rc != D3D_OK) return rc;
   D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
   const TableParts fwd = table_parts(table, plan.g.kvol, p->max_num_act_out);
-  rc = clear_rank3(plan, table ? &fwd : nullptr, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
+  rc = clear_rank3(plan, true, table ? &fwd : nullptr, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
@@ -1508,10 +1511,11 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
   }
   const int32_t max_out = p->max_num_act_out;
   const Geometry& g = plan.g;
-  // The forward table is filled from the outputs when the inputs have ranks: no clearing, no atomics, whole columns.
-  const bool walk_outputs = voxel_grid && !g.transpose && g.dil[2] < 16;
-  if (!cleared) {
-    rc = clear_rank3(plan, walk_outputs ? nullptr : &fwd, max_out, st);
+  const bool walk_outputs = walks_outputs(g, voxel_grid);
+  // d3d_spconv_conv_tables_clear has had no table where a voxel_grid was announced, whatever this kernel makes of it
+  const bool clear_table = !walk_outputs && (!cleared || voxel_grid);
+  if (!cleared || clear_table) {
+    rc = clear_rank3(plan, !cleared, clear_table ? &fwd : nullptr, max_out, st);
     if (rc != D3D_OK) return rc;
   }
   uint2* words = rank_words(plan);

@@ -226,3 +226,27 @@ def test_subm_tables_cleared_ahead(d3d, grid, n):
     p.clear(coors_t, num, shp, device=torch.device(DEV))
     p.enqueue(coors_t, num, shp, tables=[got], cleared=True)
     assert_tables_equal(table_parts(got, 27, cap), table_parts(want, 27, cap))
+
+
+@pytest.mark.parametrize("ks,st,pd,dil,tr", [((2, 2, 2), (2, 2, 2), ZERO, ONE, True), ((3, 3, 3), (3, 2, 1), ONE, ONE, True),
+                                             ((3, 3, 3), ONE, (1, 1, 16), (1, 1, 16), False)])
+def test_conv_tables_cleared_for_a_voxel_grid_they_cannot_walk(d3d, ks, st, pd, dil, tr):
+    """Transposed and widely dilated kernels scatter into the forward table although a voxel grid is given: a clear that
+    was made without the table, as it is for a voxel grid, is enough all the same."""
+    from deploy3d_b200.plugins import deserialize_plugin
+    shape, first, n = [2, 13, 24, 67], ((3, 3, 3), (1, 2, 1), ONE, ONE, False), 700
+    coors_t, num, shp = _t(unique_coors(rng(n), n, shape)), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape)
+    mid = _out_shape(shape, *first)
+    mid_max = _conv_tables_expected(d3d, coors_t, num, shp, mid, first, 1)[0]
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(*first[:4], ZERO, mid_max, False, False))
+    oc, on, _, _ = _conv_tables(d3d, plug, coors_t, num, shp, mid_max, 27)
+    grid = plug.tables_grid(coors_t, num, shp, device=DEV)
+    params, out = (ks, st, pd, dil, tr), _out_shape(mid, ks, st, pd, dil, tr)
+    max_out = _conv_tables_expected(d3d, oc, on, _carrier(mid), out, params, 1)[0]
+    want = _conv_tables_expected(d3d, oc, on, _carrier(mid), out, params, max_out)
+    second = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(ks, st, pd, dil, ZERO, max_out, False, tr))
+    assert second.tables_ok(oc, on, _carrier(mid))
+    for cleared in (False, True):
+        got = _conv_tables(d3d, second, oc, on, _carrier(mid), max_out, int(np.prod(ks)), voxel_grid=grid, cleared=cleared)
+        _check_conv_tables(got, want, max_out)
+        second._workspace.fill_(1)
