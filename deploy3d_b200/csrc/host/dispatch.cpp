@@ -159,12 +159,14 @@ bool stream_of(PyObject* obj, c10::Device device, void** out) {
 namespace {
 
 // enqueue(plugin, params address, params size (0: an opaque handle), number of outputs, inputs, outputs | None,
-//         stream | None) -> tuple of the output tensors
+//         stream | None, keep the workspace) -> tuple of the output tensors
+// The workspace is the plugin's `_workspace`, replaced when it is too small.  With keep = False the call takes one of its
+// own and never looks at that attribute: calls of one plugin from several threads or streams then share nothing.
 PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Call* c = reinterpret_cast<Call*>(self);
-  if (nargs != 7) {
-    PyErr_SetString(PyExc_TypeError, "enqueue takes seven arguments");
+  if (nargs != 8) {
+    PyErr_SetString(PyExc_TypeError, "enqueue takes eight arguments");
     return nullptr;
   }
   PyObject* plugin = args[0];
@@ -172,6 +174,7 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
   const size_t params_size = PyLong_AsSize_t(args[2]);
   const long n_out = PyLong_AsLong(args[3]);
   PyObject *inputs = args[4], *outputs = args[5];
+  const int keep = PyObject_IsTrue(args[7]);
   if (PyErr_Occurred()) return nullptr;
   const Py_ssize_t n_in = PyTuple_Check(inputs) ? PyTuple_GET_SIZE(inputs) : -1;
   if (n_in < 0 || n_in > kMaxTensors || n_out < 0 || n_out > kMaxTensors) {
@@ -238,7 +241,9 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
   }
   const size_t ws_bytes = s->workspace;
   at::Tensor ws;  // held until the launches are in the stream, whatever another thread does to the plugin meanwhile
-  if (ws_bytes) {
+  if (ws_bytes && !keep) {
+    ws = at::empty({(int64_t)ws_bytes}, at::TensorOptions().dtype(at::kByte).device(device));
+  } else if (ws_bytes) {
     PyObject* have = PyObject_GetAttr(plugin, g_workspace);
     if (!have) {
       Py_DECREF(result);
@@ -304,7 +309,7 @@ void call_dealloc(PyObject* self) {
 
 PyMethodDef call_methods[] = {
     {"enqueue", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_enqueue)), METH_FASTCALL,
-     "enqueue(plugin, params, params_size, n_out, inputs, outputs, stream) -> tuple of output tensors"},
+     "enqueue(plugin, params, params_size, n_out, inputs, outputs, stream, keep) -> tuple of output tensors"},
     {nullptr, nullptr, 0, nullptr}};
 PyTypeObject call_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 

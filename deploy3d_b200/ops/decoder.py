@@ -20,8 +20,7 @@ def nms3d(scores, boxes, iou_threshold=None):
         plug = _NMS[thr] = deserialize_plugin("NMS3d", b"")
         if thr is not None:
             plug.p = type(plug.p)(thr)
-    plug._workspace = None  # a mask of its own for every call: calls on several streams may overlap
-    return plug.enqueue(scores, boxes)[0]
+    return plug.enqueue(scores, boxes, keep_workspace=False)[0]
 
 
 def data_s_yolox3d_decode(stride, class_ids, topk):

@@ -102,13 +102,16 @@ class _Plugin:
                                                                                                device))
         return ws
 
-    def enqueue(self, *inputs, outputs=None, stream=None):
-        """Runs the plugin on the current (or given) CUDA stream and returns the tuple of output tensors."""
+    def enqueue(self, *inputs, outputs=None, stream=None, keep_workspace=True):
+        """Runs the plugin on the current (or given) CUDA stream and returns the tuple of output tensors.  With
+        keep_workspace=False the call has a workspace of its own, so that calls from several threads and streams may
+        overlap (give no `stream` then: the memory belongs to the current one)."""
         call = self._call
         if call is None:
             call = self._call = _host.call(self.name, self._prefix)
         address, size = self._params_address()
-        return call.enqueue(self, address, size, self._num_outputs(), inputs, outputs, stream)
+        return call.enqueue(self, address, size, self._num_outputs(), inputs, outputs, stream,
+                            keep_workspace)
 
 
 class SPConvIdxPlugin(_Plugin):

@@ -64,3 +64,21 @@ def test_refusals(d3d):
                         torch.zeros(3, dtype=torch.int32, device=DEV))
     with pytest.raises(D3DError):
         d3d.nms3d(torch.zeros((1, 4), device=DEV), torch.zeros((1, 4, 5), device=DEV))
+
+
+def test_nms_calls_share_no_mask(d3d):
+    """nms3d runs with a mask of its own: not with one that a call in another thread has just installed in the plugin
+    both use, whatever moment the threads switch at."""
+    from deploy3d_b200 import synth
+    from deploy3d_b200.ops import decoder
+    case = synth.config4_boxes(2, 300)
+    scores, boxes = (torch.from_numpy(case[k]).to(DEV) for k in ("scores", "boxes"))
+    want = d3d.nms3d(scores, boxes, 0.17)
+    plug = decoder._NMS[0.17]
+    others = torch.full((1 << 20,), 77, dtype=torch.uint8, device=DEV)
+    plug.__class__ = type("Contended", (type(plug),), {"_workspace": property(lambda s: others, lambda s, v: None)})
+    try:
+        assert torch.equal(d3d.nms3d(scores, boxes, 0.17), want)
+        assert (others == 77).all()
+    finally:
+        del decoder._NMS[0.17]
