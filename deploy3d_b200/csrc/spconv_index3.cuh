@@ -415,6 +415,20 @@ template <int kTaps> __device__ __forceinline__ int offset_of(const Geometry& g,
   return (r.tap[0] * g.ksize[1] + r.tap[1]) * g.ksize[2] + r.tap[2];
 }
 
+// Row `id` of the output coordinates: one store where the rows start on 16 bytes (`rows16`), else four -- the buffer is the
+// caller's, maybe a piece of an arena of words.
+__device__ __forceinline__ bool rows_on_16_bytes(const int32_t* out_coors) {
+  return (reinterpret_cast<uintptr_t>(out_coors) & 15) == 0;
+}
+__device__ __forceinline__ void store_coor(int32_t* __restrict__ out_coors, bool rows16, int64_t id, const int4& c) {
+  if (rows16) {
+    reinterpret_cast<int4*>(out_coors)[id] = c;
+  } else {
+    int32_t* row = out_coors + id * 4;
+    row[0] = c.x, row[1] = c.y, row[2] = c.z, row[3] = c.w;
+  }
+}
+
 // Every candidate pair (input i, offset k) leaves i * kvol + k in its output's cell if it is the smallest so far.
 template <int kTaps>
 __global__ void __launch_bounds__(kIdxThreads)
@@ -502,6 +516,7 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
     if (all > max_out) report_status(status, D3D_STATUS_OUTPUT_OVERFLOW);
   }
   if (!bits) return;
+  const bool rows16 = rows_on_16_bytes(out_coors);
   constexpr int kCombos = kTaps * kTaps * kTaps;
   const Taps<kTaps> t = taps_of<kTaps>(g, c, true);
 #pragma unroll
@@ -510,7 +525,7 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
     const Combo<kTaps> r = combo(t, e);
     if (id < max_out) {
       grid[cell_of(g, r, c.x)] = kIdBit | id;
-      reinterpret_cast<int4*>(out_coors)[id] = make_int4(c.x, r.x[0], r.x[1], r.x[2]);
+      store_coor(out_coors, rows16, id, make_int4(c.x, r.x[0], r.x[1], r.x[2]));
     } else {
       grid[cell_of(g, r, c.x)] = kDropped;  // the pairs of this output are dropped (index.cu:158-172)
     }

@@ -92,6 +92,7 @@ rank_number3_kernel(uint2* __restrict__ words, int64_t count, const int32_t* __r
   const uint32_t s1 = (uint32_t)g.shape[1], s2 = (uint32_t)g.shape[2], s3 = (uint32_t)g.shape[3];
   const uint32_t cell = (uint32_t)(at << 5), row = cell / s3, plane = row / s2;
   uint32_t b = plane / s1, z = plane - b * s1, y = row - plane * s2, x = cell - row * s3;
+  const bool rows16 = rows_on_16_bytes(out_coors);
   for (int seen = 0; rest && id < max_out; rest &= rest - 1u, ++id) {
     const int bit = __ffs(rest) - 1;
     x += (uint32_t)(bit - seen), seen = bit;
@@ -102,7 +103,7 @@ rank_number3_kernel(uint2* __restrict__ words, int64_t count, const int32_t* __r
         if (++z == s1) z = 0, ++b;
       }
     }
-    reinterpret_cast<int4*>(out_coors)[id] = make_int4((int)b, (int)z, (int)y, (int)x);
+    store_coor(out_coors, rows16, id, make_int4((int)b, (int)z, (int)y, (int)x));
   }
 }
 

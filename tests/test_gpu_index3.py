@@ -250,3 +250,29 @@ def test_conv_tables_cleared_for_a_voxel_grid_they_cannot_walk(d3d, ks, st, pd, 
         got = _conv_tables(d3d, second, oc, on, _carrier(mid), max_out, int(np.prod(ks)), voxel_grid=grid, cleared=cleared)
         _check_conv_tables(got, want, max_out)
         second._workspace.fill_(1)
+
+
+@pytest.mark.parametrize("words", [0, 1, 2])
+def test_output_coordinates_in_an_arena_of_words(d3d, words):
+    """Output coordinates that start on any 4 bytes, as a piece of a caller's flat buffer may."""
+    from deploy3d_b200.plugins import SPConvMMPlugin, deserialize_plugin
+    shape, n = [2, 13, 24, 25], 700
+    coors_t, num, shp = _t(unique_coors(rng(n), n, shape)), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape)
+    args = (3, 3, 3), (2, 2, 2), ONE, ONE, ZERO, 2000, False, False
+    index, num_index, want, on, carrier = d3d.spconv_index(coors_t, num, shp, *args)
+    m = int(on.item())
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(*args))
+
+    def piece():
+        flat = torch.full((4 * 2000 + 4,), -9, dtype=torch.int32, device=DEV)
+        return flat, flat[words:words + 8000].view(2000, 4)
+
+    flat, oc = piece()
+    plug.enqueue(coors_t, num, shp, outputs=[index, num_index, oc, on, carrier])
+    assert torch.equal(oc[:m], want[:m]) and (flat[:words] == -9).all() and (oc[m:] == -9).all()
+    flat, oc = piece()
+    table = torch.empty(SPConvMMPlugin.table_bytes(27, 2000), dtype=torch.uint8, device=DEV)
+    plug.tables(coors_t, num, shp, out_coors=oc, num_act_out=on, table=table)
+    key = lambda c: ((c[:, 0] * 7 + c[:, 1]) * 12 + c[:, 2]) * 13 + c[:, 3]
+    assert int(on.item()) == m and torch.equal(oc[:m], want[:m][torch.argsort(key(want[:m]))])
+    assert (flat[:words] == -9).all() and (oc[m:] == -9).all()
