@@ -205,9 +205,13 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
   }
   const Signature* s = signature(c, params, params_size, in_desc, (int)n_in, (int)n_out);
   if (!s) return nullptr;
+  // Copied before anything below can run Python code or let another thread in: a call of the same plugin with another
+  // shape may take the entry over.
+  const size_t ws_bytes = s->workspace;
   d3d_tensor_desc out_desc[kMaxTensors];
   void* out_ptr[kMaxTensors] = {};
   memcpy(out_desc, s->out.data(), n_out * sizeof(d3d_tensor_desc));
+  s = nullptr;
   PyObject* result;
   if (outputs == Py_None) {
     result = PyTuple_New(n_out);
@@ -239,7 +243,6 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
       out_ptr[i] = t.numel() ? t.data_ptr() : nullptr;
     }
   }
-  const size_t ws_bytes = s->workspace;
   at::Tensor ws;  // held until the launches are in the stream, whatever another thread does to the plugin meanwhile
   if (ws_bytes && !keep) {
     ws = at::empty({(int64_t)ws_bytes}, at::TensorOptions().dtype(at::kByte).device(device));

@@ -82,3 +82,23 @@ def test_nms_calls_share_no_mask(d3d):
         assert (others == 77).all()
     finally:
         del decoder._NMS[0.17]
+
+
+def test_other_shapes_between_the_steps_of_a_call(d3d):
+    """The caller's `outputs` may be any iterable; one that calls the same plugin with more shapes than it keeps does not
+    change what its own call runs with."""
+    from deploy3d_b200.plugins import deserialize_plugin
+    plug = deserialize_plugin("NMS3d", b"")
+    case = [torch.rand((1, 400), device=DEV).sort(descending=True)[0], torch.rand((1, 400, 7), device=DEV) + 1]
+    want = plug.enqueue(*case)[0]
+
+    class Outputs:
+        def __iter__(self):
+            for k in range(1, 10):  # nine smaller shapes, the workspace with them
+                plug.enqueue(case[0][:, :k], case[1][:, :k])
+            plug._workspace = None
+            return iter([out])
+
+    for _ in range(9):
+        out = torch.zeros_like(want)
+        assert plug.enqueue(*case, outputs=Outputs())[0] is out and torch.equal(out, want)
