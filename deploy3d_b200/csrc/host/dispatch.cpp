@@ -24,6 +24,7 @@
 #include <condition_variable>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -316,62 +317,79 @@ PyMethodDef call_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 PyTypeObject call_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// Compares two large buffers with three helper threads beside the caller: one core reads two 1.8 MB weight arrays in
-// 93 us (they come from its neighbours' caches), four in 30-40 us.  Helpers sleep between calls; a second caller that
-// finds them busy compares alone.  They are started at first use, and not in a forked child.
+// Compares two large buffers with up to three helper threads beside the caller: one core reads two 1.8 MB weight arrays in
+// 93 us (they come from its neighbours' caches), four in 30-40 us.  The buffers are dealt out in pieces and the caller takes
+// pieces too, so it waits only for helpers that are in the middle of one: a helper that is asleep, or was never started
+// because the process may have no more threads, costs nothing but its share.  Helpers sleep between calls; a second caller
+// that finds them busy compares alone.  They are started at first use, and not in a forked child.
 class Comparer {
  public:
   static constexpr int kHelpers = 3;
-  static constexpr size_t kWorthIt = 256 << 10;
+  static constexpr size_t kWorthIt = 256 << 10, kPiece = 64 << 10;
 
   bool same(const char* a, const char* b, size_t n) {
-    if (n < kWorthIt || getpid() != pid_ || !turn_.try_lock()) return memcmp(a, b, n) == 0;
+    const uint64_t pieces = (n + kPiece - 1) / kPiece;
+    if (n < kWorthIt || pieces > kPieces || getpid() != pid_ || !turn_.try_lock()) return memcmp(a, b, n) == 0;
     std::lock_guard<std::mutex> turn(turn_, std::adopt_lock);
     if (!started_) {
-      for (int i = 0; i < kHelpers; ++i) std::thread([this, i] { help(i); }).detach();
       started_ = true;
+      try {
+        for (int i = 0; i < kHelpers; ++i) std::thread([this] { help(); }).detach();
+      } catch (const std::system_error&) {  // as many as there are
+      }
     }
-    part_ = (n / (kHelpers + 1) + 63) & ~size_t(63);
+    a_ = a, b_ = b, n_ = n;
     differ_.store(false, std::memory_order_relaxed);
-    left_.store(kHelpers, std::memory_order_relaxed);
+    done_.store(0, std::memory_order_relaxed);
+    uint64_t job;
     {
       std::lock_guard<std::mutex> g(lock_);
-      a_ = a, b_ = b, n_ = n;
-      ++job_;
+      job = ++job_;
+      left_.store(job << 32 | pieces, std::memory_order_release);
     }
     wake_.notify_all();
-    const bool same = memcmp(a, b, part_) == 0;
-    while (left_.load(std::memory_order_acquire) > 0) std::this_thread::yield();
-    return same && !differ_.load(std::memory_order_relaxed);
+    work(job);
+    while (done_.load(std::memory_order_acquire) < pieces) std::this_thread::yield();  // pieces in helpers' hands
+    return !differ_.load(std::memory_order_relaxed);
   }
 
  private:
-  void help(int i) {
-    unsigned long seen = 0;
+  static constexpr uint64_t kPieces = 0xffffffffu;
+
+  // Takes pieces of `job` while there are any.  `left_` holds the job and the number of its pieces nobody has taken in one
+  // word: a helper that comes late finds another job or none left, and reads nothing else.  The buffers of a job stay as
+  // they are while one of its pieces is taken and not done.
+  void work(uint64_t job) {
+    uint64_t at = left_.load(std::memory_order_acquire);
+    while ((uint32_t)(at >> 32) == (uint32_t)job && (at & kPieces) != 0) {
+      if (!left_.compare_exchange_weak(at, at - 1, std::memory_order_acq_rel, std::memory_order_acquire)) continue;
+      const size_t from = ((at & kPieces) - 1) * kPiece, len = n_ - from < kPiece ? n_ - from : kPiece;
+      if (!differ_.load(std::memory_order_relaxed) && memcmp(a_ + from, b_ + from, len) != 0)
+        differ_.store(true, std::memory_order_relaxed);
+      done_.fetch_add(1, std::memory_order_release);
+      at = left_.load(std::memory_order_acquire);
+    }
+  }
+  void help() {
+    uint64_t seen = 0;
     for (;;) {
-      const char *a, *b;
-      size_t from, to;
       {
         std::unique_lock<std::mutex> g(lock_);
         wake_.wait(g, [&] { return job_ != seen; });
         seen = job_;
-        a = a_, b = b_;
-        from = part_ * (i + 1);
-        to = i + 1 == kHelpers ? n_ : from + part_;
       }
-      if (memcmp(a + from, b + from, to - from) != 0) differ_.store(true, std::memory_order_relaxed);
-      left_.fetch_sub(1, std::memory_order_release);
+      work(seen);
     }
   }
   const pid_t pid_ = getpid();
   std::mutex turn_, lock_;
   std::condition_variable wake_;
-  std::atomic<int> left_{0};
+  std::atomic<uint64_t> left_{0}, done_{0};
   std::atomic<bool> differ_{false};
   bool started_ = false;
-  unsigned long job_ = 0;
+  uint64_t job_ = 0;
   const char *a_ = nullptr, *b_ = nullptr;
-  size_t n_ = 0, part_ = 0;
+  size_t n_ = 0;
 };
 Comparer* comparer() {
   static Comparer* c = new Comparer();  // never destroyed: the helpers outlive the module's statics

@@ -40,3 +40,62 @@ def test_extras_of_the_mean_encoder_keep_their_size():
     from deploy3d_b200 import _lib
     assert ctypes.sizeof(_lib.MeanEncoderExtras) == 24
     assert [f[0] for f in _lib.MeanEncoderExtras._fields_] == ["lp_feats", "lp_dtype", "lp_channels", "status"]
+
+
+def _run_python(code):
+    """Runs `code` in a fresh process (threads, limits and forks of its own); its output."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, "exit %s\n%s" % (r.returncode, r.stderr[-2000:])
+    return r.stdout.split()
+
+
+def test_compare_where_no_thread_can_start(d3d):
+    """The compare of large weights does without its helpers where the process may not have another thread."""
+    assert _run_python("""
+import resource
+import numpy as np
+from deploy3d_b200 import _host
+same = _host.module().same_bytes
+a = np.random.default_rng(1).integers(0, 255, 1 << 20, dtype=np.uint8)
+b, c = a.tobytes(), a.copy()
+c[-1] ^= 1
+now = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (now + (1 << 20), resource.getrlimit(resource.RLIMIT_AS)[1]))  # no room for a stack
+print(same(a, b, 0), same(c, b, 0))
+""") == ["True", "False"]
+
+
+@pytest.mark.parametrize("busy", [False, True])
+def test_compare_finds_every_difference(d3d, busy):
+    """Sizes around the pieces the compare deals out, one byte off anywhere, by several callers at once; `busy`: on one
+    core, where helpers are rarely scheduled when they are wanted."""
+    out = _run_python("""
+import os
+import threading
+if %r:
+    os.sched_setaffinity(0, {next(iter(os.sched_getaffinity(0)))})
+import numpy as np
+from deploy3d_b200 import _host
+same = _host.module().same_bytes
+wrong = []
+def caller(seed):
+    r = np.random.default_rng(seed)
+    for n in [1, 262143, 262144, 262145, 327679, 327680, 327681, 1000003] * 10:
+        a = r.integers(0, 255, n, dtype=np.uint8)
+        b = b"head" + a.tobytes()
+        if not same(a, b, 4):
+            wrong.append(("equal", n))
+        at = int(r.choice([0, n - 1, r.integers(0, n)]))
+        a[at] ^= 1
+        if same(a, b, 4):
+            wrong.append((at, n))
+threads = [threading.Thread(target=caller, args=(s,)) for s in range(3)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+print(len(wrong), *wrong[:5])
+""" % busy)
+    assert out == ["0"]
