@@ -139,6 +139,15 @@ const Signature* signature(Call* c, const void* params, size_t params_size, cons
   return &slot;
 }
 
+// Whether a kernel can follow the tensor's address: on a GPU, in pinned host memory, or without elements (a shape).
+bool reachable(const at::Tensor& t) { return t.is_cuda() || t.numel() == 0 || (t.is_cpu() && t.is_pinned()); }
+
+int64_t volume(const d3d_tensor_desc& d) {
+  int64_t v = 1;
+  for (int i = 0; i < d.nb_dims; ++i) v *= d.dims[i];
+  return v;
+}
+
 bool stream_of(PyObject* obj, c10::Device device, void** out) {
   if (obj == Py_None) {
     *out = c10::cuda::getCurrentCUDAStream(device.index()).stream();
@@ -200,6 +209,10 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
   const c10::Device device = in[0].device();
   c10::cuda::CUDAGuard guard(device);
   for (Py_ssize_t i = 0; i < n_in; ++i) {
+    if (!reachable(in[i])) {
+      PyErr_Format(PyExc_RuntimeError, "%s: input %zd is not in CUDA memory", c->name->c_str(), i);
+      return nullptr;
+    }
     if (!in[i].is_contiguous()) in[i] = in[i].contiguous();
     if (!describe(in[i], &in_desc[i])) return nullptr;
     in_ptr[i] = in[i].numel() ? in[i].data_ptr() : nullptr;
@@ -226,7 +239,14 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
   } else {  // the caller's buffers say which of the accepted output types it wants (GatherBack can widen)
     result = PySequence_Tuple(outputs);
     if (!result) return nullptr;
-    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(result) && i < n_out; ++i) {
+    const Py_ssize_t given = PyTuple_GET_SIZE(result);
+    for (Py_ssize_t i = given; i < n_out; ++i)
+      if (volume(out_desc[i]) != 0) {
+        PyErr_Format(PyExc_ValueError, "%s: %zd of %ld outputs given", c->name->c_str(), given, n_out);
+        Py_DECREF(result);
+        return nullptr;
+      }
+    for (Py_ssize_t i = 0; i < given && i < n_out; ++i) {
       PyObject* o = PyTuple_GET_ITEM(result, i);
       if (!THPVariable_Check(o)) {
         PyErr_Format(PyExc_TypeError, "%s: output %zd is no tensor", c->name->c_str(), i);
@@ -237,6 +257,11 @@ PyObject* call_enqueue(PyObject* self, PyObject* const* args, Py_ssize_t nargs) 
       const int dt = dtype_of(t);
       if (dt < 0) {
         PyErr_Format(PyExc_KeyError, "unsupported tensor dtype %s", c10::toString(t.scalar_type()));
+        Py_DECREF(result);
+        return nullptr;
+      }
+      if (!reachable(t)) {
+        PyErr_Format(PyExc_RuntimeError, "%s: output %zd is not in CUDA memory", c->name->c_str(), i);
         Py_DECREF(result);
         return nullptr;
       }

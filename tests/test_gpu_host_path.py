@@ -102,3 +102,31 @@ def test_other_shapes_between_the_steps_of_a_call(d3d):
     for _ in range(9):
         out = torch.zeros_like(want)
         assert plug.enqueue(*case, outputs=Outputs())[0] is out and torch.equal(out, want)
+
+
+def test_missing_and_unreachable_tensors_are_refused(d3d):
+    """What would become a null or a host address in a kernel is an error; an output without elements, a shape on the host
+    and pinned memory are not."""
+    from deploy3d_b200.plugins import deserialize_plugin
+    nms = deserialize_plugin("NMS3d", b"")
+    scores, boxes = torch.rand((1, 70), device=DEV).sort(descending=True)[0], torch.rand((1, 70, 7), device=DEV) + 1
+    want, = nms.enqueue(scores, boxes)
+    with pytest.raises(ValueError, match="0 of 1 outputs"):
+        nms.enqueue(scores, boxes, outputs=[])
+    with pytest.raises(RuntimeError, match="input 1 is not in CUDA memory"):
+        nms.enqueue(scores, boxes.cpu())
+    with pytest.raises(RuntimeError, match="output 0 is not in CUDA memory"):
+        nms.enqueue(scores, boxes, outputs=[torch.zeros_like(scores, device="cpu")])
+    assert torch.equal(nms.enqueue(scores, boxes.cpu().pin_memory())[0], want)
+
+    blob = d3d.data_s_spconv_index((3, 3, 3), (2, 2, 2), (1, 1, 1), (1, 1, 1), (0, 0, 0), 50, False, False)
+    plug = deserialize_plugin("SPConvIdx3d", blob)
+    ids = torch.arange(60)
+    coors = torch.stack([0 * ids, ids // 20, ids % 20, ids % 7], 1).int().to(DEV)
+    num = torch.tensor([60], dtype=torch.int32, device=DEV)
+    want = plug.enqueue(coors, num, torch.empty((1, 0, 4, 20, 8), dtype=torch.int32, device=DEV))
+    outs = [torch.empty_like(t) for t in want[:4]]  # without the shape carrier, which has no elements
+    got = plug.enqueue(coors, num, torch.empty((1, 0, 4, 20, 8), dtype=torch.int32), outputs=outs)
+    assert len(got) == 4 and torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])
+    with pytest.raises(ValueError, match="3 of 5 outputs"):
+        plug.enqueue(coors, num, torch.empty((1, 0, 4, 20, 8), dtype=torch.int32), outputs=outs[:3])
