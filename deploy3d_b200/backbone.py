@@ -253,10 +253,10 @@ class _SubmGroup:
     def clear(self, src, shape, device):
         self._pass().clear(*_shapes_of(src), shape, device=device)
 
-    def enqueue(self, coors, num, shape, voxel_grid=None, cleared=False):
+    def enqueue(self, coors, num, shape, voxel_grid=None, cleared=False, status=None):
         p = self._pass()
         p.enqueue(coors, num, shape, tables=[self.by_ksize[k] for k in p.kernel_sizes], voxel_grid=voxel_grid,
-                  cleared=cleared)
+                  cleared=cleared, status=status)
 
 
 def _shapes_of(voxels):
@@ -272,6 +272,9 @@ class SparseNet:
     spatial     [B, Z, Y, X] of the input voxel grid
     caps        dict voxel-set name -> maximum active voxels ('in' for the input set, otherwise the key of the
                 'conv' layer that creates the set)
+    status      int32 device word that collects the D3D_STATUS_* bits of every table build (not in plugin order, where a
+                node has none): D3D_STATUS_OUTPUT_OVERFLOW says that some set had more voxels than its buffer and
+                lost the last ones in the order of their cells.  The caller reads and clears it when it likes.
     The network input is available to later layers under the tag 'input'.  A first layer with 4, 5 or 9 input
     channels runs with its input zero-padded to 16 channels (zero weight rows) and a last layer whose output
     channel count is not a multiple of 16 with zero-padded output channels, which makes both eligible for the
@@ -301,6 +304,7 @@ class SparseNet:
         weights = make_weights(layers, seed)
         self.rulebooks = {}
         self.groups = {}  # voxel set -> _SubmGroup
+        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._cleared = False
         self.tables_done = None  # event of the last forward: all tables built (overlap_rulebooks)
         self._concatenated = None  # the concatenation layer whose result is in place already
@@ -488,7 +492,7 @@ class SparseNet:
             return
         if rb.group is not None:
             rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor, voxel_grid=self._voxel_grid(rb.in_set),
-                             cleared=self._cleared)
+                             cleared=self._cleared, status=self.status)
             for other in self.rulebooks.values():
                 if other.group is rb.group and other.regroup:
                     SPConvMMPlugin.regroup(other.kvol, dst["cap"], other.raw_fwd, other.table_fwd, other.scratch_fwd)
@@ -498,7 +502,7 @@ class SparseNet:
         if rb.direct:
             rb.plugin.tables(src["coors"], src["num"], rb.shape_tensor, out_coors=dst["coors"],
                              num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv,
-                             voxel_grid=self._voxel_grid(rb.in_set), cleared=self._cleared)
+                             voxel_grid=self._voxel_grid(rb.in_set), cleared=self._cleared, status=self.status)
         else:  # kernels or grids the direct builders do not take
             first = rb.calls == 0
             rb.calls += 1
@@ -506,7 +510,8 @@ class SparseNet:
             if rb.kind != "subm":
                 outs += [dst["coors"], dst["num"], rb.out_shape_tensor]
             rb.plugin.enqueue_ex(src["coors"], src["num"], rb.shape_tensor, outputs=outs, persistent=True,
-                                 first_call=first, subm_table=plain_fwd if rb.fused_table else None)
+                                 first_call=first, subm_table=plain_fwd if rb.fused_table else None,
+                                 status=self.status)
             if not rb.fused_table:
                 SPConvMMPlugin.prepare(rb.kvol, False, dst["cap"], outs[0], outs[1], table=plain_fwd, mirror=rb.mirror)
             if plain_inv is not None:

@@ -73,6 +73,12 @@ class DetectionPipeline:
         self.graph = None
         self.side = torch.cuda.Stream(device=self.device)
 
+    @property
+    def status(self):
+        """Device word that collects what frames have lost (D3D_STATUS_* bits), 0 when every voxel had room: see
+        SparseNet.  Nothing is collected in plugin order."""
+        return self.net.status
+
     def default_caps(self):
         """Static buffer sizes (the reference fixes them per model, e.g. [131072, 65536, 32768, 16384] in
         tests/cylinder/test_cylinder3d.py:391): generous here, tightened by calibrate()."""
@@ -114,14 +120,18 @@ class DetectionPipeline:
         fork / join of the graph."""
         main = torch.cuda.current_stream(self.device)
         self.net.begin()
+        outputs = [self.vox_feats, self.vox_coors, self.vox_num]
         if self.plugin_order or self.dtype == torch.float32:
-            self.vfe.enqueue(self.points, self.batch, self.cfg, self.shape_tensor,
-                             outputs=[self.vox_feats, self.vox_coors, self.vox_num])
+            if self.plugin_order:
+                self.vfe.enqueue(self.points, self.batch, self.cfg, self.shape_tensor, outputs=outputs)
+            else:
+                self.vfe.enqueue_lp(self.points, self.batch, self.cfg, self.shape_tensor, outputs=outputs,
+                                    status=self.status)
             # fp32 -> fp16 reformat (TensorRT inserts this layer itself); padding columns stay zero
             self.vox_feats_lp[:, :self.c_pts].copy_(self.vox_feats)
         else:  # the encoder writes the half-precision, channel-padded copy itself
-            self.vfe.enqueue_lp(self.points, self.batch, self.cfg, self.shape_tensor,
-                                outputs=[self.vox_feats, self.vox_coors, self.vox_num], lp_feats=self.vox_feats_lp)
+            self.vfe.enqueue_lp(self.points, self.batch, self.cfg, self.shape_tensor, outputs=outputs,
+                                lp_feats=self.vox_feats_lp, status=self.status)
         feats, coors, num = self.net.forward(self.vox_feats_lp)
         beside = not self.plugin_order
         if beside:
@@ -228,6 +238,12 @@ class SegmentationPipeline:
             self.logits = torch.zeros((self.n_pts, n_class), dtype=torch.float32, device=dev)
             self.labels = torch.zeros(self.n_pts, dtype=torch.int32, device=dev)
         self.graph = None
+
+    @property
+    def status(self):
+        """Device word that collects the voxels the network's tables have lost: see SparseNet.  (The encoder's own set is
+        full when vox_num has reached its buffer.)"""
+        return self.net.status
 
     def load_frame(self, frame):
         self.points.copy_(torch.from_numpy(frame["points"]))

@@ -46,3 +46,21 @@ def test_device_without_an_index(d3d):
     pipe = _pipe(frame, device="cuda")
     for _ in range(2):
         _assert_same_frame(_run(pipe), want)
+
+
+@pytest.mark.parametrize("small", [None, "in", "down2", "down4"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_lost_voxels_are_reported(d3d, small, dtype):
+    """A frame whose voxels do not fit one of the buffers sets the pipeline's status word, eagerly and from the graph."""
+    frame = _frame()
+    caps = {k: v + 5 for k, v in _run(_pipe(frame))[2].items()}
+    if small:
+        caps[small] -= 6
+    pipe = _pipe(frame, caps=caps, dtype=dtype)
+    _run(pipe)
+    assert int(pipe.status.item()) == (2 if small else 0)  # D3D_STATUS_OUTPUT_OVERFLOW
+    pipe.capture()
+    pipe.status.zero_()
+    pipe.replay()
+    torch.cuda.synchronize()
+    assert int(pipe.status.item()) == (2 if small else 0)
