@@ -202,27 +202,46 @@ class _Rulebook:
 
     def _current(self):
         if self.group is not None or self.direct:
-            src = self.sets[self.in_set]
-            outs = list(self.buffers())
-            if self.kind != "subm":  # the same output voxels again, beside the live ones
-                dst = self.sets[self.out_set]
-                outs += [torch.empty_like(dst["coors"]), torch.empty_like(dst["num"]), self.out_shape_tensor]
-            self.plugin.enqueue(src["coors"], src["num"], self.shape_tensor, outputs=outs)
-            if self.kind != "subm":
-                self._renumber(outs[0], outs[2][:int(outs[3])], dst["coors"][:int(dst["num"])])
+            src, outs = self.sets[self.in_set], list(self.buffers())
+            if self.kind == "subm":
+                self.plugin.enqueue(src["coors"], src["num"], self.shape_tensor, outputs=outs)
+            else:
+                self._rulebook_of_live_tables(src, self.sets[self.out_set], *outs)
         return self.buffers()
 
-    def _renumber(self, index, by_touch, by_cell):
-        """The rulebook numbers its outputs by first touch, the live tables in the order of their cells."""
+    def _rulebook_of_live_tables(self, src, dst, index, num_index):
+        """The rulebook numbers its outputs by first touch, the live tables in the order of their cells; of a set that has
+        overflowed its buffer the tables keep the first cells.  The plugin that makes it is not the one whose workspace
+        holds the look-up of the tables, cleared or filled."""
+        live = dst["coors"][:int(dst["num"])]
         shape = [int(v) for v in self.out_shape_tensor.shape]
+        full = len(live) == dst["cap"]
+        cap = min(self.kvol * src["cap"], int(np.prod(shape[:1] + shape[2:]))) if full else dst["cap"]
+        plug = deserialize_plugin("SPConvIdx3d", data_s_spconv_index(self.ksize, self.stride, self.padding, (1, 1, 1),
+                                                                     (0, 0, 0), cap, False, False))
+        coors = torch.empty((cap, 4), dtype=torch.int32, device=index.device)
+        num = torch.empty_like(num_index)
+        plug.enqueue(src["coors"], src["num"], self.shape_tensor,
+                     outputs=[index, num_index, coors, num, self.out_shape_tensor])
         key = lambda c: ((c[:, 0].long() * shape[2] + c[:, 1]) * shape[3] + c[:, 2]) * shape[4] + c[:, 3]
-        order = torch.argsort(key(by_touch))
-        if not torch.equal(key(by_touch)[order], key(by_cell)):
-            raise RuntimeError("the voxel set overflowed its buffer: its rulebook would keep other voxels")
-        ids = torch.empty_like(order)
-        ids[order] = torch.arange(len(order), device=order.device)
-        live = index[1] >= 0
-        index[1, live] = ids[index[1, live].long()].int()
+        found, kept = key(coors[:int(num)]), key(live)
+        ids = torch.searchsorted(kept, found)
+        ids[kept[ids.clamp(max=max(len(kept) - 1, 0))] != found] = -1
+        pairs = index[:, :int(num_index)].long()
+        at = torch.nonzero(pairs[2] >= 0).view(-1)
+        to = ids[pairs[1, at]]
+        if len(found) == len(kept):
+            index[1, at] = to.int()
+            return
+        # without the pairs of voxels that were dropped: segments move up, each still from a multiple of 128 on
+        gather, offset = pairs[0, at][to >= 0], pairs[2, at][to >= 0]
+        count = torch.bincount(offset, minlength=self.kvol)
+        padded = (count + 127) // 128 * 128
+        first = (padded.cumsum(0) - padded) - (count.cumsum(0) - count)
+        at = first[offset] + torch.arange(len(offset), device=index.device)
+        index.fill_(-1)
+        index[:, at] = torch.stack([gather, to[to >= 0], offset]).int()
+        num_index.fill_(int(padded.sum()))
 
     @property
     def index(self):
@@ -332,7 +351,7 @@ class SparseNet:
                     assert L.kind != "inverse", "an inverse layer needs the rulebook of its conv"
                     rb = _Rulebook()
                     rb.sets = self.sets  # (not the net: no reference cycles, a dropped net frees its plugins at once)
-                    rb.kind, rb.in_set, rb.ksize = L.kind, cur, L.ksize
+                    rb.kind, rb.in_set, rb.ksize, rb.stride, rb.padding = L.kind, cur, L.ksize, L.stride, L.padding
                     # SubM with an odd kernel and 'same' padding: offsets k and kVol-1-k mirror each other
                     rb.mirror = (L.kind == "subm" and all(k % 2 == 1 for k in L.ksize) and
                                  tuple(L.padding) == tuple(k // 2 for k in L.ksize))

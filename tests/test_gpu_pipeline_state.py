@@ -64,3 +64,47 @@ def test_lost_voxels_are_reported(d3d, small, dtype):
     pipe.replay()
     torch.cuda.synchronize()
     assert int(pipe.status.item()) == (2 if small else 0)
+
+
+def test_reading_a_rulebook_leaves_the_cleared_tables_alone(d3d):
+    """The rulebook of a strided layer is made on demand; between `begin` and `forward` that must not touch the look-up that
+    `begin` has cleared for the tables."""
+    frame = _frame()
+    want = _run(_pipe(frame))
+    pipe = _pipe(frame)
+    _run(pipe)
+    net = pipe.net
+    net.begin()
+    read = {k: net.rulebooks[k].index.clone() for k in ("down2", "down3", "out")}
+    feats, coors, num = net.forward(pipe.vox_feats_lp)
+    torch.cuda.synchronize()
+    assert net.counts() == want[2] and torch.equal(coors[:int(num)], want[1])
+    for k, index in read.items():
+        assert torch.equal(net.rulebooks[k].index, index)
+
+
+@pytest.mark.parametrize("room", [1.2, 1.0, 0.6])
+def test_rulebook_of_the_live_voxel_set(d3d, orc, room):
+    """The rulebook of a strided layer lists the pairs between the voxels the network has, also where a set has lost some."""
+    frame = _frame()
+    caps = {k: (v + 9 if k == "in" else max(1, int(v * room))) for k, v in _run(_pipe(frame))[2].items()}
+    pipe = _pipe(frame, caps=caps)
+    _run(pipe)
+    for key in ("down2", "down4", "out"):
+        rb = pipe.net.rulebooks[key]
+        src, dst = ({k: v.cpu().numpy() for k, v in pipe.net.sets[s].items() if k in ("coors", "num")}
+                    for s in (rb.in_set, rb.out_set))
+        index, num = rb.index.cpu().numpy(), int(rb.num_index.item())
+        orc.check_layout(index, num, rb.kvol)
+        inputs, outputs = src["coors"][:src["num"][0]], dst["coors"][:dst["num"][0]]
+        ids = {tuple(c): i for i, c in enumerate(outputs.tolist())}
+        taps = np.stack(np.meshgrid(*[np.arange(k) for k in rb.ksize], indexing="ij"), -1).reshape(-1, 3)
+        want = set()
+        for i, c in enumerate(inputs):
+            at = c[1:] + np.array(rb.padding) - taps
+            for k in np.flatnonzero(((at % np.array(rb.stride)) == 0).all(1)):
+                o = ids.get((int(c[0]),) + tuple((at[k] // np.array(rb.stride)).tolist()))
+                if o is not None:
+                    want.add((i, o, int(k)))
+        live = index[:, :num][:, index[2, :num] >= 0]
+        assert len(want) == live.shape[1] > 100 and set(map(tuple, live.T.tolist())) == want
