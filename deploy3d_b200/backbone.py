@@ -324,7 +324,7 @@ class SparseNet:
         self.rulebooks = {}
         self.groups = {}  # voxel set -> _SubmGroup
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._cleared = False
+        self._cleared = None  # what `begin` has cleared and no build used: "eager" or "captured"
         self.tables_done = None  # event of the last forward: all tables built (overlap_rulebooks)
         self._concatenated = None  # the concatenation layer whose result is in place already
         self.mm = []
@@ -487,7 +487,11 @@ class SparseNet:
                 seen.add(rb.group)
                 with torch.cuda.stream(self.side_subm):
                     rb.group.clear(self.sets[rb.in_set], rb.shape_tensor, self.device)
-        self._cleared = True
+        self._cleared = self._mode()
+
+    @staticmethod
+    def _mode():
+        return "captured" if torch.cuda.is_current_stream_capturing() else "eager"
 
     def ranked(self, name):
         """Whether voxel set `name` is made by a strided pass that leaves a look-up of its voxels behind."""
@@ -511,7 +515,7 @@ class SparseNet:
             return
         if rb.group is not None:
             rb.group.enqueue(src["coors"], src["num"], rb.shape_tensor, voxel_grid=self._voxel_grid(rb.in_set),
-                             cleared=self._cleared, status=self.status)
+                             cleared=self._cleared is not None, status=self.status)
             for other in self.rulebooks.values():
                 if other.group is rb.group and other.regroup:
                     SPConvMMPlugin.regroup(other.kvol, dst["cap"], other.raw_fwd, other.table_fwd, other.scratch_fwd)
@@ -521,7 +525,7 @@ class SparseNet:
         if rb.direct:
             rb.plugin.tables(src["coors"], src["num"], rb.shape_tensor, out_coors=dst["coors"],
                              num_act_out=dst["num"], table=plain_fwd, table_inverse=plain_inv,
-                             voxel_grid=self._voxel_grid(rb.in_set), cleared=self._cleared, status=self.status)
+                             voxel_grid=self._voxel_grid(rb.in_set), cleared=self._cleared is not None, status=self.status)
         else:  # kernels or grids the direct builders do not take
             first = rb.calls == 0
             rb.calls += 1
@@ -567,7 +571,7 @@ class SparseNet:
         of its own rulebook.  Inside a CUDA graph capture these become further branches of the graph."""
         main = torch.cuda.current_stream(self.device)
         ready = {}
-        if not self._cleared:
+        if self._cleared != self._mode():  # an eager clear is no part of a graph, one in a graph has not run
             self.begin()
         if self.overlap_rulebooks:
             # two chains: the strided rulebooks follow each other (each creates the voxel set of the next); the SubM
@@ -591,7 +595,7 @@ class SparseNet:
                     ev = torch.cuda.Event()
                     ev.record(stream)
                     ready.update((k, ev) for k in keys)
-            self._cleared = False
+            self._cleared = None
             self.side.wait_stream(self.side_subm)
             self.tables_done = torch.cuda.Event()
             self.tables_done.record(self.side)

@@ -108,3 +108,28 @@ def test_rulebook_of_the_live_voxel_set(d3d, orc, room):
                     want.add((i, o, int(k)))
         live = index[:, :num][:, index[2, :num] >= 0]
         assert len(want) == live.shape[1] > 100 and set(map(tuple, live.T.tolist())) == want
+
+
+def test_clear_outside_a_graph_is_no_part_of_it(d3d):
+    """`begin` before a capture and `forward` inside it: the graph clears for itself, on every replay; and a clear that a
+    graph has recorded is not taken for one that has run."""
+    frame = _frame()
+    want = _run(_pipe(frame))
+    pipe = _pipe(frame)
+    _run(pipe)
+    net, graph = pipe.net, torch.cuda.CUDAGraph()
+    net.begin()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        feats, coors, num = net.forward(pipe.vox_feats_lp)
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert net.counts() == want[2] and torch.equal(coors[:int(num)], want[1])
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        net.begin()
+        torch.cuda.current_stream().wait_stream(net.side)
+        torch.cuda.current_stream().wait_stream(net.side_subm)
+    _, coors, num = net.forward(pipe.vox_feats_lp)
+    torch.cuda.synchronize()
+    assert net.counts() == want[2] and torch.equal(coors[:int(num)], want[1])
