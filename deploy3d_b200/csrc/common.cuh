@@ -314,8 +314,14 @@ __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.lau
 // Sum of the counts of the blocks in front of this one, by the whole block: a few hundred to a few thousand words that
 // every block reads for itself.  (A scan kernel between the count and its use costs a launch and runs on one CTA; blocks
 // that wait for each other's prefixes in one pass poll the same lines a thousand at a time: 28 us where the count kernel
-// and this take 11, 300 k points.)  `scratch`: a word per warp.
-template <int kThreads> __device__ __forceinline__ int preceding_sum(const int32_t* __restrict__ counts, int blk, int* scratch) {
+// and this take 11, 300 k points.)  What all blocks read together grows with the square of their number, so beyond
+// kMaxSummedBlocks scan_counts() is launched in between after all and `scanned` counts are prefixes already: mean encoder
+// by summing / scanning 32 / 35 us at 1172 blocks, 53.7 / 51.7 at 4096, 156 / 144 at 16 k, 736 / 525 at 65 k; strided tables
+// 66 / 71 us at 2594 blocks of words, 84 / 80 at 8458, 1482 / 635 at 122 k.  `scratch`: a word per warp.
+constexpr int kMaxSummedBlocks = 4096;
+template <int kThreads>
+__device__ __forceinline__ int preceding_sum(const int32_t* __restrict__ counts, int blk, bool scanned, int* scratch) {
+  if (scanned) return __ldg(counts + blk);
   int s = 0;
   for (int j = threadIdx.x; j < blk; j += kThreads) s += __ldg(counts + j);
   s = __reduce_add_sync(0xffffffffu, s);
@@ -325,6 +331,59 @@ template <int kThreads> __device__ __forceinline__ int preceding_sum(const int32
 #pragma unroll
   for (int w = 0; w < kThreads / 32; ++w) s += scratch[w];
   return s;
+}
+
+// Single CTA, in place: counts[i] becomes the sum of the counts in front of it.  Eight counts a thread and turn, the next
+// turn's loads ahead of this one's barriers.  counts: on 16 bytes.
+static __global__ void __launch_bounds__(1024) scan_counts_kernel(int32_t* __restrict__ counts, int n) {
+  __shared__ int scratch[40];
+  pdl_release();
+  pdl_wait();
+  constexpr int kItems = 8, kTurn = 1024 * kItems;
+  int carry = 0;
+  int4 next[2];
+  auto load = [&](int at) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = at + 4 * h;
+      int4 v = make_int4(0, 0, 0, 0);
+      if (i + 3 < n) v = *reinterpret_cast<const int4*>(counts + i);
+      else if (i < n) v.x = counts[i], v.y = i + 1 < n ? counts[i + 1] : 0, v.z = i + 2 < n ? counts[i + 2] : 0;
+      next[h] = v;
+    }
+  };
+  load(threadIdx.x * kItems);
+  for (int at0 = 0; at0 < n; at0 += kTurn) {
+    const int at = at0 + threadIdx.x * kItems;
+    int v[kItems] = {next[0].x, next[0].y, next[0].z, next[0].w, next[1].x, next[1].y, next[1].z, next[1].w};
+    if (at < n - kTurn) load(at + kTurn);  // n - kTurn: no overflow near the largest n
+    else next[0] = next[1] = make_int4(0, 0, 0, 0);
+    int mine = 0;
+#pragma unroll
+    for (int e = 0; e < kItems; ++e) mine += v[e];
+    int total, sum = carry + block_exclusive_scan(mine, scratch, &total);
+#pragma unroll
+    for (int e = 0; e < kItems; ++e) {
+      const int c = v[e];
+      v[e] = sum, sum += c;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = at + 4 * h;
+      if (i + 3 < n) *reinterpret_cast<int4*>(counts + i) = make_int4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+      else
+        for (int q = 0; q < 4; ++q)
+          if (i + q < n) counts[i + q] = v[4 * h + q];
+    }
+    carry += total;
+  }
+}
+
+// Between the kernel that counts per block and the one that numbers: whether the counts are prefixes now (`*scanned`).
+static inline int scan_counts(int32_t* counts, int blocks, bool chained, cudaStream_t st, bool* scanned) {
+  *scanned = blocks > kMaxSummedBlocks;
+  if (*scanned) D3D_LAUNCH(chained, scan_counts_kernel, 1, 1024, 0, st, counts, blocks);
+  return D3D_OK;
 }
 
 // Single CTA: in-place exclusive scan of `totals[0..n)`; *clamped_total = min(sum, limit).  A sum above the limit

@@ -1119,8 +1119,12 @@ int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
   D3D_LAUNCH3(chained, two ? conv_mark3_kernel<2> : conv_mark3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors, num_act_in, plan.n_max, plan.g);
   D3D_LAUNCH3(chained, two ? conv_count3_kernel<2> : conv_count3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid, coors,
               num_act_in, plan.n_max, plan.g, plan.win_bits, plan.winners);
+  bool scanned;
+  const int rc = scan_counts(plan.winners, plan.nblk, chained, st, &scanned);
+  if (rc != D3D_OK) return rc;
   D3D_LAUNCH3(chained, two ? conv_number3_kernel<2> : conv_number3_kernel<3>, plan.nblk, kIdxThreads, st, plan.grid,
-              coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, out_coors, num_act_out, status);
+              coors, num_act_in, plan.n_max, plan.g, max_out, plan.win_bits, plan.winners, scanned, out_coors, num_act_out,
+              status);
   D3D_LAUNCH(chained, (two ? conv_find3_kernel<2> : conv_find3_kernel<3>), plan.nblk, kIdxThreads, kFindSpare, st, plan.grid,
              coors, num_act_in, plan.n_max, plan.g, lists);
   return D3D_OK;
@@ -1526,7 +1530,10 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
   D3D_LAUNCH3(false, two ? rank_mark3_kernel<2> : rank_mark3_kernel<3>, plan.nblk, kIdxThreads, st, words, coors,
               num_act_in, plan.n_max, g);
   D3D_LAUNCH3(false, rank_count3_kernel, blocks, kRankWords, st, words, count, block_counts);
-  D3D_LAUNCH3(false, rank_number3_kernel, blocks, kRankWords, st, words, count, block_counts, g, max_out, out_coors,
+  bool scanned;
+  rc = scan_counts(block_counts, (int)blocks, false, st, &scanned);
+  if (rc != D3D_OK) return rc;
+  D3D_LAUNCH3(false, rank_number3_kernel, blocks, kRankWords, st, words, count, block_counts, scanned, g, max_out, out_coors,
               num_act_out, status);
   if (walk_outputs) {
     Targets forward = {};

@@ -495,7 +495,7 @@ template <int kTaps>
 __global__ void __launch_bounds__(kIdxThreads)
 conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coors, const int32_t* num_act_in,
                     int64_t n_max, const Geometry g, int32_t max_out, const uint32_t* __restrict__ wins,
-                    const int32_t* __restrict__ counts, int32_t* __restrict__ out_coors,
+                    const int32_t* __restrict__ counts, bool scanned, int32_t* __restrict__ out_coors,
                     int32_t* __restrict__ num_act_out, int32_t* status) {
   __shared__ int scratch[40], sums[kBlockWarps];
   pdl_release();
@@ -507,7 +507,7 @@ conv_number3_kernel(int32_t* __restrict__ grid, const int32_t* __restrict__ coor
   const uint32_t bits = i < n ? __ldg(wins + i) : 0u;
   int4 c = make_int4(-1, 0, 0, 0);
   if (bits) c = __ldg(reinterpret_cast<const int4*>(coors) + i);
-  const int base = preceding_sum<kIdxThreads>(counts, blockIdx.x, sums);
+  const int base = preceding_sum<kIdxThreads>(counts, blockIdx.x, scanned, sums);
   int total;
   int id = base + block_exclusive_scan(__popc(bits), scratch, &total);
   if (threadIdx.x == 0 && ((int64_t)blockIdx.x + 1) * kIdxThreads >= n) {

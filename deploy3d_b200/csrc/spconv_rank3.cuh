@@ -73,13 +73,13 @@ rank_count3_kernel(const uint2* __restrict__ words, int64_t count, int32_t* __re
 // its word one after the other, so what counts on dense levels is a short step: coordinates advance by carries instead of
 // divisions, one word a thread instead of four (the deepest level, 2 blocks then: 43 us beside a convolution).
 __global__ void __launch_bounds__(kRankWords)
-rank_number3_kernel(uint2* __restrict__ words, int64_t count, const int32_t* __restrict__ block_counts, const Geometry g,
+rank_number3_kernel(uint2* __restrict__ words, int64_t count, const int32_t* __restrict__ block_counts, bool scanned, const Geometry g,
                     int32_t max_out, int32_t* __restrict__ out_coors, int32_t* __restrict__ num_act_out,
                     int32_t* status) {
   __shared__ int scratch[40], sums[kRankWords / 32];
   const int64_t at = (int64_t)blockIdx.x * kRankWords + threadIdx.x;
   uint32_t rest = at < count ? words[at].x : 0u;
-  const int base = preceding_sum<kRankWords>(block_counts, blockIdx.x, sums);
+  const int base = preceding_sum<kRankWords>(block_counts, blockIdx.x, scanned, sums);
   int total;
   int id = base + block_exclusive_scan(__popc(rest), scratch, &total);
   if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {

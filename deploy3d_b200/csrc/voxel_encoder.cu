@@ -167,7 +167,7 @@ count_owners_kernel(const Voxels vox, int32_t* __restrict__ slot_of, int64_t n, 
 template <bool kMean>
 __global__ void __launch_bounds__(kEncThreads)
 number_voxels_kernel(const Voxels vox, int32_t* __restrict__ slot_of, int64_t n, int64_t m_max, int e1, int e2, int e3,
-                     const int32_t* __restrict__ owners, const float* __restrict__ pts, int c,
+                     const int32_t* __restrict__ owners, bool scanned, const float* __restrict__ pts, int c,
                      int32_t* __restrict__ out_coors, int32_t* __restrict__ count, float* __restrict__ out_feats,
                      int32_t* __restrict__ scatter_to, int32_t* __restrict__ num_act_out, int32_t* status) {
   __shared__ int scratch[40], sums[kEncThreads / 32];
@@ -178,7 +178,7 @@ number_voxels_kernel(const Voxels vox, int32_t* __restrict__ slot_of, int64_t n,
   const bool owner = mark <= -3;
   const int slot = owner_mark(mark);
   const uint32_t key = !owner ? 0u : vox.grid ? (uint32_t)slot : (uint32_t)(__ldcg(vox.slots + slot) >> 32);
-  const int base = preceding_sum<kEncThreads>(owners, blockIdx.x, sums);
+  const int base = preceding_sum<kEncThreads>(owners, blockIdx.x, scanned, sums);
   int total;
   const int rank = block_exclusive_scan(owner, scratch, &total);
   if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {
@@ -420,8 +420,11 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   D3D_LAUNCH(chained, voxelize_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pts, batch, cfg, pl.n, pl.c, pl.dims[0],
              pl.dims[1], pl.dims[2], pl.dims[3], pl.slot_of, status);
   D3D_LAUNCH(chained, count_owners_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, pl.owners);
+  bool scanned;
+  rc = scan_counts(pl.owners, pl.nblk, chained, st, &scanned);
+  if (rc != D3D_OK) return rc;
   D3D_LAUNCH(chained, number_voxels_kernel<true>, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, m_max,
-             pl.dims[1], pl.dims[2], pl.dims[3], pl.owners, pts, pl.c, out_coors, pl.count, out_feats, nullptr,
+             pl.dims[1], pl.dims[2], pl.dims[3], pl.owners, scanned, pts, pl.c, out_coors, pl.count, out_feats, nullptr,
              num_act_out, status);
   if (m_max > 0) {
     D3D_LAUNCH(chained, mean_accumulate_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pts, pl.n, pl.c,
@@ -474,8 +477,11 @@ extern "C" int d3d_cylinder_encoder_enqueue(const d3d_voxel_encoder_params* p, c
              fits ? staged : 0, st, pl.vox, pts, batch, cfg, pl.n, pl.c, pl.dims[0], pl.dims[1], pl.dims[2], pl.dims[3],
              pl.slot_of, aug);
   D3D_LAUNCH(true, count_owners_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, pl.owners);
+  bool scanned;
+  rc = scan_counts(pl.owners, pl.nblk, true, st, &scanned);
+  if (rc != D3D_OK) return rc;
   D3D_LAUNCH(true, number_voxels_kernel<false>, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, m_max, pl.dims[1],
-             pl.dims[2], pl.dims[3], pl.owners, pts, pl.c, out_coors, scatter_count, nullptr, scatter_to, num_act_out,
+             pl.dims[2], pl.dims[3], pl.owners, scanned, pts, pl.c, out_coors, scatter_count, nullptr, scatter_to, num_act_out,
              nullptr);
   D3D_LAUNCH(true, scatter_ids_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, num_act_out, m_max,
              scatter_to, scatter_count);

@@ -274,3 +274,37 @@ def test_mean_encoder_status_word(d3d):
         status.zero_()
         plug.enqueue_lp(pts, batch, cfg, shp, outputs=outs, status=status)
         assert int(status.item()) == want and int(outs[2].item()) <= cap
+
+
+@pytest.mark.parametrize("which", ["mean", "cylinder"])
+@pytest.mark.parametrize("n", [4096 * 256, 4096 * 256 + 1, 4100 * 256 + 77, 13000 * 256])
+def test_voxel_numbers_of_many_blocks(d3d, which, n):
+    """Up to 4096 blocks of points each sums the counts in front of it, beyond that they are scanned: voxels are numbered by
+    first touch either way."""
+    g = torch.Generator(device="cuda:0").manual_seed(n)
+    pts = torch.rand((n, 3), generator=g, device="cuda:0")
+    batch = torch.zeros(n, dtype=torch.int32, device="cuda:0")
+    cells = (7, 160, 150)
+    if which == "mean":
+        cfg = torch.tensor([0, 0, 0, 1 / 150, 1 / 160, 1 / 7], device="cuda:0")
+        run, pts = d3d.simple_mean_encoder, pts * 0.999
+    else:  # points on a quarter disc of radius up to 1.42
+        cfg = torch.tensor([0, 0, 0, 1, 1.6, 1.5], device="cuda:0")
+        run = d3d.cylinder_encoder
+    outs = run(pts, batch, cfg, torch.empty((1, 0) + cells, dtype=torch.int32, device="cuda:0"), 200000)
+    if which == "mean":
+        _, coors, num = outs
+        m = int(num.item())
+        div = lambda d, e: (pts[:, d] / cfg[e]).int().long()
+        at = (div(2, 5) * 160 + div(1, 4)) * 150 + div(0, 3)
+    else:
+        _, to, count, coors, num = outs
+        m = int(num.item())
+        c = coors[:m].long()
+        at = ((c[:, 1] * 160 + c[:, 2]) * 150 + c[:, 3])[to.long()]  # the map is taken on trust, the numbering is not
+        assert torch.equal(torch.bincount(to, minlength=m).int(), count[:m])
+    cell, back = torch.unique(at, return_inverse=True)
+    first = torch.full((len(cell),), n, device="cuda:0").scatter_reduce_(0, back, torch.arange(n, device="cuda:0"), "amin")
+    want = cell[torch.argsort(first)]
+    c = coors[:m].long()
+    assert m == len(cell) and torch.equal((c[:, 1] * 160 + c[:, 2]) * 150 + c[:, 3], want)

@@ -276,3 +276,41 @@ def test_output_coordinates_in_an_arena_of_words(d3d, words):
     key = lambda c: ((c[:, 0] * 7 + c[:, 1]) * 12 + c[:, 2]) * 13 + c[:, 3]
     assert int(on.item()) == m and torch.equal(oc[:m], want[:m][torch.argsort(key(want[:m]))])
     assert (flat[:words] == -9).all() and (oc[m:] == -9).all()
+
+
+# More blocks than read the counts in front of them for themselves (4096): a scan is launched in between.
+def test_conv_numbering_beyond_the_summed_blocks(d3d):
+    shape, n, cap = [1, 31, 200, 200], 1060000, 4200 * 256 + 3
+    coors = np.zeros((cap, 4), np.int32)
+    coors[:n] = unique_coors(rng(9), n, shape)
+    args = (3, 1, 1), (2, 1, 1), ZERO, ONE, ZERO
+    outs = d3d.spconv_index(_t(coors), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape), *args, 700000, False,
+                            False)
+    at = coors[:n, None, 1] - np.arange(3)[None]
+    ok = (at % 2 == 0) & (at >= 0) & (at // 2 < 15)
+    key = (at // 2 * 40000 + (coors[:n, 2] * 200 + coors[:n, 3])[:, None])[ok]
+    _, first = np.unique(key, return_index=True)
+    want = key[np.sort(first)]
+    m = int(outs[3].item())
+    got = outs[2].cpu().numpy()[:m]
+    assert m == len(want) and (got[:, 1] * 40000 + got[:, 2] * 200 + got[:, 3] == want).all()
+
+
+def test_conv_tables_beyond_the_summed_blocks(d3d):
+    from deploy3d_b200.plugins import deserialize_plugin
+    shape, n, max_out = [1, 41, 909, 907], 100000, 220000  # 34 M cells, 4127 blocks of words
+    params, out = ((3, 1, 1), ONE, (1, 0, 0), ONE, False), shape
+    coors_t, num, shp = _t(unique_coors(rng(4), n, shape)), torch.tensor([n], dtype=torch.int32, device=DEV), _carrier(shape)
+    plug = deserialize_plugin("SPConvIdx3d", d3d.data_s_spconv_index(*params[:4], ZERO, max_out, False, False))
+    assert plug.tables_ok(coors_t, num, shp)
+    got = _conv_tables(d3d, plug, coors_t, num, shp, max_out, 3)
+    index, num_index, oc, on, _ = d3d.spconv_index(coors_t, num, shp, *params[:4], ZERO, 600000, False, False)
+    m, oc = int(on.item()), oc[:int(on.item())].long()
+    order = torch.argsort((oc[:, 1] * out[2] + oc[:, 2]) * out[3] + oc[:, 3])
+    ids = torch.empty_like(order)
+    ids[order] = torch.arange(m, device=DEV)
+    pairs = index[:, :int(num_index.item())].long()
+    pairs = pairs[:, pairs[2] >= 0]
+    trip = torch.stack([ids[pairs[1]], pairs[2], pairs[0]], 1)
+    assert m > max_out
+    _check_conv_tables(got, (m, oc[order][:max_out].int(), trip[trip[:, 0] < max_out]), max_out)
