@@ -153,6 +153,8 @@ SIGNATURES = {
     "d3d_simple_mean_encoder_enqueue": (ctypes.c_int, _enqueue_sig(ctypes.POINTER(VoxelEncoderParams))),
     "d3d_simple_mean_encoder_enqueue_ex": (ctypes.c_int, _enqueue_sig(ctypes.POINTER(VoxelEncoderParams)) +
                                            [ctypes.POINTER(MeanEncoderExtras)]),
+    "d3d_simple_mean_encoder_enqueue_event": (ctypes.c_int, _enqueue_sig(ctypes.POINTER(VoxelEncoderParams)) +
+                                              [ctypes.POINTER(MeanEncoderExtras), _vp]),
     "d3d_cylinder_encoder_parse": (ctypes.c_int, [_vp, _sz, ctypes.POINTER(VoxelEncoderParams)]),
     "d3d_cylinder_encoder_output_desc": (ctypes.c_int, [ctypes.POINTER(VoxelEncoderParams), _descp, ctypes.c_int, ctypes.c_int, _descp]),
     "d3d_cylinder_encoder_workspace": (ctypes.c_int, _workspace_sig(ctypes.POINTER(VoxelEncoderParams))),

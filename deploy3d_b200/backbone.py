@@ -562,9 +562,10 @@ class SparseNet:
         out_buf.copy_(ew_apply(L.ew[0], [x.float() for x in xs], torch))
         return out_buf
 
-    def forward(self, feats):
+    def forward(self, feats, coors_ready=None):
         """feats [cap_in, Cin] in the net dtype; coordinates / count as given to set_input.  Returns
-        (out_feats, out_coors, num_act_out); every tensor is a static buffer of the net.
+        (out_feats, out_coors, num_act_out); every tensor is a static buffer of the net.  `coors_ready`: an event from which
+        on the coordinates are final, when the features come later: the tables start there (overlap_rulebooks).
 
         Rulebooks and neighbour tables depend on coordinates only, never on features, so with `overlap_rulebooks`
         the chains of them are enqueued on two side streams ahead of the convolutions; a layer waits for the event
@@ -577,8 +578,8 @@ class SparseNet:
             # two chains: the strided rulebooks follow each other (each creates the voxel set of the next); the SubM
             # rulebook of a level needs only that level's coordinates, so it runs beside the next strided one.
             # (A third stream for the strided rulebooks' neighbour tables measured no further gain.)
-            self.side.wait_stream(main)
-            self.side_subm.wait_stream(main)
+            for stream in (self.side, self.side_subm):
+                stream.wait_stream(main) if coors_ready is None else stream.wait_event(coors_ready)
             done = set()
             for L in self.layers:
                 if L.kind == "ew" or L.key in done:

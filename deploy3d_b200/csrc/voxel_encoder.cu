@@ -373,21 +373,11 @@ extern "C" int d3d_cylinder_encoder_workspace(const d3d_voxel_encoder_params* p,
   return rc;
 }
 
-extern "C" int d3d_simple_mean_encoder_enqueue(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
-                                               const d3d_tensor_desc* out, int n_out, const void* const* inputs,
-                                               void* const* outputs, void* workspace, size_t workspace_bytes,
-                                               void* stream) {
-  D3D_NVTX_RANGE("d3d_simple_mean_encoder_enqueue");
-  return d3d_simple_mean_encoder_enqueue_ex(p, in, n_in, out, n_out, inputs, outputs, workspace, workspace_bytes,
-                                            stream, nullptr);
-}
-
-extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in,
-                                                  int n_in, const d3d_tensor_desc* out, int n_out,
-                                                  const void* const* inputs, void* const* outputs, void* workspace,
-                                                  size_t workspace_bytes, void* stream,
-                                                  const d3d_mean_encoder_extras* extras) {
-  D3D_NVTX_RANGE("d3d_simple_mean_encoder_enqueue_ex");
+// `coors_event` (may be null): recorded where coordinates and count are final.
+static int enqueue_mean(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in, const d3d_tensor_desc* out,
+                        int n_out, const void* const* inputs, void* const* outputs, void* workspace,
+                        size_t workspace_bytes, void* stream, const d3d_mean_encoder_extras* extras,
+                        cudaEvent_t coors_event) {
   D3D_REQUIRE(inputs && outputs && out && n_out >= 3, D3D_ERR_INVALID_ARGUMENT);
   void* lp = extras ? extras->lp_feats : nullptr;
   int32_t* status = extras ? extras->status : nullptr;
@@ -410,6 +400,7 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   if (pl.n == 0) {
     cudaMemsetAsync(num_act_out, 0, sizeof(int32_t), st);
     if (m_max > 0) cudaMemsetAsync(out_feats, 0, (size_t)m_max * pl.c * sizeof(float), st);
+    if (coors_event && cudaEventRecord(coors_event, st) != cudaSuccess) return D3D_ERR_CUDA;
     D3D_CHECK_LAUNCH();
     return D3D_OK;
   }
@@ -426,6 +417,7 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   D3D_LAUNCH(chained, number_voxels_kernel<true>, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pl.n, m_max,
              pl.dims[1], pl.dims[2], pl.dims[3], pl.owners, scanned, pts, pl.c, out_coors, pl.count, out_feats, nullptr,
              num_act_out, status);
+  if (coors_event && cudaEventRecord(coors_event, st) != cudaSuccess) return D3D_ERR_CUDA;
   if (m_max > 0) {
     D3D_LAUNCH(chained, mean_accumulate_kernel, pl.nblk, kEncThreads, 0, st, pl.vox, pl.slot_of, pts, pl.n, pl.c,
                out_feats, pl.count);
@@ -439,6 +431,32 @@ extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params
   }
   D3D_CHECK_LAUNCH();
   return D3D_OK;
+}
+
+extern "C" int d3d_simple_mean_encoder_enqueue(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
+                                               const d3d_tensor_desc* out, int n_out, const void* const* inputs,
+                                               void* const* outputs, void* workspace, size_t workspace_bytes,
+                                               void* stream) {
+  D3D_NVTX_RANGE("d3d_simple_mean_encoder_enqueue");
+  return enqueue_mean(p, in, n_in, out, n_out, inputs, outputs, workspace, workspace_bytes, stream, nullptr, nullptr);
+}
+
+extern "C" int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
+                                                  const d3d_tensor_desc* out, int n_out, const void* const* inputs,
+                                                  void* const* outputs, void* workspace, size_t workspace_bytes,
+                                                  void* stream, const d3d_mean_encoder_extras* extras) {
+  D3D_NVTX_RANGE("d3d_simple_mean_encoder_enqueue_ex");
+  return enqueue_mean(p, in, n_in, out, n_out, inputs, outputs, workspace, workspace_bytes, stream, extras, nullptr);
+}
+
+extern "C" int d3d_simple_mean_encoder_enqueue_event(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
+                                                     const d3d_tensor_desc* out, int n_out, const void* const* inputs,
+                                                     void* const* outputs, void* workspace, size_t workspace_bytes,
+                                                     void* stream, const d3d_mean_encoder_extras* extras,
+                                                     void* coors_event) {
+  D3D_NVTX_RANGE("d3d_simple_mean_encoder_enqueue_event");
+  return enqueue_mean(p, in, n_in, out, n_out, inputs, outputs, workspace, workspace_bytes, stream, extras,
+                      reinterpret_cast<cudaEvent_t>(coors_event));
 }
 
 extern "C" int d3d_cylinder_encoder_enqueue(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,

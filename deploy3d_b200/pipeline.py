@@ -120,6 +120,7 @@ class DetectionPipeline:
         fork / join of the graph."""
         main = torch.cuda.current_stream(self.device)
         self.net.begin()
+        coors_ready = None
         outputs = [self.vox_feats, self.vox_coors, self.vox_num]
         if self.plugin_order or self.dtype == torch.float32:
             if self.plugin_order:
@@ -130,9 +131,10 @@ class DetectionPipeline:
             # fp32 -> fp16 reformat (TensorRT inserts this layer itself); padding columns stay zero
             self.vox_feats_lp[:, :self.c_pts].copy_(self.vox_feats)
         else:  # the encoder writes the half-precision, channel-padded copy itself
+            coors_ready = torch.cuda.Event()
             self.vfe.enqueue_lp(self.points, self.batch, self.cfg, self.shape_tensor, outputs=outputs,
-                                lp_feats=self.vox_feats_lp, status=self.status)
-        feats, coors, num = self.net.forward(self.vox_feats_lp)
+                                lp_feats=self.vox_feats_lp, status=self.status, coors_event=coors_ready)
+        feats, coors, num = self.net.forward(self.vox_feats_lp, coors_ready)
         beside = not self.plugin_order
         if beside:
             if self.net.tables_done is not None:
@@ -271,9 +273,11 @@ class SegmentationPipeline:
         self.encoder.enqueue(self.points, self.batch, self.cfg, self.shape_tensor,
                              outputs=[self.pts_feats, self.scatter_index, self.scatter_count, self.vox_coors,
                                       self.vox_num])
+        coors_ready = torch.cuda.Event()
+        coors_ready.record()
         self.scatter.enqueue(self.pts_feats, self.scatter_index, self.scatter_count, outputs=[self.vox_feats])
         self.vox_feats_lp[:, :self.c_pts + 5].copy_(self.vox_feats)
-        feats, _, _ = self.net.forward(self.vox_feats_lp)
+        feats, _, _ = self.net.forward(self.vox_feats_lp, coors_ready)
         # GatherBack and the label pass of the reference (test_cylinder3d.py:322) in one
         if feats.shape[1] <= MAX_LABEL_CLASSES:
             gather_labels(feats, self.scatter_index, 0.0, self.logits, self.labels)

@@ -430,9 +430,10 @@ class SimpleMeanEncoderPlugin(_PodPlugin):
     num_outputs = 3
 
 
-    def enqueue_lp(self, *inputs, outputs, lp_feats=None, status=None, stream=None):
+    def enqueue_lp(self, *inputs, outputs, lp_feats=None, status=None, stream=None, coors_event=None):
         """enqueue that also writes the voxel means in half / bfloat16, zero-padded to lp_feats.shape[1] channels,
-        and / or reports soft failures (D3D_STATUS_* bits) in the int32 device tensor `status`."""
+        and / or reports soft failures (D3D_STATUS_* bits) in the int32 device tensor `status`.  `coors_event`, a
+        torch.cuda.Event, is recorded once the coordinates are final, in front of the means."""
         inputs = [t if t.is_contiguous() else t.contiguous() for t in inputs]
         device = inputs[0].device
         in_descs = [_desc_of(t) for t in inputs]
@@ -444,12 +445,15 @@ class SimpleMeanEncoderPlugin(_PodPlugin):
                                         int(lp_feats.shape[1]) if lp_feats is not None else 0,
                                         status.data_ptr() if status is not None else None)
         with torch.cuda.device(device):
-            status = lib().d3d_simple_mean_encoder_enqueue_ex(
+            if coors_event is not None:
+                coors_event.record(stream) if stream is not None else coors_event.record()  # makes the handle
+            status = lib().d3d_simple_mean_encoder_enqueue_event(
                 ctypes.byref(self.p), desc_array(in_descs), len(in_descs), desc_array(out_descs), len(out_descs),
                 ptr_array([t.data_ptr() for t in inputs]), ptr_array([t.data_ptr() for t in outputs]),
                 ctypes.c_void_p(ws.data_ptr() if ws is not None else 0), ctypes.c_size_t(ws_bytes),
-                _stream_ptr(stream), ctypes.byref(extras))
-        check("d3d_simple_mean_encoder_enqueue_ex", status)
+                _stream_ptr(stream), ctypes.byref(extras),
+                ctypes.c_void_p(coors_event.cuda_event if coors_event is not None else 0))
+        check("d3d_simple_mean_encoder_enqueue_event", status)
         return tuple(outputs)
 
 

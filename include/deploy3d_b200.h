@@ -355,6 +355,12 @@ int d3d_simple_mean_encoder_enqueue_ex(const d3d_voxel_encoder_params* p, const 
                                        const d3d_tensor_desc* out, int n_out, const void* const* inputs,
                                        void* const* outputs, void* workspace, size_t workspace_bytes, void* stream,
                                        const d3d_mean_encoder_extras* extras);
+/* enqueue_ex that also records `coors_event` (a cudaEvent_t, may be NULL) in `stream` as soon as coordinates and numActOut
+ * are final, in front of the means: what depends on the voxels alone can start there on another stream. */
+int d3d_simple_mean_encoder_enqueue_event(const d3d_voxel_encoder_params* p, const d3d_tensor_desc* in, int n_in,
+                                          const d3d_tensor_desc* out, int n_out, const void* const* inputs,
+                                          void* const* outputs, void* workspace, size_t workspace_bytes, void* stream,
+                                          const d3d_mean_encoder_extras* extras, void* coors_event);
 
 /* ---------------------------------------------------------------------------------------------
  * CylinderEncoder.  Replaces voxel_encoder::CylinderEncoderPlugin
