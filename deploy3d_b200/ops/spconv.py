@@ -12,14 +12,19 @@ _BLOB_HEADER = 19  # bytes of an SPConvMM blob before the weights
 
 
 def _plugin(name, data_s):
+    return _plugin_and_blob(name, data_s)[0]
+
+
+def _plugin_and_blob(name, data_s):
+    """The plugin and the one copy of its blob that is kept, however many equal ones are passed."""
     key = (name, data_s)
-    plug = _CACHE.get(key)
-    if plug is None:
+    found = _CACHE.get(key)
+    if found is None:
         if len(_CACHE) > 256:
             _CACHE.clear()
             _BY_ARGS.clear()
-        plug = _CACHE[key] = deserialize_plugin(name, data_s)
-    return plug
+        found = _CACHE[key] = (deserialize_plugin(name, data_s), data_s)
+    return found
 
 
 def _plugin_by_args(name, args, data_s):
@@ -101,12 +106,12 @@ def spconv_mm(in_feats, num_act_in, num_act_out, index, num_index, kernel_size, 
             if same(weight, blob, _BLOB_HEADER) and (bias is None or same(bias, blob, end)):
                 return out
     data = data_s_spconv_mm(kernel_size, in_channels, out_channels, max_num_act_out, subm, inverse, weight, bias)
-    plug = _plugin("SPConvMM", data)
+    found = _plugin_and_blob("SPConvMM", data)
     if key is not None:
         if len(_BY_ARGS) > 1024:
             _BY_ARGS.clear()
-        _BY_ARGS[key] = (plug, data)
-    return plug.enqueue(*inputs)[0]
+        _BY_ARGS[key] = found
+    return found[0].enqueue(*inputs)[0]
 
 
 def data_s_bev_densify(out_channels):

@@ -99,3 +99,39 @@ threads = [threading.Thread(target=caller, args=(s,)) for s in range(3)]
 print(len(wrong), *wrong[:5])
 """ % busy)
     assert out == ["0"]
+
+
+class _Recorder:
+    """Stands in for a plugin object: keeps what it is called with."""
+
+    def __init__(self, name, data_s):
+        self.name, self.data_s, self.calls = name, data_s, []
+
+    def enqueue(self, *inputs, **how):
+        self.calls.append(inputs)
+        return (self,)
+
+
+@pytest.fixture
+def operators(d3d, monkeypatch):
+    """The operator layer over recorders, with empty look-ups."""
+    from deploy3d_b200.ops import spconv
+    monkeypatch.setattr(spconv, "deserialize_plugin", _Recorder)
+    monkeypatch.setattr(spconv, "_CACHE", {})
+    monkeypatch.setattr(spconv, "_BY_ARGS", {})
+    return spconv
+
+
+def _layer(w, b=None, ksize=(3, 3, 3), cap=10):
+    return (None,) * 5 + (ksize, 2, 4, cap, True, False, w, b)
+
+
+def test_weights_at_many_addresses_are_kept_once(operators):
+    import numpy as np
+    w = np.random.default_rng(0).standard_normal((27, 2, 4)).astype(np.float32)
+    copies = [w.copy() for _ in range(20)]
+    plugs = {operators.spconv_mm(*_layer(c)) for c in copies}
+    plugs |= {operators.spconv_mm(*_layer(c)) for c in copies}  # found by address now
+    assert len(plugs) == 1
+    blobs = [v[1] for k, v in operators._BY_ARGS.items() if k[0] == "SPConvMM"]
+    assert len(blobs) == 20 and len({id(b) for b in blobs}) == 1
