@@ -95,7 +95,7 @@ def spconv_mm(in_feats, num_act_in, num_act_out, index, num_index, kernel_size, 
     key = None
     if type(weight) is np.ndarray and weight.dtype == np.float32 and weight.flags.c_contiguous and (
             bias is None or (type(bias) is np.ndarray and bias.dtype == np.float32 and bias.flags.c_contiguous)):
-        key = ("SPConvMM", tuple(kernel_size), in_channels, out_channels, max_num_act_out, bool(subm), bool(inverse),
+        key = ("SPConvMM", int(np.prod(kernel_size)), in_channels, out_channels, max_num_act_out, bool(subm), bool(inverse),
                weight.ctypes.data, weight.nbytes, None if bias is None else bias.nbytes)
         found = _BY_ARGS.get(key)
         if found is not None:

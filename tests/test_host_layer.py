@@ -135,3 +135,13 @@ def test_weights_at_many_addresses_are_kept_once(operators):
     assert len(plugs) == 1
     blobs = [v[1] for k, v in operators._BY_ARGS.items() if k[0] == "SPConvMM"]
     assert len(blobs) == 20 and len({id(b) for b in blobs}) == 1
+
+
+@pytest.mark.parametrize("ksize", [27, [3, 3, 3], (27,), "array"])
+def test_kernel_size_in_any_form(operators, ksize):
+    """The blob holds the kernel volume only, so a number does for kernel_size as well as extents in any container."""
+    import numpy as np
+    w = np.ones((27, 2, 4), np.float32)
+    form = np.array([3, 3, 3]) if ksize == "array" else ksize
+    for _ in range(2):
+        assert operators.spconv_mm(*_layer(w, ksize=form)) is operators.spconv_mm(*_layer(w))
