@@ -27,8 +27,25 @@ def _plugin_and_blob(name, data_s):
     return found
 
 
+def _plain(v):
+    """Whether equal keys mean equal values for good: numbers and tuples of them, not tensors (equal to themselves whatever
+    they hold by now)."""
+    return v is None or isinstance(v, (int, float, str, np.generic)) or (type(v) is tuple and all(map(_plain, v)))
+
+
+def _volume(kernel_size):
+    """Kernel volume of extents in any container, or of the volume itself."""
+    try:
+        v = 1
+        for k in kernel_size:
+            v *= int(k)
+        return v
+    except TypeError:
+        return int(kernel_size)
+
+
 def _plugin_by_args(name, args, data_s):
-    """The plugin `name` whose blob is data_s(*args); `args` are hashable values that determine the blob."""
+    """The plugin `name` whose blob is data_s(*args); kept for arguments that determine the blob."""
     key = (name,) + args
     try:
         plug = _BY_ARGS.get(key)
@@ -36,9 +53,10 @@ def _plugin_by_args(name, args, data_s):
         return _plugin(name, data_s(*args))
     if plug is None:
         plug = _plugin(name, data_s(*args))
-        if len(_BY_ARGS) > 1024:
-            _BY_ARGS.clear()
-        _BY_ARGS[key] = plug
+        if _plain(key):
+            if len(_BY_ARGS) > 1024:
+                _BY_ARGS.clear()
+            _BY_ARGS[key] = plug
     return plug
 
 
@@ -95,7 +113,7 @@ def spconv_mm(in_feats, num_act_in, num_act_out, index, num_index, kernel_size, 
     key = None
     if type(weight) is np.ndarray and weight.dtype == np.float32 and weight.flags.c_contiguous and (
             bias is None or (type(bias) is np.ndarray and bias.dtype == np.float32 and bias.flags.c_contiguous)):
-        key = ("SPConvMM", int(np.prod(kernel_size)), in_channels, out_channels, max_num_act_out, bool(subm), bool(inverse),
+        key = ("SPConvMM", _volume(kernel_size), in_channels, out_channels, max_num_act_out, bool(subm), bool(inverse),
                weight.ctypes.data, weight.nbytes, None if bias is None else bias.nbytes)
         found = _BY_ARGS.get(key)
         if found is not None:
@@ -107,7 +125,7 @@ def spconv_mm(in_feats, num_act_in, num_act_out, index, num_index, kernel_size, 
                 return out
     data = data_s_spconv_mm(kernel_size, in_channels, out_channels, max_num_act_out, subm, inverse, weight, bias)
     found = _plugin_and_blob("SPConvMM", data)
-    if key is not None:
+    if key is not None and _plain(key):
         if len(_BY_ARGS) > 1024:
             _BY_ARGS.clear()
         _BY_ARGS[key] = found

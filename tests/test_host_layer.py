@@ -145,3 +145,19 @@ def test_kernel_size_in_any_form(operators, ksize):
     form = np.array([3, 3, 3]) if ksize == "array" else ksize
     for _ in range(2):
         assert operators.spconv_mm(*_layer(w, ksize=form)) is operators.spconv_mm(*_layer(w))
+
+
+def test_arguments_that_change_in_place(operators):
+    """A size held in a tensor is read on every call, as a number would be."""
+    import numpy as np
+    rows = torch.tensor(10)
+    k, one = (3, 3, 3), (1, 1, 1)
+    w = np.ones((27, 2, 4), np.float32)
+    for n in (10, 25, 10):
+        rows.fill_(n)
+        plug = operators._plugin_by_args("SPConvIdx3d", (k, one, one, one, (0, 0, 0), rows, True, False),
+                                         operators.data_s_spconv_index)
+        assert plug.data_s == operators.data_s_spconv_index(k, one, one, one, (0, 0, 0), n, True, False)
+        plug = operators.spconv_mm(*_layer(w, cap=rows))
+        assert plug.data_s == operators.data_s_spconv_mm(k, 2, 4, n, True, False, w)
+    assert all(operators._plain(key) for key in operators._BY_ARGS)
