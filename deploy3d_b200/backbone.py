@@ -14,7 +14,8 @@ import torch
 
 from . import synth
 from .ops import data_s_spconv_index, data_s_spconv_mm
-from .plugins import SPConvMMPlugin, SubmTables, activation, cuda_device, deserialize_plugin, recon
+from .plugins import (SPConvMMPlugin, SubmTables, activation, activation_ok, cuda_device, deserialize_plugin, recon,
+                      recon_ok)
 
 
 class Layer:
@@ -547,7 +548,7 @@ class SparseNet:
     def _elementwise(self, li, L, out_buf, xs):
         """One element-wise graph op, in fp32, rounded to the net's type.  A ReconBlock is one pass, and the concatenation
         of its result with its input right behind it is part of that pass."""
-        if L.ew[0] == "recon" and L.cout * out_buf.element_size() % 16 == 0:
+        if L.ew[0] == "recon" and recon_ok(*xs, out_buf):
             nxt = self.layers[li + 1] if li + 1 < len(self.layers) else None
             users = [U for U in self.layers if L.save is not None and
                      (L.save in (U.source, U.residual) or (U.kind == "ew" and L.save in U.ew[1]))]
@@ -647,8 +648,17 @@ class SparseNet:
         if self.plugin_order:
             in_set = rb.out_set if L.kind == "inverse" else rb.in_set
             plug.enqueue(x, self.sets[in_set]["num"], self.sets[out_set]["num"], *rb.buffers(), outputs=[out_buf])
-            if L.relu or res is not None:  # the element-wise layer an engine fuses sum and activation into
-                activation(out_buf, res, L.relu_mode)
+            # the element-wise layer an engine fuses sum and activation into; a residual it cannot read as it is (the caller's
+            # features, with strides of their own) goes through the layers one by one
+            if activation_ok(out_buf, res):
+                if L.relu or res is not None:
+                    activation(out_buf, res, L.relu_mode)
+                return out_buf
+            if L.relu_mode == 2:
+                out_buf.relu_()
+            out_buf.add_(res)
+            if L.relu_mode == 1:
+                out_buf.relu_()
             return out_buf
         return plug.run(x, self.sets[out_set]["num"], rb.table_inv if L.kind == "inverse" else rb.table_fwd, out=out_buf,
                         relu=L.relu_mode, residual=res, regrouped=rb.regroup)

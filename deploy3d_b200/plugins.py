@@ -201,8 +201,16 @@ class SPConvIdxPlugin(_Plugin):
                 int(bool(cleared))))
 
 
+def activation_ok(x, residual=None):
+    """Whether `activation` takes these tensors."""
+    return all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, residual) if t is not None) and (
+        residual is None or (residual.shape == x.shape and residual.dtype == x.dtype))
+
+
 def activation(x, residual=None, relu=1, stream=None):
     """x (+= residual), ReLU after (relu=1) or before (2) the sum, in place and in one pass (d3d_activation)."""
+    if not activation_ok(x, residual):
+        raise ValueError("activation takes contiguous tensors of one shape and type that start on 16 bytes")
     with torch.cuda.device(x.device):
         check("d3d_activation", lib().d3d_activation(_TORCH2D3D[x.dtype], x.data_ptr(),
                                                      residual.data_ptr() if residual is not None else None, x.numel(),
@@ -210,10 +218,18 @@ def activation(x, residual=None, relu=1, stream=None):
     return x
 
 
+def recon_ok(a, b, c, x, out):
+    """Whether `recon` takes these tensors."""
+    same = all(t.is_contiguous() and t.shape == x.shape and t.dtype == x.dtype for t in (a, b, c, x))
+    return (same and out.dtype == x.dtype and out.stride(1) == 1 and x.shape[1] * x.element_size() % 16 == 0 and
+            out.stride(0) * x.element_size() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (a, b, c, x, out)))
+
+
 def recon(a, b, c, x, out, copy_x=False, stream=None):
     """out[:, :C] = (sigmoid(a) + sigmoid(b) + sigmoid(c)) * x and, with copy_x, out[:, C:2C] = x (d3d_recon).  a, b, c, x
     contiguous [M, C]; `out` may be columns of a wider tensor."""
-    assert out.stride(1) == 1 and all(t.is_contiguous() and t.shape == x.shape for t in (a, b, c, x))
+    if not recon_ok(a, b, c, x, out):
+        raise ValueError("recon takes contiguous tensors of one shape and type, rows of 16-byte multiples")
     with torch.cuda.device(x.device):
         check("d3d_recon", lib().d3d_recon(_TORCH2D3D[x.dtype], a.data_ptr(), b.data_ptr(), c.data_ptr(), x.data_ptr(),
                                            x.shape[0], x.shape[1], out.data_ptr(), out.stride(0), int(copy_x),
