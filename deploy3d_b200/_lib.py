@@ -117,6 +117,7 @@ SIGNATURES = {
     "d3d_spconv_subm_tables": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_int32), _vpp, _descp, ctypes.c_int,
                                               _vpp, _vp, _sz, _vp, _vp, _vp, ctypes.c_int]),
     "d3d_spconv_subm_tables_clear": (ctypes.c_int, [_descp, ctypes.c_int, _vp, _sz, _vp]),
+    "d3d_spconv_conv_tables_workspace": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int, _szp]),
     "d3d_spconv_conv_tables_grid": (_vp, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int, _vp]),
     "d3d_spconv_conv_tables_clear": (ctypes.c_int, [ctypes.POINTER(SpconvIndexParams), _descp, ctypes.c_int, _vp, _vp,
                                                     _sz, _vp]),

@@ -973,6 +973,7 @@ Plan::Path pick_lookup(const d3d_spconv_index_params* p, const Geometry& g, int6
 
 int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* workspace, Plan* plan,
               bool tables = false) {
+  *plan = Plan();
   D3D_REQUIRE(p && in && n_in >= 3, D3D_ERR_INVALID_ARGUMENT);
   int ndim = p->ndim;
   D3D_REQUIRE(ndim >= 1 && ndim <= D3D_MAX_NDIM, D3D_ERR_INVALID_ARGUMENT);
@@ -1035,6 +1036,10 @@ int make_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n
   plan->table = plan->path == Plan::kDirect ? nullptr : w.take<unsigned long long>(plan->cap_max);
   plan->grid = plan->path == Plan::kDirect ? w.take<int32_t>((size_t)(vol + 63) / 64 * 64) : nullptr;
   plan->bits = plan->path == Plan::kBits ? w.take<uint32_t>((size_t)((vol + 31) / 32 + 63) / 64 * 64) : nullptr;
+  if (tables) {  // a look-up is all they need
+    plan->bytes = w.off;
+    return D3D_OK;
+  }
   plan->pair_out = w.take<int32_t>((size_t)g.kvol * (plan->n_max > 0 ? (size_t)plan->nblk * kIdxThreads : 1));
   plan->list_local = plan->path == Plan::kHash ? nullptr : w.take<uint8_t>((size_t)g.kvol * plan->nblk * kIdxThreads);
   plan->block_counts = w.take<int32_t>((size_t)g.kvol * plan->nblk);
@@ -1130,21 +1135,41 @@ int launch_conv3(const Plan& plan, const int32_t* coors, const int32_t* num_act_
   return D3D_OK;
 }
 
-// Strided tables by ranks (spconv_rank3.cuh), in the memory of the grid; launched plainly, beside other streams' work.
-uint2* rank_words(const Plan& plan) { return reinterpret_cast<uint2*>(plan.grid); }
-int64_t rank_count(const Plan& plan) { return ((plan.cells + 31) / 32 + 3) / 4 * 4; }
+// Strided tables by ranks (spconv_rank3.cuh): the geometry of a rulebook and, as workspace, the words and the voxels per
+// block of words (a tenth and less of the grid of ids a rulebook takes).
+struct RankPlan {
+  Plan plan;
+  bool ok;  // whether the kernel and the grid allow it
+  uint2* words;
+  int64_t count;
+  int32_t* block_counts;
+  unsigned blocks;
+  size_t bytes;
+};
+int make_rank_plan(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* workspace, RankPlan* r) {
+  const int rc = make_plan(p, in, n_in, nullptr, &r->plan);
+  if (rc != D3D_OK) return rc;
+  r->ok = !p->subm && r->plan.path == Plan::kDirect && r->plan.g.kvol <= 32;
+  r->count = ((r->plan.cells + 31) / 32 + 3) / 4 * 4;
+  r->blocks = (unsigned)ceil_div(r->count, kRankWords);
+  Carver w(workspace);
+  r->words = w.take<uint2>((size_t)r->count);  // first: d3d_spconv_conv_tables_grid
+  r->block_counts = w.take<int32_t>(r->blocks);
+  r->bytes = w.off;
+  return D3D_OK;
+}
 // Whether the forward table is filled from the outputs (when the inputs have ranks): no clearing, no atomics, whole columns.
 // Otherwise the inputs scatter into it, and its row masks and output map have to be clear.
 bool walks_outputs(const Geometry& g, const void* voxel_grid) { return voxel_grid && !g.transpose && g.dil[2] < 16; }
 // `words`: the ranks; `fwd`: the forward table will be scattered into.  Nothing here depends on the voxels.
-int clear_rank3(const Plan& plan, bool words, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
+int clear_rank3(const RankPlan& r, bool words, const TableParts* fwd, int64_t fwd_rows, cudaStream_t st) {
   ClearArgs a = {};
-  if (words) a.look.bits = reinterpret_cast<uint32_t*>(plan.grid), a.bit_words = 2 * rank_count(plan);
+  if (words) a.look.bits = reinterpret_cast<uint32_t*>(r.words), a.bit_words = 2 * r.count;
   if (fwd) {
-    a.rows = fwd->row_masks, a.row_words = fwd->tiles * plan.g.kvol * 4;
+    a.rows = fwd->row_masks, a.row_words = fwd->tiles * r.plan.g.kvol * 4;
     a.perm = fwd->perm, a.perm_words = fwd->tiles * 128, a.m_max = fwd_rows;
   }
-  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, (const int32_t*)nullptr, plan.n_max);
+  D3D_LAUNCH3(false, clear3_kernel, clear_grid(a), 256, st, a, (const int32_t*)nullptr, r.plan.n_max);
   return D3D_OK;
 }
 int launch_find_rank3(const RankWalk& walk, const int32_t* coors, const int32_t* num_act, int64_t n_max,
@@ -1462,29 +1487,39 @@ extern "C" int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, 
 }
 
 extern "C" int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in) {
-  Plan plan;
-  if (!p || p->subm || make_plan(p, in, n_in, nullptr, &plan) != D3D_OK) return 0;
-  return plan.path == Plan::kDirect && plan.g.kvol <= 32;
+  RankPlan r;
+  return p && make_rank_plan(p, in, n_in, nullptr, &r) == D3D_OK && r.ok;
+}
+
+extern "C" int d3d_spconv_conv_tables_workspace(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
+                                                size_t* bytes) {
+  D3D_REQUIRE(p && bytes, D3D_ERR_INVALID_ARGUMENT);
+  RankPlan r;
+  const int rc = make_rank_plan(p, in, n_in, nullptr, &r);
+  if (rc != D3D_OK) return rc;
+  D3D_REQUIRE(r.ok, D3D_ERR_INVALID_ARGUMENT);
+  *bytes = r.bytes;
+  return D3D_OK;
 }
 
 extern "C" const void* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                                    void* workspace) {
-  Plan plan;
-  if (!workspace || !d3d_spconv_conv_tables_ok(p, in, n_in) || make_plan(p, in, n_in, workspace, &plan) != D3D_OK)
-    return nullptr;
-  return plan.grid;
+  RankPlan r;
+  if (!workspace || !p || make_rank_plan(p, in, n_in, workspace, &r) != D3D_OK || !r.ok) return nullptr;
+  return r.words;
 }
 
 extern "C" int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                             void* table, void* workspace, size_t workspace_bytes, void* stream) {
   D3D_NVTX_RANGE("d3d_spconv_conv_tables_clear");
-  D3D_REQUIRE(p && d3d_spconv_conv_tables_ok(p, in, n_in) && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
-  Plan plan;
-  int rc = make_plan(p, in, n_in, workspace, &plan);
+  D3D_REQUIRE(p, D3D_ERR_INVALID_ARGUMENT);
+  RankPlan r;
+  int rc = make_rank_plan(p, in, n_in, workspace, &r);
   if (rc != D3D_OK) return rc;
-  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
-  const TableParts fwd = table_parts(table, plan.g.kvol, p->max_num_act_out);
-  rc = clear_rank3(plan, true, table ? &fwd : nullptr, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
+  D3D_REQUIRE(r.ok && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
+  D3D_REQUIRE(workspace && workspace_bytes >= r.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  const TableParts fwd = table_parts(table, r.plan.g.kvol, p->max_num_act_out);
+  rc = clear_rank3(r, true, table ? &fwd : nullptr, p->max_num_act_out, reinterpret_cast<cudaStream_t>(stream));
   if (rc != D3D_OK) return rc;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
@@ -1496,11 +1531,12 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
                                       int32_t* status, const void* voxel_grid, int cleared) {
   D3D_NVTX_RANGE("d3d_spconv_conv_tables");
   D3D_REQUIRE(p && inputs && out_coors && num_act_out && table, D3D_ERR_INVALID_ARGUMENT);
-  Plan plan;
-  int rc = make_plan(p, in, n_in, workspace, &plan);
+  RankPlan r;
+  int rc = make_rank_plan(p, in, n_in, workspace, &r);
   if (rc != D3D_OK) return rc;
-  D3D_REQUIRE(!p->subm && plan.path == Plan::kDirect && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
-  D3D_REQUIRE(workspace && workspace_bytes >= plan.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
+  const Plan& plan = r.plan;
+  D3D_REQUIRE(r.ok && p->max_num_act_out >= 1, D3D_ERR_INVALID_ARGUMENT);
+  D3D_REQUIRE(workspace && workspace_bytes >= r.bytes, D3D_ERR_WORKSPACE_TOO_SMALL);
   const int32_t* coors = reinterpret_cast<const int32_t*>(inputs[0]);
   const int32_t* num_act_in = reinterpret_cast<const int32_t*>(inputs[1]);
   D3D_REQUIRE(coors && num_act_in, D3D_ERR_INVALID_ARGUMENT);
@@ -1519,13 +1555,13 @@ extern "C" int d3d_spconv_conv_tables(const d3d_spconv_index_params* p, const d3
   // d3d_spconv_conv_tables_clear has had no table where a voxel_grid was announced, whatever this kernel makes of it
   const bool clear_table = !walk_outputs && (!cleared || voxel_grid);
   if (!cleared || clear_table) {
-    rc = clear_rank3(plan, !cleared, clear_table ? &fwd : nullptr, max_out, st);
+    rc = clear_rank3(r, !cleared, clear_table ? &fwd : nullptr, max_out, st);
     if (rc != D3D_OK) return rc;
   }
-  uint2* words = rank_words(plan);
-  const int64_t count = rank_count(plan);
-  const unsigned blocks = (unsigned)ceil_div(count, kRankWords);  // <= n_max / 16 + 1, see pick_lookup: fits win_bits
-  int32_t* block_counts = reinterpret_cast<int32_t*>(plan.win_bits);
+  uint2* words = r.words;
+  const int64_t count = r.count;
+  const unsigned blocks = r.blocks;
+  int32_t* block_counts = r.block_counts;
   const bool two = plan.two_taps;
   D3D_LAUNCH3(false, two ? rank_mark3_kernel<2> : rank_mark3_kernel<3>, plan.nblk, kIdxThreads, st, words, coors,
               num_act_in, plan.n_max, g);

@@ -165,11 +165,17 @@ class SPConvIdxPlugin(_Plugin):
         d = [_desc_of(t) for t in inputs]
         return bool(lib().d3d_spconv_conv_tables_ok(ctypes.byref(self.p), desc_array(d), len(d)))
 
+    def _tables_workspace_size(self, in_descs):
+        n = ctypes.c_size_t(0)
+        check("d3d_spconv_conv_tables_workspace", lib().d3d_spconv_conv_tables_workspace(
+            ctypes.byref(self.p), desc_array(in_descs), len(in_descs), ctypes.byref(n)))
+        return n.value
+
     def tables_clear(self, *inputs, table, device, stream=None):
         """The part of `tables` that does not depend on the voxels, ahead of them (d3d_spconv_conv_tables_clear); `inputs`
         give shapes only.  `table`: None when the build will be given a voxel_grid."""
         d = [_desc_of(t) for t in inputs]
-        nbytes = self.workspace_size(d)
+        nbytes = self._tables_workspace_size(d)
         ws = self._get_workspace(nbytes, device)
         with torch.cuda.device(device):
             check("d3d_spconv_conv_tables_clear", lib().d3d_spconv_conv_tables_clear(
@@ -180,7 +186,7 @@ class SPConvIdxPlugin(_Plugin):
         """Address of the look-up of its outputs the last `tables` over such inputs has left in this plugin's workspace;
         raises when there is none."""
         d = [_desc_of(t) for t in inputs]
-        ws = self._filled_workspace(self.workspace_size(d), device)
+        ws = self._filled_workspace(self._tables_workspace_size(d), device)
         return lib().d3d_spconv_conv_tables_grid(ctypes.byref(self.p), desc_array(d), len(d), ws.data_ptr())
 
     def tables(self, *inputs, out_coors, num_act_out, table, table_inverse=None, status=None, stream=None,
@@ -190,7 +196,7 @@ class SPConvIdxPlugin(_Plugin):
         inputs; `cleared`: tables_clear was called for this build."""
         device = inputs[0].device
         d = [_desc_of(t) for t in inputs]
-        nbytes = self.workspace_size(d)
+        nbytes = self._tables_workspace_size(d)
         ws = self._filled_workspace(nbytes, device) if cleared else self._get_workspace(nbytes, device)
         with torch.cuda.device(device):
             check("d3d_spconv_conv_tables", lib().d3d_spconv_conv_tables(

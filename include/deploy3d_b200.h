@@ -173,7 +173,8 @@ int d3d_spconv_index_enqueue_ex(const d3d_spconv_index_params* p, const d3d_tens
  *  d3d_spconv_conv_tables_grid  where in its workspace a strided pass leaves the look-up of its outputs.  Given as
  *      `voxel_grid` (else NULL) to the passes over those voxels they are not inserted again; that workspace must stay
  *      as it was left until then, and d3d_spconv_subm_tables needs none of its own.
- * Workspace: d3d_spconv_subm_tables_workspace; for conv_tables, d3d_spconv_index_workspace. */
+ * Workspace: d3d_spconv_subm_tables_workspace, d3d_spconv_conv_tables_workspace (that of d3d_spconv_index_workspace does
+ * as well: it is larger). */
 int d3d_spconv_subm_tables_workspace(const d3d_tensor_desc* in, int n_in, size_t* bytes);
 int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const* tables, const d3d_tensor_desc* in,
                            int n_in, const void* const* inputs, void* workspace, size_t workspace_bytes, void* stream,
@@ -181,6 +182,7 @@ int d3d_spconv_subm_tables(int n_tables, const int32_t* kernel_size, void* const
 int d3d_spconv_subm_tables_clear(const d3d_tensor_desc* in, int n_in, void* workspace, size_t workspace_bytes,
                                  void* stream);
 int d3d_spconv_conv_tables_ok(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in);
+int d3d_spconv_conv_tables_workspace(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, size_t* bytes);
 const void* d3d_spconv_conv_tables_grid(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in,
                                         void* workspace);
 int d3d_spconv_conv_tables_clear(const d3d_spconv_index_params* p, const d3d_tensor_desc* in, int n_in, void* table,

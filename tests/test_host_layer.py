@@ -161,3 +161,31 @@ def test_arguments_that_change_in_place(operators):
         plug = operators.spconv_mm(*_layer(w, cap=rows))
         assert plug.data_s == operators.data_s_spconv_mm(k, 2, 4, n, True, False, w)
     assert all(operators._plain(key) for key in operators._BY_ARGS)
+
+
+def test_tables_ask_for_what_they_use(d3d):
+    """Strided tables: 8 bytes per 32 cells and a count per 8192 of them; submanifold tables: their look-up.  Not the grid
+    and the pair lists of a rulebook."""
+    import ctypes
+    from deploy3d_b200 import _lib
+    from deploy3d_b200.plugins import SPConvIdxPlugin, _desc_of
+    for shape, n in (([1, 41, 1440, 1440], 300000), ([1, 21, 720, 720], 500000), ([2, 5, 9, 11], 64)):
+        descs = [_desc_of(t) for t in (torch.empty((n, 4), **META), torch.empty(1, **META),
+                                       torch.empty(shape[:1] + [0] + shape[1:], **META))]
+        plug = _strided(d3d)
+        out = [shape[0]] + [(e - 1) // 2 + 1 for e in shape[1:]]
+        cells = out[0] * out[1] * out[2] * out[3]
+        nbytes = plug._tables_workspace_size(descs)
+        assert cells // 4 <= nbytes <= cells // 4 + cells // 2048 + 1024 < plug.workspace_size(descs)
+        size = ctypes.c_size_t(0)
+        _lib.check("workspace", _lib.lib().d3d_spconv_subm_tables_workspace(_lib.desc_array(descs), 3, ctypes.byref(size)))
+        cells = shape[0] * shape[1] * shape[2] * shape[3]
+        if cells <= 64 * n:
+            assert cells * 4 <= size.value <= cells * 4 + 256
+        else:  # a bit per cell and hash slots for four to eight times the rows
+            assert size.value <= cells // 8 + 64 * n + 1024
+    far = [_desc_of(t) for t in (torch.empty((8, 4), **META), torch.empty(1, **META), torch.empty((1, 0, 41, 800, 800), **META))]
+    assert not SPConvIdxPlugin.tables_ok(plug, torch.empty((8, 4), **META), torch.empty(1, **META),
+                                         torch.empty((1, 0, 41, 800, 800), **META))
+    with pytest.raises(_lib.D3DError):
+        plug._tables_workspace_size(far)
