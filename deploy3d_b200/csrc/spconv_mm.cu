@@ -127,7 +127,10 @@ __device__ __forceinline__ unsigned mix32(unsigned x, unsigned m) {
   x *= 0x846ca68bu;
   return x ^ x >> 16;
 }
-// Two 32-bit mixes over different odd multiples (64-bit multiplications cost four times as many instructions).
+// Two 32-bit mixes over different odd multiples (64-bit multiplications cost four times as many instructions).  The constants
+// are published ones: the multiples of `a` and the first two of `b` are the five primes of xxHash32 (Y. Collet), mix32 has the
+// shifts and, for `a`, the multipliers of lowbias32 (C. Wellons, hash-prospector), for `b` the first multiplier of another
+// mixer found there.  Nothing but the spread of the sums depends on them.
 __device__ __forceinline__ unsigned long long entry_mix(int g, int s, int k) {
   const unsigned a = (unsigned)g * 0x9e3779b1u + (unsigned)s * 0x85ebca77u + (unsigned)k * 0xc2b2ae3du;
   const unsigned b = (unsigned)g * 0x27d4eb2fu + (unsigned)s * 0x165667b1u + (unsigned)k * 0xd3a2646du;
