@@ -750,7 +750,7 @@ def main():
                     help="pipelines (buffers + CUDA graph + stream each) that take the frames in turn")
     ap.add_argument("--layers", action="store_true", help="print the per-layer SPConvMM table to stderr")
     ap.add_argument("--tc-plan", type=int, nargs=3, default=None, metavar=("GROUP", "STAGES", "PRODUCER_WARPS"),
-                    help="override the tensor-core kernel's pipeline plan for every layer (0 = automatic)")
+                    help="override the tensor-core kernel's plan for every layer: 16 or 24 producer warps (0 = automatic)")
     ap.add_argument("--regroup", action="store_true",
                     help="rebuild every neighbour table with its outputs grouped by offset mask (d3d_spconv_mm_regroup): "
                          "fewer (tile, offset) blocks for the convolutions, three more kernels per rulebook")

@@ -8,10 +8,8 @@ torch's headers: one translation unit per .cu file, objects cached by content ha
 
 Run as ``python -m deploy3d_b200.build`` or through ``__graft_entry__.build()``.
 
-Tuning builds: ``python -m deploy3d_b200.build --tuning NAME -DD3D_TC_PROFILE [-DD3D_TC_NO_MMA] [-DD3D_TC_NO_COPY]``
-writes ``libs/libdeploy3d_b200_NAME.so`` with the given macros defined for spconv_mm_tc.cu (per-role cycle
-accounting; MMAs / row copies predicated off, which makes the results meaningless and only the timing
-informative).  ``microbench.py --lib NAME`` loads such a build; nothing else does.
+Tuning builds: ``python -m deploy3d_b200.build --tuning NAME -DMACRO ...`` writes ``libs/libdeploy3d_b200_NAME.so``
+with the given macros defined for spconv_mm_tc.cu.  ``microbench.py --lib NAME`` loads such a build; nothing else does.
 
 Checked build: ``python -m deploy3d_b200.build --checked`` writes ``libs/libdeploy3d_b200_checked.so`` with
 ``-DDEPLOY3D_BOUNDS_CHECK -rdc=true`` on every file: every id a kernel indexes with is range-checked and the first

@@ -9,6 +9,7 @@
 //
 // This file holds the host side (blob parsing, weight upload, C ABI) and the SIMT kernel that serves fp32 and
 // channel counts the tensor-core kernel cannot take; spconv_mm_tc.cu holds the tcgen05/TMEM kernel.
+#include <math.h>
 #include <string.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -565,15 +566,29 @@ static void release_device(d3d_spconv_mm_s* h) {
   h->dtype = -1;
 }
 
+// Whether a weight is an infinity or not a number: all exponent bits set.
+static bool not_finite(float v) { return !isfinite(v); }
+static bool not_finite(__half v) { return (__half_as_ushort(v) & 0x7c00u) == 0x7c00u; }
+static bool not_finite(__nv_bfloat16 v) { return (__bfloat16_as_ushort(v) & 0x7f80u) == 0x7f80u; }
+
 template <class T, class Cvt> static int upload_weights(d3d_spconv_mm_s* h, Cvt cvt) {
   const int kvol = h->p.kernel_vol, cin = h->p.in_channels, cout = h->p.out_channels;
   size_t nw = (size_t)kvol * cin * cout;
   std::vector<T> w(nw), wt(nw);
-  for (size_t i = 0; i < nw; ++i) w[i] = cvt(h->wb[i]);
+  bool bad = false;
+  for (size_t i = 0; i < nw; ++i) {
+    w[i] = cvt(h->wb[i]);
+    bad |= not_finite(w[i]);
+  }
+  h->finite = !bad;  // the tensor-core kernel multiplies rows without an input as zeros, so its weights have to be
+  std::vector<int> order(cin);  // of the input channels in a weight row of the tensor-core kernel
+  for (int ci = 0; ci < cin; ++ci) order[ci] = cin == 16 || cin == 32 || cin % 64 == 0 ? spconv_mm_tc_channel(cin, ci) : ci;
   for (int k = 0; k < kvol; ++k)
-    for (int ci = 0; ci < cin; ++ci)
-      for (int co = 0; co < cout; ++co)
-        wt[((size_t)k * cout + co) * cin + ci] = w[((size_t)k * cin + ci) * cout + co];
+    for (int ci = 0; ci < cin; ++ci) {
+      const T* row = &w[((size_t)k * cin + order[ci]) * cout];
+      T* column = &wt[(size_t)k * cout * cin + ci];
+      for (int co = 0; co < cout; ++co) column[(size_t)co * cin] = row[co];
+    }
   if (cudaMalloc(&h->w_dev, nw * sizeof(T)) != cudaSuccess) return D3D_ERR_CUDA;
   if (cudaMalloc(&h->wt_dev, nw * sizeof(T)) != cudaSuccess) return D3D_ERR_CUDA;
   if (cudaMemcpy(h->w_dev, w.data(), nw * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) return D3D_ERR_CUDA;
@@ -771,9 +786,10 @@ static int run(d3d_spconv_mm_t h, int dtype, const void* in_feats, int64_t max_n
   bool tc_ok = spconv_mm_tc_eligible(h, dtype);
   if (h->kernel_choice == 2 || h->kernel_choice == 3) {
     D3D_REQUIRE(tc_ok, D3D_ERR_INVALID_ARGUMENT);
-    return launch_spconv_mm_tc(a);
   }
-  if (h->kernel_choice == 0 && tc_ok) return launch_spconv_mm_tc(a);
+  // weights that are not finite in the compute type: a row without an input would be a zero times an infinity on the
+  // tensor-core path, and there only where it has one
+  if (h->kernel_choice != 1 && tc_ok && h->finite) return launch_spconv_mm_tc(a);
   return launch_spconv_mm_simt(a);
 }
 

@@ -15,6 +15,7 @@ struct d3d_spconv_mm_s {
   void* w_dev = nullptr;     // [kVol][Cin][Cout] in `dtype` (reference layout; SIMT kernel)
   void* wt_dev = nullptr;    // [kVol][Cout][Cin] in `dtype` (K-major B operand of the tcgen05 kernel)
   float* b_dev = nullptr;    // bias in fp32 (zeros when the blob has no bias)
+  bool finite = true;        // every weight is finite in `dtype`
   int kernel_choice = 0;     // 0 auto, 1 SIMT, 2 tcgen05
   int dependent_launch = 0;  // tcgen05 path: launch with the programmatic stream-serialisation attribute
   void* tc_state = nullptr;  // tensor map of the tcgen05 path (owned by spconv_mm_tc.cu, created by configure)
@@ -89,6 +90,8 @@ int launch_spconv_mm_simt(const MmLaunch& a);
 // Returns D3D_ERR_INVALID_ARGUMENT when the shape/dtype is not eligible for the tensor-core path.
 bool spconv_mm_tc_eligible(const d3d_spconv_mm_s* h, int dtype);
 int launch_spconv_mm_tc(const MmLaunch& a);
+// The input channel at position `pos` of a weight row in the order the tensor-core kernel multiplies in.
+int spconv_mm_tc_channel(int cin, int pos);
 // Per-handle state of the tensor-core path: created while configuring (device weights exist), freed with them.
 int spconv_mm_tc_prepare(d3d_spconv_mm_s* h, int dtype);
 void spconv_mm_tc_release(d3d_spconv_mm_s* h);

@@ -1,63 +1,58 @@
 // SPConvMM on the 5th-generation tensor cores: output-stationary implicit GEMM.
 //
 // For a tile of 128 consecutive output voxels and every kernel offset k that feeds at least one of them:
-//   A = the input rows named by the neighbour table, staged in shared memory in the K-major swizzled layout the
-//       tensor core reads -- only the rows that exist: the table carries a 128-bit row mask per (tile, offset),
-//   B = W[k]^T, K-major, loaded by a tiled TMA copy (once per kernel when all offsets fit, else once per stage),
-//   D += A * B with tcgen05.mma (M = 128, N = Cout, K = 16 per instruction), fp32 accumulator in tensor memory,
-//       issued with the inverted row mask as disable_output_lane: accumulator lanes of rows without an input are
-//       not updated, so whatever an unused row of the operand ring holds is never seen (no zero fill).
-// All offsets of a tile accumulate into the same TMEM columns; the epilogue reads them once with tcgen05.ld, adds
-// bias (+ residual), applies ReLU, converts and stores the row, and writes zeros back (tcgen05.st) for the next tile.
-// No atomics, no bias-initialisation pass.
+//   A = the input rows named by the neighbour table, gathered into registers and stored into tensor memory, from where
+//       tcgen05.mma takes its A operand; rows without an input are zeros (the table carries a 128-bit row mask per
+//       (tile, offset), and nothing is loaded for them),
+//   B = W[k]^T, K-major in shared memory, by TMA (once per kernel when all offsets fit into 112 KB, else window by window),
+//   D (+)= A * B (M = 128, N = Cout, K = 16 per instruction), fp32 accumulator in tensor memory.
+// All offsets of a tile accumulate into the same columns, in ascending order; the epilogue reads them once, adds bias
+// (+ residual), applies ReLU, converts and stores the row.  No atomics, no bias-initialisation pass.
 // (The reference: gather iterator + mma.sync tiles of 64 pairs of one offset, fp16 accumulate, half2 atomicAdd
 // scatter, trt/spconv/mm/kernel.h:84-179, mm/output_iterator.h:189-206.)
 //
-// The A rows are gathered with 16-byte cp.async written straight into the swizzled layout.  A TMA tile::gather4
-// producer was measured on B200 at 11.4 ns per gathered row whatever the row width (a request-rate limit), three
-// times slower than cp.async for these row sizes (microbench/gather_rows.cu measures both), and is not used.
+// Why A goes through registers into tensor memory (B200).  From shared memory an M128 K16 MMA takes 46 / 46 / 51 / 64 cycles
+// at N = 16 / 32 / 64 / 128: the tensor core fetches 4 KB of A each time.  From tensor memory it takes 16 / 21 / 32 / 64.
+// Zeros for missing rows cost nothing in registers, so no MMA carries a lane mask.  Plain loads go through L1, which the
+// operand ring in shared memory had taken: in cell order 61-66 % of the gathered bytes are hits (neighbouring offsets and
+// rows of a tile read the same voxels).  And a weight block is fetched once for the two or three tiles a CTA works on
+// together, not once per tile.  Weights have to be finite for that (a row without an input is 0 * W): layers with others
+// take the SIMT kernel.  27 offsets, us per launch, before (rows copied by cp.async into a shared-memory
+// ring, MMAs under lane masks) and now: 16 -> 16 at 281 k voxels 33 / 31, 32 -> 32 at 463 k
+// 81 / 72, 32 -> 64 at 463 k 96 / 77, 64 -> 64 at 238 k 80 / 70, 64 -> 128 101 / 87, 128 -> 128 at 66 k 59 / 51, 256 -> 128 at
+// 50 k 82 / 73, 256 -> 256 115 / 114; nine offsets and 90 k voxels: 64 -> 64 22 / 21, 128 -> 128 36 / 33.
 //
-// What bounds this kernel, measured on B200 (tuning builds with D3D_TC_PROFILE / D3D_TC_NO_MMA / D3D_TC_NO_COPY below,
-// microbench/mma_issue.cu):
-//   * the instruction streams of its roles.  With every MMA and every gather copy predicated off the layers still
-//     take 52-80 % of their time.  One warp that waits for a stage, fences and issues eight M128 K16 MMAs needs about
-//     750 cycles for what the tensor core executes in 320 to 512; two such warps on one SM keep it busy.  A lone
-//     warp issues a dependent instruction every four cycles or so, so what a role executes per stage besides its
-//     copies / MMAs (walking the stage sequence, waits, address arithmetic) costs as much as the work itself.
-//   * for layers of 64 channels and more, weight traffic from L2 (W[k] is fetched again for every tile: as many
-//     bytes as the gathered rows) and the shared-memory data pipe (128 B per clock and SM): every A row is written
-//     once by cp.async and the whole block read once by the tensor core, every B block likewise.
-// Hence:
-//   * layers run TWO CTAs per SM wherever shared and tensor memory allow (two independent issue streams);
-//   * the MMA warp keeps every value that feeds an MMA warp-uniform in a way the compiler can see (offset masks
-//     pass through a shuffle from lane 0), computes all descriptors of a stage first and lets the lane chosen by
-//     elect.sync issue the MMAs as straight-line code; it probes the following stage's barrier before it issues;
-//     the row masks of a tile are loaded a tile ahead and parked, inverted, in shared memory;
-//   * the neighbour ids and row-mask words are read from global memory by the producer lanes themselves, a stage
-//     ahead (and the table lines of the next tile are prefetched into L2), not staged in shared memory;
-//   * the producer warps work in teams of four that take the stages in turn, so that the per-stage overhead of a
-//     warp is paid once per two stages of the pipeline; address arithmetic of all copies of a stage comes first,
-//     the copies follow as independent instruction groups, predicated by the row-mask bit of their row;
-//   * every role loads the offset mask of its next tile while it works on the current one;
-//   * the epilogue handles 16 columns per tensor-memory load (two CTAs of 320 or 448 threads per SM fit).
-// Roles of a CTA, for W = 4 or 8 producer warps:
-//   W producer warps   teams of four; warp q of a team copies rows [32q, 32q + 32) of every A block of the team's
-//                      stages: lane = (row, 16-byte piece), so its shared-memory offsets are constants
-//   1 MMA warp         waits for a stage, one elected lane issues its tcgen05.mma and commits; owns the TMEM allocation
-//   1 control warp     one lane loads B by TMA (all offsets once when they fit, else per stage)
-//   4 epilogue warps   TMEM -> registers -> global, then zeros -> TMEM
+// What bounds it now: the instruction streams of the roles, again.  An SM needs 600 warp instructions for a unit (128 rows x
+// 128 bytes) and issues 1.7 a cycle; a lone warp executes a dependent one every four to six cycles, and a trip through a
+// full memory pipe (a barrier test, a shared-memory load) takes 70 cycles and more.  Hence:
+//   * two or three MMA warps, each with a tile of the round and two producer teams of its own: one warp needs about 450
+//     cycles from one product to the next, whatever the tensor core could do;
+//   * an MMA warp waits and issues in one elected lane, two units at a time, from values that the whole warp has computed
+//     by counters: fed from memory or by a loop of one lane, the compiler cannot keep the descriptors in uniform registers,
+//     and four MMAs with a commit take 273 cycles to issue instead of 74;
+//   * the control warp lists the units of a round, so that a producer finds its next one with a single load;
+//   * a lane of a producer holds two or four rows (rows_per_lane): 16-byte pieces dealt out lane by lane cost four times
+//     the address arithmetic;
+//   * ids, row masks, input and residual rows of the next round are prefetched into L2: the loads run one unit ahead, which
+//     covers L2 but not DRAM (128 -> 128 at 66 k voxels behind other layers: 66.0 us without, 61.4 with).
+// For 128 output channels and more the tensor pipe is busy two thirds of the time, and 128-row tiles round up (520 tiles on
+// 148 SMs are 3.5, so 4).
+//
+// Roles of a CTA (persistent, one per SM) with T = 2 or 3 MMA warps: 8 T producer warps, 4 epilogue warps (8 for T = 2), T MMA
+// warps, 1 control warp (lists, weights by TMA, prefetches).  Units pass through a ring of 2 T slots in tensor memory, one per team
+// of four producer warps (a warp can only write its quarter of the lanes).  Everything is handed over through mbarriers; every
+// wait is bounded (about one second) and on expiry raises an error word, lets the CTA drain and return instead of spinning.
+// A barrier is always waited for by the side that has seen its phase before (same team, same MMA warp, same epilogue warps):
+// a waiter two phases ahead would take the phase before last for the one it waits for.
+//
 // A tile row need not stand for output tile * 128 + row: the table carries the output row of every tile row, and a
 // table rebuilt by d3d_spconv_mm_regroup lists its outputs sorted by offset mask, so that a tile keeps only the few
-// offsets its like outputs share.  For such tables the kernel is instantiated with a second stage walk (kPacked: a
-// stage takes the next offsets that are present instead of a fixed window of offsets) and a tile order that hands
-// every CTA a like share of the costly tiles.
-// Every role derives the stage sequence of a tile from the tile's offset mask (built with the neighbour table), so
-// no per-stage metadata is exchanged.  Stages and accumulators are handed over through mbarriers; every wait is
-// bounded (about one second) and on expiry raises an error word, lets the CTA drain and return instead of spinning.
+// offsets its like outputs share; windows no tile of a round has are left out of it.
 #include <cuda.h>
 
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 #include "common.cuh"
 #include "spconv_mm_internal.h"
@@ -66,61 +61,47 @@ namespace d3d {
 namespace {
 
 constexpr int kTileRows = 128;
-constexpr int kMaxStages = 8;
-constexpr int kNumAcc = 2;
-constexpr int kMaxGroup = 8;  // kernel offsets that may share one pipeline stage
-// Warp roles for W producer warps: producers first, then the MMA warp, the control warp and four epilogue warps
-// (whose index mod 4 covers the four TMEM lane quarters).
-__host__ __device__ constexpr int threads_of(int prod_warps) { return (prod_warps + 6) * 32; }
-constexpr unsigned long long kWaitLimitNs = 1000ull * 1000ull * 1000ull;
+constexpr int kUnitCols = 32;    // tensor-memory columns of one unit of A: 128 rows x 128 bytes
+constexpr int kMaxAcc = 8;       // accumulators in tensor memory
+constexpr int kMaxBSlots = 8;    // weight blocks in flight
+constexpr int kTmemCols = 512;
+constexpr int kMaxMmaWarps = 3;  // MMA warps, each with a tile of the round and two producer teams
+constexpr int kListUnits = 128;  // units of a tile: 32 offsets of four parts
+// Warp roles for T MMA warps: 8 T producer warps (2 T teams of four), four epilogue warps (whose index mod 4 covers the four
+// TMEM lane quarters), the MMA warps and the control warp.
+__host__ __device__ constexpr int epilogue_sets(int mma_warps) { return mma_warps == 2 ? 2 : 1; }
+__host__ __device__ constexpr int threads_of(int mma_warps) { return (9 * mma_warps + 4 * epilogue_sets(mma_warps) + 1) * 32; }
+constexpr long long kWaitLimitCycles = 2000ll * 1000ll * 1000ll;  // about a second
 
 __device__ int g_tc_error;  // 0 ok; otherwise the code of the first wait that gave up
 
-// Tuning builds (python -m deploy3d_b200.build --tuning NAME -D...):
-//   D3D_TC_PROFILE  cycle accounting per role (CTA 0 only), read back with d3d_debug_copy_prof
-//   D3D_TC_NO_MMA   every tcgen05.mma predicated off     } timing experiments: what is left when a part of the
-//   D3D_TC_NO_COPY  every gather copy predicated off     } work is removed (the results are meaningless)
-#ifdef D3D_TC_NO_MMA
-#define D3D_TC_MMA_RUN(run) ((run) & 0u)
-#else
-#define D3D_TC_MMA_RUN(run) (run)
-#endif
-#ifdef D3D_TC_NO_COPY
-#define D3D_TC_COPY_RUN(run) ((run) & 0u)
-#else
-#define D3D_TC_COPY_RUN(run) (run)
-#endif
-#ifdef D3D_TC_PROFILE
-__device__ long long g_prof[3][8];
-#define PROF_DECL long long prof_[8] = {0, 0, 0, 0, 0, 0, 0, 0}; long long tprev_ = clock64();
-#define PROF(x) do { long long n_ = clock64(); prof_[x] += n_ - tprev_; tprev_ = n_; } while (0)
-#define PROF_STORE(role, cond) if (blockIdx.x == 0 && (cond)) for (int i_ = 0; i_ < 8; ++i_) g_prof[role][i_] = prof_[i_];
-#else
-#define PROF_DECL
-#define PROF(x)
-#define PROF_STORE(role, cond)
-#endif
+// How the lanes of a producer warp share its 32 rows of a unit.  Rows of 128 bytes: four lanes to a row, 32 bytes of four
+// rows each -- a load then takes 64 bytes of a line at a time instead of 32, and the L1 data pipe is what these layers run
+// into.  Shorter rows: two lanes to a row, 64 bytes of two rows each (over all offsets of the unit): half the addresses,
+// and the loaded registers are stored as they lie.
+__host__ __device__ constexpr int rows_per_lane(int offs) { return offs == 1 ? 4 : 2; }
 
 struct TcParams {
   const int32_t* table;        // [tiles][kvol][128]
   const uint32_t* tile_mask;   // [tiles] bit k set: offset k feeds the tile
   const uint32_t* row_masks;   // [tiles][kvol][4] bit r of word q set: row 32 q + r has an input under the offset
   const int32_t* perm;         // [tiles][128] output row of every tile row, -1 = none
+  const int32_t* num_out;      // live outputs (may be null): only how the tiles are dealt out depends on it
   const void* in_feats;        // [n_in_rows][cin]
   int64_t m_max;
-  int32_t n_in_rows;  // rows of the gathered tensor (an id outside [0, n_in_rows) = zero row)
+  int32_t n_in_rows;  // rows of the gathered tensor
   int kvol, cin, cout;
   int num_tiles;
-  int stages;
-  uint32_t a_bytes, b_bytes;  // per (offset, K part) block
-  int row_bytes;              // bytes of one smem row = min(cin, 64) * 2
-  int kchunk;                 // input channels per block (cin, or a 64-multiple part of it when cin is large)
-  int kparts;                 // cin / kchunk: blocks per kernel offset
-  int chunks;                 // kchunk / 64 (at least 1): swizzle-span wide column blocks per block
+  int parts;          // units per kernel offset: cin / 64, at least 1
+  int num_acc;        // accumulators
+  int ring_col;       // first tensor-memory column of the ring
+  int regrouped;      // tiles in ascending order of their offset masks: dealt out costly ones first
+  uint32_t b_bytes;   // one weight block: cout rows of row_bytes, per (offset, part)
+  int b_slots;        // ring of weight windows; 0: all kvol blocks stay in shared memory
+  int row_bytes;      // bytes of one weight row of a block = min(cin, 64) * 2
   uint32_t idesc;
   uint32_t layout_type;  // UMMA smem layout code: 6 = 32B, 4 = 64B, 2 = 128B swizzle
-  uint32_t tmem_cols;
-  int b_resident;  // all kvol weight blocks stay in smem for the whole kernel (small layers)
+  const void* weights;  // all of them, in the layout of the tensor map
   const float* bias;
   void* out;
   const void* residual;
@@ -151,7 +132,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Non-blocking test of a barrier phase.
+// Whether the phase is over, without waiting for it.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -163,36 +144,21 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 // Bounded wait.  Returns false (and records `code`) when the barrier did not flip within the limit or another role
 // already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  unsigned long long t0 = global_ns();
-  for (;;) {
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
     if (*abort_flag) return false;
-    if (global_ns() - t0 > kWaitLimitNs) {
+    if (clock64() - t0 > kWaitLimitCycles) {
       *abort_flag = code;
       atomicCAS(&g_tc_error, 0, code);
       return false;
     }
   }
+  return true;
 }
-// One lane waits, the warp learns the outcome.  __syncwarp orders the other lanes' later accesses after the
-// observation of lane 0.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, code) ? 1 : 0;
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-
 __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -200,23 +166,6 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
       : "r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// 16-byte asynchronous copy, predicated on `run` != 0 instead of branched around.  No memory clobber: it touches
-// only the operand ring, which the issuing thread never accesses with ordinary loads or stores, and the compiler may
-// then overlap the id loads of the next stage with these copies.
-__device__ __forceinline__ void cp_async_16_if(uint32_t run, uint32_t dst, const void* src) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %2, 0;\n\t"
-      "@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(dst),
-      "l"(src), "r"(D3D_TC_COPY_RUN(run)));
-}
-// The barrier receives one arrival (counted in its expected arrivals) once all cp.async issued so far by this
-// thread have landed.
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols)
                : "memory");
@@ -247,27 +196,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-// D += A * B on the accumulator lanes whose bit in `off` (lanes 0-31 in .x, ... 96-127 in .w) is clear; the other
-// lanes keep their value whatever the corresponding rows of A hold.  Issued only when `run` != 0 (predicated, not
-// branched around).
-__device__ __forceinline__ void umma_f16_rows_if(uint32_t run, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                                 uint32_t idesc, const uint4& off) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.eq.b32 p, 0, 0;\n\t"
-      "setp.ne.b32 q, %4, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(D3D_TC_MMA_RUN(run)), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w)
-      : "memory");
-}
-// Writes `v` into 16 consecutive columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_st16_same(uint32_t taddr, uint32_t v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
-      ::"r"(taddr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -276,206 +204,216 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for this thread's tensor-memory loads; `r` is what they have loaded.
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
 
+// D (+)= A * B, A in tensor memory.
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Lane t of the warp writes registers 4c, 4c + 1 to columns 8c + 2 (t % 4) and the next of TMEM lane t / 4, registers
+// 4c + 2, 4c + 3 to the same columns of lane t / 4 + 8, for c = 0..3.
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// Lane t of the warp writes register k to column 2k + t / 2 % 2 of TMEM lane t / 4 + 8 * (t % 2), for k = 0..15.
+__device__ __forceinline__ void tmem_st_16x64b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x64b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// Loads 16 (kWords = 4) or 32 bytes (8) where `has`, else leaves v as it is; kWide: 32 bytes in one go, from an address
+// that is a multiple of them.
+template <int kWords, bool kWide> __device__ __forceinline__ void load_words(uint32_t* v, const unsigned char* src, bool has) {
+  if (kWords == 4) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q ld.global.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
+        : "l"(src), "r"((int)has));
+  } else if (kWide) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %9, 0;\n\t"
+        "@q ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+        : "l"(src), "r"((int)has));
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %9, 0;\n\t"
+        "@q ld.global.v4.b32 {%0, %1, %2, %3}, [%8];\n\t"
+        "@q ld.global.v4.b32 {%4, %5, %6, %7}, [%8 + 16];\n\t}"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+        : "l"(src), "r"((int)has));
+  }
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// A unit of work is 128 rows of a tile under the kOffs offsets of a window (one 64-channel part of them).  The producers'
+// list of a round names for every unit the first (tile, offset) block of the table (x) and, in y, the part (bits 0-1) and
+// the number of offsets (at most kOffs, bits 4-6).
 struct __align__(16) Shared {
-  uint64_t full[kMaxStages];   // producers (+ the B load) -> MMA
-  uint64_t empty[kMaxStages];  // MMA (tcgen05.commit) -> producers, control
-  uint64_t acc_full[kNumAcc];
-  uint64_t acc_empty[kNumAcc];
+  uint2 units[2][kMaxMmaWarps][kListUnits];
+  int4 round[2];              // tiles (none: the end), windows, units of a tile
+  uint64_t list_full[2];      // control -> producers, MMA
+  uint64_t list_empty[2];     // producers, MMA -> control
+  uint64_t full[2 * kMaxMmaWarps];   // producers -> MMA
+  uint64_t empty[2 * kMaxMmaWarps];  // MMA (tcgen05.commit) -> producers
+  uint64_t acc_full[kMaxAcc];
+  uint64_t acc_empty[kMaxAcc];
+  uint64_t b_full[kMaxBSlots];
+  uint64_t b_empty[kMaxBSlots];
   uint64_t b_ready;  // resident weights have landed
   uint32_t tmem_base;
   int abort_flag;
-  // row masks of the MMA warp's current and next tile, inverted (bit set = accumulator lane left alone), four words
-  // per kernel offset; sized so that a whole window of kMaxGroup offsets starting below 32 stays inside
-  __align__(16) uint32_t lanes_off[2][(32 + kMaxGroup) * 4];
 };
 
-// Carved dynamic shared memory: [stages x (group A blocks | group B blocks)] aligned to 1024, the resident weights,
-// the bias, the control block.
+// Carved dynamic shared memory: weights (resident blocks or the ring of windows) aligned to 1024, bias, control block.
 struct Smem {
-  unsigned char* tiles;
-  unsigned char* bres;  // resident weights [kvol][b_bytes] (when p.b_resident)
+  unsigned char* weights;
   float* bias;
   Shared* sh;
-  uint32_t stage_bytes;
 };
-template <int kGroup> __device__ __forceinline__ Smem carve_smem(unsigned char* raw, const TcParams& p) {
+template <int kOffs> __device__ __forceinline__ Smem carve_smem(unsigned char* raw, const TcParams& p) {
   Smem s;
-  const uint32_t raw_addr = smem_u32(raw);
-  s.tiles = raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  s.stage_bytes = (uint32_t)kGroup * (p.a_bytes + (p.b_resident ? 0u : p.b_bytes));
-  s.bres = s.tiles + (size_t)p.stages * s.stage_bytes;
-  s.bias = reinterpret_cast<float*>(s.bres + (p.b_resident ? (size_t)p.kvol * p.b_bytes : 0));
+  s.weights = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
+  const size_t blocks = p.b_slots ? (size_t)p.b_slots * 2 * kOffs : (size_t)((p.kvol + kOffs - 1) / kOffs * kOffs);
+  s.bias = reinterpret_cast<float*>(s.weights + blocks * p.b_bytes);
   s.sh = reinterpret_cast<Shared*>(s.bias + ((p.cout + 3) & ~3));
   return s;
 }
 
-// The stage sequence of a tile is derived identically by every role from the tile's offset mask, in ascending order of
-// the offsets, one stage per K part (see stage_bits for the two ways a stage picks its offsets).
-struct StageIter {
-  int tile;
-  int round;           // how many tiles of this CTA came before `tile`
-  uint32_t rest;       // offsets of `tile` not yet handed out, including those of the current stage
-  uint32_t mask_next;  // of the CTA's next tile, loaded while this one is walked (a load per tile is a round trip to L2)
-  uint32_t bits;       // the offsets of the current stage: packed stages, absolute; windows, relative to `base`
-  int base;            // windows only: first offset of the stage's window
-  int part;
+// ---- the order of the work -----------------------------------------------------------------------------------------
+// A CTA takes its tiles in rounds, one for each of its MMA warps; a round walks the windows of kOffs kernel offsets that any of
+// its tiles has, in ascending order (each window in `parts` units of 64 input channels), two (window, part)s at a time: one unit
+// per (window, part, tile).  A weight block is thus used by all tiles of the round while it is in shared memory.  The control
+// warp lists the units of a round for the producers; the MMA warps and the epilogue count along.
+//
+// Rounds cover the live tiles first, in whole rounds and one of the remaining tiles shared out evenly, then whatever lies
+// behind them (tiles no offset feeds).
+struct Round {
+  int start;      // index of the round's first tile over all CTAs
+  int limit;      // tiles below this index belong to it
+  int tiles;      // tiles per CTA
+  uint32_t mask;  // lane i (mod 4): offset mask of the CTA's tile i, 0 = no such tile
 };
-__device__ __forceinline__ uint32_t load_mask(const TcParams& p, int tile) {
-  return tile < p.num_tiles ? __ldg(p.tile_mask + tile) : 0u;
+__device__ __forceinline__ int live_tiles(const TcParams& p) {
+  if (!p.num_out || p.regrouped) return p.num_tiles;
+  const int64_t n = ((int64_t)*reinterpret_cast<const volatile int32_t*>(p.num_out) + kTileRows - 1) / kTileRows;
+  return n < 0 ? 0 : n < p.num_tiles ? (int)n : p.num_tiles;
 }
-// The CTA's tile of round r, or num_tiles when it has none.  A regrouped table holds its tiles in ascending order of
-// their offset masks, the costly ones last: there the CTAs take the tiles round by round from the last tile down, in
-// alternating direction, so that every CTA starts with a costly tile and the rounds pair a CTA's costlier tiles with
-// cheaper ones.
-template <bool kPacked> __device__ __forceinline__ int tile_at(const TcParams& p, int round) {
+// Index of the CTA's tile i in a round, and the tile it stands for.
+__device__ __forceinline__ int tile_index(const TcParams& p, const Round& r, int i) {
   const int g = (int)gridDim.x, c = (int)blockIdx.x;
-  if (!kPacked) {  // plain tables: every tile costs about the same, the CTAs sweep them front to back
-    const int idx = round * g + c;
-    return idx < p.num_tiles ? idx : p.num_tiles;
-  }
-  const int idx = round * g + ((round & 1) ? g - 1 - c : c);
-  return idx < p.num_tiles ? p.num_tiles - 1 - idx : p.num_tiles;
+  if (!p.regrouped) return r.start + c * r.tiles + i;
+  return r.start + i * g + ((i & 1) ? g - 1 - c : c);
 }
-// Two ways a stage picks its offsets.  kPacked: the kGroup lowest offsets still present (tables whose outputs were
-// regrouped have few offsets per tile, anywhere among the kVol).  Otherwise: the present offsets of the next window
-// of kGroup consecutive offsets that has any -- a plain table has nearly all offsets in every tile, and with fixed
-// windows the offset of slot e is window + e, so every address is the window's plus a constant.
-template <int kGroup> __device__ __forceinline__ uint32_t lowest_bits(uint32_t m) {
-  uint32_t r = m;
-#pragma unroll
-  for (int e = 0; e < kGroup; ++e) r &= r - 1u;
-  return m & ~r;
+__device__ __forceinline__ int tile_of(const TcParams& p, int index) {
+  return p.regrouped ? p.num_tiles - 1 - index : index;
 }
-// Offset of every slot of a stage (always a valid index) and, as bit e of the result, whether slot e is in use.
-template <int kGroup, bool kPacked>
-__device__ __forceinline__ uint32_t slot_offsets(uint32_t bits, int base, int (&k)[kGroup]) {
-  if (kPacked) {
-    const uint32_t used = (1u << __popc(bits)) - 1u;
-#pragma unroll
-    for (int e = 0; e < kGroup; ++e) {
-      k[e] = bits ? __ffs(bits) - 1 : 0;
-      bits &= bits - 1u;
-    }
-    return used;
-  }
-#pragma unroll
-  for (int e = 0; e < kGroup; ++e) k[e] = base + e;
-  return bits;
+template <int kMma> __device__ __forceinline__ void open_round(const TcParams& p, int live, int start, Round& r) {
+  const int g = (int)gridDim.x;
+  r.start = start;
+  r.limit = start < live ? live : p.num_tiles;
+  // With few accumulators one tile at a time: an MMA warp that had no tile in the round before must not be able to wait for
+  // an accumulator whose use before last has not been read yet -- the phase would be taken for the one it waits for.  It is
+  // at most 2 kMma - 2 tiles ahead of the first tile that another warp may still be at.
+  const int rest = r.limit - start, most = p.num_acc >= 2 * kMma - 1 ? kMma : 1;
+  r.tiles = rest >= most * g ? most : rest <= 0 ? 0 : (rest + g - 1) / g;
+  const int i = threadIdx.x & 3;
+  const int index = tile_index(p, r, i);
+  r.mask = (i < r.tiles && index < r.limit) ? __ldg(p.tile_mask + tile_of(p, index)) : 0u;
 }
-template <int kGroup, bool kPacked> __device__ __forceinline__ void first_tile(const TcParams& p, StageIter& it) {
-  it.round = 0;
-  it.tile = tile_at<kPacked>(p, 0);
-  it.rest = load_mask(p, it.tile);
-  it.mask_next = load_mask(p, tile_at<kPacked>(p, 1));
-  it.bits = 0;
-  it.base = -kGroup;
-  it.part = p.kparts - 1;
+__device__ __forceinline__ int after_round(const Round& r) {
+  const int next = r.start + r.tiles * (int)gridDim.x;
+  return next < r.limit ? next : r.limit;
 }
-// Moves to the next stage of this CTA's tiles; false when there is none.
-template <int kGroup, bool kPacked> __device__ __forceinline__ bool next_stage(const TcParams& p, StageIter& it) {
-  constexpr uint32_t gmask = (1u << kGroup) - 1u;
-  if (++it.part < p.kparts) return true;
-  it.part = 0;
-  if (kPacked) it.rest &= ~it.bits;
-  else it.base += kGroup;
-  for (;;) {
-    if (it.tile >= p.num_tiles) return false;
-    if (kPacked) {
-      if (it.rest) {
-        it.bits = lowest_bits<kGroup>(it.rest);
-        return true;
-      }
-    } else {
-      while (it.base < p.kvol) {
-        const uint32_t take = (it.rest >> it.base) & gmask;
-        if (take) {
-          it.bits = take;
-          return true;
-        }
-        it.base += kGroup;
-      }
-      it.base = 0;
-    }
-    if (kPacked) {
-      it.tile = tile_at<true>(p, ++it.round);
-      it.rest = it.mask_next;
-      it.mask_next = load_mask(p, tile_at<true>(p, it.round + 1));
-    } else {  // front to back: the next tile is gridDim.x further
-      it.tile += gridDim.x;
-      it.rest = it.mask_next;
-      it.mask_next = load_mask(p, it.tile + (int)gridDim.x);
-    }
-  }
-}
-
-// 16 accumulator columns starting at col0 of this thread's row: bias (+ residual), ReLU, convert, two 16-byte stores.
-template <bool kBf16>
-__device__ __forceinline__ void store_chunk(const uint32_t* acc, const float* bias_s, int col0, void* out_row,
-                                            const void* res_row, int relu) {
-  float v[16];
+// 16 accumulator columns of this thread's row: bias (+ residual), ReLU, convert, 32 bytes stored.  Two columns to an
+// instruction where there is one for it: this runs on four warps that share the SM's issue slots with all producers.
+template <bool kBf16, bool kAdd>
+__device__ __forceinline__ void store_chunk(const uint32_t (&acc)[16], const float* bias_s, unsigned short* o,
+                                            const uint4 (&res)[2], int relu, bool wide) {
+  uint32_t w[8];
+  const uint4* b4 = reinterpret_cast<const uint4*>(bias_s);
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc[j]) + bias_s[col0 + j];
-  if (relu == 2) {  // activation before the residual is added (sum of two activated branches)
+  for (int q = 0; q < 4; ++q) {
+    const uint4 b = b4[q];
+    const uint32_t bb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.f);
-  }
-  if (res_row) {
-    const uint4* r4 = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(res_row) + col0);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      uint4 raw = __ldg(r4 + q);
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float lo, hi;
+    for (int h = 0; h < 2; ++h) {
+      float x, y;
+      asm("{\n\t.reg .b64 s, t;\n\tmov.b64 s, {%2, %3};\n\tmov.b64 t, {%4, %5};\n\tadd.rn.f32x2 s, s, t;\n\t"
+          "mov.b64 {%0, %1}, s;\n\t}"
+          : "=f"(x), "=f"(y)
+          : "r"(acc[4 * q + 2 * h]), "r"(acc[4 * q + 2 * h + 1]), "r"(bb[2 * h]), "r"(bb[2 * h + 1]));
+      if (kAdd) {
+        const uint4& r4 = res[q / 2];
+        const uint32_t r = q % 2 == 0 ? (h == 0 ? r4.x : r4.y) : (h == 0 ? r4.z : r4.w);
+        if (relu == 2) x = fmaxf(x, 0.f), y = fmaxf(y, 0.f);  // activation before the residual is added
         if (kBf16) {
-          lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xFFFF0000u);
+          x += __uint_as_float(r << 16), y += __uint_as_float(r & 0xFFFF0000u);
         } else {
-          __half2 h = *reinterpret_cast<const __half2*>(&w[e]);
-          lo = __low2float(h), hi = __high2float(h);
+          const __half2 hh = *reinterpret_cast<const __half2*>(&r);
+          x += __low2float(hh), y += __high2float(hh);
         }
-        v[q * 8 + 2 * e] += lo, v[q * 8 + 2 * e + 1] += hi;
+      }
+      // the activation after the rounding: the same values (the maximum of a NaN and zero is zero either way)
+      const bool clamp = relu == 1 || (relu == 2 && !kAdd);
+      if (kBf16) {
+        __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
+        if (clamp) t = __hmax2(t, __float2bfloat162_rn(0.f));
+        w[2 * q + h] = *reinterpret_cast<uint32_t*>(&t);
+      } else {
+        __half2 t = __floats2half2_rn(x, y);
+        if (clamp) t = __hmax2(t, __float2half2_rn(0.f));
+        w[2 * q + h] = *reinterpret_cast<uint32_t*>(&t);
       }
     }
   }
-  uint4* o4 = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(out_row) + col0);
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    uint32_t w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float a = v[q * 8 + 2 * e], b = v[q * 8 + 2 * e + 1];
-      if (relu == 1) a = fmaxf(a, 0.f), b = fmaxf(b, 0.f);
-      if (kBf16) {
-        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        w[e] = *reinterpret_cast<uint32_t*>(&h);
-      } else {
-        __half2 h = __floats2half2_rn(a, b);
-        w[e] = *reinterpret_cast<uint32_t*>(&h);
-      }
-    }
-    o4[q] = make_uint4(w[0], w[1], w[2], w[3]);
+  if (wide) {  // a whole sector
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+  } else {
+    uint4* o4 = reinterpret_cast<uint4*>(o);
+    o4[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    o4[1] = make_uint4(w[4], w[5], w[6], w[7]);
   }
 }
 
 // Barrier initialisation, bias staging and the TMEM allocation (by the MMA warp); returns the TMEM base address.
-template <int kProdWarps>
+template <int kMma>
 __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) {
   Shared* sh = s.sh;
   if (threadIdx.x == 0) {
-    // a stage is full once every producer thread's copies have landed and, when B travels with the stage, its
-    // TMA bytes too (the control warp's expect_tx arrival)
-    const int full_count = kTileRows + (p.b_resident ? 0 : 1);  // the four warps of one producer team
-    for (int i = 0; i < p.stages; ++i) mbar_init(&sh->full[i], full_count), mbar_init(&sh->empty[i], 1);
-    for (int a = 0; a < kNumAcc; ++a) mbar_init(&sh->acc_full[a], 1), mbar_init(&sh->acc_empty[a], 4);
+    for (int i = 0; i < 2 * kMma; ++i) mbar_init(&sh->full[i], 4), mbar_init(&sh->empty[i], 1);
+    for (int a = 0; a < p.num_acc; ++a) mbar_init(&sh->acc_full[a], 1), mbar_init(&sh->acc_empty[a], 4 * epilogue_sets(kMma));
+    for (int b = 0; b < p.b_slots; ++b) mbar_init(&sh->b_full[b], 1), mbar_init(&sh->b_empty[b], kMma);
+    for (int l = 0; l < 2; ++l) mbar_init(&sh->list_full[l], 1), mbar_init(&sh->list_empty[l], 9 * kMma);
     mbar_init(&sh->b_ready, 1);
     sh->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int c = threadIdx.x; c < p.cout; c += blockDim.x) s.bias[c] = p.bias[c];
-  if ((int)(threadIdx.x >> 5) == kProdWarps) tmem_alloc(&sh->tmem_base, p.tmem_cols);
+  if ((int)(threadIdx.x >> 5) == 8 * kMma + 4 * epilogue_sets(kMma)) tmem_alloc(&sh->tmem_base, kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -483,438 +421,450 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
 }
 
 // All roles meet, then the allocating warp returns the tensor memory.
-template <int kProdWarps>
+template <int kMma>
 __device__ __forceinline__ void cta_teardown(const TcParams& p, uint32_t tmem_base) {
   tc_fence_before();
   __syncthreads();
-  if ((int)(threadIdx.x >> 5) == kProdWarps) {
+  if ((int)(threadIdx.x >> 5) == 8 * kMma + 4 * epilogue_sets(kMma)) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, p.tmem_cols);
+    tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-// ---- producers ---------------------------------------------------------------------------------------------------
-// kPieces = 16-byte pieces per row of a 64-column block (2, 4 or 8), kChunks = 64-column blocks per A block.
-// The producer warps form teams of four; a team fills a whole stage (warp q of the team copies rows [32q, 32q + 32)
-// of every block) and the teams take the stages in turn.  What a warp spends per stage besides the copies -- walking
-// the stage sequence, loading ids, waiting for the slot -- is then paid once per kTeams stages of the pipeline.
-// A warp instruction covers 32 / kPieces whole rows (lane = row * kPieces + piece: whole rows on the global side,
-// whole swizzle spans on the shared side); because a pass advances by a multiple of 4 rows and the warp's first row by
-// a multiple of 32, the XOR swizzle term of the destination is a per-lane constant (128-byte rows: two constants,
-// by pass parity).  Only rows that have an input are copied: the row mask of the (tile, offset, quarter) -- one word,
-// the same for the whole warp -- predicates the copies, and the MMA warp keeps the other accumulator lanes out of the
-// product, so whatever an unused row of the ring holds is never seen.  Ids and row masks come straight from global
-// memory; the loads of the team's next stage are issued before the copies of this one.
-template <int kPieces, int kChunks, int kGroup, int kProdWarps, bool kPacked>
-__device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, int warp, int lane) {
-  constexpr int kTeams = kProdWarps / 4;
-  constexpr int kRows = 32;                   // rows of a block per warp
-  constexpr int kRowsPerPass = 32 / kPieces;  // 16, 8 or 4
-  constexpr int kPasses = kRows / kRowsPerPass;
-  constexpr int kRowBytes = kPieces * 16;
-  constexpr uint32_t kChunkBytes = kTileRows * kRowBytes;      // one 64-column block
-  constexpr uint32_t kBlockBytes = kChunkBytes * kChunks;      // = p.a_bytes
-  constexpr int kSwzShift = kRowBytes == 128 ? 0 : kRowBytes == 64 ? 1 : 2;
-  constexpr int kSwzMask = kRowBytes == 128 ? 7 : kRowBytes == 64 ? 3 : 1;
+// ---- producers -------------------------------------------------------------------------------------------------------
+template <int kOffs, bool kWide, int kMma>
+__device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int warp, int lane) {
+  constexpr int kRows = rows_per_lane(kOffs);
+  constexpr int kWords = kOffs == 4 ? 4 : 8;               // 32-bit words a lane loads at a time
+  constexpr int kLoads = 32 / (kRows * kOffs * kWords);    // loads per row and offset
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
   const int team = warp / 4, quarter = warp % 4;
-  const int j = lane % kPieces, rsub = lane / kPieces;
-  const int row0 = kRows * quarter + rsub;  // the row this lane copies in pass 0
-  const uint32_t dst_lane =
-      (uint32_t)row0 * kRowBytes + ((uint32_t)(j ^ ((row0 >> kSwzShift) & kSwzMask)) << 4);
-  const unsigned char* src_j = reinterpret_cast<const unsigned char*>(p.in_feats) + j * 16;
-  const uint32_t row_src_bytes = (uint32_t)p.cin * 2;
+  // this lane reads piece `piece` of tile rows 32 * quarter + row0 and the next (kRows of them)
+  const int row0 = kRows == 4 ? lane >> 2 << 2 : 4 * (lane >> 2) + 2 * (lane & 1);
+  const int piece = kRows == 4 ? lane & 3 : lane >> 1 & 1;
+  const unsigned char* src_lane = reinterpret_cast<const unsigned char*>(p.in_feats) + piece * (kWords * 4);
+  const int32_t* ids_lane = p.table + quarter * 32 + row0;
+  const uint32_t* rows_lane = p.row_masks + quarter;
+  const uint32_t row_bytes = (uint32_t)p.cin * 2;
   const uint32_t last_in_row = (uint32_t)p.n_in_rows - 1u;
-  const uint32_t tiles_addr = smem_u32(s.tiles);
+  const uint32_t dst = tmem_base + (uint32_t)(p.ring_col + team * kUnitCols) + ((uint32_t)(quarter * 32) << 16);
 
-  struct Ids {
-    int id[kGroup][kPasses];
-    uint32_t rows[kGroup];  // row mask word of this warp's quarter, 0 for an offset the stage does not take
-  };
-  auto load_ids = [&](const StageIter& it, Ids& v) {
-    const int64_t blk0 = (int64_t)it.tile * p.kvol;
-    if (kPacked) {
-      int k[kGroup];
-      const uint32_t used = slot_offsets<kGroup, true>(it.bits, 0, k);
-#pragma unroll
-      for (int e = 0; e < kGroup; ++e) {
-        const bool take = (used >> e) & 1u;
-        const int32_t* base = p.table + (blk0 + k[e]) * kTileRows + row0;
-        v.rows[e] = take ? __ldg(p.row_masks + (blk0 + k[e]) * 4 + quarter) : 0u;
-#pragma unroll
-        for (int i = 0; i < kPasses; ++i) v.id[e][i] = take ? __ldg(base + i * kRowsPerPass) : -1;
+  const int owner = team % kMma;  // the MMA warp this team works for
+  int buf = 0, n = team / kMma, len = 0;  // the unit's place in that warp's list
+  uint32_t list_phase = 0;
+  bool open = false;  // list `buf` is out
+  enum { kUnit, kLater, kEnd };
+  // Makes list[n] a unit, going to the next rounds if need be.  Does not wait for a list unless `block`: with a unit in
+  // hand that would be a deadlock, for the next list comes after the last weights of this one.
+  auto settle = [&](bool block) -> int {
+    while (!open || n >= len) {
+      if (open) {  // done with this one
+        n -= len;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->list_empty[buf]);
+        if (buf) list_phase ^= 1;
+        buf ^= 1;
+        open = false;
       }
-    } else {  // the window's blocks follow each other in the table: constant offsets from its first block
-      const int32_t* base = p.table + (blk0 + it.base) * kTileRows + row0;
-      const uint32_t* rows = p.row_masks + (blk0 + it.base) * 4 + quarter;
+      if (!block && !__all_sync(0xffffffffu, mbar_test(&sh->list_full[buf], list_phase))) return kLater;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 13))) return kEnd;
+      const int4 round = sh->round[buf];
+      if (round.x == 0) return kEnd;
+      len = owner < round.x ? round.z : 0;
+      open = true;
+    }
+    return kUnit;
+  };
+  struct Unit {
+    int32_t id[kOffs][kRows];
+    uint32_t rows[kOffs];  // bit i: row i of the quarter has an input under the offset
+    int part;
+  } cur;
+  auto load_unit = [&]() {
+    const uint2 e = sh->units[buf][owner][n];
+    cur.part = e.y & 3u;
+    const int offs = (int)(e.y >> 4);
+    const int32_t* ids = ids_lane + (int64_t)e.x * kTileRows;
+    const uint32_t* rows = rows_lane + (int64_t)e.x * 4;
 #pragma unroll
-      for (int e = 0; e < kGroup; ++e) {
-        const bool take = (it.bits >> e) & 1u;
-        v.rows[e] = take ? __ldg(rows + e * 4) : 0u;
-#pragma unroll
-        for (int i = 0; i < kPasses; ++i) v.id[e][i] = take ? __ldg(base + e * kTileRows + i * kRowsPerPass) : -1;
+    for (int o = 0; o < kOffs; ++o) {
+      const bool in = o == 0 || o < offs;
+      if (kRows == 4) {
+        const int4 q = in ? __ldg(reinterpret_cast<const int4*>(ids + o * kTileRows)) : make_int4(0, 0, 0, 0);
+        cur.id[o][0] = q.x, cur.id[o][1] = q.y, cur.id[o][kRows - 2] = q.z, cur.id[o][kRows - 1] = q.w;
+      } else {
+        const int2 q = in ? __ldg(reinterpret_cast<const int2*>(ids + o * kTileRows)) : make_int2(0, 0);
+        cur.id[o][0] = q.x, cur.id[o][1] = q.y;
       }
+      cur.rows[o] = in ? __ldg(rows + o * 4) : 0u;
     }
-  };
-  // the neighbour ids of a tile are kvol * 512 contiguous bytes: one 128-byte line per lane of a team
-  auto prefetch_ids = [&](int tile) {
-    const int line = quarter * 32 + lane;
-    if (tile < p.num_tiles && line < p.kvol * 4) {
-      const int32_t* a = p.table + (int64_t)tile * p.kvol * kTileRows + line * 32;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-    }
-  };
-  // the team's next stage: kTeams stages further in the sequence
-  auto next_own = [&](StageIter& it) -> bool {
-#pragma unroll
-    for (int t = 0; t < kTeams; ++t)
-      if (!next_stage<kGroup, kPacked>(p, it)) return false;
-    return true;
   };
   pdl_wait();  // masks, ids and features may come from the preceding kernels
-  prefetch_ids(tile_at<kPacked>(p, 1));
-  int stage = team;  // slot of the team's current stage (at least two stages exist)
-  uint32_t phase = 0;
-  PROF_DECL
-  // One stage: find the team's stage after `cur` and start the loads of its ids, then wait for the slot and copy
-  // `cur`.  Returns false when `cur` was the team's last stage or a wait gave up.
-  auto step = [&](const StageIter& cur, const Ids& ids, StageIter& nxt, Ids& ids_next) -> bool {
-    PROF(0);
-    nxt = cur;
-    const bool have_next = next_own(nxt);
-    if (have_next) load_ids(nxt, ids_next);
-    // on entering a tile, pull the ids of the CTA's next tile towards the SM: they may come from DRAM, which takes
-    // longer than the one stage the loads above run ahead
-    if (have_next && nxt.tile != cur.tile)
-      prefetch_ids(kPacked ? tile_at<true>(p, nxt.round + 1) : nxt.tile + (int)gridDim.x);
-    PROF(1);
-    if (!mbar_wait_warp(&sh->empty[stage], phase ^ 1, abort_flag, 12)) return false;
-    PROF(2);
-    const unsigned char* src_part = src_j + (size_t)cur.part * p.kchunk * 2;
-    const uint32_t dst = tiles_addr + (uint32_t)stage * s.stage_bytes + dst_lane;
-    // A lone warp issues a dependent instruction every four cycles or so, and the copies (volatile asm) keep their
-    // order: so the source addresses of all copies of the stage come first -- independent chains the scheduler can
-    // interleave -- and the copies themselves follow as short, independent instruction groups.  An id without an
-    // input (-1) or beyond the tensor is clamped to the last row: its address stays inside the tensor whether or
-    // not the copy is predicated off.
-    const unsigned char* src[kGroup][kPasses];
+  uint32_t phase = 1;
+  int next = settle(true);
+  if (next == kUnit) load_unit();
+  while (next == kUnit) {
+    uint32_t v[kRows][32 / kRows];  // the words of the lane's rows
+    const unsigned char* src = src_lane + cur.part * 128;
 #pragma unroll
-    for (int e = 0; e < kGroup; ++e)
+    for (int i = 0; i < kRows; ++i)
 #pragma unroll
-      for (int i = 0; i < kPasses; ++i)
-      {
-#ifdef DEPLOY3D_BOUNDS_CHECK  // ids of rows that have an input (the others are unspecified) are recorded when off
-        if ((ids.rows[e] >> (rsub + i * kRowsPerPass)) & 1u)
-          (void)D3D_BOUNDS_OK(ids.id[e][i], 0, (long long)last_in_row + 1, kSiteMmTcId);
+      for (int q = 0; q < 32 / kRows; ++q) v[i][q] = 0u;
+#pragma unroll
+    for (int o = 0; o < kOffs; ++o) {
+      const uint32_t rows = cur.rows[o] >> row0;
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        const bool has = (rows >> i) & 1u;
+#ifdef DEPLOY3D_BOUNDS_CHECK
+        if (has) (void)D3D_BOUNDS_OK(cur.id[o][i], 0, (long long)last_in_row + 1, kSiteMmTcId);
 #endif
-        src[e][i] = src_part + (uint64_t)min((uint32_t)ids.id[e][i], last_in_row) * row_src_bytes;
-      }
+        // an id beyond the tensor is clamped to its last row
+        const unsigned char* row = src + (uint64_t)min((uint32_t)cur.id[o][i], last_in_row) * row_bytes;
 #pragma unroll
-    for (int e = 0; e < kGroup; ++e) {
-      const uint32_t mine = ids.rows[e] >> rsub;  // bit i * kRowsPerPass: this lane's row of pass i
-#pragma unroll
-      for (int i = 0; i < kPasses; ++i) {
-        const uint32_t d = (kRowBytes == 128 ? (dst ^ (uint32_t)((i & 1) << 6)) : dst) +
-                           (uint32_t)(e * kBlockBytes + i * kRowsPerPass * kRowBytes);
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c)
-          cp_async_16_if(mine & (1u << (i * kRowsPerPass)), d + c * kChunkBytes, src[e][i] + c * 128);
+        for (int c = 0; c < kLoads; ++c)
+          load_words<kWords, kWide>(&v[i][(o * kLoads + c) * kWords], row + c * 64, has);
       }
     }
-    cp_async_arrive(&sh->full[stage]);  // one arrival per producer thread once its copies have landed
-    PROF(3);
+    n += 2;
+    next = settle(false);
+    if (next == kUnit) load_unit();  // in flight while this unit's rows arrive
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->empty[team], phase, abort_flag, 12))) return;
+    tc_fence_after();
+    if constexpr (kRows == 4) {
 #pragma unroll
-    for (int t = 0; t < kTeams; ++t)
-      if (++stage == p.stages) stage = 0, phase ^= 1;
-    return have_next;
-  };
-  // two id buffers used in turn: the loaded ids are first touched a whole stage after their loads were issued
-  StageIter it_a, it_b;
-  Ids ids_a, ids_b;
-  first_tile<kGroup, kPacked>(p, it_a);
-  bool have = true;
-  for (int t = 0; t <= team && have; ++t) have = next_stage<kGroup, kPacked>(p, it_a);
-  if (have) {
-    load_ids(it_a, ids_a);
-    while (step(it_a, ids_a, it_b, ids_b) && step(it_b, ids_b, it_a, ids_a)) {
-    }
-  }
-  PROF_STORE(0, warp == 0 && lane == 0)
-}
-
-// ---- control warp (one lane) ---------------------------------------------------------------------------------------
-// Brings in the weights: all of them once when they are resident, else the blocks of every stage as soon as the
-// stage is free.
-template <int kGroup, bool kPacked>
-__device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b) {
-  Shared* sh = s.sh;
-  volatile int* abort_flag = &sh->abort_flag;
-  const uint32_t b_tx = (uint32_t)p.cout * p.kchunk * 2;
-  if ((int)blockIdx.x >= p.num_tiles) return;
-  // the weights are constants of the layer: their load does not wait for the preceding kernel
-  if (p.b_resident) {  // in the layout the per-stage loads would have produced
-    mbar_arrive_expect_tx(&sh->b_ready, (uint32_t)p.kvol * b_tx);
-    for (int k = 0; k < p.kvol; ++k)
-      for (int c = 0; c < p.chunks; ++c)
-        tma_load_2d(map_b, &sh->b_ready, s.bres + (size_t)k * p.b_bytes + (size_t)c * p.cout * p.row_bytes, c * 64,
-                    k * p.cout);
-    return;
-  }
-  pdl_wait();  // the offset masks come from the preceding kernels
-  StageIter it;
-  first_tile<kGroup, kPacked>(p, it);
-  int stage = 0;
-  uint32_t phase = 0;
-  while (next_stage<kGroup, kPacked>(p, it)) {
-    if (!mbar_wait(&sh->empty[stage], phase ^ 1, abort_flag, 11)) return;
-    mbar_arrive_expect_tx(&sh->full[stage], (uint32_t)__popc(it.bits) * b_tx);
-    unsigned char* b_dst = s.tiles + (size_t)stage * s.stage_bytes + (size_t)kGroup * p.a_bytes;
-    int k[kGroup];
-    const uint32_t used = slot_offsets<kGroup, kPacked>(it.bits, it.base, k);
+      for (int h = 0; h < 2; ++h) {  // rows 0, 1 and 2, 3, interleaved by two words
+        uint32_t w[16];
 #pragma unroll
-    for (int e = 0; e < kGroup; ++e, b_dst += p.b_bytes) {
-      if (!((used >> e) & 1u)) continue;
-      for (int c = 0; c < p.chunks; ++c)
-        tma_load_2d(map_b, &sh->full[stage], b_dst + (size_t)c * p.cout * p.row_bytes,
-                    it.part * p.kchunk + c * 64, k[e] * p.cout);
+        for (int q = 0; q < 16; ++q) w[q] = v[2 * h + (q >> 1 & 1)][(q >> 2) * 2 + (q & 1)];
+        tmem_st_16x256b_x4(dst + ((uint32_t)(16 * h) << 16), w);
+      }
+    } else {
+      tmem_st_16x64b_x16(dst, v[0]);
+      tmem_st_16x64b_x16(dst + (16u << 16), v[kRows - 1]);
     }
-    if (++stage == p.stages) stage = 0, phase ^= 1;
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->full[team]);
+    phase ^= 1;
+    if (next == kLater && (next = settle(true)) == kUnit) load_unit();
   }
 }
 
-// ---- MMA warp ----------------------------------------------------------------------------------------------------
+// ---- control warp ----------------------------------------------------------------------------------------------------
 // Low word of a K-major operand descriptor: start address in 16-byte units, leading byte offset 1 (unused for the
 // swizzled K-major layouts).  Advancing the operand by `d` bytes adds d / 16 to this word.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 
-// The whole warp walks the stage sequence; everything an MMA depends on (offset mask, stage slot) is kept
-// warp-uniform in a form the compiler can see -- the mask goes through a shuffle from lane 0 -- so that descriptor
-// arithmetic stays in the uniform datapath; one elected lane issues the straight line of predicated MMAs of a stage
-// and the commit.  Every MMA accumulates (the epilogue hands the accumulators over zeroed) and updates only the
-// accumulator lanes of rows that have an input under its offset: the row masks of a tile are loaded a tile ahead
-// (one coalesced load per 32 words), parked inverted in shared memory, and the issuing lane reads four words per offset.
-template <int kPieces, int kChunks, int kGroup, bool kPacked>
-__device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base) {
-  constexpr int kSteps = kPieces * kChunks / 2;  // tcgen05.mma instructions (K = 16 each) per block
-  constexpr uint32_t kRowBytes = kPieces * 16;
-  constexpr uint32_t a_step = (kTileRows * kRowBytes * kChunks) >> 4;  // = p.a_bytes / 16
-  constexpr uint32_t cs_a = (kTileRows * kRowBytes) >> 4;              // between the 64-column blocks of A
-  Shared* sh = s.sh;
-  volatile int* abort_flag = &sh->abort_flag;
-  const int lane = threadIdx.x & 31;
-  // descriptor high word: stride between 8-row groups, version, swizzle mode
-  const uint64_t desc_hi = (uint64_t)(((8u * kRowBytes) >> 4) | (1u << 14) | (p.layout_type << 29)) << 32;
-  const uint32_t cs_b = (uint32_t)(p.cout * kRowBytes) >> 4;
-  const uint32_t b_step = p.b_bytes >> 4, stage_step = s.stage_bytes >> 4;
-  const uint32_t tiles_lo = desc_lo(smem_u32(s.tiles)), bres_lo = desc_lo(smem_u32(s.bres));
-  const uint32_t idesc = p.idesc;
-  const bool resident = p.b_resident != 0;
-  if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23))) return;
-  int stage = 0, acc = 0, buf = 0;
-  uint32_t phase = 0, acc_phase = 0;
-  const int num_stages = p.stages, kparts = p.kparts;
-  const int row_words = p.kvol * 4;  // at most 128
-  bool landed = false;  // the stage about to be waited for was already seen full by the probe below
-  pdl_wait();
-  PROF_DECL
-  uint32_t rows_ahead[4];
-  auto load_rows = [&](int tile) {
-    const uint32_t* w = p.row_masks + (int64_t)tile * row_words + lane;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      rows_ahead[i] = (tile < p.num_tiles && lane + 32 * i < row_words) ? __ldg(w + 32 * i) : 0u;
-  };
-  uint32_t mask_ahead = load_mask(p, tile_at<kPacked>(p, 0));
-  load_rows(tile_at<kPacked>(p, 0));
-  for (int round = 0, tile; (tile = tile_at<kPacked>(p, round)) < p.num_tiles; ++round) {
-    const uint32_t mask = __shfl_sync(0xffffffffu, mask_ahead, 0);
-    uint32_t* lanes_off = sh->lanes_off[buf];
-    if (mask != 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) lanes_off[lane + 32 * i] = ~rows_ahead[i];
-    }
-    // round trips to L2: in flight while this tile is issued
-    mask_ahead = load_mask(p, tile_at<kPacked>(p, round + 1));
-    load_rows(tile_at<kPacked>(p, round + 1));
-    if (mask == 0) continue;  // a tile no offset feeds uses no accumulator: the epilogue writes its bias rows alone
-    __syncwarp();
-    PROF(0);
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase, abort_flag, 22))) return;
-    tc_fence_after();
-    PROF(4);
-    const uint32_t d_addr = tmem_base + (uint32_t)(acc * p.cout);
-    // windows: for (base = 0; base < kvol; base += kGroup) over the windows that have an offset; packed stages:
-    // while offsets are left, the kGroup lowest of them
-    uint32_t rest = mask;
-    for (int base = 0; kPacked ? rest != 0u : base < p.kvol; base += kPacked ? 0 : kGroup) {
-      uint32_t bits;  // the offsets of the tile's next stage
-      if (kPacked) {
-        bits = lowest_bits<kGroup>(rest);
-        rest &= ~bits;
-      } else {
-        bits = (mask >> base) & ((1u << kGroup) - 1u);
-        if (bits == 0u) continue;
-      }
-      int k[kGroup];
-      const uint32_t used = slot_offsets<kGroup, kPacked>(bits, base, k);
-      for (int part = 0; part < kparts; ++part) {
-        // the full barrier guards shared memory only: no tcgen05 fence is needed, but the rows written by
-        // cp.async (generic proxy) must be made visible to the tensor core's reads (async proxy)
-        PROF(0);
-        if (!__all_sync(0xffffffffu, landed || mbar_wait(&sh->full[stage], phase, abort_flag, 21))) return;
-        PROF(1);
-        fence_proxy_async();
-        PROF(2);
-        // look at the following stage's barrier now: the answer (a round trip to shared memory) arrives while
-        // this stage's MMAs are issued, and a stage that has already landed then costs no wait at all
-        const bool wrap = stage + 1 == num_stages;
-        const int stage_next = wrap ? 0 : stage + 1;
-        const uint32_t phase_next = phase ^ (wrap ? 1u : 0u);
-        const bool landed_next = mbar_test(&sh->full[stage_next], phase_next);
-        const uint32_t a_lo = tiles_lo + (uint32_t)stage * stage_step;
-        const uint32_t b_stage = a_lo + (uint32_t)kGroup * a_step;
-        // descriptors of all MMAs of the stage first (independent, warp-uniform arithmetic), then the straight
-        // line of MMAs: the issuing lane runs no dependent chain between two of them
-        uint64_t desc_a[kGroup][kSteps], desc_b[kGroup][kSteps];
-#pragma unroll
-        for (int e = 0; e < kGroup; ++e) {
-          // resident weights are indexed by the offset, streamed ones by the slot
-          const uint32_t b_lo = resident ? bres_lo + (uint32_t)k[e] * b_step
-                                         : b_stage + (uint32_t)e * b_step;
-#pragma unroll
-          for (int ks = 0; ks < kSteps; ++ks) {
-            // 32 bytes per K step inside the swizzle span, the next 64-column block every 4 steps
-            const uint32_t adv_a = (uint32_t)e * a_step + (uint32_t)(ks >> 2) * cs_a + (uint32_t)(ks & 3) * 2u;
-            const uint32_t adv_b = (uint32_t)(ks >> 2) * cs_b + (uint32_t)(ks & 3) * 2u;
-            desc_a[e][ks] = desc_hi | (a_lo + adv_a);
-            desc_b[e][ks] = desc_hi | (b_lo + adv_b);
-          }
-        }
-        if (elect_one()) {
-          const uint4* off = reinterpret_cast<const uint4*>(lanes_off);
-#pragma unroll
-          for (int e = 0; e < kGroup; ++e) {
-            const uint4 o = off[k[e]];
-#pragma unroll
-            for (int ks = 0; ks < kSteps; ++ks)
-              umma_f16_rows_if((used >> e) & 1u, d_addr, desc_a[e][ks], desc_b[e][ks], idesc, o);
-          }
-          umma_commit(&sh->empty[stage]);  // the stage may be refilled once these MMAs have read it
-        }
-        __syncwarp();
-        PROF(3);
-        stage = stage_next, phase = phase_next, landed = landed_next;
-      }
-    }
-    if (elect_one()) umma_commit(&sh->acc_full[acc]);
-    __syncwarp();
-    buf ^= 1;
-    if (++acc == kNumAcc) acc = 0, acc_phase ^= 1;
-  }
-  PROF_STORE(1, (threadIdx.x & 31) == 0)
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// Brings what a round reads towards the SM: ids and row masks of its tiles, the rows of the input that lie where the outputs
+// do (a submanifold layer gathers each of them, here or in a tile nearby), the rows of the residual.  The producers are only
+// one unit ahead with their loads, which covers L2 but not DRAM (64 -> 64 at 238 k voxels behind other layers: 77.8 us without).
+__device__ __forceinline__ void prefetch_round(const TcParams& p, int live, const Round& r) {
+  const int i = threadIdx.x & 31, index = tile_index(p, r, i);
+  if (i >= r.tiles || index >= r.limit || index >= live) return;
+  const int64_t tile = tile_of(p, index), row = tile * kTileRows;
+  prefetch_l2(p.table + tile * p.kvol * kTileRows, (uint32_t)(p.kvol * kTileRows * 4));
+  prefetch_l2(p.row_masks + tile * p.kvol * 4, (uint32_t)(p.kvol * 16));
+  if (p.regrouped) return;
+  const int64_t in = p.n_in_rows == p.m_max && row < p.n_in_rows ? p.n_in_rows - row : 0, out = p.m_max - row;
+  prefetch_l2(reinterpret_cast<const unsigned char*>(p.in_feats) + row * p.cin * 2,
+              (uint32_t)(in < kTileRows ? in : kTileRows) * p.cin * 2);
+  if (p.residual)
+    prefetch_l2(reinterpret_cast<const unsigned char*>(p.residual) + row * p.cout * 2,
+                (uint32_t)(out < kTileRows ? out : kTileRows) * p.cout * 2);
 }
 
-// ---- epilogue ----------------------------------------------------------------------------------------------------
-// Epilogue warp `quad` (= warp index mod 4: it may touch TMEM lanes [32*quad, 32*quad + 32)).  The accumulators are
-// handed to the MMA warp zeroed: once at the start, then every time one has been read.
-template <bool kPacked>
-__device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int quad) {
+// Lists the units of every round and brings in the weights: all of them once when they are resident, else the block of
+// every (window, part) as soon as a slot is free.
+template <int kOffs, int kMma>
+__device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b) {
+  constexpr uint32_t kWindow = kOffs == 1 ? 1u : kOffs == 2 ? 3u : 15u;
+  constexpr int kWindows = 32 / kOffs;
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
   const int lane = threadIdx.x & 31;
+  const uint32_t b_tx = (uint32_t)p.cout * p.row_bytes;
+  const bool resident = p.b_slots == 0;
+  const int parts = p.parts;
+  // the weights are constants of the layer: their load does not wait for the preceding kernel
+  if (resident && lane == 0) {
+    // blocks behind the last offset, up to a whole window: rows beyond the tensor, which TMA fills with zeros
+    const int blocks = (p.kvol + kOffs - 1) / kOffs * kOffs;
+    mbar_arrive_expect_tx(&sh->b_ready, (uint32_t)blocks * b_tx);
+    for (int k = 0; k < blocks; ++k) tma_load_2d(map_b, &sh->b_ready, s.weights + (size_t)k * p.b_bytes, 0, k * p.cout);
+  }
+  if (!resident && lane == 0) {  // a slice of the weights for every CTA, towards L2
+    const uint32_t bytes = (uint32_t)p.kvol * (uint32_t)p.cout * (uint32_t)p.cin * 2u;
+    const uint32_t slice = (bytes / gridDim.x + 127u) & ~127u, from = blockIdx.x * slice;
+    if (from < bytes)
+      prefetch_l2(reinterpret_cast<const unsigned char*>(p.weights) + from, bytes - from < slice ? bytes - from : slice);
+  }
+  __syncwarp();
+  pdl_wait();  // the offset masks come from the preceding kernels
+  const int live = live_tiles(p);
+  int buf = 0, b_slot = 0;
+  uint32_t list_phase = 0, b_phase = 0;
+  Round r;
+  open_round<kMma>(p, live, 0, r);
+  prefetch_round(p, live, r);
+  for (;;) {
+    const bool end = r.tiles == 0;
+    uint32_t masks[kMma], all = 0;
+    int count = 0;
+#pragma unroll
+    for (int i = 0; i < kMma; ++i) {
+      masks[i] = __shfl_sync(0xffffffffu, r.mask, i);
+      all |= masks[i], count += masks[i] != 0u;
+    }
+    const Round done = r;
+    if (!end) {  // the next round's masks are on their way
+      open_round<kMma>(p, live, after_round(done), r);
+      prefetch_round(p, live, r);
+    }
+    if (all == 0u && !end) continue;
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14))) return;
+    // lane w lists window w
+    const uint32_t bits = lane < kWindows ? kWindow << (lane * kOffs) : 0u;
+    const bool present = (all & bits) != 0u;
+    const uint32_t windows = __ballot_sync(0xffffffffu, present);
+    const int rank = __popc(windows & lanemask_lt());  // of the window in the round
+    const int steps = __popc(windows) * parts;
+    const int offs = p.kvol - lane * kOffs < kOffs ? p.kvol - lane * kOffs : kOffs;
+    if (present) {
+      int place = 0;  // of the tile among the round's tiles that have an offset
+#pragma unroll
+      for (int i = 0; i < kMma; ++i) {
+        if (masks[i] == 0u) continue;
+        const uint32_t blk = (uint32_t)tile_of(p, tile_index(p, done, i)) * (uint32_t)p.kvol + (uint32_t)(lane * kOffs);
+        for (int part = 0; part < parts; ++part)
+          sh->units[buf][place][rank * parts + part] = make_uint2(blk, (uint32_t)part | (uint32_t)offs << 4);
+        ++place;
+      }
+    }
+    if (lane == 0) sh->round[buf] = make_int4(count, (int)windows, steps, 0);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->list_full[buf]);
+    if (buf) list_phase ^= 1;
+    buf ^= 1;
+    if (end) return;
+    if (!resident) {
+      // two (window, part)s to a slot
+      uint32_t rest = windows;
+      for (int seq = 0, part = 0; seq < steps; seq += 2) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11))) return;
+        const int both = seq + 1 < steps ? 2 : 1;
+        if (lane == 0) mbar_arrive_expect_tx(&sh->b_full[b_slot], (uint32_t)(both * kOffs) * b_tx);
+        for (int h = 0; h < both; ++h) {
+          const int k = (__ffs(rest) - 1) * kOffs;
+          if (lane == 0) {
+#pragma unroll
+            for (int o = 0; o < kOffs; ++o)  // behind the last offset: zeros, as above
+              tma_load_2d(map_b, &sh->b_full[b_slot], s.weights + (size_t)((b_slot * 2 + h) * kOffs + o) * p.b_bytes, part * 64,
+                          (k + o) * p.cout);
+          }
+          if (++part == parts) part = 0, rest &= rest - 1u;
+        }
+        __syncwarp();
+        if (++b_slot == p.b_slots) b_slot = 0, b_phase ^= 1;
+      }
+    }
+  }
+}
+
+// ---- MMA warps -------------------------------------------------------------------------------------------------------
+// Every other tile of a round.  The warp walks the round together and by counters: what feeds an MMA has to be the same for
+// the whole warp in a way the compiler can see.  (Four MMAs and a commit issued from a loop run by one lane take 273 cycles, by
+// the elected lane of such a warp 74, at 32 output channels.)
+template <int kOffs, int kMma>
+__device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int me) {
+  constexpr int kSteps = 4 / kOffs;  // MMAs (K = 16) per offset of a unit
+  Shared* sh = s.sh;
+  volatile int* abort_flag = &sh->abort_flag;
+  // descriptor high word: stride between 8-row groups, version, swizzle mode
+  const uint64_t desc_hi = (uint64_t)(((8u * (uint32_t)p.row_bytes) >> 4) | (1u << 14) | (p.layout_type << 29)) << 32;
+  const uint32_t b_step = p.b_bytes >> 4, b_lo0 = desc_lo(smem_u32(s.weights));
+  const uint32_t idesc = p.idesc;
+  const uint32_t ring = tmem_base + (uint32_t)p.ring_col;
+  const bool resident = p.b_slots == 0;
+  const int parts = p.parts, num_acc = p.num_acc, b_slots = p.b_slots;
+  const uint32_t cout = (uint32_t)p.cout;
+  if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23))) return;
+  // the slots of this warp's two teams, taken in turn
+  const uint32_t a_of[2] = {ring + (uint32_t)(me * kUnitCols), ring + (uint32_t)((me + kMma) * kUnitCols)};
+  uint64_t* const full_of[2] = {&sh->full[me], &sh->full[me + kMma]};
+  uint64_t* const empty_of[2] = {&sh->empty[me], &sh->empty[me + kMma]};
+  int buf = 0, b_slot = 0, acc0 = 0;
+  uint32_t list_phase = 0, b_phase = 0, turn = 0, acc_phase = 0;  // turn: bit 0 the slot, bit 1 its phase
+  for (;;) {
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 15))) return;
+    const int4 round = sh->round[buf];
+    const int count = (int)__reduce_or_sync(0xffffffffu, (unsigned)round.x);
+    const uint32_t windows = __reduce_or_sync(0xffffffffu, (unsigned)round.y);
+    if (count == 0) break;
+    // this warp's tile of the round, if there is one, and its accumulator
+    const bool mine = me < count;
+    const bool wrap = acc0 + me >= num_acc;
+    const int acc = wrap ? acc0 + me - num_acc : acc0 + me;
+    const uint32_t d_addr = tmem_base + (uint32_t)acc * cout;
+    if (mine && !__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22)))
+      return;
+    tc_fence_after();
+    uint32_t add = 0u;  // the first products of a round start the sums
+    uint32_t rest = windows;
+    const int steps = __popc(windows) * parts;
+    for (int seq = 0; seq < steps; seq += 2) {  // two (window, part)s at a time
+      const bool both = seq + 1 < steps;
+      uint32_t b_lo[2];
+      if (resident) {
+        b_lo[0] = b_lo0 + (uint32_t)((__ffs(rest) - 1) * kOffs) * b_step;
+        rest &= rest - 1u;
+        b_lo[1] = b_lo0 + (uint32_t)((__ffs(rest) - 1) * kOffs) * b_step;
+        rest &= rest - 1u;
+      } else {
+        b_lo[0] = b_lo0 + (uint32_t)(b_slot * 2 * kOffs) * b_step;
+        b_lo[1] = b_lo[0] + (uint32_t)kOffs * b_step;
+      }
+      uint64_t desc[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          desc[h][m] = desc_hi | (b_lo[h] + (uint32_t)(m / kSteps) * b_step + 2u * (m % kSteps));
+      const bool odd = turn & 1u;
+      const uint32_t a_addr[2] = {odd ? a_of[1] : a_of[0], odd ? a_of[0] : a_of[1]};
+      uint64_t* const full[2] = {odd ? full_of[1] : full_of[0], odd ? full_of[0] : full_of[1]};
+      uint64_t* const empty[2] = {odd ? empty_of[1] : empty_of[0], odd ? empty_of[0] : empty_of[1]};
+      // One lane waits and issues, for both windows at once: every instruction of this warp between two products is one too
+      // many.  After a wait that gave up all others give up at once, and what is issued then does not matter.
+      if (elect_one()) {
+        if (!resident) mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24);
+        auto unit = [&](int h) {
+          mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21);
+          tc_fence_after();
+          umma_f16_ta(d_addr, a_addr[h], desc[h][0], idesc, h ? 1u : add);
+#pragma unroll
+          for (int m = 1; m < 4; ++m) umma_f16_ta(d_addr, a_addr[h] + 8 * m, desc[h][m], idesc, 1u);
+          umma_commit(empty[h]);  // the slot may be refilled once these MMAs have read it
+        };
+        if (mine) {
+          unit(0);
+          if (both) unit(1);
+        }
+        if (!resident) umma_commit(&sh->b_empty[b_slot]);
+      }
+      __syncwarp();
+      add = 1u;
+      if (mine) turn = (turn + (both ? 2u : 1u)) & 3u;
+      if (!resident && ++b_slot == b_slots) b_slot = 0, b_phase ^= 1;
+    }
+    if (elect_one()) {
+      if (mine) umma_commit(&sh->acc_full[acc]);
+      mbar_arrive(&sh->list_empty[buf]);
+    }
+    __syncwarp();
+    if (*abort_flag) return;
+    if (buf) list_phase ^= 1;
+    buf ^= 1;
+    acc0 += count;
+    if (acc0 >= num_acc) acc0 -= num_acc, acc_phase ^= 1;
+  }
+}
+
+// ---- epilogue --------------------------------------------------------------------------------------------------------
+// Epilogue warp `quad` (= warp index mod 4: it may touch TMEM lanes [32*quad, 32*quad + 32)) of set `set`: the sets share
+// the columns of every tile, so that an accumulator is free again soon (of 256 output channels there is only one).
+template <int kOffs, int kMma>
+__device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int quad, int set) {
+  Shared* sh = s.sh;
+  volatile int* abort_flag = &sh->abort_flag;
+  const int lane = threadIdx.x & 31;
+  // the tile row the producers put into this TMEM lane
+  const int row_in_tile = quad * 32 + 4 * (lane & 7) + (rows_per_lane(kOffs) == 4 ? lane >> 3 : 2 * (lane >> 3 & 1) + (lane >> 4));
+  const bool wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
+  const int half = epilogue_sets(kMma) == 2 ? (p.cout + 31) / 32 * 16 : p.cout;
+  const int from = set ? half : 0, to = set ? p.cout : half;
   int acc = 0;
   uint32_t acc_phase = 0;
   const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-  for (int a = 0; a < kNumAcc; ++a) {
-    for (int c0 = 0; c0 < p.cout; c0 += 16) tmem_st16_same(lane_base + (uint32_t)(a * p.cout + c0), 0u);
-    tmem_st_wait();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sh->acc_empty[a]);
-  }
   pdl_wait();  // residual rows come from an earlier layer; output rows may still be read by the preceding kernel
-  uint32_t mask = load_mask(p, tile_at<kPacked>(p, 0));
-  // the output a tile row stands for (the row itself, unless the table's outputs were regrouped): loaded a tile ahead
-  auto load_row = [&](int tile) -> int {
-#ifdef D3D_TC_NO_PERM
-    return tile < p.num_tiles ? tile * kTileRows + quad * 32 + lane : -1;
-#else
-    return tile < p.num_tiles ? __ldg(p.perm + (int64_t)tile * kTileRows + quad * 32 + lane) : -1;
-#endif
-  };
-  int row_ahead = load_row(tile_at<kPacked>(p, 0));
-  PROF_DECL
-  for (int round = 0, tile; (tile = tile_at<kPacked>(p, round)) < p.num_tiles; ++round) {
-    const int next = tile_at<kPacked>(p, round + 1);
-    const uint32_t next_mask = next < p.num_tiles ? __ldg(p.tile_mask + next) : 0u;
-    const int64_t row = row_ahead;
-    row_ahead = load_row(next);
-    const bool empty_tile = mask == 0;  // bias (+ residual) only, no accumulator involved
-    PROF(0);
-    if (!empty_tile) {
-      if (!mbar_wait(&sh->acc_full[acc], acc_phase, abort_flag, 31)) return;
-      tc_fence_after();
-    }
-    PROF(1);
-    const bool row_ok = row >= 0 && row < p.m_max;
-    unsigned short* out_row = reinterpret_cast<unsigned short*>(p.out) + row * p.cout;
-    const unsigned short* res_row =
-        (p.residual && row_ok) ? reinterpret_cast<const unsigned short*>(p.residual) + row * p.cout : nullptr;
-    const uint32_t taddr = lane_base + (uint32_t)(acc * p.cout);
-    for (int c0 = 0; c0 < p.cout; c0 += 16) {
-      uint32_t v[16];
-      if (empty_tile) {
+  const int live = live_tiles(p);
+  Round r;
+  for (open_round<kMma>(p, live, 0, r); r.tiles; open_round<kMma>(p, live, after_round(r), r)) {
+    for (int i = 0; i < r.tiles; ++i) {
+      const uint32_t mask = __shfl_sync(0xffffffffu, r.mask, i);
+      const int index = tile_index(p, r, i);
+      if (index >= r.limit) continue;
+      const int64_t row = __ldg(p.perm + (int64_t)tile_of(p, index) * kTileRows + row_in_tile);
+      const bool empty_tile = mask == 0;  // bias (+ residual) only, no accumulator involved
+      const bool row_ok = row >= 0 && row < p.m_max;
+      unsigned short* out_row = reinterpret_cast<unsigned short*>(p.out) + row * p.cout;
+      const uint4* res_row = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.residual) + row * p.cout);
+      const uint32_t taddr = lane_base + (uint32_t)(acc * p.cout);
+      auto columns = [&](auto with_residual) {
+        constexpr bool kAdd = decltype(with_residual)::value;
+        uint4 res[2];  // of the next 16 columns, on their way
+        if (kAdd && row_ok && from < to) res[0] = __ldg(res_row + from / 8), res[1] = __ldg(res_row + from / 8 + 1);
+        if (!empty_tile) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc], acc_phase, abort_flag, 31))) return false;
+          tc_fence_after();
+        }
+        for (int c0 = from; c0 < to; c0 += 16) {
+          uint32_t v[16];
+          if (empty_tile) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = 0u;
-      } else {
-        tmem_ld16(taddr + c0, v);
-        tmem_ld_wait();
-        tmem_st16_same(taddr + c0, 0u);  // the next tile of this accumulator starts from zero
-      }
-      if (row_ok) {
-        if (p.is_bf16) store_chunk<true>(v, s.bias, c0, out_row, res_row, p.relu);
-        else store_chunk<false>(v, s.bias, c0, out_row, res_row, p.relu);
+            for (int q = 0; q < 16; ++q) v[q] = 0u;
+          } else {
+            tmem_ld16(taddr + c0, v);
+          }
+          const uint4 now[2] = {res[0], res[1]};
+          if (kAdd && row_ok && c0 + 16 < to) res[0] = __ldg(res_row + c0 / 8 + 2), res[1] = __ldg(res_row + c0 / 8 + 3);
+          if (!empty_tile) tmem_ld_wait(v);
+          if (row_ok) {
+            if (p.is_bf16) store_chunk<true, kAdd>(v, s.bias + c0, out_row + c0, now, p.relu, wide);
+            else store_chunk<false, kAdd>(v, s.bias + c0, out_row + c0, now, p.relu, wide);
+          }
+        }
+        return true;
+      };
+      if (!(p.residual ? columns(std::true_type{}) : columns(std::false_type{}))) return;
+      if (!empty_tile) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
+        if (++acc == p.num_acc) acc = 0, acc_phase ^= 1;
       }
     }
-    if (!empty_tile) {
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
-      if (++acc == kNumAcc) acc = 0, acc_phase ^= 1;
-    }
-    PROF(2);
-    mask = next_mask;
   }
-  PROF_STORE(2, quad == 0 && lane == 0)
 }
 
-// kPieces x kChunks = 16-byte pieces per A row (2, 4, 8, 16), kGroup = offsets per stage, kProdWarps = 4 or 8,
-// kCtas = CTAs per SM the launch is planned for (1 or 2).
-template <int kPieces, int kChunks, int kGroup, int kProdWarps, int kCtas, bool kPacked>
-__global__ void __launch_bounds__(threads_of(kProdWarps), kCtas)
+template <int kOffs, bool kWide, int kMma>
+__global__ void __launch_bounds__(threads_of(kMma), 1)
 spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  const Smem s = carve_smem<kGroup>(smem_raw, p);
+  constexpr int kEpilogue = 4 * epilogue_sets(kMma);
+  const Smem s = carve_smem<kOffs>(smem_raw, p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup<kProdWarps>(p, s);
+  const uint32_t tmem_base = cta_setup<kMma>(p, s);
   pdl_release();
-  if (warp < kProdWarps) {
-    producer_role<kPieces, kChunks, kGroup, kProdWarps, kPacked>(p, s, warp, lane);
-  } else if (warp == kProdWarps) {
-    mma_role<kPieces, kChunks, kGroup, kPacked>(p, s, tmem_base);
-    __syncwarp();
-  } else if (warp == kProdWarps + 1) {
-    if (lane == 0) control_role<kGroup, kPacked>(p, s, &map_b);
-    __syncwarp();
+  if (warp < 8 * kMma) {
+    producer_role<kOffs, kWide, kMma>(p, s, tmem_base, warp, lane);
+  } else if (warp < 8 * kMma + kEpilogue) {
+    epilogue_role<kOffs, kMma>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
+  } else if (warp < 9 * kMma + kEpilogue) {
+    mma_role<kOffs, kMma>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
   } else {
-    epilogue_role<kPacked>(p, s, tmem_base, warp & 3);
+    control_role<kOffs, kMma>(p, s, &map_b);
   }
-  cta_teardown<kProdWarps>(p, tmem_base);
+  __syncwarp();
+  cta_teardown<kMma>(p, tmem_base);
 }
 
-// ---- host --------------------------------------------------------------------------------------------------------
+// ---- host ------------------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -953,34 +903,25 @@ struct TcState {
   bool map_b_ok = false;
 };
 
-// Tuning override for experiments (0 = automatic): offsets per stage and pipeline stages.
-int g_plan_group = 0, g_plan_stages = 0, g_plan_prod_warps = 0;
+// Tuning override for experiments (0 = automatic).
+int g_plan_mma_warps = 0;
 
 typedef void (*KernelFn)(const CUtensorMap, const TcParams);
 struct KernelEntry {
-  int pieces, chunks, group, prod_warps, ctas;
-  KernelFn fn[2];  // fixed windows of offsets per stage / the offsets present packed into the stages
+  int offs, wide, mma_warps;
+  KernelFn fn;
 };
-#define D3D_TC_K(P, C, G, W, N) \
-  {P, C, G, W, N, {spconv_mm_tc_kernel<P, C, G, W, N, false>, spconv_mm_tc_kernel<P, C, G, W, N, true>}}
-// One kernel instance per (row width of a block, offsets per stage, CTAs per SM).
+#define D3D_TC_K(O, V, M) {O, V, M, spconv_mm_tc_kernel<O, V, M>}
 const KernelEntry kKernels[] = {
-    D3D_TC_K(2, 1, 8, 8, 2), D3D_TC_K(2, 1, 4, 8, 2), D3D_TC_K(2, 1, 2, 8, 2), D3D_TC_K(2, 1, 1, 8, 2),
-    D3D_TC_K(4, 1, 4, 8, 2), D3D_TC_K(4, 1, 3, 8, 2), D3D_TC_K(4, 1, 2, 8, 2), D3D_TC_K(4, 1, 1, 8, 2),
-    D3D_TC_K(8, 1, 2, 8, 2), D3D_TC_K(8, 1, 1, 8, 2),
-    D3D_TC_K(2, 1, 8, 4, 2), D3D_TC_K(4, 1, 3, 4, 2), D3D_TC_K(8, 1, 1, 4, 2), D3D_TC_K(8, 1, 2, 4, 2),
-    D3D_TC_K(2, 1, 8, 8, 1), D3D_TC_K(2, 1, 4, 8, 1), D3D_TC_K(2, 1, 2, 8, 1), D3D_TC_K(2, 1, 1, 8, 1),
-    D3D_TC_K(4, 1, 4, 8, 1), D3D_TC_K(4, 1, 3, 8, 1), D3D_TC_K(4, 1, 2, 8, 1), D3D_TC_K(4, 1, 1, 8, 1),
-    D3D_TC_K(8, 1, 2, 8, 1), D3D_TC_K(8, 1, 1, 8, 1), D3D_TC_K(8, 2, 1, 8, 1),
+    D3D_TC_K(4, true, 2), D3D_TC_K(2, true, 2), D3D_TC_K(2, false, 2), D3D_TC_K(1, true, 2), D3D_TC_K(1, false, 2),
+    D3D_TC_K(4, true, 3), D3D_TC_K(2, true, 3), D3D_TC_K(2, false, 3), D3D_TC_K(1, true, 3), D3D_TC_K(1, false, 3),
 };
 #undef D3D_TC_K
 constexpr int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
 
-const KernelEntry* find_kernel(int pieces, int chunks, int group, int prod_warps, int ctas) {
+const KernelEntry* find_kernel(int offs, int wide, int mma_warps) {
   for (int i = 0; i < kNumKernels; ++i)
-    if (kKernels[i].pieces == pieces && kKernels[i].chunks == chunks && kKernels[i].group == group &&
-        kKernels[i].prod_warps == prod_warps && kKernels[i].ctas == ctas)
-      return &kKernels[i];
+    if (kKernels[i].offs == offs && kKernels[i].wide == wide && kKernels[i].mma_warps == mma_warps) return &kKernels[i];
   return nullptr;
 }
 
@@ -993,6 +934,16 @@ bool spconv_mm_tc_eligible(const d3d_spconv_mm_s* h, int dtype) {
   if (cout % 16 != 0 || cout < 16 || cout > 256) return false;
   if (kvol > 32) return false;
   return encode_fn() != nullptr;
+}
+
+// The channel at position `pos` of a weight row in the order the kernel multiplies in.
+int spconv_mm_tc_channel(int cin, int pos) {
+  const int width = cin < 64 ? cin : 64;  // channels of a unit's row
+  const int in = pos % width;
+  if (rows_per_lane(64 / width) == 4)  // four lanes of 16 channels each; a store puts two words of each side by side
+    return pos - in + in / 4 % 4 * 16 + in / 16 * 4 + in % 4;
+  const int run = width / 2, word = in / 4, half = in / 2 % 2;  // two lanes of half the channels each, word by word
+  return pos - in + half * run + word * 2 + in % 2;
 }
 
 void spconv_mm_tc_release(d3d_spconv_mm_s* h) {
@@ -1026,143 +977,79 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   D3D_REQUIRE(st && st->map_b_ok, D3D_ERR_INVALID_ARGUMENT);  // configure() creates it
 
   TcParams p;
-  p.table = a.table;
-  p.tile_mask = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(a.table) +
-                                                  table_ids_bytes(kvol, m_max));
-  p.row_masks = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(p.tile_mask) +
-                                                  table_mask_bytes(m_max));
-  p.perm = reinterpret_cast<const int32_t*>(reinterpret_cast<const unsigned char*>(p.row_masks) +
-                                            table_rows_bytes(kvol, m_max));
+  const TableParts t = table_parts(const_cast<int32_t*>(a.table), kvol, m_max);
+  p.table = t.ids, p.tile_mask = t.tile_mask, p.row_masks = t.row_masks, p.perm = t.perm;
+  p.num_out = a.num_act_out;
   p.in_feats = a.in_feats;
   p.m_max = m_max;
   p.n_in_rows = (int32_t)a.max_num_act_in;
   p.kvol = kvol, p.cin = cin, p.cout = cout;
-  p.num_tiles = (int)((m_max + kTileRows - 1) / kTileRows);
-  const int box_cols = cin < 64 ? cin : 64;
-  p.row_bytes = box_cols * 2;
+  p.num_tiles = (int)t.tiles;
+  const int width = cin < 64 ? cin : 64, offs = 64 / width;
+  p.parts = cin / width;
+  p.row_bytes = width * 2;
   p.layout_type = p.row_bytes == 32 ? 6u : p.row_bytes == 64 ? 4u : 2u;
   const uint32_t fmt = a.dtype == D3D_BF16 ? 1u : 0u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(cout >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
-  uint32_t cols = 32;
-  while (cols < (uint32_t)(kNumAcc * cout)) cols <<= 1;
-  p.tmem_cols = cols;
+  p.regrouped = a.regrouped ? 1 : 0;
+  const int wide = offs == 4 || reinterpret_cast<uintptr_t>(a.in_feats) % 32 == 0;
+  p.weights = h->wt_dev;
   p.bias = h->b_dev;
   p.out = a.out_feats;
   p.residual = a.residual;
   p.relu = a.relu;
   p.is_bf16 = a.dtype == D3D_BF16;
 
-  // Shared-memory plan.  Control data of a CTA: alignment slack, bias, barriers and row flags.
-  const size_t ctrl = 1024 + align_up((size_t)cout * 4 + 8, 16) + sizeof(Shared);
-  const size_t swizzle_repeat = (size_t)8 * p.row_bytes;  // operand blocks start on a multiple of it
-  struct Plan {
-    int kchunk, resident, group, stages;
-    size_t smem;
-    const KernelEntry* kernel;
-  };
-  // `two_per_sm`: 4 producer warps and half the SM's shared memory and tensor-memory columns per CTA.
-  auto make_plan = [&](bool two_per_sm, int kchunk, Plan* out) -> bool {
-    if (two_per_sm && (kchunk > 64 || cols > 256)) return false;
-    const int pieces = kchunk >= 64 ? 8 : kchunk / 8, chunks = kchunk > 64 ? kchunk / 64 : 1;
-    const int ksteps = kchunk / 16, kparts = cin / kchunk;
-    const size_t a_bytes = (size_t)kTileRows * kchunk * 2;
-    const size_t b_bytes = align_up((size_t)cout * kchunk * 2, swizzle_repeat);
-    const size_t limit = two_per_sm ? 113 * 1024 : 227 * 1024;
-    if (ctrl + 2 * (a_bytes + b_bytes) > limit) return false;
-    // two producer teams, except for 32-channel blocks, which measured better with one (B200: 94 vs 102 us at
-    // 463 k voxels; 64 channels: 102 vs 116 us, 128: 68 vs 73 us the other way round)
-    const int prod_warps = g_plan_prod_warps ? g_plan_prod_warps : (two_per_sm && kchunk == 32 ? 4 : 8);
-    const size_t budget = limit - ctrl;
-    const size_t bres_bytes = (size_t)kvol * b_bytes;
-    Plan best;
-    best.stages = 0, best.group = 0, best.kernel = nullptr;
-    int best_score = -1;
-    for (int resident = 1; resident >= 0; --resident) {
-      // resident weights whenever two stages still fit beside them, streamed per stage only otherwise: a streamed
-      // W[k] crosses from L2 once per tile and sits in the hand-over loop (B200, 463 k voxels: 32 -> 32 85.6 vs
-      // 88.2 us, 16 -> 32 36.9 vs 39.9 us)
-      if (resident && (kparts != 1 || bres_bytes + 2 * a_bytes > budget)) continue;
-      if (!resident && best_score >= 0) continue;
-      const size_t ring = budget - (resident ? bres_bytes : 0);
-      const size_t blk = a_bytes + (resident ? 0 : b_bytes);
-      for (int group = kMaxGroup; group >= 1; --group) {
-        const KernelEntry* k = find_kernel(pieces, chunks, group, prod_warps, two_per_sm ? 2 : 1);
-        if (!k) continue;
-        if (g_plan_group && group != g_plan_group) continue;
-        if (group > 1 && (group * ksteps > 8 || group > kvol)) continue;
-        // with K parts, offsets that share a stage would accumulate part by part instead of offset by offset: keep
-        // the one accumulation order every plan produces
-        if (group > 1 && kparts > 1) continue;
-        int stages = (int)(ring / ((size_t)group * blk));
-        if (stages > kMaxStages) stages = kMaxStages;
-        if (g_plan_stages && stages > g_plan_stages) stages = g_plan_stages;
-        if (stages < 2) continue;
-        // eight MMAs per hand-over first (B200, 64 -> 64 at 238 k voxels: two offsets per stage in two stages 84 us,
-        // one offset per stage in four stages 94 us), then up to three stages (more add little), then more MMAs
-        const int depth = stages >= 3 ? 3 : stages;
-        const int mmas = group * ksteps;
-        const int score = (mmas > 8 ? 8 : mmas) * 400 + depth * 1000 + mmas * 10 + (stages > 4 ? 4 : stages) + resident * 5;
-        if (score > best_score) {
-          best_score = score;
-          best.kchunk = kchunk, best.resident = resident, best.group = group, best.stages = stages, best.kernel = k;
-          best.smem = ctrl + (size_t)stages * group * blk + (resident ? bres_bytes : 0);
-        }
-      }
-    }
-    if (best_score < 0) return false;
-    // pin the number of CTAs per SM through the request: more than a third (half) of the SM's shared memory
-    const size_t floor_bytes = two_per_sm ? 80 * 1024 : 120 * 1024;
-    if (best.smem < floor_bytes) best.smem = floor_bytes;
-    *out = best;
-    return true;
-  };
-  Plan pl;
-  bool two_per_sm = false;
-  if (h->kernel_choice != 3) two_per_sm = make_plan(true, cin < 64 ? cin : 64, &pl) && pl.stages >= 2;
-  if (!two_per_sm) {
-    Plan wide, narrow;
-    const bool have_wide = cin >= 128 && make_plan(false, 128, &wide);
-    const bool have_narrow = make_plan(false, cin < 64 ? cin : 64, &narrow);
-    D3D_REQUIRE(have_wide || have_narrow, D3D_ERR_TOO_LARGE);
-    // 128-channel blocks (eight MMAs per hand-over) when three of them fit, else 64-channel K parts
-    pl = (have_wide && (wide.stages >= 3 || !have_narrow)) ? wide : narrow;
+  // Three MMA warps where a unit's products are short (up to 64 columns: 24 producer warps then feed them), two where the tensor
+  // pipe is the longer part, where few offsets make the epilogue it (it has eight warps then) and for 16 input channels, whose
+  // units take the most instructions.  us with two / three: 27 offsets 32 -> 32 83 / 72, 64 -> 64 77 / 69, 128 -> 64 61 / 58,
+  // 64 -> 128 94 / 113, 128 -> 128 50 / 55, 256 -> 256 116 / 120, 16 -> 32 31 / 34; nine offsets 32 -> 32 15.8 / 17.2; three
+  // offsets 64 -> 64 15.3 / 18.2.
+  const int mma_warps = g_plan_mma_warps ? g_plan_mma_warps : (cin >= 32 && cout <= 64 && kvol > 9) ? 3 : 2;
+  const KernelEntry* k = find_kernel(offs, wide, mma_warps);
+  D3D_REQUIRE(k, D3D_ERR_INVALID_ARGUMENT);
+  // tensor memory: a slot for every producer team, the rest accumulators
+  p.ring_col = kTmemCols - 2 * mma_warps * kUnitCols;
+  p.num_acc = p.ring_col / cout;
+  if (p.num_acc > kMaxAcc) p.num_acc = kMaxAcc;
+  // shared memory: weights
+  p.b_bytes = (uint32_t)align_up((size_t)cout * p.row_bytes, (size_t)8 * p.row_bytes);
+  const size_t ctrl = 1024 + align_up((size_t)cout * 4 + 16, 16) + sizeof(Shared);
+  size_t weights = align_up(kvol, offs) * p.b_bytes;
+  p.b_slots = 0;
+  // in shared memory for good up to 112 KB, which leaves L1 as much (16 -> 16 to 32 -> 64, held or streamed: the same to 1 %)
+  if (p.parts > 1 || weights > 112 * 1024) {
+    const size_t window = (size_t)2 * offs * p.b_bytes;  // two of them to a slot
+    p.b_slots = (int)(128 * 1024 / window);
+    if (p.b_slots < 3) p.b_slots = 3;
+    if (p.b_slots > kMaxBSlots) p.b_slots = kMaxBSlots;
+    weights = p.b_slots * window;
   }
-  p.kchunk = pl.kchunk;
-  p.kparts = cin / pl.kchunk;
-  p.chunks = pl.kchunk <= 64 ? 1 : pl.kchunk / 64;
-  p.a_bytes = (uint32_t)((size_t)kTileRows * pl.kchunk * 2);
-  p.b_bytes = (uint32_t)align_up((size_t)cout * pl.kchunk * 2, swizzle_repeat);
-  p.b_resident = pl.resident, p.stages = pl.stages;
-  const int packed = a.regrouped ? 1 : 0;
-  const KernelFn kernel = pl.kernel->fn[packed];
+  const size_t smem = ctrl + weights;
+  D3D_REQUIRE(smem <= 227 * 1024, D3D_ERR_TOO_LARGE);
   {
     // raising the dynamic shared memory limit is per function and per device; once each, under a lock
     static std::mutex attr_lock;
-    static bool attr_set[64][kNumKernels][2] = {};
+    static bool attr_set[64][kNumKernels] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return D3D_ERR_CUDA;
-    const int ki = (int)(pl.kernel - kKernels);
+    const int ki = (int)(k - kKernels);
     std::lock_guard<std::mutex> guard(attr_lock);
-    if (!attr_set[dev][ki][packed]) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    if (!attr_set[dev][ki]) {
+      if (cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
         return D3D_ERR_CUDA;
-      attr_set[dev][ki][packed] = true;
+      attr_set[dev][ki] = true;
     }
   }
-  const int ctas = kNumSMs * (two_per_sm ? 2 : 1);
-  const int grid = p.num_tiles < ctas ? p.num_tiles : ctas;
-  // programmatic dependent launch (opt-in per handle): the prologue of this kernel (barriers, tensor memory,
-  // weights) may overlap the tail of the preceding kernel of the stream; every role waits for that kernel before
-  // it touches its data.  Measured on B200: 3-4 us less per launch for layers run back to back on one stream; a
-  // loss where other streams have kernels that would otherwise fill the tail of the preceding kernel.
+  const int grid = p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid), cfg.blockDim = dim3(threads_of(pl.kernel->prod_warps));
-  cfg.dynamicSmemBytes = pl.smem, cfg.stream = reinterpret_cast<cudaStream_t>(a.stream);
+  cfg.gridDim = dim3(grid), cfg.blockDim = dim3(threads_of(mma_warps));
+  cfg.dynamicSmemBytes = smem, cfg.stream = reinterpret_cast<cudaStream_t>(a.stream);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = a.chained ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kernel, st->map_b, p) != cudaSuccess) return D3D_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, k->fn, st->map_b, p) != cudaSuccess) return D3D_ERR_CUDA;
   D3D_CHECK_LAUNCH();
   return D3D_OK;
 }
@@ -1181,19 +1068,13 @@ extern "C" int d3d_debug_take_kernel_error(int* code) {
   return D3D_OK;
 }
 
-#ifdef D3D_TC_PROFILE
-extern "C" int d3d_debug_copy_prof(long long* dst) {
-  cudaDeviceSynchronize();
-  return (int)cudaMemcpyFromSymbol(dst, d3d::g_prof, sizeof(long long) * 24);
-}
-#endif
-
-// Tuning aid without a reference counterpart: overrides the pipeline plan of the tensor-core kernel for every later
-// launch of this process (kernel offsets per stage, maximum number of stages, producer warps; 0 = automatic).  Not thread-safe.
+// Tuning aid without a reference counterpart: overrides the plan of the tensor-core kernel for every later launch of
+// this process.  16 or 24 producer warps (two or three MMA warps), 0 = automatic; offsets per stage and stages belong to an
+// earlier kernel and have no effect.  Not thread-safe.
 extern "C" int d3d_debug_set_tc_plan(int group, int max_stages, int prod_warps) {
-  if (group < 0 || group > d3d::kMaxGroup || max_stages < 0 || max_stages > d3d::kMaxStages ||
-      !(prod_warps == 0 || prod_warps == 4 || prod_warps == 8))
+  if (group < 0 || group > 8 || max_stages < 0 || max_stages > 8 ||
+      !(prod_warps == 0 || prod_warps == 4 || prod_warps == 8 || prod_warps == 16 || prod_warps == 24))
     return D3D_ERR_INVALID_ARGUMENT;
-  d3d::g_plan_group = group, d3d::g_plan_stages = max_stages, d3d::g_plan_prod_warps = prod_warps;
+  d3d::g_plan_mma_warps = prod_warps >= 16 ? prod_warps / 8 : 0;
   return D3D_OK;
 }

@@ -83,8 +83,8 @@ int d3d_debug_take_kernel_error(int* code);
  * D3D_ERR_INVALID_ARGUMENT. */
 int d3d_debug_take_bounds_violation(int32_t* record);
 /* Tuning aid (no reference counterpart): overrides the pipeline plan of the tensor-core SPConvMM kernel for every
- * later launch of the process: kernel offsets per pipeline stage, maximum number of stages, producer warps (4 or 8);
- * 0 = automatic.  Not thread-safe; results do not depend on the plan. */
+ * later launch of the process: producer warps (16 or 24), 0 = automatic.  The other arguments (0 to 8), and 4 or 8 producer
+ * warps, are accepted and have no effect.  Not thread-safe; results do not depend on the plan. */
 int d3d_debug_set_tc_plan(int group, int max_stages, int prod_warps);
 
 /* ---------------------------------------------------------------------------------------------
@@ -222,8 +222,8 @@ typedef struct {
  * tests/cylinder/test_cylinder3d.py:91-92).  `residual` (same dtype/shape as outFeats) is added to the result.
  * relu: 0 none; 1 ReLU after the residual add (residual block); 2 ReLU before it (sum of two activated branches,
  * tests/cylinder/test_cylinder3d.py:113-124).
- * regrouped: a hint, nonzero when `table` went through d3d_spconv_mm_regroup: the kernel then packs the few offsets a
- * tile has left into its pipeline stages instead of walking fixed windows of offsets.  Results do not depend on it. */
+ * regrouped: a hint, nonzero when `table` went through d3d_spconv_mm_regroup: the kernel then deals the tiles out costly
+ * ones first.  Results do not depend on it. */
 typedef struct {
   int32_t relu;
   const void* residual;
@@ -293,9 +293,8 @@ int d3d_spconv_mm_run(d3d_spconv_mm_t handle, int dtype, const void* in_feats, i
                       const int32_t* num_act_out, const void* table, void* out_feats,
                       const d3d_spconv_mm_epilogue* epilogue, void* stream);
 /* Kernel choice for tests and profiling: 0 = automatic, 1 = SIMT fp32-FMA path, 2 = tcgen05 tensor-core path (what
- * "automatic" picks for eligible shapes), 3 = tcgen05 path restricted to one CTA per SM (layers of at most 64 input
- * channels otherwise run two half-size CTAs per SM).  2 and 3 fail with D3D_ERR_INVALID_ARGUMENT at run time when
- * the shape is not eligible. */
+ * "automatic" picks for eligible shapes), 3 = the same.  2 and 3 fail with D3D_ERR_INVALID_ARGUMENT at run time when
+ * the shape is not eligible.  Weights that are not finite in the compute dtype take the SIMT path with every choice. */
 int d3d_spconv_mm_set_kernel(d3d_spconv_mm_t handle, int which);
 /* Opt-in for callers that enqueue layers back to back on ONE stream (as TensorRT does): the tensor-core kernel is
  * launched with the programmatic stream-serialisation attribute, so that its prologue overlaps the tail of the

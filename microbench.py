@@ -25,20 +25,17 @@ def main():
     ap.add_argument("--voxels", type=int, default=66000)
     ap.add_argument("--grid", type=int, nargs=3, default=[11, 360, 360], help="Z Y X of the voxel grid")
     ap.add_argument("--stride", type=int, default=1)
-    ap.add_argument("--kernel", type=int, default=0, help="0 auto, 1 SIMT, 2 tcgen05, 3 tcgen05 with one CTA per SM")
+    ap.add_argument("--kernel", type=int, default=0, help="0 auto, 1 SIMT, 2 or 3 tcgen05")
     ap.add_argument("--dtype", default="fp16", choices=["fp16", "bf16"])
     ap.add_argument("--reps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--index-reps", type=int, default=0, help="also time the rulebook + table build this many times")
     ap.add_argument("--plan", type=int, nargs=3, default=None, metavar=("GROUP", "STAGES", "PRODUCER_WARPS"),
-                    help="override the tensor-core kernel's pipeline plan (0 = automatic)")
+                    help="override the tensor-core kernel's plan: 16 or 24 producer warps (0 = automatic); the first two have no effect")
     ap.add_argument("--regroup", action="store_true",
                     help="run on the neighbour table with its outputs grouped by offset mask (d3d_spconv_mm_regroup)")
     ap.add_argument("--lib", default=None, metavar="NAME",
                     help="load the tuning build libs/libdeploy3d_b200_NAME.so (python -m deploy3d_b200.build --tuning NAME ...)")
-    ap.add_argument("--role-cycles", action="store_true",
-                    help="after the timed launches, one more launch whose per-role cycle counts (CTA 0) are printed; "
-                         "needs a tuning build with -DD3D_TC_PROFILE")
     args = ap.parse_args()
     if args.lib:
         from deploy3d_b200 import _lib
@@ -107,21 +104,6 @@ def main():
     if blocks_plain is not None:
         res["tile_offset_blocks"] = {"plain": blocks_plain, "regrouped": blocks_grouped}
         res["regroup_us"] = regroup_us
-    if args.role_cycles:
-        import ctypes
-        from deploy3d_b200 import _lib
-        mm.run(x, num_out, table, out=out, relu=True)
-        buf = (ctypes.c_longlong * 24)()
-        copy_prof = _lib.lib().d3d_debug_copy_prof  # AttributeError without -DD3D_TC_PROFILE
-        copy_prof.restype, copy_prof.argtypes = ctypes.c_int, [ctypes.POINTER(ctypes.c_longlong)]
-        _lib.check("d3d_debug_copy_prof", copy_prof(buf))
-        c = np.array(list(buf)).reshape(3, 8)
-        res["role_cycles"] = {
-            "producer_warp0": {"other": int(c[0, 0]), "walk_and_id_loads": int(c[0, 1]), "wait_empty": int(c[0, 2]),
-                               "address_and_copy_issue": int(c[0, 3])},
-            "mma_warp": {"other": int(c[1, 0]), "wait_full": int(c[1, 1]), "proxy_fence": int(c[1, 2]),
-                         "issue_and_commit": int(c[1, 3]), "wait_accumulator": int(c[1, 4])},
-            "epilogue_warp0": {"other": int(c[2, 0]), "wait_accumulator_full": int(c[2, 1]), "work": int(c[2, 2])}}
     if args.index_reps:
         torch.cuda.synchronize()
         e0.record()

@@ -1,0 +1,110 @@
+"""SPConvMM on the tensor cores at the edges of its units, rounds and accumulators: kernel volumes that leave windows of
+offsets and pairs of them half full, one to three rounds per CTA with a remainder, every number of accumulators, features and
+outputs that start on 16 bytes only, weights that are not finite.  Held against the SIMT kernel of the same library, which
+walks the offsets one by one (tests/test_gpu_spconv_tc.py holds both against the oracle)."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from tests._util import assert_feats_close, rng, unique_coors
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _error():
+    from deploy3d_b200 import _lib
+    code = ctypes.c_int(-1)
+    _lib.check("d3d_debug_take_kernel_error", _lib.lib().d3d_debug_take_kernel_error(ctypes.byref(code)))
+    return code.value
+
+
+def _setup(d3d, n, grid, ks, cin, cout, dtype, seed, cap=None, edit=None):
+    """Table of a SubM rulebook over n random voxels, features, and a plugin with random weights (`edit` may change them)."""
+    from deploy3d_b200.plugins import SPConvMMPlugin, deserialize_plugin
+    cap = cap or n
+    coors = torch.from_numpy(unique_coors(rng(seed), n, grid)).to(DEV)
+    num = torch.tensor([n], dtype=torch.int32, device=DEV)
+    outs = d3d.spconv_index(coors, num, torch.empty([grid[0], 0] + grid[1:], dtype=torch.int32, device=DEV), ks, (1,) * 3,
+                            tuple(k // 2 for k in ks), (1,) * 3, (0,) * 3, cap, True, False)
+    kvol = int(np.prod(ks))
+    table = SPConvMMPlugin.prepare(kvol, False, cap, outs[0], outs[1])
+    r = rng(seed + 1)
+    w = (r.standard_normal((kvol, cin, cout)) * np.sqrt(2.0 / (kvol * cin))).astype(np.float32)
+    b = r.standard_normal(cout).astype(np.float32)
+    if edit:
+        edit(w)
+    plug = deserialize_plugin("SPConvMM", d3d.data_s_spconv_mm(ks, cin, cout, cap, True, False, w, b))
+    plug.configure(dtype)
+    x = torch.from_numpy(r.standard_normal((n, cin)).astype(np.float32)).to(DEV, dtype)
+    return plug, x, num, table
+
+
+def _both(plug, x, num, table, **kw):
+    plug.set_kernel(1)
+    want = plug.run(x, num, table, **kw).float().cpu().numpy()
+    plug.set_kernel(2)
+    got = plug.run(x, num, table, **kw)
+    assert _error() == 0, "a bounded wait of the tensor-core kernel expired"
+    return got, want
+
+
+@pytest.mark.parametrize("ks", [(1, 1, 1), (3, 1, 1), (5, 1, 1), (1, 3, 3), (5, 3, 1), (3, 3, 3)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (32, 32), (64, 64), (128, 48), (256, 16)])
+def test_kernel_volumes(d3d, ks, cin, cout):
+    plug, x, num, table = _setup(d3d, 3000, [1, 20, 24, 22], ks, cin, cout, torch.float16, 3)
+    got, want = _both(plug, x, num, table, relu=True)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "kernel %s" % (ks,))
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 147, 149, 297, 445, 593])
+@pytest.mark.parametrize("cin,cout", [(32, 64), (64, 128)])
+def test_rounds_and_their_remainder(d3d, tiles, cin, cout):
+    n = tiles * 128 - 37
+    plug, x, num, table = _setup(d3d, n, [2, 40, 48, 44], (3, 1, 3), cin, cout, torch.bfloat16, tiles)
+    res = torch.randn((n, cout), device=DEV).bfloat16()
+    got, want = _both(plug, x, num, table, relu=True, residual=res)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d tiles" % tiles)
+
+
+@pytest.mark.parametrize("cout", [16, 32, 48, 64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 240, 256])
+def test_numbers_of_accumulators(d3d, cout):
+    plug, x, num, table = _setup(d3d, 57000, [2, 40, 48, 44], (3, 1, 1), 32, cout, torch.float16, cout)
+    got, want = _both(plug, x, num, table)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d output channels" % cout)
+
+
+@pytest.mark.parametrize("cin", [16, 32, 64, 128])
+def test_features_and_outputs_on_16_bytes(d3d, cin):
+    n, cout = 5000, 48
+    plug, x, num, table = _setup(d3d, n, [1, 24, 30, 20], (3, 3, 3), cin, cout, torch.float16, 7)
+    want = plug.run(x, num, table, relu=True)
+    at = lambda t: torch.cat([t.new_zeros(8), t.flatten()])[8:].view(t.shape)
+    out = at(torch.zeros_like(want))
+    moved = at(x)
+    assert moved.data_ptr() % 32 == 16 and out.data_ptr() % 32 == 16
+    assert torch.equal(plug.run(moved, num, table, out=out, relu=True), want)
+    assert _error() == 0
+
+
+@pytest.mark.parametrize("said", [0, 1, 700, 100000])
+def test_live_count_only_deals_out_the_tiles(d3d, said):
+    """`num_act_out` orders the work; what is computed follows from the table alone."""
+    plug, x, num, table = _setup(d3d, 5000, [1, 24, 30, 20], (3, 3, 3), 32, 32, torch.float16, 9, cap=9000)
+    want = plug.run(x, num, table)
+    got = plug.run(x, torch.tensor([said], dtype=torch.int32, device=DEV), table)
+    assert torch.equal(got, want) and _error() == 0
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1e6])
+def test_weights_that_are_not_finite(d3d, value):
+    """An infinite weight (1e6 is one in fp16) reaches the rows that have an input under its offset and no others."""
+    def edit(w):
+        w[5, 3, 2] = value
+    plug, x, num, table = _setup(d3d, 2000, [1, 24, 30, 20], (3, 3, 3), 32, 32, torch.float16, 11, edit=edit)
+    got, want = _both(plug, x, num, table)
+    got = got.float().cpu().numpy()
+    assert 0 < (~np.isfinite(want)).sum() < 2000
+    np.testing.assert_array_equal(got, want)
