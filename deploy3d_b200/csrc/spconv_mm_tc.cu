@@ -282,7 +282,9 @@ struct __align__(16) Shared {
   uint64_t acc_empty[kMaxAcc];
   uint64_t b_full[kMaxBSlots];
   uint64_t b_empty[kMaxBSlots];
-  uint64_t b_ready;  // resident weights have landed
+  uint64_t b_ready;     // resident weights have landed
+  uint64_t live_ready;  // `live` is known
+  int live;             // tiles that hold live outputs, read once so that all roles deal the tiles out alike
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -317,7 +319,8 @@ struct Round {
   uint32_t mask;  // lane i (mod 4): offset mask of the CTA's tile i, 0 = no such tile
 };
 __device__ __forceinline__ int live_tiles(const TcParams& p) {
-  if (!p.num_out || p.regrouped) return p.num_tiles;
+  // (at most one tile to a CTA: nothing to deal out, and a trip to L2 less in front of a short launch)
+  if (!p.num_out || p.regrouped || p.num_tiles <= (int)gridDim.x) return p.num_tiles;
   const int64_t n = ((int64_t)*reinterpret_cast<const volatile int32_t*>(p.num_out) + kTileRows - 1) / kTileRows;
   return n < 0 ? 0 : n < p.num_tiles ? (int)n : p.num_tiles;
 }
@@ -408,7 +411,7 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
     for (int a = 0; a < p.num_acc; ++a) mbar_init(&sh->acc_full[a], 1), mbar_init(&sh->acc_empty[a], 4 * epilogue_sets(kMma));
     for (int b = 0; b < p.b_slots; ++b) mbar_init(&sh->b_full[b], 1), mbar_init(&sh->b_empty[b], kMma);
     for (int l = 0; l < 2; ++l) mbar_init(&sh->list_full[l], 1), mbar_init(&sh->list_empty[l], 9 * kMma);
-    mbar_init(&sh->b_ready, 1);
+    mbar_init(&sh->b_ready, 1), mbar_init(&sh->live_ready, 1);
     sh->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -606,12 +609,15 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   }
   __syncwarp();
   pdl_wait();  // the offset masks come from the preceding kernels
-  const int live = live_tiles(p);
+  const int live = __shfl_sync(0xffffffffu, live_tiles(p), 0);
+  if (lane == 0) {
+    sh->live = live;
+    mbar_arrive(&sh->live_ready);
+  }
   int buf = 0, b_slot = 0;
   uint32_t list_phase = 0, b_phase = 0;
   Round r;
   open_round<kMma>(p, live, 0, r);
-  prefetch_round(p, live, r);
   for (;;) {
     const bool end = r.tiles == 0;
     uint32_t masks[kMma], all = 0;
@@ -622,11 +628,10 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
       all |= masks[i], count += masks[i] != 0u;
     }
     const Round done = r;
-    if (!end) {  // the next round's masks are on their way
+    if (all == 0u && !end) {
       open_round<kMma>(p, live, after_round(done), r);
-      prefetch_round(p, live, r);
+      continue;
     }
-    if (all == 0u && !end) continue;
     if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14))) return;
     // lane w lists window w
     const uint32_t bits = lane < kWindows ? kWindow << (lane * kOffs) : 0u;
@@ -652,6 +657,8 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     if (buf) list_phase ^= 1;
     buf ^= 1;
     if (end) return;
+    open_round<kMma>(p, live, after_round(done), r);  // the next round's masks are on their way
+    prefetch_round(p, live, r);
     if (!resident) {
       // two (window, part)s to a slot
       uint32_t rest = windows;
@@ -792,9 +799,12 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
   uint32_t acc_phase = 0;
   const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
   pdl_wait();  // residual rows come from an earlier layer; output rows may still be read by the preceding kernel
-  const int live = live_tiles(p);
+  if (!__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32))) return;
+  const int live = sh->live;
   Round r;
-  for (open_round<kMma>(p, live, 0, r); r.tiles; open_round<kMma>(p, live, after_round(r), r)) {
+  open_round<kMma>(p, live, 0, r);
+  if (quad == 0 && set == 0) prefetch_round(p, live, r);  // of the first round; the control warp sees to the others
+  for (; r.tiles; open_round<kMma>(p, live, after_round(r), r)) {
     for (int i = 0; i < r.tiles; ++i) {
       const uint32_t mask = __shfl_sync(0xffffffffu, r.mask, i);
       const int index = tile_index(p, r, i);
