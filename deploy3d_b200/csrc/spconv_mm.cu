@@ -56,7 +56,7 @@ __global__ void pack_mask_kernel(const uint4* __restrict__ row_masks, int64_t ti
 // index rows: gatherIn | scatterOut | kernelOffset (trt/spconv/index_trt.cu:211-213); `inverse` swaps the
 // first two (trt/spconv/mm_trt.cu:174-177).
 // Besides the ids, every (tile of 128 outputs, offset) gets a 128-bit mask of the rows that have an input: the
-// convolution kernel copies only those rows and lets the tensor core update only those accumulator lanes.
+// convolution kernel loads only those rows and takes zeros for the others.
 __global__ void table_scatter_kernel(const int32_t* __restrict__ index, int64_t row_len,
                                      const int32_t* __restrict__ num_index, int inverse, int mirror, int kvol,
                                      int64_t m_max, int32_t* __restrict__ table, uint32_t* __restrict__ row_masks,
@@ -215,7 +215,7 @@ __global__ void table_redo_kernel(const unsigned long long* __restrict__ checks,
 // ---------------------------------------------------------------------------------------------
 // Regrouping: tiles of outputs with like offset masks
 // ---------------------------------------------------------------------------------------------
-// A (tile, offset) block costs the convolution kernel a stage slot, a weight block and its MMAs whether one row or
+// A (tile, offset) block costs the convolution kernel a slot, a weight block and its MMAs whether one row or
 // all 128 have an input, and with the outputs in voxel order nearly every offset feeds some row of every tile.  Sorted
 // by their own offset mask (which of the kVol offsets have an input), outputs with like masks share a tile and the
 // tile's mask shrinks to little more than theirs: LiDAR frames go from 27 to 4-19 blocks per tile.  The regrouped
