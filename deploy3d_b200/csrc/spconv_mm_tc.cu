@@ -86,7 +86,6 @@ struct TcParams {
   const uint32_t* tile_mask;   // [tiles] bit k set: offset k feeds the tile
   const uint32_t* row_masks;   // [tiles][kvol][4] bit r of word q set: row 32 q + r has an input under the offset
   const int32_t* perm;         // [tiles][128] output row of every tile row, -1 = none
-  const int32_t* num_out;      // live outputs (may be null): only how the tiles are dealt out depends on it
   const void* in_feats;        // [n_in_rows][cin]
   int64_t m_max;
   int32_t n_in_rows;  // rows of the gathered tensor
@@ -284,7 +283,7 @@ struct __align__(16) Shared {
   uint64_t b_empty[kMaxBSlots];
   uint64_t b_ready;     // resident weights have landed
   uint64_t live_ready;  // `live` is known
-  int live;             // tiles that hold live outputs, read once so that all roles deal the tiles out alike
+  int live;             // where the tiles without an offset begin, found once for all roles
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -318,11 +317,29 @@ struct Round {
   int tiles;      // tiles per CTA
   uint32_t mask;  // lane i (mod 4): offset mask of the CTA's tile i, 0 = no such tile
 };
+// Where the tiles behind which no tile has an offset begin, found by the whole warp from the offset masks alone: up to a
+// 128th of them late (that many are looked at, in one trip to L2; eight to a lane instead of four made the kernel large enough
+// to cost 64 -> 128 at 238 k voxels 88 -> 93 us).  Where empty tiles lie between others the answer may be smaller; every CTA comes
+// to the same one, which is what dealing the tiles out asks for.
 __device__ __forceinline__ int live_tiles(const TcParams& p) {
-  // (at most one tile to a CTA: nothing to deal out, and a trip to L2 less in front of a short launch)
-  if (!p.num_out || p.regrouped || p.num_tiles <= (int)gridDim.x) return p.num_tiles;
-  const int64_t n = ((int64_t)*reinterpret_cast<const volatile int32_t*>(p.num_out) + kTileRows - 1) / kTileRows;
-  return n < 0 ? 0 : n < p.num_tiles ? (int)n : p.num_tiles;
+  // (at most one tile to a CTA: nothing to deal out)
+  if (p.regrouped || p.num_tiles <= (int)gridDim.x) return p.num_tiles;
+  constexpr int kProbes = 4;
+  const int step = (p.num_tiles + 32 * kProbes - 1) / (32 * kProbes);
+  uint32_t mask[kProbes];
+#pragma unroll
+  for (int i = 0; i < kProbes; ++i) {
+    const int64_t tile = (int64_t)(i * 32 + (threadIdx.x & 31)) * step;
+    mask[i] = tile < p.num_tiles ? __ldg(p.tile_mask + tile) : 0u;
+  }
+  int parts = 0;  // up to the last probe with an offset
+#pragma unroll
+  for (int i = 0; i < kProbes; ++i) {
+    const uint32_t has = __ballot_sync(0xffffffffu, mask[i] != 0u);
+    if (has) parts = i * 32 + 32 - __clz(has);
+  }
+  const int64_t live = (int64_t)parts * step;
+  return live < p.num_tiles ? (int)live : p.num_tiles;
 }
 // Index of the CTA's tile i in a round, and the tile it stands for.
 __device__ __forceinline__ int tile_index(const TcParams& p, const Round& r, int i) {
@@ -609,15 +626,16 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   }
   __syncwarp();
   pdl_wait();  // the offset masks come from the preceding kernels
-  const int live = __shfl_sync(0xffffffffu, live_tiles(p), 0);
+  Round r;
+  open_round<kMma>(p, p.num_tiles, 0, r);  // as if all were live, so that the masks are on their way
+  const int live = live_tiles(p);
   if (lane == 0) {
     sh->live = live;
     mbar_arrive(&sh->live_ready);
   }
+  if (live < r.tiles * (int)gridDim.x && live < p.num_tiles) open_round<kMma>(p, live, 0, r);  // not a whole round
   int buf = 0, b_slot = 0;
   uint32_t list_phase = 0, b_phase = 0;
-  Round r;
-  open_round<kMma>(p, live, 0, r);
   for (;;) {
     const bool end = r.tiles == 0;
     uint32_t masks[kMma], all = 0;
@@ -989,7 +1007,6 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   TcParams p;
   const TableParts t = table_parts(const_cast<int32_t*>(a.table), kvol, m_max);
   p.table = t.ids, p.tile_mask = t.tile_mask, p.row_masks = t.row_masks, p.perm = t.perm;
-  p.num_out = a.num_act_out;
   p.in_feats = a.in_feats;
   p.m_max = m_max;
   p.n_in_rows = (int32_t)a.max_num_act_in;

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests._util import assert_feats_close, rng, unique_coors
+from tests._util import assert_feats_close, rng, table_parts, unique_coors
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -91,11 +91,46 @@ def test_features_and_outputs_on_16_bytes(d3d, cin):
 
 @pytest.mark.parametrize("said", [0, 1, 700, 100000])
 def test_live_count_only_deals_out_the_tiles(d3d, said):
-    """`num_act_out` orders the work; what is computed follows from the table alone."""
+    """What is computed follows from the table alone."""
     plug, x, num, table = _setup(d3d, 5000, [1, 24, 30, 20], (3, 3, 3), 32, 32, torch.float16, 9, cap=9000)
     want = plug.run(x, num, table)
     got = plug.run(x, torch.tensor([said], dtype=torch.int32, device=DEV), table)
     assert torch.equal(got, want) and _error() == 0
+
+
+def test_count_that_changes_during_the_launch(d3d):
+    """Which CTA computes which tile follows from the table alone: the word of `num_act_out` may be rewritten meanwhile."""
+    plug, x, num, table = _setup(d3d, 41000, [2, 40, 48, 44], (3, 1, 3), 32, 32, torch.float16, 13, cap=60000)
+    want = plug.run(x, num, table).clone()
+    said = num.clone()
+    out = torch.empty_like(want)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(60):
+        with torch.cuda.stream(other):
+            for v in (0, 100, 41000, 30000, 60000):
+                said.fill_(v)
+        out.fill_(7.0)
+        plug.run(x, said, table, out=out)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and _error() == 0
+
+
+@pytest.mark.parametrize("empty", ["none", "tail", "middle", "all_but_last", "every_other", "all"])
+def test_tiles_without_an_offset(d3d, empty):
+    """Tiles no offset feeds, wherever they lie in the table, hold the bias and the residual."""
+    cap = 60000
+    plug, x, num, table = _setup(d3d, cap, [2, 40, 48, 44], (3, 1, 3), 32, 32, torch.float16, 14)
+    _, tile_mask, row_masks, _ = table_parts(table, 9, cap)
+    tiles = tile_mask.numel()
+    gone = torch.zeros(tiles, dtype=torch.bool, device=DEV)
+    gone[{"none": slice(0, 0), "tail": slice(390, tiles), "middle": slice(150, 401), "all_but_last": slice(0, tiles - 1),
+          "every_other": slice(0, tiles, 2), "all": slice(0, tiles)}[empty]] = True
+    tile_mask[gone] = 0
+    row_masks[gone] = 0
+    res = torch.randn((cap, 32), device=DEV).half()
+    got, want = _both(plug, x, num, table, residual=res)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, empty)
 
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1e6])
