@@ -100,6 +100,7 @@ SIGNATURES = {
     "d3d_version": (ctypes.c_char_p, []),
     "d3d_status_string": (ctypes.c_char_p, [ctypes.c_int]),
     "d3d_debug_take_kernel_error": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
+    "d3d_debug_set_wait_limit": (ctypes.c_int, [ctypes.c_int]),
     "d3d_spconv_mm_regroup_scratch_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int64]),
     "d3d_spconv_mm_regroup": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _vp, _vp, _vp, ctypes.c_size_t, _vp]),
     "d3d_debug_take_bounds_violation": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int32)]),

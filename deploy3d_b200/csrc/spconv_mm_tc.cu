@@ -71,7 +71,7 @@ constexpr int kListUnits = 128;  // units of a tile: 32 offsets of four parts
 // TMEM lane quarters), the MMA warps and the control warp.
 __host__ __device__ constexpr int epilogue_sets(int mma_warps) { return mma_warps == 2 ? 2 : 1; }
 __host__ __device__ constexpr int threads_of(int mma_warps) { return (9 * mma_warps + 4 * epilogue_sets(mma_warps) + 1) * 32; }
-constexpr long long kWaitLimitCycles = 2000ll * 1000ll * 1000ll;  // about a second
+constexpr uint32_t kWaitLimitCycles = 2000u * 1000u * 1000u;  // about a second; differences of the 32-bit clock hold twice that
 
 __device__ int g_tc_error;  // 0 ok; otherwise the code of the first wait that gave up
 
@@ -106,6 +106,7 @@ struct TcParams {
   const void* residual;
   int relu;
   int is_bf16;
+  uint32_t wait_limit;  // cycles after which a wait gives up
 };
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------
@@ -145,12 +146,13 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait.  Returns false (and records `code`) when the barrier did not flip within the limit or another role
 // already gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                          uint32_t limit) {
   if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
+  const uint32_t t0 = (uint32_t)clock();
   while (!mbar_try_wait(bar, parity)) {
     if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitLimitCycles) {
+    if ((uint32_t)clock() - t0 > limit) {
       *abort_flag = code;
       atomicCAS(&g_tc_error, 0, code);
       return false;
@@ -488,7 +490,7 @@ __device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, 
         open = false;
       }
       if (!block && !__all_sync(0xffffffffu, mbar_test(&sh->list_full[buf], list_phase))) return kLater;
-      if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 13))) return kEnd;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 13, p.wait_limit))) return kEnd;
       const int4 round = sh->round[buf];
       if (round.x == 0) return kEnd;
       len = owner < round.x ? round.z : 0;
@@ -550,7 +552,7 @@ __device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, 
     n += 2;
     next = settle(false);
     if (next == kUnit) load_unit();  // in flight while this unit's rows arrive
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->empty[team], phase, abort_flag, 12))) return;
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->empty[team], phase, abort_flag, 12, p.wait_limit))) return;
     tc_fence_after();
     if constexpr (kRows == 4) {
 #pragma unroll
@@ -650,7 +652,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
       open_round<kMma>(p, live, after_round(done), r);
       continue;
     }
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14))) return;
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14, p.wait_limit))) return;
     // lane w lists window w
     const uint32_t bits = lane < kWindows ? kWindow << (lane * kOffs) : 0u;
     const bool present = (all & bits) != 0u;
@@ -681,7 +683,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
       // two (window, part)s to a slot
       uint32_t rest = windows;
       for (int seq = 0, part = 0; seq < steps; seq += 2) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11))) return;
+        if (!__all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11, p.wait_limit))) return;
         const int both = seq + 1 < steps ? 2 : 1;
         if (lane == 0) mbar_arrive_expect_tx(&sh->b_full[b_slot], (uint32_t)(both * kOffs) * b_tx);
         for (int h = 0; h < both; ++h) {
@@ -718,7 +720,8 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   const bool resident = p.b_slots == 0;
   const int parts = p.parts, num_acc = p.num_acc, b_slots = p.b_slots;
   const uint32_t cout = (uint32_t)p.cout;
-  if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23))) return;
+  if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23, p.wait_limit))) return;
+  pdl_wait();  // the first list comes after the preceding kernels, which may take longer than a wait is allowed to
   // the slots of this warp's two teams, taken in turn
   const uint32_t a_of[2] = {ring + (uint32_t)(me * kUnitCols), ring + (uint32_t)((me + kMma) * kUnitCols)};
   uint64_t* const full_of[2] = {&sh->full[me], &sh->full[me + kMma]};
@@ -726,7 +729,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   int buf = 0, b_slot = 0, acc0 = 0;
   uint32_t list_phase = 0, b_phase = 0, turn = 0, acc_phase = 0;  // turn: bit 0 the slot, bit 1 its phase
   for (;;) {
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 15))) return;
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 15, p.wait_limit))) return;
     const int4 round = sh->round[buf];
     const int count = (int)__reduce_or_sync(0xffffffffu, (unsigned)round.x);
     const uint32_t windows = __reduce_or_sync(0xffffffffu, (unsigned)round.y);
@@ -736,7 +739,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
     const bool wrap = acc0 + me >= num_acc;
     const int acc = wrap ? acc0 + me - num_acc : acc0 + me;
     const uint32_t d_addr = tmem_base + (uint32_t)acc * cout;
-    if (mine && !__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22)))
+    if (mine && !__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22, p.wait_limit)))
       return;
     tc_fence_after();
     uint32_t add = 0u;  // the first products of a round start the sums
@@ -767,9 +770,9 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
       // One lane waits and issues, for both windows at once: every instruction of this warp between two products is one too
       // many.  After a wait that gave up all others give up at once, and what is issued then does not matter.
       if (elect_one()) {
-        if (!resident) mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24);
+        if (!resident) mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24, p.wait_limit);
         auto unit = [&](int h) {
-          mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21);
+          mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21, p.wait_limit);
           tc_fence_after();
           umma_f16_ta(d_addr, a_addr[h], desc[h][0], idesc, h ? 1u : add);
 #pragma unroll
@@ -817,7 +820,7 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
   uint32_t acc_phase = 0;
   const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
   pdl_wait();  // residual rows come from an earlier layer; output rows may still be read by the preceding kernel
-  if (!__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32))) return;
+  if (!__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32, p.wait_limit))) return;
   const int live = sh->live;
   Round r;
   open_round<kMma>(p, live, 0, r);
@@ -838,7 +841,7 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
         uint4 res[2];  // of the next 16 columns, on their way
         if (kAdd && row_ok && from < to) res[0] = __ldg(res_row + from / 8), res[1] = __ldg(res_row + from / 8 + 1);
         if (!empty_tile) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc], acc_phase, abort_flag, 31))) return false;
+          if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc], acc_phase, abort_flag, 31, p.wait_limit))) return false;
           tc_fence_after();
         }
         for (int c0 = from; c0 < to; c0 += 16) {
@@ -933,6 +936,7 @@ struct TcState {
 
 // Tuning override for experiments (0 = automatic).
 int g_plan_mma_warps = 0;
+uint32_t g_wait_limit = kWaitLimitCycles;  // d3d_debug_set_wait_limit
 
 typedef void (*KernelFn)(const CUtensorMap, const TcParams);
 struct KernelEntry {
@@ -1026,6 +1030,7 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   p.residual = a.residual;
   p.relu = a.relu;
   p.is_bf16 = a.dtype == D3D_BF16;
+  p.wait_limit = g_wait_limit;
 
   // Three MMA warps where a unit's products are short (up to 64 columns: 24 producer warps then feed them), two where the tensor
   // pipe is the longer part, where few offsets make the epilogue it (it has eight warps then) and for 16 input channels, whose
@@ -1092,6 +1097,14 @@ extern "C" int d3d_debug_take_kernel_error(int* code) {
   if (cudaDeviceSynchronize() != cudaSuccess) return D3D_ERR_CUDA;
   if (cudaMemcpyFromSymbol(code, d3d::g_tc_error, sizeof(int)) != cudaSuccess) return D3D_ERR_CUDA;
   if (cudaMemcpyToSymbol(d3d::g_tc_error, &zero, sizeof(int)) != cudaSuccess) return D3D_ERR_CUDA;
+  return D3D_OK;
+}
+
+// Debug aid without a reference counterpart: after how many cycles a bounded wait of the tensor-core kernel gives up, for every
+// later launch of this process (0 = the usual second).  Not thread-safe.
+extern "C" int d3d_debug_set_wait_limit(int cycles) {
+  D3D_REQUIRE(cycles >= 0, D3D_ERR_INVALID_ARGUMENT);
+  d3d::g_wait_limit = cycles ? (uint32_t)cycles : d3d::kWaitLimitCycles;
   return D3D_OK;
 }
 

@@ -73,6 +73,9 @@ const char* d3d_status_string(int status);
  * time-sliced away for longer would trip it too), the CTA then drains, part of the output stays unwritten, and the
  * asynchronous enqueue that launched it has long returned D3D_OK.  Not thread-safe. */
 int d3d_debug_take_kernel_error(int* code);
+/* Debug aid (no reference counterpart): after how many cycles such a wait gives up, for every later launch of the process;
+ * 0 = the usual second.  Tests shorten it.  Not thread-safe. */
+int d3d_debug_set_wait_limit(int cycles);
 /* Debug aid (no reference counterpart).  A checked build of the library (-DDEPLOY3D_BOUNDS_CHECK) range-checks every
  * row id, table entry and coordinate its kernels index with, skips an access that is out of range and records it:
  * this call synchronises the device, copies {violations seen, site, value, limit of the first} to record[0..3] and

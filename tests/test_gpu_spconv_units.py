@@ -21,6 +21,15 @@ def _error():
     return code.value
 
 
+@pytest.fixture
+def wait_limit():
+    """Sets the cycles after which a bounded wait gives up; the usual second again afterwards."""
+    from deploy3d_b200 import _lib
+    set_to = lambda cycles: _lib.check("d3d_debug_set_wait_limit", _lib.lib().d3d_debug_set_wait_limit(cycles))
+    yield set_to
+    set_to(0)
+
+
 def _setup(d3d, n, grid, ks, cin, cout, dtype, seed, cap=None, edit=None):
     """Table of a SubM rulebook over n random voxels, features, and a plugin with random weights (`edit` may change them)."""
     from deploy3d_b200.plugins import SPConvMMPlugin, deserialize_plugin
@@ -143,3 +152,21 @@ def test_weights_that_are_not_finite(d3d, value):
     got = got.float().cpu().numpy()
     assert 0 < (~np.isfinite(want)).sum() < 2000
     np.testing.assert_array_equal(got, want)
+
+
+def test_preceding_kernel_does_not_count_towards_a_wait(d3d, wait_limit):
+    """A layer launched while the one in front still runs waits for it without a limit: the bound is on the kernel's own
+    hand-overs.  64 voxels with 27 offsets of 256 -> 256 channels are two CTAs of 57 M multiply-adds each on the SIMT kernel, at
+    least 440 k cycles at 128 a cycle; the 256 -> 16 layer behind it takes about 40 k in all."""
+    first, x, num, table = _setup(d3d, 64, [1, 4, 4, 4], (3, 3, 3), 256, 256, torch.float16, 21)
+    second, _, _, _ = _setup(d3d, 64, [1, 4, 4, 4], (3, 3, 3), 256, 16, torch.float16, 22)
+    first.set_kernel(1)
+    want = second.run(first.run(x, num, table), num, table).clone()
+    second.set_dependent_launch(True)
+    wait_limit(150000)
+    mid, got = torch.empty_like(x), torch.empty_like(want)
+    for _ in range(3):
+        first.run(x, num, table, out=mid)
+        second.run(mid, num, table, out=got)
+    assert _error() == 0, "a wait ran out while the preceding kernel was running"
+    assert torch.equal(got, want)
