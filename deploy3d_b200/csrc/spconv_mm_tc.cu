@@ -144,7 +144,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  Returns false (and records `code`) when the barrier did not flip within the limit or another role
+// Bounded wait.  Returns false (and leaves `code` in the flag) when the barrier did not flip within the limit or another role
 // already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
                                           uint32_t limit) {
@@ -154,11 +154,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (*abort_flag) return false;
     if ((uint32_t)clock() - t0 > limit) {
       *abort_flag = code;
-      atomicCAS(&g_tc_error, 0, code);
       return false;
     }
   }
   return true;
+}
+// Waits for something the warp has set in motion itself and that needs no other role to end, whoever has given up meanwhile: a
+// CTA must not end, nor return its tensor memory, while copies or MMAs of its own are on their way.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const uint32_t t0 = (uint32_t)clock();
+  while (!mbar_try_wait(bar, parity) && (uint32_t)clock() - t0 <= kWaitLimitCycles) {
+  }
 }
 __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y) {
   asm volatile(
@@ -283,6 +289,7 @@ struct __align__(16) Shared {
   uint64_t acc_empty[kMaxAcc];
   uint64_t b_full[kMaxBSlots];
   uint64_t b_empty[kMaxBSlots];
+  uint64_t drained[kMaxMmaWarps];  // the MMAs of a warp that gave up are over
   uint64_t b_ready;     // resident weights have landed
   uint64_t live_ready;  // `live` is known
   int live;             // where the tiles without an offset begin, found once for all roles
@@ -427,6 +434,7 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
   Shared* sh = s.sh;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * kMma; ++i) mbar_init(&sh->full[i], 4), mbar_init(&sh->empty[i], 1);
+    for (int i = 0; i < kMma; ++i) mbar_init(&sh->drained[i], 1);
     for (int a = 0; a < p.num_acc; ++a) mbar_init(&sh->acc_full[a], 1), mbar_init(&sh->acc_empty[a], 4 * epilogue_sets(kMma));
     for (int b = 0; b < p.b_slots; ++b) mbar_init(&sh->b_full[b], 1), mbar_init(&sh->b_empty[b], kMma);
     for (int l = 0; l < 2; ++l) mbar_init(&sh->list_full[l], 1), mbar_init(&sh->list_empty[l], 9 * kMma);
@@ -442,14 +450,15 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
   return sh->tmem_base;
 }
 
-// All roles meet, then the allocating warp returns the tensor memory.
+// All roles meet, then the allocating warp returns the tensor memory and reports a wait that gave up.
 template <int kMma>
-__device__ __forceinline__ void cta_teardown(const TcParams& p, uint32_t tmem_base) {
+__device__ __forceinline__ void cta_teardown(const Smem& s, uint32_t tmem_base) {
   tc_fence_before();
   __syncthreads();
   if ((int)(threadIdx.x >> 5) == 8 * kMma + 4 * epilogue_sets(kMma)) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
+    if (s.sh->abort_flag && elect_one()) atomicCAS(&g_tc_error, 0, s.sh->abort_flag);
   }
 }
 
@@ -638,6 +647,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   if (live < r.tiles * (int)gridDim.x && live < p.num_tiles) open_round<kMma>(p, live, 0, r);  // not a whole round
   int buf = 0, b_slot = 0;
   uint32_t list_phase = 0, b_phase = 0;
+  bool ok = true;  // no wait for a weight slot has given up
   for (;;) {
     const bool end = r.tiles == 0;
     uint32_t masks[kMma], all = 0;
@@ -652,7 +662,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
       open_round<kMma>(p, live, after_round(done), r);
       continue;
     }
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14, p.wait_limit))) return;
+    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14, p.wait_limit))) break;
     // lane w lists window w
     const uint32_t bits = lane < kWindows ? kWindow << (lane * kOffs) : 0u;
     const bool present = (all & bits) != 0u;
@@ -676,14 +686,15 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     if (lane == 0) mbar_arrive(&sh->list_full[buf]);
     if (buf) list_phase ^= 1;
     buf ^= 1;
-    if (end) return;
+    if (end) break;
     open_round<kMma>(p, live, after_round(done), r);  // the next round's masks are on their way
     prefetch_round(p, live, r);
     if (!resident) {
       // two (window, part)s to a slot
       uint32_t rest = windows;
       for (int seq = 0, part = 0; seq < steps; seq += 2) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11, p.wait_limit))) return;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11, p.wait_limit));
+        if (!ok) break;
         const int both = seq + 1 < steps ? 2 : 1;
         if (lane == 0) mbar_arrive_expect_tx(&sh->b_full[b_slot], (uint32_t)(both * kOffs) * b_tx);
         for (int h = 0; h < both; ++h) {
@@ -699,8 +710,12 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
         __syncwarp();
         if (++b_slot == p.b_slots) b_slot = 0, b_phase ^= 1;
       }
+      if (!ok) break;
     }
   }
+  // the last weights of every slot have landed
+  if (resident) mbar_drain(&sh->b_ready, 0);
+  for (int b = 0; b < p.b_slots; ++b) mbar_drain(&sh->b_full[b], b < b_slot ? b_phase : b_phase ^ 1);
 }
 
 // ---- MMA warps -------------------------------------------------------------------------------------------------------
@@ -728,8 +743,10 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   uint64_t* const empty_of[2] = {&sh->empty[me], &sh->empty[me + kMma]};
   int buf = 0, b_slot = 0, acc0 = 0;
   uint32_t list_phase = 0, b_phase = 0, turn = 0, acc_phase = 0;  // turn: bit 0 the slot, bit 1 its phase
+  bool ok = true;  // no wait has given up
   for (;;) {
-    if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 15, p.wait_limit))) return;
+    ok = __all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 15, p.wait_limit));
+    if (!ok) break;
     const int4 round = sh->round[buf];
     const int count = (int)__reduce_or_sync(0xffffffffu, (unsigned)round.x);
     const uint32_t windows = __reduce_or_sync(0xffffffffu, (unsigned)round.y);
@@ -739,8 +756,8 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
     const bool wrap = acc0 + me >= num_acc;
     const int acc = wrap ? acc0 + me - num_acc : acc0 + me;
     const uint32_t d_addr = tmem_base + (uint32_t)acc * cout;
-    if (mine && !__all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22, p.wait_limit)))
-      return;
+    ok = !mine || __all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22, p.wait_limit));
+    if (!ok) break;
     tc_fence_after();
     uint32_t add = 0u;  // the first products of a round start the sums
     uint32_t rest = windows;
@@ -768,11 +785,12 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
       uint64_t* const full[2] = {odd ? full_of[1] : full_of[0], odd ? full_of[0] : full_of[1]};
       uint64_t* const empty[2] = {odd ? empty_of[1] : empty_of[0], odd ? empty_of[0] : empty_of[1]};
       // One lane waits and issues, for both windows at once: every instruction of this warp between two products is one too
-      // many.  After a wait that gave up all others give up at once, and what is issued then does not matter.
-      if (elect_one()) {
-        if (!resident) mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24, p.wait_limit);
+      // many.  After a wait that gave up it issues nothing.
+      if (elect_one() && ok) {
+        if (!resident) ok = mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24, p.wait_limit);
         auto unit = [&](int h) {
-          mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21, p.wait_limit);
+          ok = ok && mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21, p.wait_limit);
+          if (!ok) return;
           tc_fence_after();
           umma_f16_ta(d_addr, a_addr[h], desc[h][0], idesc, h ? 1u : add);
 #pragma unroll
@@ -783,23 +801,29 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
           unit(0);
           if (both) unit(1);
         }
-        if (!resident) umma_commit(&sh->b_empty[b_slot]);
+        if (!resident && ok) umma_commit(&sh->b_empty[b_slot]);
       }
       __syncwarp();
       add = 1u;
       if (mine) turn = (turn + (both ? 2u : 1u)) & 3u;
       if (!resident && ++b_slot == b_slots) b_slot = 0, b_phase ^= 1;
     }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
     if (elect_one()) {
       if (mine) umma_commit(&sh->acc_full[acc]);
       mbar_arrive(&sh->list_empty[buf]);
     }
     __syncwarp();
-    if (*abort_flag) return;
     if (buf) list_phase ^= 1;
     buf ^= 1;
     acc0 += count;
     if (acc0 >= num_acc) acc0 -= num_acc, acc_phase ^= 1;
+  }
+  if (!ok) {  // nobody reads these accumulators: see the MMAs out here
+    if (elect_one()) umma_commit(&sh->drained[me]);
+    __syncwarp();
+    mbar_drain(&sh->drained[me], 0);
   }
 }
 
@@ -892,7 +916,7 @@ spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p)
     control_role<kOffs, kMma>(p, s, &map_b);
   }
   __syncwarp();
-  cta_teardown<kMma>(p, tmem_base);
+  cta_teardown<kMma>(s, tmem_base);
 }
 
 // ---- host ------------------------------------------------------------------------------------------------------------

@@ -170,3 +170,22 @@ def test_preceding_kernel_does_not_count_towards_a_wait(d3d, wait_limit):
         second.run(mid, num, table, out=got)
     assert _error() == 0, "a wait ran out while the preceding kernel was running"
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (32, 64), (64, 64), (64, 128), (256, 256)])
+def test_wait_that_gives_up(d3d, wait_limit, cin, cout):
+    """A wait that gives up ends the launch with an error word, wherever in the kernel it happens; the launches after it are
+    as good as ever."""
+    plug, x, num, table = _setup(d3d, 60000, [1, 40, 60, 60], (3, 3, 3), cin, cout, torch.float16, 23)
+    want = plug.run(x, num, table, relu=True).clone()
+    scrap = torch.empty_like(want)
+    codes = set()
+    for cycles in (1, 300, 1000, 3000, 10000):
+        wait_limit(cycles)
+        for _ in range(3):
+            plug.run(x, num, table, out=scrap, relu=True)
+            codes.add(_error())
+    wait_limit(0)
+    assert codes - {0}, "no wait gave up"
+    for _ in range(3):
+        assert torch.equal(plug.run(x, num, table, relu=True), want) and _error() == 0
