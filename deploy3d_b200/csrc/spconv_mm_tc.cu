@@ -107,6 +107,7 @@ struct TcParams {
   int relu;
   int is_bf16;
   uint32_t wait_limit;  // cycles after which a wait gives up
+  int table_wide;       // the table starts on 16 bytes
 };
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------
@@ -521,7 +522,10 @@ __device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, 
 #pragma unroll
     for (int o = 0; o < kOffs; ++o) {
       const bool in = o == 0 || o < offs;
-      if (kRows == 4) {
+      if (!kWide && !p.table_wide) {
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) cur.id[o][i] = in ? __ldg(ids + o * kTileRows + i) : 0;
+      } else if (kRows == 4) {
         const int4 q = in ? __ldg(reinterpret_cast<const int4*>(ids + o * kTileRows)) : make_int4(0, 0, 0, 0);
         cur.id[o][0] = q.x, cur.id[o][1] = q.y, cur.id[o][kRows - 2] = q.z, cur.id[o][kRows - 1] = q.w;
       } else {
@@ -595,12 +599,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
 // Brings what a round reads towards the SM: ids and row masks of its tiles, the rows of the input that lie where the outputs
 // do (a submanifold layer gathers each of them, here or in a tile nearby), the rows of the residual.  The producers are only
 // one unit ahead with their loads, which covers L2 but not DRAM (64 -> 64 at 238 k voxels behind other layers: 77.8 us without).
-__device__ __forceinline__ void prefetch_round(const TcParams& p, int live, const Round& r) {
+template <bool kWide> __device__ __forceinline__ void prefetch_round(const TcParams& p, int live, const Round& r) {
   const int i = threadIdx.x & 31, index = tile_index(p, r, i);
   if (i >= r.tiles || index >= r.limit || index >= live) return;
   const int64_t tile = tile_of(p, index), row = tile * kTileRows;
-  prefetch_l2(p.table + tile * p.kvol * kTileRows, (uint32_t)(p.kvol * kTileRows * 4));
-  prefetch_l2(p.row_masks + tile * p.kvol * 4, (uint32_t)(p.kvol * 16));
+  if (kWide || p.table_wide) {
+    prefetch_l2(p.table + tile * p.kvol * kTileRows, (uint32_t)(p.kvol * kTileRows * 4));
+    prefetch_l2(p.row_masks + tile * p.kvol * 4, (uint32_t)(p.kvol * 16));
+  }
   if (p.regrouped) return;
   const int64_t in = p.n_in_rows == p.m_max && row < p.n_in_rows ? p.n_in_rows - row : 0, out = p.m_max - row;
   prefetch_l2(reinterpret_cast<const unsigned char*>(p.in_feats) + row * p.cin * 2,
@@ -612,7 +618,7 @@ __device__ __forceinline__ void prefetch_round(const TcParams& p, int live, cons
 
 // Lists the units of every round and brings in the weights: all of them once when they are resident, else the block of
 // every (window, part) as soon as a slot is free.
-template <int kOffs, int kMma>
+template <int kOffs, bool kWide, int kMma>
 __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b) {
   constexpr uint32_t kWindow = kOffs == 1 ? 1u : kOffs == 2 ? 3u : 15u;
   constexpr int kWindows = 32 / kOffs;
@@ -688,7 +694,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     buf ^= 1;
     if (end) break;
     open_round<kMma>(p, live, after_round(done), r);  // the next round's masks are on their way
-    prefetch_round(p, live, r);
+    prefetch_round<kWide>(p, live, r);
     if (!resident) {
       // two (window, part)s to a slot
       uint32_t rest = windows;
@@ -830,7 +836,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
 // ---- epilogue --------------------------------------------------------------------------------------------------------
 // Epilogue warp `quad` (= warp index mod 4: it may touch TMEM lanes [32*quad, 32*quad + 32)) of set `set`: the sets share
 // the columns of every tile, so that an accumulator is free again soon (of 256 output channels there is only one).
-template <int kOffs, int kMma>
+template <int kOffs, bool kWide, int kMma>
 __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int quad, int set) {
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
@@ -848,7 +854,7 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
   const int live = sh->live;
   Round r;
   open_round<kMma>(p, live, 0, r);
-  if (quad == 0 && set == 0) prefetch_round(p, live, r);  // of the first round; the control warp sees to the others
+  if (quad == 0 && set == 0) prefetch_round<kWide>(p, live, r);  // of the first round; the control warp sees to the others
   for (; r.tiles; open_round<kMma>(p, live, after_round(r), r)) {
     for (int i = 0; i < r.tiles; ++i) {
       const uint32_t mask = __shfl_sync(0xffffffffu, r.mask, i);
@@ -909,11 +915,11 @@ spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p)
   if (warp < 8 * kMma) {
     producer_role<kOffs, kWide, kMma>(p, s, tmem_base, warp, lane);
   } else if (warp < 8 * kMma + kEpilogue) {
-    epilogue_role<kOffs, kMma>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
+    epilogue_role<kOffs, kWide, kMma>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
   } else if (warp < 9 * kMma + kEpilogue) {
     mma_role<kOffs, kMma>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
   } else {
-    control_role<kOffs, kMma>(p, s, &map_b);
+    control_role<kOffs, kWide, kMma>(p, s, &map_b);
   }
   __syncwarp();
   cta_teardown<kMma>(s, tmem_base);
@@ -969,8 +975,8 @@ struct KernelEntry {
 };
 #define D3D_TC_K(O, V, M) {O, V, M, spconv_mm_tc_kernel<O, V, M>}
 const KernelEntry kKernels[] = {
-    D3D_TC_K(4, true, 2), D3D_TC_K(2, true, 2), D3D_TC_K(2, false, 2), D3D_TC_K(1, true, 2), D3D_TC_K(1, false, 2),
-    D3D_TC_K(4, true, 3), D3D_TC_K(2, true, 3), D3D_TC_K(2, false, 3), D3D_TC_K(1, true, 3), D3D_TC_K(1, false, 3),
+    D3D_TC_K(4, true, 2), D3D_TC_K(4, false, 2), D3D_TC_K(2, true, 2), D3D_TC_K(2, false, 2), D3D_TC_K(1, true, 2),
+    D3D_TC_K(1, false, 2), D3D_TC_K(2, true, 3), D3D_TC_K(2, false, 3), D3D_TC_K(1, true, 3), D3D_TC_K(1, false, 3),
 };
 #undef D3D_TC_K
 constexpr int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
@@ -1047,7 +1053,10 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   const uint32_t fmt = a.dtype == D3D_BF16 ? 1u : 0u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(cout >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
   p.regrouped = a.regrouped ? 1 : 0;
-  const int wide = offs == 4 || reinterpret_cast<uintptr_t>(a.in_feats) % 32 == 0;
+  // the other kernels: features that only start on 16 bytes (rows of 32 bytes are loaded 16 at a time anyway), a table that
+  // only starts on four
+  p.table_wide = reinterpret_cast<uintptr_t>(a.table) % 16 == 0;
+  const bool wide = (offs == 4 || reinterpret_cast<uintptr_t>(a.in_feats) % 32 == 0) && p.table_wide;
   p.weights = h->wt_dev;
   p.bias = h->b_dev;
   p.out = a.out_feats;
@@ -1061,7 +1070,7 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   // units take the most instructions.  us with two / three: 27 offsets 32 -> 32 83 / 72, 64 -> 64 77 / 69, 128 -> 64 61 / 58,
   // 64 -> 128 94 / 113, 128 -> 128 50 / 55, 256 -> 256 116 / 120, 16 -> 32 31 / 34; nine offsets 32 -> 32 15.8 / 17.2; three
   // offsets 64 -> 64 15.3 / 18.2.
-  const int mma_warps = g_plan_mma_warps ? g_plan_mma_warps : (cin >= 32 && cout <= 64 && kvol > 9) ? 3 : 2;
+  const int mma_warps = cin < 32 ? 2 : g_plan_mma_warps ? g_plan_mma_warps : (cout <= 64 && kvol > 9) ? 3 : 2;
   const KernelEntry* k = find_kernel(offs, wide, mma_warps);
   D3D_REQUIRE(k, D3D_ERR_INVALID_ARGUMENT);
   // tensor memory: a slot for every producer team, the rest accumulators

@@ -98,6 +98,25 @@ def test_features_and_outputs_on_16_bytes(d3d, cin):
     assert _error() == 0
 
 
+@pytest.mark.parametrize("ks", [(3, 3, 3), (3, 1, 3)])
+@pytest.mark.parametrize("cin,cout", [(16, 32), (32, 48), (32, 96), (64, 64), (64, 80)])
+def test_table_and_features_off_their_boundaries(d3d, ks, cin, cout):
+    """A table that starts on four bytes (a copy inside a larger buffer), features that start on 16, and both."""
+    n = 5000
+    plug, x, num, table = _setup(d3d, n, [1, 24, 30, 20], ks, cin, cout, torch.float16, 17)
+    want = plug.run(x, num, table, relu=True)
+    moved = torch.cat([x.new_zeros(8), x.flatten()])[8:].view(x.shape)
+    assert moved.data_ptr() % 32 == 16
+    for off in (4, 8, 12):
+        buf = torch.empty(table.numel() + 16, dtype=torch.uint8, device=DEV)
+        copy = buf[off:off + table.numel()]
+        copy.copy_(table)
+        assert copy.data_ptr() % 16 == off
+        for feats in (x, moved):
+            assert torch.equal(plug.run(feats, num, copy, relu=True), want)
+    assert torch.equal(plug.run(moved, num, table, relu=True), want) and _error() == 0
+
+
 @pytest.mark.parametrize("said", [0, 1, 700, 100000])
 def test_live_count_only_deals_out_the_tiles(d3d, said):
     """What is computed follows from the table alone."""
