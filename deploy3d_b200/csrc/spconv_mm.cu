@@ -580,7 +580,7 @@ template <class T, class Cvt> static int upload_weights(d3d_spconv_mm_s* h, Cvt 
     w[i] = cvt(h->wb[i]);
     bad |= not_finite(w[i]);
   }
-  h->finite = !bad;  // the tensor-core kernel multiplies rows without an input as zeros, so its weights have to be
+  h->finite = !bad;  // the tensor-core kernel multiplies rows without an input as zeros; where it must not, it masks them
   std::vector<int> order(cin);  // of the input channels in a weight row of the tensor-core kernel
   for (int ci = 0; ci < cin; ++ci) order[ci] = cin == 16 || cin == 32 || cin % 64 == 0 ? spconv_mm_tc_channel(cin, ci) : ci;
   for (int k = 0; k < kvol; ++k)
@@ -786,10 +786,9 @@ static int run(d3d_spconv_mm_t h, int dtype, const void* in_feats, int64_t max_n
   bool tc_ok = spconv_mm_tc_eligible(h, dtype);
   if (h->kernel_choice == 2 || h->kernel_choice == 3) {
     D3D_REQUIRE(tc_ok, D3D_ERR_INVALID_ARGUMENT);
+    return launch_spconv_mm_tc(a);
   }
-  // weights that are not finite in the compute type: a row without an input would be a zero times an infinity on the
-  // tensor-core path, and there only where it has one
-  if (h->kernel_choice != 1 && tc_ok && h->finite) return launch_spconv_mm_tc(a);
+  if (h->kernel_choice == 0 && tc_ok) return launch_spconv_mm_tc(a);
   return launch_spconv_mm_simt(a);
 }
 

@@ -81,6 +81,11 @@ __device__ int g_tc_error;  // 0 ok; otherwise the code of the first wait that g
 // and the loaded registers are stored as they lie.
 __host__ __device__ constexpr int rows_per_lane(int offs) { return offs == 1 ? 4 : 2; }
 
+// The row of a tile's quarter (32 rows) that the producers put into TMEM lane `lane` of it.
+__host__ __device__ constexpr int row_of_lane(int offs, int lane) {
+  return 4 * (lane & 7) + (rows_per_lane(offs) == 4 ? lane >> 3 : 2 * (lane >> 3 & 1) + (lane >> 4));
+}
+
 struct TcParams {
   const int32_t* table;        // [tiles][kvol][128]
   const uint32_t* tile_mask;   // [tiles] bit k set: offset k feeds the tile
@@ -108,6 +113,7 @@ struct TcParams {
   int is_bf16;
   uint32_t wait_limit;  // cycles after which a wait gives up
   int table_wide;       // the table starts on 16 bytes
+  int masked;           // a weight is not finite: products leave the accumulator rows without an input alone
 };
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------
@@ -231,6 +237,23 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, ui
       :
       : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// D += A * B for the rows (lanes of D) whose bit in `rows` is set.
+__device__ __forceinline__ void umma_f16_ta_rows(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                                 const uint32_t (&rows)[4]) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%4, %5, %6, %7}, p;\n\t}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(~rows[0]), "r"(~rows[1]), "r"(~rows[2]), "r"(~rows[3])
+      : "memory");
+}
+// Zeros in 16 columns of the warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+      ::"r"(taddr), "r"(0u) : "memory");
 }
 // Lane t of the warp writes registers 4c, 4c + 1 to columns 8c + 2 (t % 4) and the next of TMEM lane t / 4, registers
 // 4c + 2, 4c + 3 to the same columns of lane t / 4 + 8, for c = 0..3.
@@ -430,7 +453,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[16], const flo
 }
 
 // Barrier initialisation, bias staging and the TMEM allocation (by the MMA warp); returns the TMEM base address.
-template <int kMma>
+template <bool kWide, int kMma>
 __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) {
   Shared* sh = s.sh;
   if (threadIdx.x == 0) {
@@ -448,6 +471,16 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (!kWide && p.masked) {  // accumulators start as zeros, and the epilogue leaves them so
+    const int warp = (int)(threadIdx.x >> 5);
+    if (warp >= 8 * kMma && warp < 8 * kMma + 4) {
+      for (int c = 0; c < p.num_acc * p.cout; c += 16) tmem_zero16(sh->tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c);
+      tmem_st_wait();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  }
   return sh->tmem_base;
 }
 
@@ -728,7 +761,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
 // Every other tile of a round.  The warp walks the round together and by counters: what feeds an MMA has to be the same for
 // the whole warp in a way the compiler can see.  (Four MMAs and a commit issued from a loop run by one lane take 273 cycles, by
 // the elected lane of such a warp 74, at 32 output channels.)
-template <int kOffs, int kMma>
+template <int kOffs, bool kWide, int kMma>
 __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int me) {
   constexpr int kSteps = 4 / kOffs;  // MMAs (K = 16) per offset of a unit
   Shared* sh = s.sh;
@@ -790,6 +823,38 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
       const uint32_t a_addr[2] = {odd ? a_of[1] : a_of[0], odd ? a_of[0] : a_of[1]};
       uint64_t* const full[2] = {odd ? full_of[1] : full_of[0], odd ? full_of[0] : full_of[1]};
       uint64_t* const empty[2] = {odd ? empty_of[1] : empty_of[0], odd ? empty_of[0] : empty_of[1]};
+      if (!kWide && p.masked) {
+        // Under the row masks of every offset, one unit after the other.  Here a lane mask costs what it costs: 46 cycles for an
+        // MMA at least, and the masks come from L2.
+        for (int h = 0; h < (both ? 2 : 1); ++h) {
+          uint32_t rows[kOffs][4];
+          if (mine) {
+            const uint2 e = sh->units[buf][me][seq + h];
+#pragma unroll
+            for (int o = 0; o < kOffs; ++o)
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint32_t word = o < (int)(e.y >> 4) ? __ldg(p.row_masks + ((int64_t)e.x + o) * 4 + q) : 0u;
+                rows[o][q] = __ballot_sync(0xffffffffu, (word >> row_of_lane(kOffs, threadIdx.x & 31)) & 1u);
+              }
+          }
+          if (elect_one() && ok) {
+            if (!resident && h == 0) ok = mbar_wait(&sh->b_full[b_slot], b_phase, abort_flag, 24, p.wait_limit);
+            ok = ok && (!mine || mbar_wait(full[h], ((turn + (uint32_t)h) >> 1) & 1u, abort_flag, 21, p.wait_limit));
+            if (ok && mine) {
+              tc_fence_after();
+#pragma unroll
+              for (int m = 0; m < 4; ++m) {
+                const uint32_t(&r)[4] = rows[m / kSteps];
+                if (r[0] | r[1] | r[2] | r[3]) umma_f16_ta_rows(d_addr, a_addr[h] + 8 * m, desc[h][m], idesc, r);
+              }
+              umma_commit(empty[h]);
+            }
+            if (!resident && ok && h == (both ? 1 : 0)) umma_commit(&sh->b_empty[b_slot]);
+          }
+          __syncwarp();
+        }
+      } else
       // One lane waits and issues, for both windows at once: every instruction of this warp between two products is one too
       // many.  After a wait that gave up it issues nothing.
       if (elect_one() && ok) {
@@ -841,8 +906,7 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
   const int lane = threadIdx.x & 31;
-  // the tile row the producers put into this TMEM lane
-  const int row_in_tile = quad * 32 + 4 * (lane & 7) + (rows_per_lane(kOffs) == 4 ? lane >> 3 : 2 * (lane >> 3 & 1) + (lane >> 4));
+  const int row_in_tile = quad * 32 + row_of_lane(kOffs, lane);
   const bool wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const int half = epilogue_sets(kMma) == 2 ? (p.cout + 31) / 32 * 16 : p.cout;
   const int from = set ? half : 0, to = set ? p.cout : half;
@@ -894,6 +958,10 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
       };
       if (!(p.residual ? columns(std::true_type{}) : columns(std::false_type{}))) return;
       if (!empty_tile) {
+        if (!kWide && p.masked) {
+          for (int c0 = from; c0 < to; c0 += 16) tmem_zero16(taddr + c0);
+          tmem_st_wait();
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
@@ -910,14 +978,14 @@ spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p)
   constexpr int kEpilogue = 4 * epilogue_sets(kMma);
   const Smem s = carve_smem<kOffs>(smem_raw, p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup<kMma>(p, s);
+  const uint32_t tmem_base = cta_setup<kWide, kMma>(p, s);
   pdl_release();
   if (warp < 8 * kMma) {
     producer_role<kOffs, kWide, kMma>(p, s, tmem_base, warp, lane);
   } else if (warp < 8 * kMma + kEpilogue) {
     epilogue_role<kOffs, kWide, kMma>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
   } else if (warp < 9 * kMma + kEpilogue) {
-    mma_role<kOffs, kMma>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
+    mma_role<kOffs, kWide, kMma>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
   } else {
     control_role<kOffs, kWide, kMma>(p, s, &map_b);
   }
@@ -1054,9 +1122,10 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(cout >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
   p.regrouped = a.regrouped ? 1 : 0;
   // the other kernels: features that only start on 16 bytes (rows of 32 bytes are loaded 16 at a time anyway), a table that
-  // only starts on four
+  // only starts on four, weights that are not finite (a row without an input is zeros here, and 0 * W has to be 0)
   p.table_wide = reinterpret_cast<uintptr_t>(a.table) % 16 == 0;
-  const bool wide = (offs == 4 || reinterpret_cast<uintptr_t>(a.in_feats) % 32 == 0) && p.table_wide;
+  p.masked = !h->finite;
+  const bool wide = (offs == 4 || reinterpret_cast<uintptr_t>(a.in_feats) % 32 == 0) && p.table_wide && !p.masked;
   p.weights = h->wt_dev;
   p.bias = h->b_dev;
   p.out = a.out_feats;

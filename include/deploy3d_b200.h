@@ -297,7 +297,7 @@ int d3d_spconv_mm_run(d3d_spconv_mm_t handle, int dtype, const void* in_feats, i
                       const d3d_spconv_mm_epilogue* epilogue, void* stream);
 /* Kernel choice for tests and profiling: 0 = automatic, 1 = SIMT fp32-FMA path, 2 = tcgen05 tensor-core path (what
  * "automatic" picks for eligible shapes), 3 = the same.  2 and 3 fail with D3D_ERR_INVALID_ARGUMENT at run time when
- * the shape is not eligible.  Weights that are not finite in the compute dtype take the SIMT path with every choice. */
+ * the shape is not eligible. */
 int d3d_spconv_mm_set_kernel(d3d_spconv_mm_t handle, int which);
 /* Opt-in for callers that enqueue layers back to back on ONE stream (as TensorRT does): the tensor-core kernel is
  * launched with the programmatic stream-serialisation attribute, so that its prologue overlaps the tail of the
