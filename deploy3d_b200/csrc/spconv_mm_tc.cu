@@ -452,21 +452,24 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[16], const flo
   }
 }
 
-// Barrier initialisation, bias staging and the TMEM allocation (by the MMA warp); returns the TMEM base address.
+// Barrier initialisation and the TMEM allocation (by the first MMA warp); returns the TMEM base address.
 template <bool kWide, int kMma>
 __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) {
   Shared* sh = s.sh;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * kMma; ++i) mbar_init(&sh->full[i], 4), mbar_init(&sh->empty[i], 1);
-    for (int i = 0; i < kMma; ++i) mbar_init(&sh->drained[i], 1);
-    for (int a = 0; a < p.num_acc; ++a) mbar_init(&sh->acc_full[a], 1), mbar_init(&sh->acc_empty[a], 4 * epilogue_sets(kMma));
-    for (int b = 0; b < p.b_slots; ++b) mbar_init(&sh->b_full[b], 1), mbar_init(&sh->b_empty[b], kMma);
-    for (int l = 0; l < 2; ++l) mbar_init(&sh->list_full[l], 1), mbar_init(&sh->list_empty[l], 9 * kMma);
-    mbar_init(&sh->b_ready, 1), mbar_init(&sh->live_ready, 1);
-    sh->abort_flag = 0;
+  // all of this stands in front of a short launch: a barrier of every kind to a lane
+  const int i = threadIdx.x;
+  if (i < 32) {
+    if (i < 2 * kMma) mbar_init(&sh->full[i], 4), mbar_init(&sh->empty[i], 1);
+    if (i < kMma) mbar_init(&sh->drained[i], 1);
+    if (i < p.num_acc) mbar_init(&sh->acc_full[i], 1), mbar_init(&sh->acc_empty[i], 4 * epilogue_sets(kMma));
+    if (i < p.b_slots) mbar_init(&sh->b_full[i], 1), mbar_init(&sh->b_empty[i], kMma);
+    if (i < 2) mbar_init(&sh->list_full[i], 1), mbar_init(&sh->list_empty[i], 9 * kMma);
+    if (i == 0) {
+      mbar_init(&sh->b_ready, 1), mbar_init(&sh->live_ready, 1);
+      sh->abort_flag = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int c = threadIdx.x; c < p.cout; c += blockDim.x) s.bias[c] = p.bias[c];
   if ((int)(threadIdx.x >> 5) == 8 * kMma + 4 * epilogue_sets(kMma)) tmem_alloc(&sh->tmem_base, kTmemCols);
   tc_fence_before();
   __syncthreads();
@@ -913,6 +916,11 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
   int acc = 0;
   uint32_t acc_phase = 0;
   const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+  {
+    constexpr int kThreads = 128 * epilogue_sets(kMma);
+    for (int c = set * 128 + quad * 32 + lane; c < p.cout; c += kThreads) s.bias[c] = __ldg(p.bias + c);
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");  // the epilogue warps
+  }
   pdl_wait();  // residual rows come from an earlier layer; output rows may still be read by the preceding kernel
   if (!__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32, p.wait_limit))) return;
   const int live = sh->live;
