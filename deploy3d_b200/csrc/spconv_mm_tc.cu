@@ -86,6 +86,19 @@ __host__ __device__ constexpr int row_of_lane(int offs, int lane) {
   return 4 * (lane & 7) + (rows_per_lane(offs) == 4 ? lane >> 3 : 2 * (lane >> 3 & 1) + (lane >> 4));
 }
 
+// Short launches: the MMA warps share a tile, every window going to the next one.  Bit k: offset k lies in a window of warp i.
+__host__ __device__ constexpr uint32_t every(int period, int width) {
+  uint32_t bits = 0;
+  for (int k = 0; k < 32; ++k) bits |= (k % period < width ? 1u : 0u) << k;
+  return bits;
+}
+template <int kOffs, int kMma> __device__ __forceinline__ uint32_t offsets_of(int i) {
+  constexpr uint32_t bits = every(kOffs * kMma, kOffs);
+  return bits << (i * kOffs);
+}
+// Bit w: window w is warp i's.
+template <int kMma> __device__ __forceinline__ uint32_t windows_of(int i) { return offsets_of<1, kMma>(i); }
+
 struct TcParams {
   const int32_t* table;        // [tiles][kvol][128]
   const uint32_t* tile_mask;   // [tiles] bit k set: offset k feeds the tile
@@ -342,12 +355,20 @@ template <int kOffs> __device__ __forceinline__ Smem carve_smem(unsigned char* r
 // per (window, part, tile).  A weight block is thus used by all tiles of the round while it is in shared memory.  The control
 // warp lists the units of a round for the producers; the MMA warps and the epilogue count along.
 //
-// Rounds cover the live tiles first, in whole rounds and one of the remaining tiles shared out evenly, then whatever lies
-// behind them (tiles no offset feeds).
+// Rounds cover the live tiles first, in whole rounds and one of the remaining tiles shared out evenly (157 tiles of 64 -> 64: one
+// each and nine CTAs with two 14.7 us, 78 CTAs with two 16.0), then whatever lies behind them (tiles no offset feeds).
+//
+// Launches of at most one tile to a CTA (kSplit): both MMA warps work on it, each window going to the next warp -- by its number,
+// not by its place among those the tile has, so that a regrouped table gives the same sums --, with an accumulator, a list and
+// weight slots each; the epilogue adds the two sums.  27 offsets and 6 k voxels, us with one warp / both: 16 -> 16 7.3 / 6.5,
+// 32 -> 64 9.3 / 7.9, 64 -> 64 12.3 / 10.1, 128 -> 128 19.3 / 15.8.  A kernel of its own: the same by a flag costs 0.3 to 0.9 us,
+// since a short launch fetches most of its code for the first time.
 struct Round {
   int start;      // index of the round's first tile over all CTAs
-  int limit;      // tiles below this index belong to it
-  int tiles;      // tiles per CTA
+  int next;       // of the next round's
+  int first;      // of this CTA's (tiles in the order of the table)
+  int limit;      // this CTA's tiles lie below this index
+  int tiles;      // tiles of a CTA, at most
   uint32_t mask;  // lane i (mod 4): offset mask of the CTA's tile i, 0 = no such tile
 };
 // Where the tiles behind which no tile has an offset begin, found by the whole warp from the offset masks alone: up to a
@@ -377,28 +398,28 @@ __device__ __forceinline__ int live_tiles(const TcParams& p) {
 // Index of the CTA's tile i in a round, and the tile it stands for.
 __device__ __forceinline__ int tile_index(const TcParams& p, const Round& r, int i) {
   const int g = (int)gridDim.x, c = (int)blockIdx.x;
-  if (!p.regrouped) return r.start + c * r.tiles + i;
+  if (!p.regrouped) return r.first + i;
   return r.start + i * g + ((i & 1) ? g - 1 - c : c);
 }
 __device__ __forceinline__ int tile_of(const TcParams& p, int index) {
   return p.regrouped ? p.num_tiles - 1 - index : index;
 }
-template <int kMma> __device__ __forceinline__ void open_round(const TcParams& p, int live, int start, Round& r) {
+template <int kMma, bool kSplit> __device__ __forceinline__ void open_round(const TcParams& p, int live, int start, Round& r) {
   const int g = (int)gridDim.x;
-  r.start = start;
-  r.limit = start < live ? live : p.num_tiles;
+  const int end = start < live ? live : p.num_tiles;
   // With few accumulators one tile at a time: an MMA warp that had no tile in the round before must not be able to wait for
   // an accumulator whose use before last has not been read yet -- the phase would be taken for the one it waits for.  It is
   // at most 2 kMma - 2 tiles ahead of the first tile that another warp may still be at.
-  const int rest = r.limit - start, most = p.num_acc >= 2 * kMma - 1 ? kMma : 1;
+  const int rest = end - start, most = !kSplit && p.num_acc >= 2 * kMma - 1 ? kMma : 1;
   r.tiles = rest >= most * g ? most : rest <= 0 ? 0 : (rest + g - 1) / g;
+  // the first `more` CTAs take all of them, the others one less
+  const int c = (int)blockIdx.x, less = r.tiles - 1, more = rest - less * g < g ? rest - less * g : g;
+  r.start = start, r.next = start + less * g + more;
+  r.first = start + c * less + (c < more ? c : more);
+  r.limit = p.regrouped ? r.next : r.first + less + (c < more ? 1 : 0);
   const int i = threadIdx.x & 3;
   const int index = tile_index(p, r, i);
   r.mask = (i < r.tiles && index < r.limit) ? __ldg(p.tile_mask + tile_of(p, index)) : 0u;
-}
-__device__ __forceinline__ int after_round(const Round& r) {
-  const int next = r.start + r.tiles * (int)gridDim.x;
-  return next < r.limit ? next : r.limit;
 }
 // 16 accumulator columns of this thread's row: bias (+ residual), ReLU, convert, 32 bytes stored.  Two columns to an
 // instruction where there is one for it: this runs on four warps that share the SM's issue slots with all producers.
@@ -453,7 +474,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&acc)[16], const flo
 }
 
 // Barrier initialisation and the TMEM allocation (by the first MMA warp); returns the TMEM base address.
-template <bool kWide, int kMma>
+template <bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) {
   Shared* sh = s.sh;
   // all of this stands in front of a short launch: a barrier of every kind to a lane
@@ -462,7 +483,7 @@ __device__ __forceinline__ uint32_t cta_setup(const TcParams& p, const Smem& s) 
     if (i < 2 * kMma) mbar_init(&sh->full[i], 4), mbar_init(&sh->empty[i], 1);
     if (i < kMma) mbar_init(&sh->drained[i], 1);
     if (i < p.num_acc) mbar_init(&sh->acc_full[i], 1), mbar_init(&sh->acc_empty[i], 4 * epilogue_sets(kMma));
-    if (i < p.b_slots) mbar_init(&sh->b_full[i], 1), mbar_init(&sh->b_empty[i], kMma);
+    if (i < p.b_slots) mbar_init(&sh->b_full[i], 1), mbar_init(&sh->b_empty[i], kSplit ? 1 : kMma);
     if (i < 2) mbar_init(&sh->list_full[i], 1), mbar_init(&sh->list_empty[i], 9 * kMma);
     if (i == 0) {
       mbar_init(&sh->b_ready, 1), mbar_init(&sh->live_ready, 1);
@@ -500,7 +521,7 @@ __device__ __forceinline__ void cta_teardown(const Smem& s, uint32_t tmem_base) 
 }
 
 // ---- producers -------------------------------------------------------------------------------------------------------
-template <int kOffs, bool kWide, int kMma>
+template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int warp, int lane) {
   constexpr int kRows = rows_per_lane(kOffs);
   constexpr int kWords = kOffs == 4 ? 4 : 8;               // 32-bit words a lane loads at a time
@@ -539,7 +560,7 @@ __device__ __forceinline__ void producer_role(const TcParams& p, const Smem& s, 
       if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_full[buf], list_phase, abort_flag, 13, p.wait_limit))) return kEnd;
       const int4 round = sh->round[buf];
       if (round.x == 0) return kEnd;
-      len = owner < round.x ? round.z : 0;
+      len = kSplit ? __popc((uint32_t)round.y & windows_of<kMma>(owner)) * p.parts : owner < round.x ? round.z : 0;
       open = true;
     }
     return kUnit;
@@ -654,7 +675,7 @@ template <bool kWide> __device__ __forceinline__ void prefetch_round(const TcPar
 
 // Lists the units of every round and brings in the weights: all of them once when they are resident, else the block of
 // every (window, part) as soon as a slot is free.
-template <int kOffs, bool kWide, int kMma>
+template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b) {
   constexpr uint32_t kWindow = kOffs == 1 ? 1u : kOffs == 2 ? 3u : 15u;
   constexpr int kWindows = 32 / kOffs;
@@ -663,7 +684,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   const int lane = threadIdx.x & 31;
   const uint32_t b_tx = (uint32_t)p.cout * p.row_bytes;
   const bool resident = p.b_slots == 0;
-  const int parts = p.parts;
+  const int parts = p.parts, ring_slots = kSplit ? p.b_slots / kMma : p.b_slots;
   // the weights are constants of the layer: their load does not wait for the preceding kernel
   if (resident && lane == 0) {
     // blocks behind the last offset, up to a whole window: rows beyond the tensor, which TMA fills with zeros
@@ -680,13 +701,13 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   __syncwarp();
   pdl_wait();  // the offset masks come from the preceding kernels
   Round r;
-  open_round<kMma>(p, p.num_tiles, 0, r);  // as if all were live, so that the masks are on their way
-  const int live = live_tiles(p);
-  if (lane == 0) {
+  open_round<kMma, kSplit>(p, p.num_tiles, 0, r);  // as if all were live, so that the masks are on their way
+  const int live = kSplit ? p.num_tiles : live_tiles(p);
+  if (!kSplit && lane == 0) {
     sh->live = live;
     mbar_arrive(&sh->live_ready);
   }
-  if (live < r.tiles * (int)gridDim.x && live < p.num_tiles) open_round<kMma>(p, live, 0, r);  // not a whole round
+  if (!kSplit && live < r.tiles * (int)gridDim.x && live < p.num_tiles) open_round<kMma, kSplit>(p, live, 0, r);  // not a whole round
   int buf = 0, b_slot = 0;
   uint32_t list_phase = 0, b_phase = 0;
   bool ok = true;  // no wait for a weight slot has given up
@@ -701,7 +722,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     }
     const Round done = r;
     if (all == 0u && !end) {
-      open_round<kMma>(p, live, after_round(done), r);
+      open_round<kMma, kSplit>(p, live, done.next, r);
       continue;
     }
     if (!__all_sync(0xffffffffu, mbar_wait(&sh->list_empty[buf], list_phase ^ 1, abort_flag, 14, p.wait_limit))) break;
@@ -712,7 +733,12 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     const int rank = __popc(windows & lanemask_lt());  // of the window in the round
     const int steps = __popc(windows) * parts;
     const int offs = p.kvol - lane * kOffs < kOffs ? p.kvol - lane * kOffs : kOffs;
-    if (present) {
+    if (kSplit && present) {
+      const uint32_t blk = (uint32_t)tile_of(p, tile_index(p, done, 0)) * (uint32_t)p.kvol + (uint32_t)(lane * kOffs);
+      const int own = __popc(windows & windows_of<kMma>(lane % kMma) & lanemask_lt());
+      for (int part = 0; part < parts; ++part)
+        sh->units[buf][lane % kMma][own * parts + part] = make_uint2(blk, (uint32_t)part | (uint32_t)offs << 4);
+    } else if (present) {
       int place = 0;  // of the tile among the round's tiles that have an offset
 #pragma unroll
       for (int i = 0; i < kMma; ++i) {
@@ -729,42 +755,56 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
     if (buf) list_phase ^= 1;
     buf ^= 1;
     if (end) break;
-    open_round<kMma>(p, live, after_round(done), r);  // the next round's masks are on their way
+    open_round<kMma, kSplit>(p, live, done.next, r);  // the next round's masks are on their way
     prefetch_round<kWide>(p, live, r);
     if (!resident) {
-      // two (window, part)s to a slot
-      uint32_t rest = windows;
-      for (int seq = 0, part = 0; seq < steps; seq += 2) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&sh->b_empty[b_slot], b_phase ^ 1, abort_flag, 11, p.wait_limit));
-        if (!ok) break;
-        const int both = seq + 1 < steps ? 2 : 1;
-        if (lane == 0) mbar_arrive_expect_tx(&sh->b_full[b_slot], (uint32_t)(both * kOffs) * b_tx);
-        for (int h = 0; h < both; ++h) {
-          const int k = (__ffs(rest) - 1) * kOffs;
-          if (lane == 0) {
+      // two (window, part)s to a slot; the MMA warps that share a tile have slots of their own, lane i counts those of warp i
+      constexpr int kRings = kSplit ? kMma : 1;
+      uint32_t rest = kSplit ? windows & windows_of<kMma>(lane % kMma) : windows;
+      int part = 0, todo = __popc(rest) * parts;
+      while (ok && __any_sync(0xffffffffu, lane < kRings && todo > 0)) {
+#pragma unroll 1
+        for (int ring = 0; ring < kRings; ++ring) {
+          const int left = kSplit ? __shfl_sync(0xffffffffu, todo, ring) : todo;
+          if (left <= 0) continue;
+          const int slot = kSplit ? __shfl_sync(0xffffffffu, b_slot, ring) + ring * ring_slots : b_slot;
+          const uint32_t phase = kSplit ? __shfl_sync(0xffffffffu, b_phase, ring) : b_phase;
+          ok = __all_sync(0xffffffffu, mbar_wait(&sh->b_empty[slot], phase ^ 1, abort_flag, 11, p.wait_limit));
+          if (!ok) break;
+          if (lane == (kSplit ? ring : 0)) {
+            const int both = left > 1 ? 2 : 1;
+            mbar_arrive_expect_tx(&sh->b_full[slot], (uint32_t)(both * kOffs) * b_tx);
+            for (int h = 0; h < both; ++h) {
+              const int k = (__ffs(rest) - 1) * kOffs;
 #pragma unroll
-            for (int o = 0; o < kOffs; ++o)  // behind the last offset: zeros, as above
-              tma_load_2d(map_b, &sh->b_full[b_slot], s.weights + (size_t)((b_slot * 2 + h) * kOffs + o) * p.b_bytes, part * 64,
-                          (k + o) * p.cout);
+              for (int o = 0; o < kOffs; ++o)  // behind the last offset: zeros, as above
+                tma_load_2d(map_b, &sh->b_full[slot], s.weights + (size_t)((slot * 2 + h) * kOffs + o) * p.b_bytes, part * 64,
+                            (k + o) * p.cout);
+              if (++part == parts) part = 0, rest &= rest - 1u;
+            }
           }
-          if (++part == parts) part = 0, rest &= rest - 1u;
+          if (!kSplit || lane == ring) {
+            todo -= 2;
+            if (++b_slot == ring_slots) b_slot = 0, b_phase ^= 1;
+          }
+          __syncwarp();
         }
-        __syncwarp();
-        if (++b_slot == p.b_slots) b_slot = 0, b_phase ^= 1;
       }
       if (!ok) break;
     }
   }
   // the last weights of every slot have landed
   if (resident) mbar_drain(&sh->b_ready, 0);
-  for (int b = 0; b < p.b_slots; ++b) mbar_drain(&sh->b_full[b], b < b_slot ? b_phase : b_phase ^ 1);
+  for (int b = 0; b < ring_slots; ++b)
+    if (lane < (kSplit ? kMma : 1)) mbar_drain(&sh->b_full[lane * ring_slots + b], b < b_slot ? b_phase : b_phase ^ 1);
+  __syncwarp();
 }
 
 // ---- MMA warps -------------------------------------------------------------------------------------------------------
 // Every other tile of a round.  The warp walks the round together and by counters: what feeds an MMA has to be the same for
 // the whole warp in a way the compiler can see.  (Four MMAs and a commit issued from a loop run by one lane take 273 cycles, by
 // the elected lane of such a warp 74, at 32 output channels.)
-template <int kOffs, bool kWide, int kMma>
+template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int me) {
   constexpr int kSteps = 4 / kOffs;  // MMAs (K = 16) per offset of a unit
   Shared* sh = s.sh;
@@ -775,7 +815,8 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   const uint32_t idesc = p.idesc;
   const uint32_t ring = tmem_base + (uint32_t)p.ring_col;
   const bool resident = p.b_slots == 0;
-  const int parts = p.parts, num_acc = p.num_acc, b_slots = p.b_slots;
+  const int parts = p.parts, num_acc = p.num_acc;
+  const int b_first = kSplit ? me * (p.b_slots / kMma) : 0, b_end = kSplit ? b_first + p.b_slots / kMma : p.b_slots;
   const uint32_t cout = (uint32_t)p.cout;
   if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23, p.wait_limit))) return;
   pdl_wait();  // the first list comes after the preceding kernels, which may take longer than a wait is allowed to
@@ -783,7 +824,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   const uint32_t a_of[2] = {ring + (uint32_t)(me * kUnitCols), ring + (uint32_t)((me + kMma) * kUnitCols)};
   uint64_t* const full_of[2] = {&sh->full[me], &sh->full[me + kMma]};
   uint64_t* const empty_of[2] = {&sh->empty[me], &sh->empty[me + kMma]};
-  int buf = 0, b_slot = 0, acc0 = 0;
+  int buf = 0, b_slot = b_first, acc0 = 0;
   uint32_t list_phase = 0, b_phase = 0, turn = 0, acc_phase = 0;  // turn: bit 0 the slot, bit 1 its phase
   bool ok = true;  // no wait has given up
   for (;;) {
@@ -791,11 +832,11 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
     if (!ok) break;
     const int4 round = sh->round[buf];
     const int count = (int)__reduce_or_sync(0xffffffffu, (unsigned)round.x);
-    const uint32_t windows = __reduce_or_sync(0xffffffffu, (unsigned)round.y);
+    const uint32_t windows = __reduce_or_sync(0xffffffffu, kSplit ? (unsigned)round.y & windows_of<kMma>(me) : (unsigned)round.y);
     if (count == 0) break;
-    // this warp's tile of the round, if there is one, and its accumulator
-    const bool mine = me < count;
-    const bool wrap = acc0 + me >= num_acc;
+    // this warp's tile of the round, if there is one, and its accumulator (of a shared tile even where it has no window)
+    const bool mine = kSplit || me < count;
+    const bool wrap = !kSplit && acc0 + me >= num_acc;
     const int acc = wrap ? acc0 + me - num_acc : acc0 + me;
     const uint32_t d_addr = tmem_base + (uint32_t)acc * cout;
     ok = !mine || __all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[acc], acc_phase ^ (wrap ? 0u : 1u), abort_flag, 22, p.wait_limit));
@@ -880,7 +921,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
       __syncwarp();
       add = 1u;
       if (mine) turn = (turn + (both ? 2u : 1u)) & 3u;
-      if (!resident && ++b_slot == b_slots) b_slot = 0, b_phase ^= 1;
+      if (!resident && ++b_slot == b_end) b_slot = b_first, b_phase ^= 1;
     }
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) break;
@@ -891,7 +932,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
     __syncwarp();
     if (buf) list_phase ^= 1;
     buf ^= 1;
-    acc0 += count;
+    acc0 += kSplit ? kMma : count;
     if (acc0 >= num_acc) acc0 -= num_acc, acc_phase ^= 1;
   }
   if (!ok) {  // nobody reads these accumulators: see the MMAs out here
@@ -904,7 +945,7 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
 // ---- epilogue --------------------------------------------------------------------------------------------------------
 // Epilogue warp `quad` (= warp index mod 4: it may touch TMEM lanes [32*quad, 32*quad + 32)) of set `set`: the sets share
 // the columns of every tile, so that an accumulator is free again soon (of 256 output channels there is only one).
-template <int kOffs, bool kWide, int kMma>
+template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int quad, int set) {
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
@@ -922,12 +963,12 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
     asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");  // the epilogue warps
   }
   pdl_wait();  // residual rows come from an earlier layer; output rows may still be read by the preceding kernel
-  if (!__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32, p.wait_limit))) return;
-  const int live = sh->live;
+  if (!kSplit && !__all_sync(0xffffffffu, mbar_wait(&sh->live_ready, 0, abort_flag, 32, p.wait_limit))) return;
+  const int live = kSplit ? p.num_tiles : sh->live;
   Round r;
-  open_round<kMma>(p, live, 0, r);
+  open_round<kMma, kSplit>(p, live, 0, r);
   if (quad == 0 && set == 0) prefetch_round<kWide>(p, live, r);  // of the first round; the control warp sees to the others
-  for (; r.tiles; open_round<kMma>(p, live, after_round(r), r)) {
+  for (; r.tiles; open_round<kMma, kSplit>(p, live, r.next, r)) {
     for (int i = 0; i < r.tiles; ++i) {
       const uint32_t mask = __shfl_sync(0xffffffffu, r.mask, i);
       const int index = tile_index(p, r, i);
@@ -938,12 +979,17 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
       unsigned short* out_row = reinterpret_cast<unsigned short*>(p.out) + row * p.cout;
       const uint4* res_row = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.residual) + row * p.cout);
       const uint32_t taddr = lane_base + (uint32_t)(acc * p.cout);
+      constexpr int kAccs = kSplit ? kMma : 1;  // accumulators of a tile
+      int first = 0;                            // the first of them that has a product
+      while (kSplit && first + 1 < kAccs && (mask & offsets_of<kOffs, kMma>(first)) == 0u) ++first;
       auto columns = [&](auto with_residual) {
         constexpr bool kAdd = decltype(with_residual)::value;
         uint4 res[2];  // of the next 16 columns, on their way
         if (kAdd && row_ok && from < to) res[0] = __ldg(res_row + from / 8), res[1] = __ldg(res_row + from / 8 + 1);
         if (!empty_tile) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc], acc_phase, abort_flag, 31, p.wait_limit))) return false;
+#pragma unroll
+          for (int m = 0; m < kAccs; ++m)
+            if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc + m], acc_phase, abort_flag, 31, p.wait_limit))) return false;
           tc_fence_after();
         }
         for (int c0 = from; c0 < to; c0 += 16) {
@@ -952,11 +998,22 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
 #pragma unroll
             for (int q = 0; q < 16; ++q) v[q] = 0u;
           } else {
-            tmem_ld16(taddr + c0, v);
+            tmem_ld16(taddr + first * p.cout + c0, v);
           }
           const uint4 now[2] = {res[0], res[1]};
           if (kAdd && row_ok && c0 + 16 < to) res[0] = __ldg(res_row + c0 / 8 + 2), res[1] = __ldg(res_row + c0 / 8 + 3);
           if (!empty_tile) tmem_ld_wait(v);
+          if (kSplit) {  // the other warps' sums, in the order of the warps
+#pragma unroll
+            for (int m = 1; m < kAccs; ++m) {
+              if (m <= first || (mask & offsets_of<kOffs, kMma>(m)) == 0u) continue;
+              uint32_t w[16];
+              tmem_ld16(taddr + m * p.cout + c0, w);
+              tmem_ld_wait(w);
+#pragma unroll
+              for (int q = 0; q < 16; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(w[q]));
+            }
+          }
           if (row_ok) {
             if (p.is_bf16) store_chunk<true, kAdd>(v, s.bias + c0, out_row + c0, now, p.relu, wide);
             else store_chunk<false, kAdd>(v, s.bias + c0, out_row + c0, now, p.relu, wide);
@@ -967,35 +1024,36 @@ __device__ __forceinline__ void epilogue_role(const TcParams& p, const Smem& s, 
       if (!(p.residual ? columns(std::true_type{}) : columns(std::false_type{}))) return;
       if (!empty_tile) {
         if (!kWide && p.masked) {
-          for (int c0 = from; c0 < to; c0 += 16) tmem_zero16(taddr + c0);
+          for (int m = 0; m < kAccs; ++m)
+            for (int c0 = from; c0 < to; c0 += 16) tmem_zero16(taddr + m * p.cout + c0);
           tmem_st_wait();
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
-        if (++acc == p.num_acc) acc = 0, acc_phase ^= 1;
+        if (lane < kAccs) mbar_arrive(&sh->acc_empty[acc + lane]);
+        if ((acc += kAccs) == p.num_acc) acc = 0, acc_phase ^= 1;
       }
     }
   }
 }
 
-template <int kOffs, bool kWide, int kMma>
+template <int kOffs, bool kWide, int kMma, bool kSplit>
 __global__ void __launch_bounds__(threads_of(kMma), 1)
 spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   constexpr int kEpilogue = 4 * epilogue_sets(kMma);
   const Smem s = carve_smem<kOffs>(smem_raw, p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tmem_base = cta_setup<kWide, kMma>(p, s);
+  const uint32_t tmem_base = cta_setup<kWide, kMma, kSplit>(p, s);
   pdl_release();
   if (warp < 8 * kMma) {
-    producer_role<kOffs, kWide, kMma>(p, s, tmem_base, warp, lane);
+    producer_role<kOffs, kWide, kMma, kSplit>(p, s, tmem_base, warp, lane);
   } else if (warp < 8 * kMma + kEpilogue) {
-    epilogue_role<kOffs, kWide, kMma>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
+    epilogue_role<kOffs, kWide, kMma, kSplit>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
   } else if (warp < 9 * kMma + kEpilogue) {
-    mma_role<kOffs, kWide, kMma>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
+    mma_role<kOffs, kWide, kMma, kSplit>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
   } else {
-    control_role<kOffs, kWide, kMma>(p, s, &map_b);
+    control_role<kOffs, kWide, kMma, kSplit>(p, s, &map_b);
   }
   __syncwarp();
   cta_teardown<kMma>(s, tmem_base);
@@ -1046,20 +1104,23 @@ uint32_t g_wait_limit = kWaitLimitCycles;  // d3d_debug_set_wait_limit
 
 typedef void (*KernelFn)(const CUtensorMap, const TcParams);
 struct KernelEntry {
-  int offs, wide, mma_warps;
+  int offs, wide, mma_warps, split;
   KernelFn fn;
 };
-#define D3D_TC_K(O, V, M) {O, V, M, spconv_mm_tc_kernel<O, V, M>}
+#define D3D_TC_K(O, V, M, S) {O, V, M, S, spconv_mm_tc_kernel<O, V, M, S>}
 const KernelEntry kKernels[] = {
-    D3D_TC_K(4, true, 2), D3D_TC_K(4, false, 2), D3D_TC_K(2, true, 2), D3D_TC_K(2, false, 2), D3D_TC_K(1, true, 2),
-    D3D_TC_K(1, false, 2), D3D_TC_K(2, true, 3), D3D_TC_K(2, false, 3), D3D_TC_K(1, true, 3), D3D_TC_K(1, false, 3),
+    D3D_TC_K(4, true, 2, false), D3D_TC_K(4, false, 2, false), D3D_TC_K(2, true, 2, false), D3D_TC_K(2, false, 2, false),
+    D3D_TC_K(1, true, 2, false), D3D_TC_K(1, false, 2, false), D3D_TC_K(2, true, 3, false), D3D_TC_K(2, false, 3, false),
+    D3D_TC_K(1, true, 3, false), D3D_TC_K(1, false, 3, false), D3D_TC_K(4, true, 2, true), D3D_TC_K(4, false, 2, true),
+    D3D_TC_K(2, true, 2, true), D3D_TC_K(2, false, 2, true), D3D_TC_K(1, true, 2, true), D3D_TC_K(1, false, 2, true),
 };
 #undef D3D_TC_K
 constexpr int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
 
-const KernelEntry* find_kernel(int offs, int wide, int mma_warps) {
+const KernelEntry* find_kernel(int offs, int wide, int mma_warps, int split) {
   for (int i = 0; i < kNumKernels; ++i)
-    if (kKernels[i].offs == offs && kKernels[i].wide == wide && kKernels[i].mma_warps == mma_warps) return &kKernels[i];
+    if (kKernels[i].offs == offs && kKernels[i].wide == wide && kKernels[i].mma_warps == mma_warps && kKernels[i].split == split)
+      return &kKernels[i];
   return nullptr;
 }
 
@@ -1142,29 +1203,40 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   p.is_bf16 = a.dtype == D3D_BF16;
   p.wait_limit = g_wait_limit;
 
-  // Three MMA warps where a unit's products are short (up to 64 columns: 24 producer warps then feed them), two where the tensor
-  // pipe is the longer part, where few offsets make the epilogue it (it has eight warps then) and for 16 input channels, whose
+  // Three MMA warps where a unit's products are short (up to 64 columns: 24 producer warps then feed them) and a CTA has more than
+  // two tiles, two where the tensor pipe is the longer part, where few offsets make the epilogue it (it has eight warps then) and for 16 input channels, whose
   // units take the most instructions.  us with two / three: 27 offsets 32 -> 32 83 / 72, 64 -> 64 77 / 69, 128 -> 64 61 / 58,
   // 64 -> 128 94 / 113, 128 -> 128 50 / 55, 256 -> 256 116 / 120, 16 -> 32 31 / 34; nine offsets 32 -> 32 15.8 / 17.2; three
   // offsets 64 -> 64 15.3 / 18.2.
-  const int mma_warps = cin < 32 ? 2 : g_plan_mma_warps ? g_plan_mma_warps : (cout <= 64 && kvol > 9) ? 3 : 2;
-  const KernelEntry* k = find_kernel(offs, wide, mma_warps);
+  // One tile to a CTA: two MMA warps share it, since a chain of products is what such a launch lasts (an MMA warp takes 470 cycles
+  // from one unit to the next, whatever feeds it).  From the second tile on a tile each is faster: they share their weights (157
+  // tiles of 64 -> 64: 14.7 us, shared one after the other 17.8).
+  const bool is_short = p.num_tiles <= 2 * kNumSMs, split = p.num_tiles <= kNumSMs && cout <= 192 && kvol > offs;
+  const int mma_warps = cin < 32 || split        ? 2
+                        : g_plan_mma_warps       ? g_plan_mma_warps
+                        : cout <= 64 && kvol > 9 ? (is_short ? 2 : 3)
+                                                 : 2;
+  const KernelEntry* k = find_kernel(offs, wide, mma_warps, split);
   D3D_REQUIRE(k, D3D_ERR_INVALID_ARGUMENT);
   // tensor memory: a slot for every producer team, the rest accumulators
   p.ring_col = kTmemCols - 2 * mma_warps * kUnitCols;
   p.num_acc = p.ring_col / cout;
   if (p.num_acc > kMaxAcc) p.num_acc = kMaxAcc;
+  if (split) p.num_acc -= p.num_acc % mma_warps;
   // shared memory: weights
   p.b_bytes = (uint32_t)align_up((size_t)cout * p.row_bytes, (size_t)8 * p.row_bytes);
   const size_t ctrl = 1024 + align_up((size_t)cout * 4 + 16, 16) + sizeof(Shared);
   size_t weights = align_up(kvol, offs) * p.b_bytes;
   p.b_slots = 0;
   // in shared memory for good up to 112 KB, which leaves L1 as much (16 -> 16 to 32 -> 64, held or streamed: the same to 1 %)
-  if (p.parts > 1 || weights > 112 * 1024) {
+  // but not where a CTA has two tiles: the first products need not wait for all (219 tiles of 32 -> 64: 13.1 us held, 12.7 streamed;
+  // with one tile the load in front of a chained launch is worth more: 6.0 held, 6.9 streamed)
+  if (p.parts > 1 || weights > (is_short && !split ? 56 : 112) * 1024) {
     const size_t window = (size_t)2 * offs * p.b_bytes;  // two of them to a slot
     p.b_slots = (int)(128 * 1024 / window);
     if (p.b_slots < 3) p.b_slots = 3;
     if (p.b_slots > kMaxBSlots) p.b_slots = kMaxBSlots;
+    if (split) p.b_slots = p.b_slots < 2 * mma_warps ? 2 * mma_warps : p.b_slots - p.b_slots % mma_warps;
     weights = p.b_slots * window;
   }
   const size_t smem = ctrl + weights;

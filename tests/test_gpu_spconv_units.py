@@ -78,11 +78,57 @@ def test_rounds_and_their_remainder(d3d, tiles, cin, cout):
     assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d tiles" % tiles)
 
 
+@pytest.mark.parametrize("tiles", [148, 296, 297, 443, 444, 445, 593, 900])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 64), (128, 64)])
+def test_rounds_of_three_tiles(d3d, tiles, cin, cout):
+    """Three MMA warps (27 offsets, up to 64 output channels; 64 is the fewest accumulators they run with) over whole rounds and
+    remainders, with weights that are held (32 -> 32), streamed and in two parts; a stretch of tiles without an offset, so
+    that rounds of one, two and three live tiles follow each other; plain and regrouped."""
+    from deploy3d_b200.plugins import SPConvMMPlugin
+    n = tiles * 128 - 37
+    plug, x, num, table = _setup(d3d, n, [1, 60, 60, 60], (3, 3, 3), cin, cout, torch.bfloat16, tiles)
+    _, tile_mask, row_masks, _ = table_parts(table, 27, n)
+    gone = torch.zeros(tiles, dtype=torch.bool, device=DEV)
+    gone[tiles // 3:tiles // 2] = True
+    gone[::7] = True
+    gone[1::14] = True
+    tile_mask[gone] = 0
+    row_masks[gone] = 0
+    res = torch.randn((n, cout), device=DEV).bfloat16()
+    got, want = _both(plug, x, num, table, residual=res)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d tiles" % tiles)
+    grouped = SPConvMMPlugin.regroup(27, n, table)
+    assert torch.equal(plug.run(x, num, grouped, residual=res), got) and _error() == 0
+
+
 @pytest.mark.parametrize("cout", [16, 32, 48, 64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 240, 256])
 def test_numbers_of_accumulators(d3d, cout):
     plug, x, num, table = _setup(d3d, 57000, [2, 40, 48, 44], (3, 1, 1), 32, cout, torch.float16, cout)
     got, want = _both(plug, x, num, table)
     assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d output channels" % cout)
+
+
+@pytest.mark.parametrize("ks", [(3, 3, 3), (3, 1, 1), (5, 1, 3)])
+@pytest.mark.parametrize("cin", [16, 32, 64, 128])
+@pytest.mark.parametrize("cout", [16, 48, 128, 144, 192, 208])
+def test_tile_shared_by_the_mma_warps(d3d, ks, cin, cout):
+    """At most one tile to a CTA: the windows of a tile go to the MMA warps in turn.  Tiles that have only even windows, only odd
+    ones, a single one, or none; plain and regrouped, whose bytes have to be the same."""
+    from deploy3d_b200.plugins import SPConvMMPlugin
+    n, kvol = 6 * 128 - 11, int(np.prod(ks))
+    plug, x, num, table = _setup(d3d, n, [1, 8, 10, 12], ks, cin, cout, torch.float16, cout + cin)
+    _, tile_mask, row_masks, _ = table_parts(table, kvol, n)
+    offs = 64 // min(cin, 64)
+    window = torch.arange(kvol, device=DEV) // offs
+    keep = [window >= 0, window % 2 == 0, window % 2 == 1, window == 1, window < 0, window == 2]
+    for t, k in enumerate(keep):
+        row_masks[t][~k] = 0
+        tile_mask[t] = tile_mask[t] & sum(1 << i for i in range(kvol) if k[i])
+    res = torch.randn((n, cout), device=DEV).half()
+    got, want = _both(plug, x, num, table, relu=True, residual=res)
+    assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "shared tiles")
+    grouped = SPConvMMPlugin.regroup(kvol, n, table)
+    assert torch.equal(plug.run(x, num, grouped, relu=True, residual=res), got) and _error() == 0
 
 
 @pytest.mark.parametrize("cin", [16, 32, 64, 128])
