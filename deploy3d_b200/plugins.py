@@ -353,7 +353,7 @@ class SPConvMMPlugin(_Plugin):
         self._configured = (torch_dtype, torch.device("cuda", torch.cuda.current_device()))
 
     def set_kernel(self, which):
-        """0 automatic, 1 SIMT, 2 tcgen05, 3 tcgen05 with one CTA per SM."""
+        """0 automatic, 1 SIMT, 2 tcgen05 (3 is the same)."""
         check("d3d_spconv_mm_set_kernel", lib().d3d_spconv_mm_set_kernel(self.handle, int(which)))
 
     def set_dependent_launch(self, enable):

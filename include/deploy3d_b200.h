@@ -85,9 +85,10 @@ int d3d_debug_set_wait_limit(int cycles);
  * index, limit = scatter index + 1).  The regular build checks nothing of the kind and returns
  * D3D_ERR_INVALID_ARGUMENT. */
 int d3d_debug_take_bounds_violation(int32_t* record);
-/* Tuning aid (no reference counterpart): overrides the pipeline plan of the tensor-core SPConvMM kernel for every
- * later launch of the process: producer warps (16 or 24), 0 = automatic.  The other arguments (0 to 8), and 4 or 8 producer
- * warps, are accepted and have no effect.  Not thread-safe; results do not depend on the plan. */
+/* Tuning aid (no reference counterpart): 16 or 24 producer warps (two or three MMA warps) in every later launch of the
+ * tensor-core SPConvMM kernel of the process that has the choice (more than 148 tiles of 128 outputs, at least 32 input
+ * channels), 0 = automatic.  `group` and `max_stages` (0 to 8), and 4 or 8 producer warps, belong to an earlier kernel: they are
+ * accepted and have no effect.  Not thread-safe; results do not depend on the plan. */
 int d3d_debug_set_tc_plan(int group, int max_stages, int prod_warps);
 
 /* ---------------------------------------------------------------------------------------------

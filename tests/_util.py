@@ -1,4 +1,6 @@
 """Helpers shared by the parity tests: seeded inputs, tolerances, canonical comparisons."""
+import contextlib
+
 import numpy as np
 
 
@@ -50,6 +52,17 @@ def pairs_equal(a, b, kvol):
     for k in range(kvol):
         assert a[k].shape == b[k].shape, "offset %d: %s vs %s pairs" % (k, a[k].shape, b[k].shape)
         assert (a[k] == b[k]).all(), "offset %d: pair lists differ" % k
+
+
+@contextlib.contextmanager
+def producer_warps(warps):
+    """The tensor-core convolution with 16 or 24 producer warps (two or three MMA warps) where it has the choice; 0: its own."""
+    from deploy3d_b200 import _lib
+    _lib.check("d3d_debug_set_tc_plan", _lib.lib().d3d_debug_set_tc_plan(0, 0, warps))
+    try:
+        yield
+    finally:
+        _lib.check("d3d_debug_set_tc_plan", _lib.lib().d3d_debug_set_tc_plan(0, 0, 0))
 
 
 def table_parts(table, kvol, max_num_act_out):

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests._util import pairs_equal
+from tests._util import pairs_equal, producer_warps
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -165,8 +165,8 @@ def test_every_layer_matches_reference_gpu(d3d, ref, pipe):
 @pytest.mark.parametrize("cin,cout,residual", [(16, 16, False), (32, 64, True), (64, 64, True), (128, 128, False),
                                                (256, 128, True)])
 def test_tensor_core_convolution_is_deterministic(d3d, cin, cout, residual):
-    """The same launch twice gives the same bytes (no atomics, fixed accumulation order), with one and with two CTAs
-    per SM; the reference scatters with half-precision atomics and has no such property
+    """The same launch twice gives the same bytes (no atomics, fixed accumulation order), with two and with three MMA
+    warps; the reference scatters with half-precision atomics and has no such property
     (trt/spconv/mm/output_iterator.h:189-206)."""
     from deploy3d_b200 import synth
     from deploy3d_b200.ops import data_s_spconv_index, data_s_spconv_mm
@@ -186,16 +186,17 @@ def test_tensor_core_convolution_is_deterministic(d3d, cin, cout, residual):
     x = torch.randn((n, cin), device=DEV).half()
     res = torch.randn((n, cout), device=DEV).half() if residual else None
     first = None
-    for which in (2, 3):
+    for warps in (16, 24):
         plug = deserialize_plugin("SPConvMM", data_s_spconv_mm((3, 3, 3), cin, cout, n, True, False, w, b))
         plug.configure(torch.float16)
-        plug.set_kernel(which)
+        plug.set_kernel(2)
         for _ in range(3):
-            y = plug.run(x, num, table, relu=True, residual=res)
+            with producer_warps(warps):
+                y = plug.run(x, num, table, relu=True, residual=res)
             torch.cuda.synchronize()
             if first is None:
                 first = y.clone()
-            assert torch.equal(y, first), "kernel choice %d: output bytes changed between runs" % which
+            assert torch.equal(y, first), "%d producer warps: output bytes changed between runs" % warps
 
 
 def test_whole_frame_twice_is_identical(d3d):

@@ -108,7 +108,7 @@ def test_segmentation_frame_matches_cpu_pipeline(d3d, net):
 
 def test_regrouped_tables_leave_the_frames_unchanged(d3d):
     """Both pipelines with every neighbour table regrouped by offset mask (d3d_spconv_mm_regroup between the table
-    build and the layers, the packed stage walk in the kernel): the detection frame's sparse features, BEV map and
+    build and the layers, windows no tile of a round has left out in the kernel): the detection frame's sparse features, BEV map and
     NMS scores and the segmentation frame's logits are the bytes the plain tables give, eagerly and from the graph,
     and the regrouped tables have fewer (tile, offset) blocks."""
     from deploy3d_b200 import synth

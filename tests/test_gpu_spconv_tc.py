@@ -7,8 +7,8 @@ import numpy as np
 import pytest
 import torch
 
-from tests._util import (assert_feats_close, assert_table_consistent, assert_tables_equal, rng, round_to, table_pairs,
-                         table_parts, table_row_bits, unique_coors)
+from tests._util import (assert_feats_close, assert_table_consistent, assert_tables_equal, producer_warps, rng, round_to,
+                         table_pairs, table_parts, table_row_bits, unique_coors)
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -47,11 +47,12 @@ def _run(d3d, orc, outs, num_in, num_out, n_in, n_out_max, cin, cout, ks, invers
     tdt = torch.float16 if dtype == "fp16" else torch.bfloat16
     table = SPConvMMPlugin.prepare(kvol, inverse, n_out_max, outs[0], outs[1])
     got = {}
-    for which in (2, 3, 1):  # tcgen05 (two CTAs per SM where it applies), tcgen05 with one CTA per SM, SIMT
+    for which, warps in (("two", 16), ("three", 24), ("auto", 0), ("simt", 0)):  # two or three MMA warps, SIMT
         plug = deserialize_plugin("SPConvMM", d3d.data_s_spconv_mm(ks, cin, cout, n_out_max, False, inverse, w, b))
         plug.configure(tdt)
-        plug.set_kernel(which)
-        y = plug.run(_t(feats, tdt), num_out, table, relu=relu, residual=None if res is None else _t(res, tdt))
+        plug.set_kernel(1 if which == "simt" else 2)
+        with producer_warps(warps):
+            y = plug.run(_t(feats, tdt), num_out, table, relu=relu, residual=None if res is None else _t(res, tdt))
         assert _kernel_error() == 0, "a bounded wait of the tensor-core kernel expired"
         got[which] = y.float().cpu().numpy()
     want = orc.spconv_mm(round_to(feats, dtype), round_to(w, dtype), round_to(b, dtype), outs[0].cpu().numpy(),
@@ -60,10 +61,11 @@ def _run(d3d, orc, outs, num_in, num_out, n_in, n_out_max, cin, cout, ks, invers
         want = want + round_to(res, dtype)
     if relu:
         want = np.maximum(want, 0)
-    assert_feats_close(got[2], want, 1e-2, "tcgen05 vs oracle")
-    assert (got[2] == got[3]).all(), "one or two CTAs per SM accumulate in the same order: identical results"
-    assert_feats_close(got[2], got[1], 1e-2, "tcgen05 vs SIMT")
-    return got[2]
+    assert_feats_close(got["auto"], want, 1e-2, "tcgen05 vs oracle")
+    for which in ("two", "three"):
+        assert (got[which] == got["auto"]).all(), "%s MMA warps: results do not depend on their number" % which
+    assert_feats_close(got["auto"], got["simt"], 1e-2, "tcgen05 vs SIMT")
+    return got["auto"]
 
 
 def test_smallest_case(d3d, orc):
@@ -180,14 +182,15 @@ def test_regrouped_table_same_pairs_same_bytes(d3d, orc, case):
     b = r.standard_normal(cout).astype(np.float32)
     x = torch.randn((n_in_rows, cin), device=DEV).half()
     res = torch.randn((m_max, cout), device=DEV).half()
-    for which in (2, 3, 1):
+    for which, warps in ((2, 16), (2, 24), (2, 0), (1, 0)):
         plug = deserialize_plugin("SPConvMM", d3d.data_s_spconv_mm(ks, cin, cout, m_max, subm, inverse, w, b))
         plug.configure(torch.float16)
         plug.set_kernel(which)
-        y_plain = plug.run(x, num_out, plain, relu=True, residual=res).clone()
-        y_grouped = plug.run(x, num_out, grouped, relu=True, residual=res)
+        with producer_warps(warps):
+            y_plain = plug.run(x, num_out, plain, relu=True, residual=res).clone()
+            y_grouped = plug.run(x, num_out, grouped, relu=True, residual=res)
         assert _kernel_error() == 0
-        assert torch.equal(y_plain, y_grouped), "kernel choice %d: regrouped table changes the result" % which
+        assert torch.equal(y_plain, y_grouped), "kernel choice %d, %d producer warps: regrouping changes the result" % (which, warps)
 
 
 def test_dependent_launch_is_bit_identical(d3d):

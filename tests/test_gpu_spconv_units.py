@@ -1,14 +1,15 @@
 """SPConvMM on the tensor cores at the edges of its units, rounds and accumulators: kernel volumes that leave windows of
-offsets and pairs of them half full, one to three rounds per CTA with a remainder, every number of accumulators, features and
-outputs that start on 16 bytes only, weights that are not finite.  Held against the SIMT kernel of the same library, which
-walks the offsets one by one (tests/test_gpu_spconv_tc.py holds both against the oracle)."""
+offsets and pairs of them half full, tiles shared by the MMA warps, rounds of one to three tiles with a remainder, every
+number of accumulators, features, outputs and tables off their boundaries, weights that are not finite, waits that run out.
+Held against the SIMT kernel of the same library, which walks the offsets one by one (tests/test_gpu_spconv_tc.py holds both
+against the oracle)."""
 import ctypes
 
 import numpy as np
 import pytest
 import torch
 
-from tests._util import assert_feats_close, rng, table_parts, table_row_bits, unique_coors
+from tests._util import assert_feats_close, producer_warps, rng, table_parts, table_row_bits, unique_coors
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -103,9 +104,13 @@ def test_rounds_of_three_tiles(d3d, tiles, cin, cout):
 
 @pytest.mark.parametrize("cout", [16, 32, 48, 64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 240, 256])
 def test_numbers_of_accumulators(d3d, cout):
+    """With two and three MMA warps, whose bytes are the same."""
     plug, x, num, table = _setup(d3d, 57000, [2, 40, 48, 44], (3, 1, 1), 32, cout, torch.float16, cout)
     got, want = _both(plug, x, num, table)
     assert_feats_close(got.float().cpu().numpy(), want, 1e-2, "%d output channels" % cout)
+    for warps in (16, 24):
+        with producer_warps(warps):
+            assert torch.equal(plug.run(x, num, table), got) and _error() == 0
 
 
 @pytest.mark.parametrize("ks", [(3, 3, 3), (3, 1, 1), (5, 1, 3)])
