@@ -25,13 +25,15 @@ def main():
     ap.add_argument("--voxels", type=int, default=66000)
     ap.add_argument("--grid", type=int, nargs=3, default=[11, 360, 360], help="Z Y X of the voxel grid")
     ap.add_argument("--stride", type=int, default=1)
-    ap.add_argument("--kernel", type=int, default=0, help="0 auto, 1 SIMT, 2 or 3 tcgen05")
+    ap.add_argument("--kernel", type=int, default=0, help="0 auto, 1 SIMT, 2 tcgen05")
     ap.add_argument("--dtype", default="fp16", choices=["fp16", "bf16"])
     ap.add_argument("--reps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--index-reps", type=int, default=0, help="also time the rulebook + table build this many times")
-    ap.add_argument("--plan", type=int, nargs=3, default=None, metavar=("GROUP", "STAGES", "PRODUCER_WARPS"),
-                    help="override the tensor-core kernel's plan: 16 or 24 producer warps (0 = automatic); the first two have no effect")
+    ap.add_argument("--producer-warps", type=int, default=0, choices=(0, 16, 24),
+                    help="of the tensor-core kernel, where it has the choice (0 = automatic)")
+    ap.add_argument("--order", default="random", choices=["random", "cell"],
+                    help="order of the voxels: at random, as points come, or by grid cell, as the frame pipelines number them")
     ap.add_argument("--regroup", action="store_true",
                     help="run on the neighbour table with its outputs grouped by offset mask (d3d_spconv_mm_regroup)")
     ap.add_argument("--lib", default=None, metavar="NAME",
@@ -40,12 +42,14 @@ def main():
     if args.lib:
         from deploy3d_b200 import _lib
         _lib.use_tuning_build(args.lib)
-    if args.plan:
+    if args.producer_warps:
         from deploy3d_b200 import _lib
-        _lib.check("d3d_debug_set_tc_plan", _lib.lib().d3d_debug_set_tc_plan(*args.plan))
+        _lib.check("d3d_debug_set_tc_plan", _lib.lib().d3d_debug_set_tc_plan(0, 0, args.producer_warps))
     dev = "cuda:0"
     rng = np.random.Generator(np.random.PCG64(77))
     vox = synth.lidar_like_voxels(rng, args.voxels, tuple(args.grid), sigma=6.0)
+    if args.order == "cell":
+        vox = vox[np.lexsort((vox[:, 2], vox[:, 1], vox[:, 0]))]
     coors = torch.from_numpy(np.concatenate([np.zeros((len(vox), 1), np.int32), vox], 1)).to(dev)
     n = coors.shape[0]
     num_in = torch.tensor([n], dtype=torch.int32, device=dev)
