@@ -1,6 +1,6 @@
 // Stand-alone check, not part of the library:
 //     nvcc -gencode arch=compute_100a,code=sm_100a -O2 -o lane_mask lane_mask.cu && ./lane_mask
-// Two properties the SPConvMM kernel relies on: (1) tcgen05.mma with a disable_output_lane vector leaves the masked
+// Two properties SPConvMM relies on where a weight is not finite (it takes A from tensor memory, this from shared): (1) tcgen05.mma with a disable_output_lane vector leaves the masked
 // TMEM lanes untouched whatever the corresponding rows of A hold, with and without accumulation; (2) tcgen05.st
 // initialises an accumulator that a later accumulating MMA then adds to.  One CTA, M=128 N=16 K=16; A row r holds
 // r % 8 + 1 in every k, B is all ones, so D[r][n] = 16 * (r % 8 + 1).  Every wait is bounded.

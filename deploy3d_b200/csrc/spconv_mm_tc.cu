@@ -11,32 +11,35 @@
 // (The reference: gather iterator + mma.sync tiles of 64 pairs of one offset, fp16 accumulate, half2 atomicAdd
 // scatter, trt/spconv/mm/kernel.h:84-179, mm/output_iterator.h:189-206.)
 //
-// Why A goes through registers into tensor memory (B200).  From shared memory an M128 K16 MMA takes 46 / 46 / 51 / 64 cycles
-// at N = 16 / 32 / 64 / 128: the tensor core fetches 4 KB of A each time.  From tensor memory it takes 16 / 21 / 32 / 64.
-// Zeros for missing rows cost nothing in registers, so no MMA carries a lane mask.  Plain loads go through L1, which the
-// operand ring in shared memory had taken: in cell order 61-66 % of the gathered bytes are hits (neighbouring offsets and
-// rows of a tile read the same voxels).  And a weight block is fetched once for the two or three tiles a CTA works on
-// together, not once per tile.  Weights have to be finite for that (a row without an input is 0 * W): layers with others
-// take the SIMT kernel.  27 offsets, us per launch, before (rows copied by cp.async into a shared-memory
-// ring, MMAs under lane masks) and now: 16 -> 16 at 281 k voxels 33 / 31, 32 -> 32 at 463 k
-// 81 / 72, 32 -> 64 at 463 k 96 / 77, 64 -> 64 at 238 k 80 / 70, 64 -> 128 101 / 87, 128 -> 128 at 66 k 59 / 51, 256 -> 128 at
-// 50 k 82 / 73, 256 -> 256 115 / 114; nine offsets and 90 k voxels: 64 -> 64 22 / 21, 128 -> 128 36 / 33.
+// Why A goes through registers into tensor memory (B200).  From shared memory an M128 K16 MMA takes 41 / 42 / 48 / 64 cycles
+// at N = 16 / 32 / 64 / 128: the tensor core fetches 4 KB of A each time.  From tensor memory it takes 15 / 20 / 32 / 64
+// (microbench/mma_operand.cu).  Zeros for missing rows cost nothing in registers, so no MMA carries a lane mask.  Plain loads go
+// through L1, which the operand ring in shared memory had taken: neighbouring offsets and rows of a tile read the same voxels.
+// And up to 128 output channels a weight block is fetched once for the two or three tiles a CTA works on together, not once per
+// tile (with more there are too few accumulators for that, see open_round: one MMA warp and its two teams do the work).
+// 27 offsets, us per launch, before (rows copied by cp.async into a shared-memory ring, MMAs under lane masks) and now:
+// 16 -> 16 at 281 k voxels 33 / 31, 32 -> 32 at 463 k 81 / 70, 32 -> 64 at 463 k 96 / 76, 64 -> 64 at 238 k 80 / 66,
+// 64 -> 128 101 / 87, 128 -> 128 at 66 k 59 / 51, 256 -> 128 at 50 k 82 / 73, 256 -> 256 115 / 115.
+//
+// Where a weight is not finite, 0 * W is not zero.  Such a layer takes the kernels without kWide: their products then leave the
+// accumulator rows without an input alone (tcgen05.mma with a lane mask), and the accumulators start as zeros.
 //
 // What bounds it now: the instruction streams of the roles, again.  An SM needs 600 warp instructions for a unit (128 rows x
 // 128 bytes) and issues 1.7 a cycle; a lone warp executes a dependent one every four to six cycles, and a trip through a
 // full memory pipe (a barrier test, a shared-memory load) takes 70 cycles and more.  Hence:
-//   * two or three MMA warps, each with a tile of the round and two producer teams of its own: one warp needs about 450
-//     cycles from one product to the next, whatever the tensor core could do;
+//   * two or three MMA warps, each with a tile of the round (or its windows of the one tile a CTA has) and two producer teams of
+//     its own: one warp needs about 470 cycles from one product to the next, whatever the tensor core could do -- four or six
+//     teams to one warp are no faster;
 //   * an MMA warp waits and issues in one elected lane, two units at a time, from values that the whole warp has computed
-//     by counters: fed from memory or by a loop of one lane, the compiler cannot keep the descriptors in uniform registers,
-//     and four MMAs with a commit take 273 cycles to issue instead of 74;
+//     by counters: fed from memory or by a loop of one lane, the compiler cannot keep the descriptors in uniform registers, and
+//     four MMAs with a commit take 223 cycles to issue instead of 143 (microbench/mma_operand.cu);
 //   * the control warp lists the units of a round, so that a producer finds its next one with a single load;
 //   * a lane of a producer holds two or four rows (rows_per_lane): 16-byte pieces dealt out lane by lane cost four times
 //     the address arithmetic;
 //   * ids, row masks, input and residual rows of the next round are prefetched into L2: the loads run one unit ahead, which
 //     covers L2 but not DRAM (128 -> 128 at 66 k voxels behind other layers: 66.0 us without, 61.4 with).
-// For 128 output channels and more the tensor pipe is busy two thirds of the time, and 128-row tiles round up (520 tiles on
-// 148 SMs are 3.5, so 4).
+// For 128 output channels the tensor pipe is busy half of the launch, and 128-row tiles round up (520 tiles on 148 SMs are 3.5,
+// so 4).
 //
 // Roles of a CTA (persistent, one per SM) with T = 2 or 3 MMA warps: 8 T producer warps, 4 epilogue warps (8 for T = 2), T MMA
 // warps, 1 control warp (lists, weights by TMA, prefetches).  Units pass through a ring of 2 T slots in tensor memory, one per team
@@ -801,9 +804,8 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
 }
 
 // ---- MMA warps -------------------------------------------------------------------------------------------------------
-// Every other tile of a round.  The warp walks the round together and by counters: what feeds an MMA has to be the same for
-// the whole warp in a way the compiler can see.  (Four MMAs and a commit issued from a loop run by one lane take 273 cycles, by
-// the elected lane of such a warp 74, at 32 output channels.)
+// One tile of a round (kSplit: its windows of the tile).  The warp walks the round together and by counters: what feeds an MMA
+// has to be the same for the whole warp in a way the compiler can see.
 template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int me) {
   constexpr int kSteps = 4 / kOffs;  // MMAs (K = 16) per offset of a unit
@@ -868,8 +870,8 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
       uint64_t* const full[2] = {odd ? full_of[1] : full_of[0], odd ? full_of[0] : full_of[1]};
       uint64_t* const empty[2] = {odd ? empty_of[1] : empty_of[0], odd ? empty_of[0] : empty_of[1]};
       if (!kWide && p.masked) {
-        // Under the row masks of every offset, one unit after the other.  Here a lane mask costs what it costs: 46 cycles for an
-        // MMA at least, and the masks come from L2.
+        // Under the row masks of every offset, one unit after the other; the masks come from L2 (64 -> 64 at 238 k voxels: 94 us,
+        // without them 76).
         for (int h = 0; h < (both ? 2 : 1); ++h) {
           uint32_t rows[kOffs][4];
           if (mine) {

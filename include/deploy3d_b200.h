@@ -293,6 +293,7 @@ int d3d_spconv_mm_regroup(int kernel_vol, int64_t max_num_act_out, const void* t
                           void* scratch, size_t scratch_bytes, void* stream);
 int d3d_spconv_mm_prepare(int kernel_vol, int mode, int64_t max_num_act_out, const int32_t* index,
                           int64_t index_row_len, const int32_t* num_index, void* table, void* stream);
+/* `num_act_out` is part of the plugin's inputs and is not read: which outputs exist, and their inputs, is what the table says. */
 int d3d_spconv_mm_run(d3d_spconv_mm_t handle, int dtype, const void* in_feats, int64_t max_num_act_in,
                       const int32_t* num_act_out, const void* table, void* out_feats,
                       const d3d_spconv_mm_epilogue* epilogue, void* stream);
