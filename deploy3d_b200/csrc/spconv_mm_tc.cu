@@ -42,7 +42,8 @@
 // so 4).
 //
 // Roles of a CTA (persistent, one per SM) with T = 2 or 3 MMA warps: 8 T producer warps, 4 epilogue warps (8 for T = 2), T MMA
-// warps, 1 control warp (lists, weights by TMA, prefetches).  Units pass through a ring of 2 T slots in tensor memory, one per team
+// warps, 1 control warp (lists, weights by TMA -- those that are held are fetched by
+// the last MMA warp --, prefetches).  Units pass through a ring of 2 T slots in tensor memory, one per team
 // of four producer warps (a warp can only write its quarter of the lanes).  Everything is handed over through mbarriers; every
 // wait is bounded (about one second) and on expiry raises an error word, lets the CTA drain and return instead of spinning.
 // A barrier is always waited for by the side that has seen its phase before (same team, same MMA warp, same epilogue warps):
@@ -115,6 +116,7 @@ struct TcParams {
   int parts;          // units per kernel offset: cin / 64, at least 1
   int num_acc;        // accumulators
   int ring_col;       // first tensor-memory column of the ring
+  int spread;         // the tiles of a CTA lie a grid apart, instead of side by side
   int regrouped;      // tiles in ascending order of their offset masks: dealt out costly ones first
   uint32_t b_bytes;   // one weight block: cout rows of row_bytes, per (offset, part)
   int b_slots;        // ring of weight windows; 0: all kvol blocks stay in shared memory
@@ -359,12 +361,14 @@ template <int kOffs> __device__ __forceinline__ Smem carve_smem(unsigned char* r
 // warp lists the units of a round for the producers; the MMA warps and the epilogue count along.
 //
 // Rounds cover the live tiles first, in whole rounds and one of the remaining tiles shared out evenly (157 tiles of 64 -> 64: one
-// each and nine CTAs with two 14.7 us, 78 CTAs with two 16.0), then whatever lies behind them (tiles no offset feeds).
+// each and nine CTAs with two 14.7 us, 78 CTAs with two 16.0), then whatever lies behind them (tiles no offset feeds).  Launches
+// of at most two tiles to a CTA are one round (p.spread).
 //
 // Launches of at most one tile to a CTA (kSplit): both MMA warps work on it, each window going to the next warp -- by its number,
 // not by its place among those the tile has, so that a regrouped table gives the same sums --, with an accumulator, a list and
 // weight slots each; the epilogue adds the two sums.  27 offsets and 6 k voxels, us with one warp / both: 16 -> 16 7.3 / 6.5,
-// 32 -> 64 9.3 / 7.9, 64 -> 64 12.3 / 10.1, 128 -> 128 19.3 / 15.8.  A kernel of its own: the same by a flag costs 0.3 to 0.9 us,
+// 32 -> 64 9.3 / 7.9, 64 -> 64 12.3 / 10.1, 128 -> 128 19.3 / 15.8 (7.1 and 5.8 at 32 -> 64 and 16 -> 16 since weights that are
+// held are not asked for by the control warp).  A kernel of its own: the same by a flag costs 0.3 to 0.9 us,
 // since a short launch fetches most of its code for the first time.
 struct Round {
   int start;      // index of the round's first tile over all CTAs
@@ -380,7 +384,7 @@ struct Round {
 // to the same one, which is what dealing the tiles out asks for.
 __device__ __forceinline__ int live_tiles(const TcParams& p) {
   // (at most one tile to a CTA: nothing to deal out)
-  if (p.regrouped || p.num_tiles <= (int)gridDim.x) return p.num_tiles;
+  if (p.spread || p.num_tiles <= (int)gridDim.x) return p.num_tiles;
   constexpr int kProbes = 4;
   const int step = (p.num_tiles + 32 * kProbes - 1) / (32 * kProbes);
   uint32_t mask[kProbes];
@@ -401,8 +405,8 @@ __device__ __forceinline__ int live_tiles(const TcParams& p) {
 // Index of the CTA's tile i in a round, and the tile it stands for.
 __device__ __forceinline__ int tile_index(const TcParams& p, const Round& r, int i) {
   const int g = (int)gridDim.x, c = (int)blockIdx.x;
-  if (!p.regrouped) return r.first + i;
-  return r.start + i * g + ((i & 1) ? g - 1 - c : c);
+  if (!p.spread) return r.first + i;
+  return r.start + i * g + (p.regrouped && (i & 1) ? g - 1 - c : c);
 }
 __device__ __forceinline__ int tile_of(const TcParams& p, int index) {
   return p.regrouped ? p.num_tiles - 1 - index : index;
@@ -419,7 +423,7 @@ template <int kMma, bool kSplit> __device__ __forceinline__ void open_round(cons
   const int c = (int)blockIdx.x, less = r.tiles - 1, more = rest - less * g < g ? rest - less * g : g;
   r.start = start, r.next = start + less * g + more;
   r.first = start + c * less + (c < more ? c : more);
-  r.limit = p.regrouped ? r.next : r.first + less + (c < more ? 1 : 0);
+  r.limit = p.spread ? r.next : r.first + less + (c < more ? 1 : 0);
   const int i = threadIdx.x & 3;
   const int index = tile_index(p, r, i);
   r.mask = (i < r.tiles && index < r.limit) ? __ldg(p.tile_mask + tile_of(p, index)) : 0u;
@@ -676,8 +680,8 @@ template <bool kWide> __device__ __forceinline__ void prefetch_round(const TcPar
                 (uint32_t)(out < kTileRows ? out : kTileRows) * p.cout * 2);
 }
 
-// Lists the units of every round and brings in the weights: all of them once when they are resident, else the block of
-// every (window, part) as soon as a slot is free.
+// Lists the units of every round and brings in weights that are not held, the block of every (window, part) as soon as a slot
+// is free.
 template <int kOffs, bool kWide, int kMma, bool kSplit>
 __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b) {
   constexpr uint32_t kWindow = kOffs == 1 ? 1u : kOffs == 2 ? 3u : 15u;
@@ -688,14 +692,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
   const uint32_t b_tx = (uint32_t)p.cout * p.row_bytes;
   const bool resident = p.b_slots == 0;
   const int parts = p.parts, ring_slots = kSplit ? p.b_slots / kMma : p.b_slots;
-  // the weights are constants of the layer: their load does not wait for the preceding kernel
-  if (resident && lane == 0) {
-    // blocks behind the last offset, up to a whole window: rows beyond the tensor, which TMA fills with zeros
-    const int blocks = (p.kvol + kOffs - 1) / kOffs * kOffs;
-    mbar_arrive_expect_tx(&sh->b_ready, (uint32_t)blocks * b_tx);
-    for (int k = 0; k < blocks; ++k) tma_load_2d(map_b, &sh->b_ready, s.weights + (size_t)k * p.b_bytes, 0, k * p.cout);
-  }
-  if (!resident && lane == 0) {  // a slice of the weights for every CTA, towards L2
+  if (!resident && lane == 0) {  // (constants of the layer) a slice of the weights for every CTA, towards L2
     const uint32_t bytes = (uint32_t)p.kvol * (uint32_t)p.cout * (uint32_t)p.cin * 2u;
     const uint32_t slice = (bytes / gridDim.x + 127u) & ~127u, from = blockIdx.x * slice;
     if (from < bytes)
@@ -807,7 +804,7 @@ __device__ __forceinline__ void control_role(const TcParams& p, const Smem& s, c
 // One tile of a round (kSplit: its windows of the tile).  The warp walks the round together and by counters: what feeds an MMA
 // has to be the same for the whole warp in a way the compiler can see.
 template <int kOffs, bool kWide, int kMma, bool kSplit>
-__device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint32_t tmem_base, int me) {
+__device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, const CUtensorMap* map_b, uint32_t tmem_base, int me) {
   constexpr int kSteps = 4 / kOffs;  // MMAs (K = 16) per offset of a unit
   Shared* sh = s.sh;
   volatile int* abort_flag = &sh->abort_flag;
@@ -820,6 +817,15 @@ __device__ __forceinline__ void mma_role(const TcParams& p, const Smem& s, uint3
   const int parts = p.parts, num_acc = p.num_acc;
   const int b_first = kSplit ? me * (p.b_slots / kMma) : 0, b_end = kSplit ? b_first + p.b_slots / kMma : p.b_slots;
   const uint32_t cout = (uint32_t)p.cout;
+  // Weights that are held: constants of the layer, whose load does not wait for the preceding kernel.  The last MMA warp asks for
+  // them: 28 loads take a lane 1.1 us, which the control warp would spend in front of the first list.
+  if (resident && me == kMma - 1 && elect_one()) {
+    // blocks behind the last offset, up to a whole window: rows beyond the tensor, which TMA fills with zeros
+    const int blocks = (p.kvol + kOffs - 1) / kOffs * kOffs;
+    mbar_arrive_expect_tx(&sh->b_ready, (uint32_t)blocks * (cout * p.row_bytes));
+    for (int k = 0; k < blocks; ++k) tma_load_2d(map_b, &sh->b_ready, s.weights + (size_t)k * p.b_bytes, 0, k * p.cout);
+  }
+  __syncwarp();
   if (resident && !__all_sync(0xffffffffu, mbar_wait(&sh->b_ready, 0, abort_flag, 23, p.wait_limit))) return;
   pdl_wait();  // the first list comes after the preceding kernels, which may take longer than a wait is allowed to
   // the slots of this warp's two teams, taken in turn
@@ -1053,7 +1059,7 @@ spconv_mm_tc_kernel(const __grid_constant__ CUtensorMap map_b, const TcParams p)
   } else if (warp < 8 * kMma + kEpilogue) {
     epilogue_role<kOffs, kWide, kMma, kSplit>(p, s, tmem_base, warp & 3, (warp - 8 * kMma) / 4);
   } else if (warp < 9 * kMma + kEpilogue) {
-    mma_role<kOffs, kWide, kMma, kSplit>(p, s, tmem_base, warp - 8 * kMma - kEpilogue);
+    mma_role<kOffs, kWide, kMma, kSplit>(p, s, &map_b, tmem_base, warp - 8 * kMma - kEpilogue);
   } else {
     control_role<kOffs, kWide, kMma, kSplit>(p, s, &map_b);
   }
@@ -1213,11 +1219,15 @@ int launch_spconv_mm_tc(const MmLaunch& a) {
   // One tile to a CTA: two MMA warps share it, since a chain of products is what such a launch lasts (an MMA warp takes 470 cycles
   // from one unit to the next, whatever feeds it).  From the second tile on a tile each is faster: they share their weights (157
   // tiles of 64 -> 64: 14.7 us, shared one after the other 17.8).
+  //   Two tiles of a CTA lie a grid apart: that is balanced wherever the live tiles end, so that these need not be looked for, which
+  // costs two trips to L2 in front of the first list (219 live of 256 tiles, 16 -> 32 9.7 / 8.6 us; the CTAs that start first have
+  // two: the other way round 64 -> 64 behind another launch 13.1 / 13.8).
   const bool is_short = p.num_tiles <= 2 * kNumSMs, split = p.num_tiles <= kNumSMs && cout <= 192 && kvol > offs;
   const int mma_warps = cin < 32 || split        ? 2
                         : g_plan_mma_warps       ? g_plan_mma_warps
                         : cout <= 64 && kvol > 9 ? (is_short ? 2 : 3)
                                                  : 2;
+  p.spread = p.regrouped || is_short;
   const KernelEntry* k = find_kernel(offs, wide, mma_warps, split);
   D3D_REQUIRE(k, D3D_ERR_INVALID_ARGUMENT);
   // tensor memory: a slot for every producer team, the rest accumulators
