@@ -151,10 +151,11 @@ def test_features_and_outputs_on_16_bytes(d3d, cin):
 
 @pytest.mark.parametrize("ks", [(3, 3, 3), (3, 1, 3)])
 @pytest.mark.parametrize("cin,cout", [(16, 32), (32, 48), (32, 96), (64, 64), (64, 80)])
-def test_table_and_features_off_their_boundaries(d3d, ks, cin, cout):
-    """A table that starts on four bytes (a copy inside a larger buffer), features that start on 16, and both."""
-    n = 5000
-    plug, x, num, table = _setup(d3d, n, [1, 24, 30, 20], ks, cin, cout, torch.float16, 17)
+@pytest.mark.parametrize("n", [5000, 30000, 45000])
+def test_table_and_features_off_their_boundaries(d3d, n, ks, cin, cout):
+    """A table that starts on four bytes (a copy inside a larger buffer), features that start on 16, and both; one tile to a
+    CTA, two, and more, which 27 offsets and up to 64 channels run with three MMA warps."""
+    plug, x, num, table = _setup(d3d, n, [1, 40, 40, 40], ks, cin, cout, torch.float16, 17)
     want = plug.run(x, num, table, relu=True)
     moved = torch.cat([x.new_zeros(8), x.flatten()])[8:].view(x.shape)
     assert moved.data_ptr() % 32 == 16
@@ -266,11 +267,10 @@ def test_wait_that_gives_up(d3d, wait_limit, cin, cout):
 
 @pytest.mark.parametrize("ks", [(3, 3, 3), (3, 1, 3)])
 @pytest.mark.parametrize("cin,cout", [(16, 16), (32, 32), (64, 64), (64, 128), (128, 48), (256, 256)])
-def test_weights_that_are_not_finite_stay_on_the_tensor_cores(d3d, ks, cin, cout):
+@pytest.mark.parametrize("n", [4000, 20000, 45000])
+def test_weights_that_are_not_finite_stay_on_the_tensor_cores(d3d, n, ks, cin, cout):
     """An infinite weight reaches its own output channel in the rows that have an input under its offset, and nothing else:
     the other channels come out with the same bytes as without it, which another kernel's would not."""
-    n = 20000
-
     def edit(w):
         w[5, cin - 3, 2] = np.inf
 
