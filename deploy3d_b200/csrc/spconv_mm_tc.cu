@@ -18,14 +18,14 @@
 // And up to 128 output channels a weight block is fetched once for the two or three tiles a CTA works on together, not once per
 // tile (with more there are too few accumulators for that, see open_round: one MMA warp and its two teams do the work).
 // 27 offsets, us per launch, before (rows copied by cp.async into a shared-memory ring, MMAs under lane masks) and now:
-// 16 -> 16 at 281 k voxels 33 / 31, 32 -> 32 at 463 k 81 / 70, 32 -> 64 at 463 k 96 / 76, 64 -> 64 at 238 k 80 / 66,
+// 16 -> 16 at 281 k voxels 33 / 31, 32 -> 32 at 463 k 81 / 67, 32 -> 64 at 463 k 96 / 75, 64 -> 64 at 238 k 80 / 65,
 // 64 -> 128 101 / 87, 128 -> 128 at 66 k 59 / 51, 256 -> 128 at 50 k 82 / 73, 256 -> 256 115 / 115.
 //
 // Where a weight is not finite, 0 * W is not zero.  Such a layer takes the kernels without kWide: their products then leave the
 // accumulator rows without an input alone (tcgen05.mma with a lane mask), and the accumulators start as zeros.
 //
-// What bounds it now: the instruction streams of the roles, again.  An SM needs 600 warp instructions for a unit (128 rows x
-// 128 bytes) and issues 1.7 a cycle; a lone warp executes a dependent one every four to six cycles, and a trip through a
+// What bounds it now: the instruction streams of the roles, again.  An SM needs 720 to 770 warp instructions for a unit (128 rows
+// x 128 bytes) and issues 1.7 to 2.4 a cycle; a lone warp executes a dependent one every four to six cycles, and a trip through a
 // full memory pipe (a barrier test, a shared-memory load) takes 70 cycles and more.  Hence:
 //   * two or three MMA warps, each with a tile of the round (or its windows of the one tile a CTA has) and two producer teams of
 //     its own: one warp needs about 470 cycles from one product to the next, whatever the tensor core could do -- four or six
